@@ -3,11 +3,11 @@
 // multiple of 8 up to 256, any number of heads and groups, with or without a window.
 // It is the attention of the 32-bit path and the yardstick of the tensor-core kernels.
 //
-// One block per (query row, query head).  Keys are cut into chunks of 32 by absolute
-// position; chunk c goes to warp c mod 4, one key per lane.  Each warp keeps a running
-// (max, sum, accumulator) in 32-bit; the four are merged at the end in a fixed order.
+// Keys are cut into chunks of 32 by absolute position, one key per lane; a few warps take the chunks in turn, each
+// with a running (max, sum, accumulator) in 32-bit, merged at the end in a fixed order.
 // The partition depends only on the query's position, so the result for a position is
-// the same whatever else is in the batch and however the prompt was cut.
+// the same whatever else is in the batch and however the prompt was cut.  Two kernels: tiles of query rows whose keys
+// and values wait in shared memory (heads whose rows are whole 16-byte units), and one block per (query row, head).
 //
 // Formulas: rust/engine/src/runner/model/qwen2/kernels.rs:702-853 (scores scaled by
 // 1/sqrt(d), mask key <= query, online softmax with max/sum/accumulator in 32-bit,
@@ -125,17 +125,329 @@ __global__ void __launch_bounds__(WARPS * 32) attention_plain_kernel(
     else reinterpret_cast<T*>(out)[at] = from_f32<T>(o);
   }
 }
+
+// ---- tiles of query rows ------------------------------------------------------------------------
+// A CTA takes 8 WPG rows: neighbouring tokens with the query heads that share one kv head (or some of them, where they
+// are more than the tile).  PARTS groups of WPG warps: chunk c of 32 keys goes to group c mod PARTS, whose keys and
+// values come to its own buffers by cp.async, the next chunk's keys while the values of this one are used and the other
+// way round.  A warp takes 8 rows: scores with a key per lane (the row's query as broadcasts, two products an
+// instruction: sums of even and odd entries apart), the weights left in shared memory, then the weighted sum with two
+// neighbouring entries of the head per lane.  A row's own arithmetic is the same in every tile and batch; rows of other
+// requests in the tile take a pass of their own.
+//
+// What bounds it: multiply-adds and loads from shared memory, about even with 8 rows to a warp.  The other kernel's block
+// per (row, head) reads a row's keys and values once per head and row.  Measured on a B200, 32-bit, 14 query and 2 kv
+// heads of 64 (the other kernel in brackets): a prompt of 517 53 us (560), 8 single tokens after 520 36 us (57), one after
+// 3,000 155 us (296), where a row's chain of chunks bounds it; 12 and 2 heads of 128, 300 rows after 500 174 us (1,330).
+constexpr int RW = 8;      // rows a warp takes
+
+__device__ __forceinline__ void cp_async16(void* dst, const void* src, bool has) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(has ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+__device__ __forceinline__ void fma_pair(unsigned long long& d, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pair_of(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float low_of(unsigned long long d) { return __uint_as_float((uint32_t)d); }
+__device__ __forceinline__ float high_of(unsigned long long d) { return __uint_as_float((uint32_t)(d >> 32)); }
+__device__ __forceinline__ float2 load2(const float* p) { return *reinterpret_cast<const float2*>(p); }
+__device__ __forceinline__ float2 load2(const __nv_bfloat16* p) {
+  const uint32_t u = *reinterpret_cast<const uint32_t*>(p);
+  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+
+struct RowsParams {
+  void* out;
+  const void* q;
+  const void* cache_k;
+  const void* cache_v;
+  const int* row_req;
+  const int* row_pos;
+  const int* block_table;
+  const float* sinks;
+  const float* dist_bias;
+  int out_stride, q_stride, max_blocks, tokens, n_q, n_kv, d, page_size, num_pages, window, keep_first, sink, bias_len,
+      out_f32, tile_tokens, head_tiles;      // tokens of a tile; tiles that share a token's heads
+  float scale, softcap;
+};
+
+template <typename T> __host__ __device__ constexpr int rows_ld(int d) { return d + 16 / (int)sizeof(T); }
+template <typename T> static int rows_smem(int d, int parts, int wpg) {
+  return 4 * RW * wpg * d + (int)sizeof(T) * parts * 2 * 32 * rows_ld<T>(d) + 4 * parts * wpg * 32 * RW;
+}
+
+template <typename T, int D, int PARTS, int WPG>
+__global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsParams p) {
+  extern __shared__ __align__(16) char ap_smem[];
+  constexpr int R = RW * WPG, NT = PARTS * 32 * WPG, DP = D ? (D + 63) / 64 : 4;
+  const int d = D ? D : p.d, ld = rows_ld<T>(d);
+  float* qs = reinterpret_cast<float*>(ap_smem);                                       // [R][d]
+  T* kv = reinterpret_cast<T*>(ap_smem + 4 * R * d);                                   // [PARTS][keys, values][32][ld]
+  float* weights = reinterpret_cast<float*>(kv + PARTS * 2 * 32 * ld);                 // [PARTS][WPG][32][RW]
+  __shared__ int s_req[R], s_pos[R];
+  pdl_trigger();
+  const int tid = threadIdx.x, lane = tid & 31, part = tid / (32 * WPG), warp = (tid >> 5) % WPG;
+  const int kvh = blockIdx.y, group = p.n_q / p.n_kv;
+  const int tile = gridDim.x - 1 - blockIdx.x;      // the last rows see the most keys: they go first
+  const int t0 = tile / p.head_tiles * p.tile_tokens, h0 = tile % p.head_tiles * R;
+  const int heads = min(R, group - h0);             // of a token in this tile
+  auto token_of = [&](int r) { return t0 + r / heads; };
+  auto head_of = [&](int r) { return kvh * group + h0 + r % heads; };
+  pdl_wait();
+  for (int r = tid; r < R; r += NT) {
+    const int t = token_of(r);
+    const bool has = r < heads * p.tile_tokens && t < p.tokens;
+    s_req[r] = has ? p.row_req[t] : -1;
+    s_pos[r] = has ? p.row_pos[t] : -1;
+  }
+  __syncthreads();
+  for (int i = tid; i < R * d; i += NT) {
+    const int r = i / d;
+    qs[i] = s_req[r] >= 0 ? to_f32<T>(static_cast<const T*>(p.q)[(size_t)token_of(r) * p.q_stride + (size_t)head_of(r) * d + i % d]) : 0.f;
+  }
+  __syncthreads();
+
+  T* keys = kv + (size_t)part * 2 * 32 * ld;
+  T* values = keys + 32 * ld;
+  float* mine = weights + (part * WPG + warp) * 32 * RW;
+  const float* qw = qs + warp * RW * d;
+  auto group_sync = [&]() {      // the warps of this group
+    if (WPG == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + part), "r"(32 * WPG) : "memory");
+  };
+
+  for (int r0 = 0; r0 < R && s_req[r0] >= 0;) {
+    // the rows of one request: [r0, r1)
+    const int req = s_req[r0];
+    int r1 = r0, p_max = -1, lo_min = 0x7fffffff, kept_max = 0;
+    for (; r1 < R && s_req[r1] == req; ++r1) {
+      const int first = lab_first_key(s_pos[r1], p.window);
+      p_max = max(p_max, s_pos[r1]);
+      lo_min = min(lo_min, first);
+      if (p.window > 0 && p.keep_first > 0) kept_max = max(kept_max, min(p.keep_first, first));
+    }
+    const int* bt = p.block_table + (size_t)req * p.max_blocks;
+    const int last = p_max < 0 ? -1 : p_max / 32;      // (a row of padding sees nothing)
+    // chunks that no row sees lie between the kept first positions and the window
+    auto settle = [&](int c) {
+      if (c * 32 >= kept_max && c < lo_min / 32) c += (lo_min / 32 - c + PARTS - 1) / PARTS * PARTS;
+      return c;
+    };
+    // where key 32 c + lane lies, or -1
+    auto place = [&](int c) -> long long {
+      const int j = c * 32 + lane;
+      if (c > last || j > p_max) return -1;
+      const bool seen = j >= lo_min || j < kept_max;
+      if (!seen) return -1;
+      const int page = bt[j / p.page_size];
+      if (page < 0 || page >= p.num_pages) {
+        lab_set_error(LAB_ERR_PAGE_RANGE);
+        return -1;
+      }
+      return (((long long)page * p.n_kv + kvh) * p.page_size + j % p.page_size) * d;
+    };
+    const int units = d * (int)sizeof(T) / 16;
+    auto fetch = [&](T* to, const void* cache, long long base, bool any) {
+      if (any) {
+        // a warp brings 32 / WPG rows, its lanes units side by side
+        for (int e = lane; e - lane < 32 / WPG * units; e += 32) {
+          const int row = e / units, u = e - row * units;
+          const bool in = row < 32 / WPG;
+          const long long at = __shfl_sync(0xffffffffu, base, (warp * (32 / WPG) + row) & 31);
+          if (in)
+            cp_async16(to + (warp * (32 / WPG) + row) * ld + u * (16 / (int)sizeof(T)),
+                       static_cast<const T*>(cache) + (at < 0 ? 0 : at) + u * (16 / (int)sizeof(T)), at >= 0);
+        }
+      }
+      cp_async_commit();
+    };
+
+    float m[RW], l[RW];
+    unsigned long long acc[RW][DP];
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+      m[i] = -INFINITY, l[i] = 0.f;
+#pragma unroll
+      for (int u = 0; u < DP; ++u) acc[i][u] = 0ull;
+    }
+    int c = settle(part);
+    long long base = place(c);
+    fetch(keys, p.cache_k, base, c <= last);
+    fetch(values, p.cache_v, base, c <= last);
+    while (c <= last) {
+      const int cn = settle(c + PARTS);
+      const long long base_n = place(cn);
+      cp_async_wait<1>();
+      group_sync();
+      // scores of the warp's rows with key 32 c + lane
+      unsigned long long dot[RW];
+#pragma unroll
+      for (int i = 0; i < RW; ++i) dot[i] = 0ull;
+      const T* kr = keys + lane * ld;
+#pragma unroll 4
+      for (int e = 0; e < d; e += 4) {
+        const float4 kq = load4(kr + e);
+        const unsigned long long k_lo = pair_of(kq.x, kq.y), k_hi = pair_of(kq.z, kq.w);
+        ulonglong2 qv[RW];
+#pragma unroll
+        for (int i = 0; i < RW; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(qw + i * d + e);
+#pragma unroll
+        for (int i = 0; i < RW; ++i) fma_pair(dot[i], qv[i].x, k_lo);
+#pragma unroll
+        for (int i = 0; i < RW; ++i) fma_pair(dot[i], qv[i].y, k_hi);
+      }
+      group_sync();
+      fetch(keys, p.cache_k, base_n, cn <= last);      // the keys' buffer is free
+      const int j = c * 32 + lane;
+#pragma unroll
+      for (int i = 0; i < RW; ++i) {
+        const int r = warp * RW + i, pos = s_pos[r];
+        const int first = lab_first_key(pos, p.window);
+        const int kept = p.window > 0 && p.keep_first > 0 ? min(p.keep_first, first) : 0;
+        float s = -INFINITY;
+        if (r >= r0 && r < r1 && base >= 0 && j <= pos && (j >= first || j < kept)) {
+          s = (low_of(dot[i]) + high_of(dot[i])) * p.scale;
+          if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
+          if (p.dist_bias != nullptr) s += p.dist_bias[(size_t)head_of(r) * p.bias_len + min(pos - j, p.bias_len - 1)];
+        }
+        const float m_new = fmaxf(m[i], warp_max(s));
+        float pj = 0.f;
+        if (m_new != -INFINITY) {      // (else no readable key so far)
+          pj = s == -INFINITY ? 0.f : expf(s - m_new);
+          const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+          l[i] = l[i] * corr + pj;
+          const unsigned long long cc = pair_of(corr, corr);
+#pragma unroll
+          for (int u = 0; u < DP; ++u) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][u]) : "l"(cc));
+          m[i] = m_new;
+        }
+        mine[lane * RW + i] = pj;
+      }
+      cp_async_wait<1>();
+      group_sync();
+      // the weighted sum: a key's weights of all rows, its entries 2 lane, 2 lane + 1 (and 64 further on)
+#pragma unroll 4
+      for (int jj = 0; jj < 32; ++jj) {
+        const float4 w0 = load4(mine + jj * RW), w1 = load4(mine + jj * RW + 4);
+        const float w[RW] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+        for (int u = 0; u < DP; ++u) {
+          const int e = 2 * lane + 64 * u;
+          if (D % 64 != 0 || D == 0) {
+            if (e >= d) break;
+          }
+          const float2 v = load2(values + jj * ld + e);
+          const unsigned long long vv = pair_of(v.x, v.y);
+          if (v.x * 0.f + v.y * 0.f == 0.f) {
+#pragma unroll
+            for (int i = 0; i < RW; ++i) fma_pair(acc[i][u], pair_of(w[i], w[i]), vv);
+          } else {      // an infinity or NaN counts for the rows that give it a weight only
+#pragma unroll
+            for (int i = 0; i < RW; ++i)
+              if (w[i] != 0.f) fma_pair(acc[i][u], pair_of(w[i], w[i]), vv);
+          }
+        }
+      }
+      group_sync();
+      fetch(values, p.cache_v, base_n, cn <= last);
+      c = cn;
+      base = base_n;
+    }
+    cp_async_wait<0>();
+    __syncthreads();      // every buffer has been read: the parts' results take their place
+    float* results = reinterpret_cast<float*>(kv);      // [PARTS][R][d + 2]
+#pragma unroll
+    for (int i = 0; i < RW; ++i) {
+      float* to = results + (part * R + warp * RW + i) * (d + 2);
+      const float all = warp_sum(l[i]);
+      if (lane == 0) to[d] = m[i], to[d + 1] = all;
+#pragma unroll
+      for (int u = 0; u < DP; ++u) {
+        const int e = 2 * lane + 64 * u;
+        if (e < d) to[e] = low_of(acc[i][u]);
+        if (e + 1 < d) to[e + 1] = high_of(acc[i][u]);
+      }
+    }
+    __syncthreads();
+    for (int x = tid; x < (r1 - r0) * d; x += NT) {
+      const int r = r0 + x / d, i = x % d, h = head_of(r);
+      const float sink_at = p.sinks != nullptr ? p.sinks[h] : 0.f;      // the score of the key without a value
+      float big = -INFINITY;
+#pragma unroll
+      for (int w = 0; w < PARTS; ++w) big = fmaxf(big, results[(w * R + r) * (d + 2) + d]);
+      if (p.sink) big = fmaxf(big, sink_at);
+      float num = 0.f, den = p.sink ? expf(sink_at - big) : 0.f;
+#pragma unroll
+      for (int w = 0; w < PARTS; ++w) {
+        const float* from = results + (w * R + r) * (d + 2);
+        const float wt = from[d] == -INFINITY ? 0.f : expf(from[d] - big);
+        num += wt * from[i];
+        den += wt * from[d + 1];
+      }
+      const size_t at = (size_t)token_of(r) * p.out_stride + (size_t)h * d + i;
+      const float o = den > 0.f ? num / den : 0.f;
+      if (p.out_f32) static_cast<float*>(p.out)[at] = o;
+      else static_cast<T*>(p.out)[at] = from_f32<T>(o);
+    }
+    __syncthreads();
+    r0 = r1;
+  }
+}
+
+template <typename T, int D, int PARTS, int WPG>
+int launch_rows(RowsParams p, cudaStream_t stream) {
+  const int smem = rows_smem<T>(p.d, PARTS, WPG);
+  const cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<T, D, PARTS, WPG>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  const long long tiles = ((long long)p.tokens + p.tile_tokens - 1) / p.tile_tokens * p.head_tiles;
+  return (int)lab_launch(attention_rows_kernel<T, D, PARTS, WPG>, dim3((unsigned)tiles, p.n_kv), dim3(PARTS * 32 * WPG),
+                         smem, stream, p);
+}
+
+// Sixteen rows a CTA halve what it reads, eight give twice the CTAs: sixteen once they fill every multiprocessor twice.
+template <typename T>
+int pick_rows(RowsParams p, bool single, cudaStream_t stream) {
+  const int group = p.n_q / p.n_kv;
+  auto shape = [&](int rows) {
+    p.tile_tokens = single || group >= rows ? 1 : rows / group;
+    p.head_tiles = (group + rows - 1) / rows;
+    return ((long long)p.tokens + p.tile_tokens - 1) / p.tile_tokens * p.head_tiles * p.n_kv;
+  };
+  const bool wide = shape(2 * RW) >= 2 * 148;
+  if (!wide) shape(RW);
+  if (p.d == 64) return wide ? launch_rows<T, 64, 4, 2>(p, stream) : launch_rows<T, 64, 4, 1>(p, stream);
+  if (p.d == 128) return wide ? launch_rows<T, 128, 4, 2>(p, stream) : launch_rows<T, 128, 4, 1>(p, stream);
+  if (p.d < 128) return wide ? launch_rows<T, 0, 4, 2>(p, stream) : launch_rows<T, 0, 4, 1>(p, stream);
+  return wide ? launch_rows<T, 0, 2, 2>(p, stream) : launch_rows<T, 0, 2, 1>(p, stream);
+}
 }  // namespace
 
+// `single`: no request brings more than one row (rows of one token then make up a tile).
 LAB_EXPORT int lab_attention_plain(void* out, int out_stride, const void* q, int q_stride, const void* cache_k,
                                    const void* cache_v, const int* row_req, const int* row_pos, const int* block_table,
                                    int max_blocks, int tokens, int n_q, int n_kv, int d, int page_size, int num_pages,
                                    int window, float scale, int keep_first, int sink, const float* sinks,
-                                   const float* dist_bias, int bias_len, float softcap, int out_f32, int dtype,
-                                   cudaStream_t stream) {
+                                   const float* dist_bias, int bias_len, float softcap, int out_f32, int single,
+                                   int dtype, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (d > 32 * MAX_DPL || d <= 0 || n_q % n_kv || (dist_bias != nullptr && bias_len < 1)) return (int)cudaErrorInvalidValue;
   if (sinks != nullptr) sink = 1;
+  if (d % (dtype == LAB_F32 ? 4 : 8) == 0 && (((uintptr_t)cache_k | (uintptr_t)cache_v) & 15) == 0 && n_kv <= 65535) {
+    const RowsParams p{out, q, cache_k, cache_v, row_req, row_pos, block_table, sinks, dist_bias, out_stride, q_stride,
+                       max_blocks, tokens, n_q, n_kv, d, page_size, num_pages, window, keep_first, sink, bias_len,
+                       out_f32, 1, 1, scale, softcap};
+    return dtype == LAB_F32 ? pick_rows<float>(p, single != 0, stream) : pick_rows<__nv_bfloat16>(p, single != 0, stream);
+  }
   dim3 grid(tokens, n_q);
   const size_t smem = (size_t)(d + WARPS * (d + 2)) * sizeof(float);
   if (dtype == LAB_F32)

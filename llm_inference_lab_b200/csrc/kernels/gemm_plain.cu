@@ -608,19 +608,28 @@ int launch_tile(void* out, const void* x, const void* w, const void* bias, int M
   const auto kernel = gemm_plain_kernel<T, OutT, GATED, MI, VEC>;
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::BYTES);
   if (e != cudaSuccess) return (int)e;
-  const dim3 grid((N + cols - 1) / cols, (M + Shape::ROWS - 1) / Shape::ROWS, batch);
-  return (int)lab_launch(kernel, grid, dim3(Shape::THREADS), Shape::BYTES, stream, (OutT*)out, (const T*)x, (const T*)w,
-                         (const T*)bias, M, N, K, ldx, ldo, batch_x, batch_w, batch_o, GATED ? 0 : act, row_src, row_div,
-                         tile_group, GATED ? act : 0, gate_limit, row_scale);
+  constexpr int most = 65534 * Shape::ROWS;      // rows of a launch: the grid's limit, whole tiles of groups
+  for (int m0 = 0; m0 < M; m0 += most) {
+    const int rows = M - m0 < most ? M - m0 : most;
+    const dim3 grid((N + cols - 1) / cols, (rows + Shape::ROWS - 1) / Shape::ROWS, batch);
+    const cudaError_t f = lab_launch(
+        kernel, grid, dim3(Shape::THREADS), Shape::BYTES, stream, (OutT*)out + (size_t)m0 * ldo,
+        (const T*)x + (row_src == nullptr ? (size_t)m0 * ldx : 0), (const T*)w, (const T*)bias, rows, N, K, ldx, ldo, batch_x,
+        batch_w, batch_o, GATED ? 0 : act, row_src == nullptr ? nullptr : row_src + m0, row_div,
+        tile_group == nullptr ? nullptr : tile_group + m0 / BM, GATED ? act : 0, gate_limit, row_scale);
+    if (f != cudaSuccess) return (int)f;
+    if (M - m0 <= most) break;
+  }
+  return 0;
 }
 
 // Whether tiles of 16 rows serve M rows of N accumulator columns, rather than tiles of 32.  A launch takes as long as the
 // multiprocessor with the most tiles, and a tile of 16 rows costs 0.54 of one of 32 (measured: 0.49 where a
 // multiprocessor has one, 0.57 where it has four).  517 x 896 x 4864: 155 us in tiles of 32, 176 of 16; 517 x 1152 x 896:
-// 47 and 43; 100 x 896 x 4864: 93 and 74.  (A grid has at most 65,535 rows of tiles.)
+// 47 and 43; 100 x 896 x 4864: 93 and 74.
 static inline bool flat_tiles(long long M, long long N, int batch) {
   const long long columns = (N + 63) / 64 * batch;
-  return M <= 16ll * 65535 && ((M + 15) / 16 * columns + 147) / 148 * 54 < ((M + 31) / 32 * columns + 147) / 148 * 100;
+  return ((M + 15) / 16 * columns + 147) / 148 * 54 < ((M + 31) / 32 * columns + 147) / 148 * 100;
 }
 
 template <typename T, typename OutT>

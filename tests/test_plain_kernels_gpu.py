@@ -35,3 +35,90 @@ def test_product_rows_do_not_depend_on_their_batch(N, K, gated):
     bias = torch.randn(w.shape[0], device=DEV, generator=g)
     if not gated:
         assert torch.equal(ops().gemm_plain(x[3:40], w, bias), ops().gemm_plain(x, w, bias)[3:40])
+
+
+def paged(rng, lens, n_kv, d, page, dtype):
+    """(keys, values, block table, keys and values per request); what no request holds is NaN"""
+    blocks = [-(-n // page) for n in lens]
+    order = rng.permutation(sum(blocks))
+    ck = np.full((sum(blocks), n_kv, page, d), np.nan, dtype=np.float32)
+    cv, bt, held, at = ck.copy(), -np.ones((len(lens), max(blocks)), dtype=np.int32), [], 0
+    for r, n in enumerate(lens):
+        bt[r, :blocks[r]] = order[at: at + blocks[r]]
+        at += blocks[r]
+        k, v = (rng.standard_normal((n, n_kv, d)).astype(np.float32) for _ in range(2))
+        for c, src in ((ck, k), (cv, v)):
+            for j in range(n):
+                c[bt[r, j // page], :, j % page] = src[j]
+        held.append((k, v))
+    t = lambda a: torch.from_numpy(a).to(DEV)  # noqa: E731
+    return t(ck).to(dtype), t(cv).to(dtype), t(bt), held
+
+
+ATTENTION = [
+    # heads, kv heads, head size, page, window, first positions kept, requests (positions held, new rows)
+    (14, 2, 64, 16, 0, 0, [(517, 517), (40, 1), (33, 1), (1, 1)]),
+    (7, 1, 128, 16, 0, 0, [(100, 40), (300, 1)]),
+    (40, 2, 64, 8, 0, 0, [(70, 5), (64, 64)]),          # more heads to a kv head than a tile has rows
+    (3, 3, 20, 4, 0, 0, [(90, 90), (31, 31), (32, 32), (33, 2)]),
+    (4, 2, 256, 16, 0, 0, [(150, 60), (65, 1)]),
+    (2, 2, 200, 16, 40, 7, [(260, 130), (9, 9)]),
+    (6, 2, 8, 16, 33, 70, [(400, 200), (50, 1)]),
+    (6, 3, 18, 16, 0, 0, [(70, 33)]),                    # rows of no whole 16-byte units: the block-per-row kernel
+    (5, 1, 96, 32, -64, 0, [(200, 150), (129, 1)]),      # chunks
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_q,n_kv,d,page,window,keep,requests", ATTENTION)
+def test_attention_rows(n_q, n_kv, d, page, window, keep, requests, dtype):
+    rng = np.random.default_rng(d + n_q)
+    ck, cv, bt, held = paged(rng, [n for n, _ in requests], n_kv, d, page, dtype)
+    pos = np.concatenate([np.arange(n - new, n) for n, new in requests]).astype(np.int32)
+    req = np.concatenate([np.full(new, r) for r, (_, new) in enumerate(requests)]).astype(np.int32)
+    q = torch.from_numpy(rng.standard_normal((len(pos), n_q * d)).astype(np.float32)).to(DEV).to(dtype)
+
+    def run(rows, single=False):
+        rows = np.asarray(rows)
+        t = lambda a: torch.from_numpy(np.ascontiguousarray(a[rows])).to(DEV)  # noqa: E731
+        out = ops().attention_plain(q[torch.from_numpy(rows).to(DEV)], ck, cv, t(req), t(pos), bt, n_q, n_kv, d, window, d ** -0.5,
+                                    keep_first=keep, single=single)
+        ops().take_device_errors()
+        return out
+
+    full = run(np.arange(len(pos)))
+    want = np.zeros((len(pos), n_q, d))
+    for i, (r, p) in enumerate(zip(req, pos)):
+        k, v = (torch.from_numpy(a[: p + 1]).to(dtype).double().numpy() for a in held[r])
+        j = np.arange(p + 1)
+        first = max(0, p - window + 1) if window > 0 else p // -window * -window if window else 0
+        seen = (j >= first) | (j < (keep if window > 0 else 0))
+        for h in range(n_q):
+            s = (k[seen, h // (n_q // n_kv)] @ q[i, h * d: (h + 1) * d].double().cpu().numpy()) * d ** -0.5
+            e = np.exp(s - s.max())
+            want[i, h] = e @ v[seen, h // (n_q // n_kv)] / e.sum()
+    err = np.linalg.norm(full.double().cpu().numpy().reshape(want.shape) - want) / np.linalg.norm(want)
+    assert err < (2e-6 if dtype == torch.float32 else 4e-3)     # roundings of sums; of the result to 8 bits
+    # a row alone, in tiles of its own, and in another neighbourhood gives the same bits
+    some = [0, len(pos) // 2, len(pos) - 1]
+    for i in some:
+        assert torch.equal(run([i], single=True)[0], full[i])
+    assert torch.equal(run(some), full[torch.tensor(some, device=DEV)])
+
+
+def test_attention_rows_keep_infinities_and_nans_to_the_rows_that_see_them():
+    rng = np.random.default_rng(3)
+    n, n_q, n_kv, d = 70, 4, 2, 64
+    ck, cv, bt, _ = paged(rng, [n], n_kv, d, 16, torch.float32)
+    q = torch.from_numpy(rng.standard_normal((n, n_q * d)).astype(np.float32)).to(DEV)
+    t = lambda a: torch.from_numpy(np.asarray(a, dtype=np.int32)).to(DEV)  # noqa: E731
+    run = lambda: ops().attention_plain(q, ck, cv, t([0] * n), t(range(n)), bt, n_q, n_kv, d, 0, 0.125)  # noqa: E731
+    clean = run()
+    page, at = int(bt[0, 40 // 16]), 40 % 16
+    cv[page, 0, at, 5], cv[page, 0, at, 9], ck[page, 1, at, 3] = float("nan"), float("inf"), float("nan")
+    got = run()
+    assert torch.equal(got[:40], clean[:40])
+    heads, before = got[40:].view(n - 40, n_q, d), clean[40:].view(n - 40, n_q, d)
+    assert bool(heads[:, :2, 5].isnan().all()) and bool((heads[:, :2, 9] == float("inf")).all())
+    assert not bool(heads[:, 2:].any())      # a denominator that is no positive number leaves zeros, as the other kernel does
+    assert torch.equal(heads[:, :2, 10:], before[:, :2, 10:])
