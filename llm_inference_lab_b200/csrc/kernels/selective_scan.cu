@@ -8,12 +8,18 @@
 // everything here is 32-bit, the output is rounded once for the output projection.
 //
 // Kernels: the causal convolution of x with the request's last inputs kept between steps (+ SiLU), and
-// the walk.  The walk is sequential in tokens; a CTA takes 16 channels of one request, 8 lanes a channel,
+// the walk.  The walk is sequential in tokens; a CTA takes some channels of one request, WL lanes a channel,
 // each lane a share of the state's entries in registers.  A chunk of tokens waits in shared memory while the
 // next one arrives there (cp.async); step sizes are formed once per channel and token before the chunk is
 // walked.  From token to token passes only the state's own update: every lane leaves its share of the sum
 // over the state in shared memory, and the sums, the skip term and the gate are formed after the chunk, a
 // thread per channel and token.
+//
+// A long portion is cut into segments of tokens that are walked side by side, in two launches: the first walks every
+// segment but the last from zeros (the first one from the request's state) for its closing state and the sum of its
+// step sizes, the second takes every segment again from its opening state, which follows from the segments before it
+// (S <- exp(A sum dt) S + S_segment), and leaves the outputs.  Everything stays 32-bit; the errors against 64-bit are
+// those of the walk in one piece.
 #include "common.cuh"
 
 namespace {
@@ -89,10 +95,9 @@ __global__ void __launch_bounds__(kThreads) conv_keep_inputs_kernel(ConvParams p
 }
 
 // ---- the walk ----------------------------------------------------------------------------------------
-constexpr int WC = 16;        // channels a CTA takes
-constexpr int WL = 8;         // lanes a channel: lane l holds the state entries l, l + 8, ...
 constexpr int WT = 32;        // tokens a chunk
-constexpr int WTHREADS = WC * WL;
+constexpr int WTHREADS = 128;
+constexpr int SCAN_MAX_STATE = 256;
 
 struct ScanParams {
   const float* x;        // [tokens, ld_x] after the convolution and SiLU
@@ -103,34 +108,96 @@ struct ScanParams {
   const int* q_start;
   const int* state_slot;
   int ld_x, ld_dt, ld_bc, ld_z, b_at, c_at, channels, N, n_slots, write, ld_out;
+  int vec;               // rows of all inputs may be copied 16 bytes at a time
+  int segments;          // a request's rows are cut into at most that many segments of whole chunks
+  float* states;         // [requests, segments, channels, N]: 0, a copy of the request's state; i, the state at the end
+                         // of segment i - 1 (from zeros, of segment 0 from the request's state)
+  float* sums;           // [requests, segments, channels]: the sum of the step sizes of segment i - 1
 };
+// What a launch of the walk does: everything in one piece, the segments' closing states, or the outputs.
+enum { SCAN_WHOLE, SCAN_CLOSE, SCAN_OUTPUT };
 
-// 4 bytes from global to shared memory without a register in between; waited for by cp_async_wait_all.
+// 4 or 16 bytes from global to shared memory without a register in between; waited for by cp_async_wait_all.
 __device__ __forceinline__ void cp_async_f32(float* dst, const float* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
                : "memory");
 }
+__device__ __forceinline__ void cp_async_f32x4(float* dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// Floats of one chunk's inputs as they arrive: dt_pre, x, z [WT][WC] each, then B and C [WT][N] each.
-__host__ __device__ inline int scan_chunk_floats(int N) { return 3 * WT * WC + 2 * WT * N; }
+// ---- two 32-bit numbers an instruction, each rounded as by itself -------------------------------------
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float low_of(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high_of(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// exp of two numbers that are not positive, to the hardware's 2^x (relative error about 2^-22): x log2(e) is cut into the
+// nearest integer and a rest of at most a half, the rest formed from log2(e) in two pieces (the range reduction of Cody
+// and Waite), so that a slow decay, whose error comes with the same sign at every token and adds up over the state's
+// memory, is off by no more than a fast one.  Below -86 the result stays at exp(-86), 4e-38.
+__device__ __forceinline__ f32x2 exp2_of(f32x2 x) {
+  const float magic = 12582912.f;      // 1.5 * 2^23: adding it rounds to an integer, which is left in the low bits
+  x = pair_of(fmaxf(low_of(x), -86.f), fmaxf(high_of(x), -86.f));
+  const f32x2 hi = pair_of(1.44269502f, 1.44269502f), lo = pair_of(1.92596299e-8f, 1.92596299e-8f);
+  const f32x2 t = fma2(x, hi, pair_of(magic, magic));
+  const f32x2 minus_j = fma2(t, pair_of(-1.f, -1.f), pair_of(magic, magic));
+  const f32x2 rest = fma2(x, lo, fma2(x, hi, minus_j));
+  return pair_of(__uint_as_float(__float_as_uint(fast_exp2(low_of(rest))) + ((uint32_t)t << 23)),
+                 __uint_as_float(__float_as_uint(fast_exp2(high_of(rest))) + ((uint32_t)(t >> 32) << 23)));
+}
 
-template <typename T, int R>
+// Floats of one chunk's inputs as they arrive: dt_pre, x, z [WT][channels] each, then B and C [WT][N4] each, N4 the
+// state's entries in whole quads.
+__host__ __device__ inline int scan_chunk_floats(int wc, int n4) { return 3 * WT * wc + 2 * WT * n4; }
+
+// Lane l of a channel's WL holds the quads l, l + WL, ... of its state, R entries in all.  What bounds the walk, once
+// there are CTAs enough, is the issue of instructions: an entry and token takes eight, most of them for two entries at
+// once; a token of a CTA also takes its step sizes, gates and copies.  Measured on a B200, 1,792 channels of 16 entries:
+// 8 requests of 250 tokens 69 us (102 with eight lanes a channel, an entry an instruction and expf); one of 2,048
+// 114 us in eleven segments (344 in one piece of that form).
+template <typename T, int WL, int R, int MODE>
 __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict__ out, const T* __restrict__ a_log,
                                                                   const T* __restrict__ skip,
                                                                   const T* __restrict__ dt_bias, ScanParams p) {
-  extern __shared__ float smem[];
-  const int N = p.N, chunk_floats = scan_chunk_floats(N);
+  extern __shared__ __align__(16) float smem[];
+  constexpr int WC = WTHREADS / WL, Q = R / 4;
+  const int N = p.N, n4 = (N + 3) & ~3, chunk_floats = scan_chunk_floats(WC, n4);
   float* s_in = smem;                          // two chunks of inputs: one walked, one arriving
   float* s_dx = smem + 2 * chunk_floats;       // [WT][WC] step size times x
   float* s_part = s_dx + WT * WC;              // [WT][WC][WL] every lane's share of the sum over the state
-  pdl_trigger();
   pdl_wait();
   const int r = blockIdx.y, c0 = blockIdx.x * WC;
-  const int first = p.q_start[r], n = p.q_start[r + 1] - first, slot = p.state_slot[r];
+  int first = p.q_start[r], n = p.q_start[r + 1] - first;
+  const int slot = p.state_slot[r];
+  int seg = 0, last = 0;      // this CTA's segment, the request's last one
+  if (MODE != SCAN_WHOLE && n > 0) {
+    const int len = (((n + p.segments - 1) / p.segments) + WT - 1) / WT * WT;
+    seg = blockIdx.z;
+    last = (n - 1) / len;
+    if (MODE == SCAN_CLOSE && seg >= last) return;
+    first += seg * len;
+    n = min(len, n - seg * len);
+  }
   if (n <= 0) return;
   const int tid = threadIdx.x, ch = tid / WL, l = tid % WL, c = c0 + ch;
   const bool live = c < p.channels;
+  if (MODE == SCAN_CLOSE && (slot < 0 || slot >= p.n_slots)) return;      // (the next launch deals with these)
   if (slot == -1) {       // rows of padding leave zeros
     for (int i = tid; i < n * WC; i += WTHREADS)
       if (c0 + i % WC < p.channels) out[(size_t)(first + i / WC) * p.ld_out + c0 + i % WC] = from_f32<T>(0.f);
@@ -140,39 +207,85 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
     if (tid == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
     return;
   }
+  if (N != n4) {      // the last quad's missing entries of B and C are zeros, which no copy touches
+    for (int i = tid; i < 2 * chunk_floats; i += WTHREADS) s_in[i] = 0.f;
+    __syncthreads();
+  }
   // a chunk's inputs set out for shared memory; channels beyond the last read nothing and stay unused
   auto fetch = [&](int t0, float* buf) {
     const int nt = min(WT, n - t0);
-    float *b_dt = buf, *b_x = buf + WT * WC, *b_z = buf + 2 * WT * WC, *b_b = buf + 3 * WT * WC, *b_c = b_b + WT * N;
+    float *b_dt = buf, *b_x = buf + WT * WC, *b_z = buf + 2 * WT * WC, *b_b = buf + 3 * WT * WC, *b_c = b_b + WT * n4;
+    const size_t row0 = (size_t)(first + t0);
+    if (p.vec) {
+      for (int i = tid; i < nt * (WC / 4); i += WTHREADS) {
+        const int cc = c0 + 4 * (i % (WC / 4));
+        if (cc >= p.channels) continue;
+        const size_t row = row0 + i / (WC / 4);
+        cp_async_f32x4(b_dt + 4 * i, p.dt_pre + row * p.ld_dt + cc);
+        cp_async_f32x4(b_x + 4 * i, p.x + row * p.ld_x + cc);
+        if (MODE != SCAN_CLOSE) cp_async_f32x4(b_z + 4 * i, p.z + row * p.ld_z + cc);
+      }
+      for (int i = tid; i < nt * (n4 / 4); i += WTHREADS) {
+        const float* row = p.bc + (row0 + i / (n4 / 4)) * p.ld_bc + 4 * (i % (n4 / 4));
+        cp_async_f32x4(b_b + 4 * i, row + p.b_at);
+        if (MODE != SCAN_CLOSE) cp_async_f32x4(b_c + 4 * i, row + p.c_at);
+      }
+      return;
+    }
     for (int i = tid; i < nt * WC; i += WTHREADS) {
       const int cc = c0 + i % WC;
       if (cc >= p.channels) continue;
-      const size_t row = (size_t)(first + t0 + i / WC);
+      const size_t row = row0 + i / WC;
       cp_async_f32(b_dt + i, p.dt_pre + row * p.ld_dt + cc);
       cp_async_f32(b_x + i, p.x + row * p.ld_x + cc);
-      cp_async_f32(b_z + i, p.z + row * p.ld_z + cc);
+      if (MODE != SCAN_CLOSE) cp_async_f32(b_z + i, p.z + row * p.ld_z + cc);
     }
     for (int i = tid; i < nt * N; i += WTHREADS) {
-      const float* row = p.bc + (size_t)(first + t0 + i / N) * p.ld_bc + i % N;
-      cp_async_f32(b_b + i, row + p.b_at);
-      cp_async_f32(b_c + i, row + p.c_at);
+      const float* row = p.bc + (row0 + i / N) * p.ld_bc + i % N;
+      cp_async_f32(b_b + i / N * n4 + i % N, row + p.b_at);
+      if (MODE != SCAN_CLOSE) cp_async_f32(b_c + i / N * n4 + i % N, row + p.c_at);
     }
   };
   fetch(0, s_in);
+  auto entry = [&](int i) { return ((i / 4) * WL + l) * 4 + i % 4; };      // the state's entry that S[i] holds
   float S[R], A[R];
   float* st = p.state + ((size_t)slot * p.channels + (live ? c : 0)) * N;
+  const size_t per_segment = (size_t)p.channels * N;
+  float* kept = MODE == SCAN_WHOLE ? nullptr : p.states + (size_t)r * p.segments * per_segment + (size_t)(live ? c : 0) * N;
+  const float* sums = MODE == SCAN_WHOLE ? nullptr : p.sums + (size_t)r * p.segments * p.channels + (live ? c : 0);
 #pragma unroll
   for (int i = 0; i < R; ++i) {
-    const int e = i * WL + l;
+    const int e = entry(i);
     const bool has = live && e < N;
-    S[i] = has ? st[e] : 0.f;
     A[i] = has ? -expf(to_f32(a_log[(size_t)c * N + e])) : 0.f;
+    S[i] = 0.f;
+    if (!has) continue;
+    if (MODE == SCAN_WHOLE || (MODE == SCAN_OUTPUT && last == 0)) {
+      S[i] = st[e];
+    } else if (MODE == SCAN_CLOSE) {
+      // (the last segment's CTA of the next launch writes the request's state while others still open theirs)
+      if (seg == 0) kept[e] = S[i] = st[e];
+    } else {
+      S[i] = kept[(seg == 0 ? 0 : per_segment) + e];
+    }
   }
+  if (MODE == SCAN_OUTPUT) {
+    for (int g = 2; g <= seg; ++g) {
+      const float dt = sums[(size_t)g * p.channels];
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (live && entry(i) < N) S[i] = fmaf(expf(dt * A[i]), S[i], kept[g * per_segment + entry(i)]);
+    }
+  }
+  f32x2 S2[R / 2], A2[R / 2];
+#pragma unroll
+  for (int i = 0; i < R / 2; ++i) S2[i] = pair_of(S[2 * i], S[2 * i + 1]), A2[i] = pair_of(A[2 * i], A[2 * i + 1]);
+  float dt_sum = 0.f;      // SCAN_CLOSE: of channel tid % WC, over this thread's tokens
   int which = 0;
   for (int t0 = 0; t0 < n; t0 += WT, which ^= 1) {
     const int nt = min(WT, n - t0);
     float* buf = s_in + which * chunk_floats;
-    float *b_dt = buf, *b_x = buf + WT * WC, *b_z = buf + 2 * WT * WC, *b_b = buf + 3 * WT * WC, *b_c = b_b + WT * N;
+    float *b_dt = buf, *b_x = buf + WT * WC, *b_z = buf + 2 * WT * WC, *b_b = buf + 3 * WT * WC, *b_c = b_b + WT * n4;
     cp_async_wait_all();
     __syncthreads();       // the chunk is here; the chunk before has been written out, its buffer is free
     if (t0 + WT < n) fetch(t0 + WT, s_in + (which ^ 1) * chunk_floats);
@@ -186,75 +299,104 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
       }
       b_dt[i] = dt;
       s_dx[i] = dx;
+      if (MODE == SCAN_CLOSE) dt_sum += dt;
     }
     __syncthreads();
     // the walk: nothing but the state's own update passes from token to token
-#pragma unroll 4
+#pragma unroll 2
     for (int tt = 0; tt < nt; ++tt) {
       const float dt = b_dt[tt * WC + ch], dx = s_dx[tt * WC + ch];
-      float acc = 0.f;
+      const f32x2 dt2 = pair_of(dt, dt), dx2 = pair_of(dx, dx);
+      f32x2 acc = 0ull;      // two zeros
 #pragma unroll
-      for (int i = 0; i < R; ++i) {
-        const int e = i * WL + l;
-        if (e < N) {
-          // expf, not a power of two with A scaled: a slow decay's error of one more unit in the last place
-          // comes with the same sign at every token and adds up over the state's memory
-          S[i] = fmaf(expf(dt * A[i]), S[i], dx * b_b[tt * N + e]);
-          acc = fmaf(S[i], b_c[tt * N + e], acc);
+      for (int q = 0; q < Q; ++q) {
+        const int e = (q * WL + l) * 4;
+        if (Q * WL * 4 > 16 && e >= n4) break;
+        if (Q * WL * 4 == 16 && e >= n4) continue;
+        const ulonglong2 bq = *reinterpret_cast<const ulonglong2*>(b_b + tt * n4 + e);
+        S2[2 * q] = fma2(exp2_of(mul2(dt2, A2[2 * q])), S2[2 * q], mul2(dx2, bq.x));
+        S2[2 * q + 1] = fma2(exp2_of(mul2(dt2, A2[2 * q + 1])), S2[2 * q + 1], mul2(dx2, bq.y));
+        if (MODE != SCAN_CLOSE) {
+          const ulonglong2 cq = *reinterpret_cast<const ulonglong2*>(b_c + tt * n4 + e);
+          acc = fma2(S2[2 * q], cq.x, acc);
+          acc = fma2(S2[2 * q + 1], cq.y, acc);
         }
       }
-      s_part[tt * WTHREADS + tid] = acc;
+      if (MODE != SCAN_CLOSE) s_part[tt * WTHREADS + tid] = low_of(acc) + high_of(acc);
     }
+    if (MODE == SCAN_CLOSE) continue;
     __syncthreads();
     // the sum over the lanes (in their order), the skip term and the gate, a thread per channel and token
     for (int i = tid; i < nt * WC; i += WTHREADS) {
       const int cc = c0 + i % WC;
       if (cc >= p.channels) continue;
-      const float4 lo = *reinterpret_cast<const float4*>(s_part + (size_t)i * WL);
-      const float4 hi = *reinterpret_cast<const float4*>(s_part + (size_t)i * WL + 4);
-      const float acc = ((lo.x + hi.x) + (lo.z + hi.z)) + ((lo.y + hi.y) + (lo.w + hi.w));
+      float4 sum = *reinterpret_cast<const float4*>(s_part + (size_t)i * WL);
+      if (WL == 8) {
+        const float4 hi = *reinterpret_cast<const float4*>(s_part + (size_t)i * WL + 4);
+        sum.x += hi.x, sum.y += hi.y, sum.z += hi.z, sum.w += hi.w;
+      }
+      const float acc = (sum.x + sum.z) + (sum.y + sum.w);
       out[(size_t)(first + t0 + i / WC) * p.ld_out + cc] =
           from_f32<T>(fmaf(to_f32(skip[cc]), b_x[i], acc) * silu_f(b_z[i]));
     }
   }
-  if (p.write && live) {
+  pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
+  if (MODE == SCAN_CLOSE) {
+    s_part[tid] = dt_sum;      // WC threads apart: the same channel
+    __syncthreads();
+    if (tid < WC && c0 + tid < p.channels) {
+      float all = 0.f;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-      const int e = i * WL + l;
-      if (e < N) st[e] = S[i];
+      for (int i = 0; i < WTHREADS / WC; ++i) all += s_part[i * WC + tid];
+      p.sums[((size_t)r * p.segments + seg + 1) * p.channels + c0 + tid] = all;
     }
   }
+  float* to = MODE == SCAN_CLOSE ? kept + (seg + 1) * per_segment : st;
+  if (live && (MODE == SCAN_CLOSE || (p.write && seg == last))) {
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+      if (entry(i) < N) to[entry(i)] = i % 2 == 0 ? low_of(S2[i / 2]) : high_of(S2[i / 2]);
+  }
 }
 
-template <typename T, int R>
-int launch_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
-                cudaStream_t stream) {
-  const size_t smem = sizeof(float) * ((size_t)2 * scan_chunk_floats(p.N) + (size_t)WT * WC + (size_t)WT * WC * WL);
+template <typename T, int WL, int R, int MODE>
+int launch_scan_as(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
+                   cudaStream_t stream) {
+  constexpr int WC = WTHREADS / WL;
+  const size_t smem = sizeof(float) * ((size_t)2 * scan_chunk_floats(WC, (p.N + 3) & ~3) + WT * WC + WT * WTHREADS);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, WL, R, MODE>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  return (int)lab_launch(selective_scan_kernel<T, R>, dim3((p.channels + WC - 1) / WC, requests), dim3(WTHREADS), smem,
-                         stream, (T*)out, (const T*)a_log, (const T*)skip, (const T*)dt_bias, p);
+  const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
+  return (int)lab_launch(selective_scan_kernel<T, WL, R, MODE>, dim3((p.channels + WC - 1) / WC, requests, segments),
+                         dim3(WTHREADS), smem, stream, (T*)out, (const T*)a_log, (const T*)skip, (const T*)dt_bias, p);
 }
 
+template <typename T, int WL, int R>
+int launch_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
+                cudaStream_t stream) {
+  if (p.segments <= 1) return launch_scan_as<T, WL, R, SCAN_WHOLE>(out, a_log, skip, dt_bias, p, requests, stream);
+  const int e = launch_scan_as<T, WL, R, SCAN_CLOSE>(out, a_log, skip, dt_bias, p, requests, stream);
+  return e != 0 ? e : launch_scan_as<T, WL, R, SCAN_OUTPUT>(out, a_log, skip, dt_bias, p, requests, stream);
+}
+
+// Four lanes a channel up to 64 entries; eight beyond, where a lane's registers would not hold a quarter.
 template <typename T>
 int pick_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
               cudaStream_t stream) {
-  const int per_lane = (p.N + WL - 1) / WL;
-  if (per_lane <= 1) return launch_scan<T, 1>(out, a_log, skip, dt_bias, p, requests, stream);
-  if (per_lane <= 2) return launch_scan<T, 2>(out, a_log, skip, dt_bias, p, requests, stream);
-  if (per_lane <= 3) return launch_scan<T, 3>(out, a_log, skip, dt_bias, p, requests, stream);
-  if (per_lane <= 4) return launch_scan<T, 4>(out, a_log, skip, dt_bias, p, requests, stream);
-  if (per_lane <= 8) return launch_scan<T, 8>(out, a_log, skip, dt_bias, p, requests, stream);
-  if (per_lane <= 16) return launch_scan<T, 16>(out, a_log, skip, dt_bias, p, requests, stream);
-  if (per_lane <= 32) return launch_scan<T, 32>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (p.N <= 16) return launch_scan<T, 4, 4>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (p.N <= 32) return launch_scan<T, 4, 8>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (p.N <= 64) return launch_scan<T, 4, 16>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (p.N <= 128) return launch_scan<T, 8, 16>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (p.N <= SCAN_MAX_STATE) return launch_scan<T, 8, 32>(out, a_log, skip, dt_bias, p, requests, stream);
   return (int)cudaErrorInvalidValue;
 }
 }  // namespace
 
 // The largest state (entries per channel) the walk takes.
-LAB_EXPORT int lab_selective_scan_max_state() { return 32 * WL; }
+LAB_EXPORT int lab_selective_scan_max_state() { return SCAN_MAX_STATE; }
 
 LAB_EXPORT int lab_conv_silu(float* out32, void* out_t, const float* proj, int ld, int conv_at, int channels, int taps,
                              const void* taps_w, const void* taps_b, float* kept, const int* row_req,
@@ -280,17 +422,24 @@ LAB_EXPORT int lab_conv_silu(float* out32, void* out_t, const float* proj, int l
   return 0;
 }
 
+// segments > 1: every request's rows are cut into at most that many; `states` [requests, segments, channels, N] and
+// `sums` [requests, segments, channels] are scratch.
 LAB_EXPORT int lab_selective_scan(void* out, int ld_out, const float* x, int ld_x, const float* dt_pre, int ld_dt,
                                   const float* bc, int ld_bc, int b_at, int c_at, const float* z, int ld_z,
                                   const void* a_log, const void* skip, const void* dt_bias, float* state,
                                   const int* q_start, const int* state_slot, int requests, int channels, int N,
-                                  int n_slots, int write, int dtype, cudaStream_t stream) {
+                                  int n_slots, int write, int segments, float* states, float* sums, int dtype,
+                                  cudaStream_t stream) {
   if (requests <= 0) return 0;
-  if (channels <= 0 || N <= 0 || N > 32 * WL) return (int)cudaErrorInvalidValue;
+  if (channels <= 0 || N <= 0 || N > SCAN_MAX_STATE) return (int)cudaErrorInvalidValue;
+  if (segments > 65535 || (segments > 1 && (states == nullptr || sums == nullptr))) return (int)cudaErrorInvalidValue;
   ScanParams p;
   p.x = x; p.dt_pre = dt_pre; p.bc = bc; p.z = z; p.state = state; p.q_start = q_start; p.state_slot = state_slot;
   p.ld_x = ld_x; p.ld_dt = ld_dt; p.ld_bc = ld_bc; p.ld_z = ld_z; p.b_at = b_at; p.c_at = c_at; p.channels = channels;
   p.N = N; p.n_slots = n_slots; p.write = write; p.ld_out = ld_out;
+  p.segments = segments; p.states = states; p.sums = sums;
+  p.vec = ((ld_x | ld_dt | ld_bc | ld_z | b_at | c_at | channels | N) & 3) == 0 &&
+          ((((uintptr_t)x) | ((uintptr_t)dt_pre) | ((uintptr_t)bc) | ((uintptr_t)z)) & 15) == 0;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
   if (dtype == LAB_F32) return pick_scan<float>(out, a_log, skip, dt_bias, p, requests, stream);
   return pick_scan<__nv_bfloat16>(out, a_log, skip, dt_bias, p, requests, stream);

@@ -1637,6 +1637,15 @@ def conv_silu(proj: torch.Tensor, conv_at: int, channels: int, taps: int, w: tor
     return out32, out_t
 
 
+def scan_segments(ctas: int, longest: int) -> int:
+    """Into how many segments `selective_scan` cuts a request's rows, `ctas` CTAs walking the step in one piece and a
+    multiprocessor holding four.  Segments cost a second launch and most of the walk's work once more, so they pay while
+    they bring idle multiprocessors to work: measured with its mixer, 56 CTAs and 2,048 tokens 684 us in one piece, 327
+    in 4, 238 in 8, 223 in 12; 112 CTAs and 700 tokens 259, 189 in 4, 171 in 6, 181 in 8; 224 CTAs and 500 tokens 247, 233
+    in 2; 448 CTAs and 250 tokens 175, 196 in 2.  Segments of 32 tokens (a chunk) still pay: 128 tokens 118, 100 in 4."""
+    return max(1, min(longest // 32, 9 * sm_count() // (2 * max(1, ctas)), 32))
+
+
 def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int, z: torch.Tensor,
                    a_log: torch.Tensor, skip: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, ctx,
                    write: bool = True) -> torch.Tensor:
@@ -1654,11 +1663,16 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
     if N > SELECTIVE_SCAN_MAX_STATE:
         raise KernelError(f"selective_scan: a state of {N} entries a channel exceeds {SELECTIVE_SCAN_MAX_STATE}")
     out = torch.empty((tokens, channels), dtype=a_log.dtype, device=x.device)
+    segments = scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
+    states = sums = None
+    if segments > 1:
+        states = torch.empty((ctx.n_requests, segments, channels, N), dtype=torch.float32, device=x.device)
+        sums = torch.empty((ctx.n_requests, segments, channels), dtype=torch.float32, device=x.device)
     _check(lib("selective_scan").lab_selective_scan(
         _ptr(out), out.stride(0), _ptr(x), x.stride(0), _ptr(dt_pre), dt_pre.stride(0), _ptr(bc), bc.stride(0), b_at,
         c_at, _ptr(z), z.stride(0), _ptr(a_log), _ptr(skip), _ptr(dt_bias), _ptr(state), _ptr(ctx.q_start),
-        _ptr(ctx.state_slot), ctx.n_requests, channels, N, state.shape[0], int(write), dtype_code(a_log.dtype),
-        _stream()), "selective_scan")
+        _ptr(ctx.state_slot), ctx.n_requests, channels, N, state.shape[0], int(write), segments, _ptr(states),
+        _ptr(sums), dtype_code(a_log.dtype), _stream()), "selective_scan", 2 if segments > 1 else 1)
     return out
 
 
