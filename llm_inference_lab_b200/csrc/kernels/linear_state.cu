@@ -5,10 +5,11 @@
 // a_t is a constant of the head (linear attention with a fixed decay) or a number per token and head (a
 // state-space mixer, where a_t = exp(-exp(A_log) * dt_t) and s_t = dt_t); q and k may be shared by the
 // heads of a group.  The state is 32-bit, is read at a request's first row of the step and written back
-// after its last, and every product and sum of the recurrence is 32-bit, token by token in order, so a
-// position's result does not depend on how the sequence was cut into steps.
+// after its last, and every product and sum of the recurrence is 32-bit.
 //
-//   decay_scan        the recurrence over each request's rows (any number of rows, single tokens included)
+//   decay_scan        the recurrence over each request's rows (any number of rows, single tokens included), token by
+//                     token in order; rows of a long portion in segments side by side, whose opening states follow
+//                     from the segments before them (S <- (product of decays) S + S_segment)
 //   ssm_prepare       for a state-space mixer, from the 32-bit input projection [z | x | B | C | dt]: the
 //                     causal convolution per channel of x, B, C over the last `taps` inputs (the inputs
 //                     before a step's first row come from the request's kept inputs) with bias and SiLU;
@@ -63,39 +64,72 @@ struct ScanParams {
   const int* state_slot;
   int n_slots, H, G, N, V, act, write;
   int vec;               // q, k, v rows may be copied 16 bytes at a time
+  int segments;          // a request's rows are cut into at most that many segments of whole chunks
+  float* states;         // [requests, segments, H, N, V]: 0, a copy of the request's state; i, the state at the end of
+                         // segment i - 1 (from zeros, of segment 0 from the request's state)
+  float* decays;         // [requests, segments, H]: the product of the decays of segment i - 1
 };
+// What a launch does: everything in one piece, the segments' closing states, or the outputs.
+enum { SCAN_WHOLE, SCAN_CLOSE, SCAN_OUTPUT };
+
+// two 32-bit numbers an instruction, each rounded as by itself
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float low_of(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high_of(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 
 // grid (slices of V, heads, requests); block 2 * SCAN_P * Vs threads in two halves.
 //
 // Walkers (the first SCAN_P * Vs threads): thread (j, part) keeps rows part * R .. part * R + R - 1 of column
 // slice * Vs + j of the state in registers (R a multiple of 4: the rows' keys and queries come from shared
 // memory four at a time; the four threads' shares of a token's keys lie R + 4 floats apart, which spreads
-// their 16-byte loads over the banks).  A token costs a walker 2 R multiply-adds behind R / 2 loads; the four
+// their 16-byte loads over the banks).  A token costs a walker 3 R / 2 instructions on two rows each behind R / 2 loads; the four
 // walkers of a column add their shares of the output by two shuffles.  The next token's keys, queries and
 // value are loaded before the current token's arithmetic (up to R = 16; beyond, registers do not allow it).
-// The walk is one dependent chain per request and head: its time is the number of tokens times that step,
-// whatever the number of CTAs, so nothing else may sit on it.
+// The walk of a segment is one dependent chain: its time is the number of tokens times that step, whatever the number
+// of CTAs, so nothing else may sit on it.  (A launch for the closing states forms no outputs: no queries, two thirds
+// of the instructions.)
 //
 // Helpers (the other half) keep everything else off that chain: while the walkers are on chunk c (16 tokens),
 // the helpers apply the SiLU to chunk c + 1, whose rows their cp.async copies have brought (16 bytes a copy
 // where the operands' addresses allow it: `vec`), and start the copies of chunk c + 2 into the buffer the
 // walkers left one chunk ago.  Three buffers, one barrier of the whole CTA per chunk.
-template <int R>
+template <int R, int MODE>
 __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
   extern __shared__ __align__(16) float smem[];
   constexpr int RS = R + 4;                      // floats between two threads' shares of a token's keys
   constexpr int NP = SCAN_P * RS;                // floats of a token's keys (or queries) in shared memory
-  constexpr bool AHEAD = R <= 16;                // the next token's operands are loaded a token ahead
-  pdl_trigger();
+  constexpr bool OUT = MODE != SCAN_CLOSE;
   const int walkers = blockDim.x / 2, Vs = walkers / SCAN_P;
   const int tok_floats = 2 * NP + Vs + 4;        // k | q | v | a | s | (two unused, which keep rows 16-byte aligned)
-  const int h = blockIdx.y, r = blockIdx.z, g = h / (p.H / p.G);
+  const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
+  const int h = blockIdx.y, r = blockIdx.z / segments, seg = blockIdx.z % segments, g = h / (p.H / p.G);
   const bool helper = threadIdx.x >= walkers;
   const int tid = helper ? threadIdx.x - walkers : threadIdx.x;      // index within the half
   const int j = tid / SCAN_P, part = tid % SCAN_P;
   const int col0 = blockIdx.x * Vs, col = col0 + j;
-  const int t0 = p.q_start[r], n_tok = p.q_start[r + 1] - t0;
+  int t0 = p.q_start[r], n_tok = p.q_start[r + 1] - t0, last = 0;      // last: the request's last segment
   const int slot = p.state_slot[r];
+  if (MODE != SCAN_WHOLE && n_tok > 0) {
+    const int len = ((n_tok + p.segments - 1) / p.segments + SCAN_CT - 1) / SCAN_CT * SCAN_CT;
+    last = (n_tok - 1) / len;
+    t0 += seg * len;
+    n_tok = MODE == SCAN_CLOSE && seg >= last ? 0 : min(len, n_tok - seg * len);
+  }
   if (n_tok <= 0 || slot == -1) {      // nothing to do, or rows of padding (their output is never read)
     pdl_wait();
     return;
@@ -130,7 +164,7 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
         const int tt = e / per, c = e - tt * per;
         float* dst = base + tt * tok_floats;
         if (c < nk) cp_async16(dst + at(4 * c), k0 + (size_t)tt * p.ld_qk + 4 * c);
-        else if (c < 2 * nk) cp_async16(dst + NP + at(4 * (c - nk)), q0 + (size_t)tt * p.ld_qk + 4 * (c - nk));
+        else if (c < 2 * nk) { if (OUT) cp_async16(dst + NP + at(4 * (c - nk)), q0 + (size_t)tt * p.ld_qk + 4 * (c - nk)); }
         else cp_async16(dst + 2 * NP + 4 * (c - 2 * nk), v0 + (size_t)tt * p.ld_v + 4 * (c - 2 * nk));
       }
     } else {
@@ -139,7 +173,7 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
         const int tt = e / per, c = e - tt * per;
         float* dst = base + tt * tok_floats;
         if (c < p.N) cp_async4(dst + at(c), k0 + (size_t)tt * p.ld_qk + c);
-        else if (c < 2 * p.N) cp_async4(dst + NP + at(c - p.N), q0 + (size_t)tt * p.ld_qk + (c - p.N));
+        else if (c < 2 * p.N) { if (OUT) cp_async4(dst + NP + at(c - p.N), q0 + (size_t)tt * p.ld_qk + (c - p.N)); }
         else cp_async4(dst + 2 * NP + (c - 2 * p.N), v0 + (size_t)tt * p.ld_v + (c - 2 * p.N));
       }
     }
@@ -165,8 +199,12 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
     }
   };
 
-  float S[R];
+  f32x2 S[R / 2];
+  float decayed = 1.f;      // SCAN_CLOSE: the product of the decays
   float* st = p.state + ((size_t)slot * p.H + h) * p.N * p.V;
+  const size_t per_segment = (size_t)p.H * p.N * p.V;
+  float* kept = MODE == SCAN_WHOLE ? nullptr : p.states + (size_t)r * p.segments * per_segment + (size_t)h * p.N * p.V;
+  float* decays = MODE == SCAN_WHOLE ? nullptr : p.decays + (size_t)r * p.segments * p.H + h;
   float a_const = 0.f;
   if (helper) {
     issue(0);
@@ -176,11 +214,31 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
     cp_async_wait_group<1>();
     finish(0);
   } else {
+    float s[R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-      const int n = part * R + i;
-      S[i] = (n < p.N && col < p.V) ? st[(size_t)n * p.V + col] : 0.f;
+      const size_t at = (size_t)(part * R + i) * p.V + col;
+      s[i] = 0.f;
+      if (part * R + i >= p.N || col >= p.V) continue;
+      if (MODE == SCAN_WHOLE || (MODE == SCAN_OUTPUT && last == 0)) {
+        s[i] = st[at];
+      } else if (MODE == SCAN_CLOSE) {
+        // (the last segment's CTA of the next launch writes the request's state while others still open theirs)
+        if (seg == 0) kept[at] = s[i] = st[at];
+      } else {
+        s[i] = kept[(seg == 0 ? 0 : per_segment) + at];
+      }
     }
+    if (MODE == SCAN_OUTPUT) {
+      for (int e = 2; e <= seg; ++e) {
+        const float a = decays[(size_t)e * p.H];
+#pragma unroll
+        for (int i = 0; i < R; ++i)
+          if (part * R + i < p.N && col < p.V) s[i] = fmaf(a, s[i], kept[e * per_segment + (size_t)(part * R + i) * p.V + col]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < R / 2; ++i) S[i] = pair_of(s[2 * i], s[2 * i + 1]);
     if (p.a_tok == nullptr) a_const = p.a_head[h];
   }
   __syncthreads();
@@ -197,60 +255,67 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
       const int cnt = min(SCAN_CT, n_tok - c * SCAN_CT);
       const float* base = buffer(c);
       float* out = p.out + (size_t)(t0 + c * SCAN_CT) * p.ld_o + h * p.V + col;
-      float4 kk[R / 4], qq[R / 4];
-      float a, vj;
-      auto load = [&](int tt, float4* k_to, float4* q_to, float& a_to, float& v_to) {
+      // a token's update; the walker's share of its output
+      auto step = [&](int tt) {
         const float* tok = base + tt * tok_floats;
-        const float4* k4 = reinterpret_cast<const float4*>(tok + part * RS);
-        const float4* q4 = reinterpret_cast<const float4*>(tok + NP + part * RS);
-#pragma unroll
-        for (int i = 0; i < R / 4; ++i) k_to[i] = k4[i], q_to[i] = q4[i];
-        a_to = p.a_tok != nullptr ? tok[2 * NP + Vs] : a_const;
-        v_to = tok[2 * NP + j];
-        if (p.s_tok != nullptr) v_to *= tok[2 * NP + Vs + 1];
-      };
-      if (AHEAD) load(0, kk, qq, a, vj);
-      for (int tt = 0; tt < cnt; ++tt) {
-        float4 kn[AHEAD ? R / 4 : 1], qn[AHEAD ? R / 4 : 1];
-        float an = 0.f, vn = 0.f;
-        if (AHEAD) {
-          if (tt + 1 < cnt) load(tt + 1, kn, qn, an, vn);
-        } else {
-          load(tt, kk, qq, a, vj);
-        }
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        const ulonglong2* k4 = reinterpret_cast<const ulonglong2*>(tok + part * RS);
+        const ulonglong2* q4 = reinterpret_cast<const ulonglong2*>(tok + NP + part * RS);
+        const float a = p.a_tok != nullptr ? tok[2 * NP + Vs] : a_const;
+        float vj = tok[2 * NP + j];
+        if (p.s_tok != nullptr) vj *= tok[2 * NP + Vs + 1];
+        const f32x2 aa = pair_of(a, a), vv = pair_of(vj, vj);
+        f32x2 acc[2] = {0ull, 0ull};      // zeros
 #pragma unroll
         for (int i = 0; i < R / 4; ++i) {
-          S[4 * i + 0] = fmaf(a, S[4 * i + 0], kk[i].x * vj);
-          S[4 * i + 1] = fmaf(a, S[4 * i + 1], kk[i].y * vj);
-          S[4 * i + 2] = fmaf(a, S[4 * i + 2], kk[i].z * vj);
-          S[4 * i + 3] = fmaf(a, S[4 * i + 3], kk[i].w * vj);
-          acc[0] = fmaf(S[4 * i + 0], qq[i].x, acc[0]);
-          acc[1] = fmaf(S[4 * i + 1], qq[i].y, acc[1]);
-          acc[2] = fmaf(S[4 * i + 2], qq[i].z, acc[2]);
-          acc[3] = fmaf(S[4 * i + 3], qq[i].w, acc[3]);
+          const ulonglong2 k = k4[i];
+          S[2 * i] = fma2(aa, S[2 * i], mul2(k.x, vv));
+          S[2 * i + 1] = fma2(aa, S[2 * i + 1], mul2(k.y, vv));
+          if (OUT) {
+            const ulonglong2 q = q4[i];
+            acc[0] = fma2(S[2 * i], q.x, acc[0]);
+            acc[1] = fma2(S[2 * i + 1], q.y, acc[1]);
+          }
         }
-        float total = (acc[0] + acc[1]) + (acc[2] + acc[3]);
-        total += __shfl_xor_sync(0xffffffffu, total, 1);
-        total += __shfl_xor_sync(0xffffffffu, total, 2);
-        if (part == 0 && col < p.V) out[(size_t)tt * p.ld_o] = total;
-        if (AHEAD) {
+        if (!OUT) decayed *= a;
+        return (low_of(acc[0]) + high_of(acc[0])) + (low_of(acc[1]) + high_of(acc[1]));
+      };
+      // four tokens at a time: their sums over a column's four walkers take three shuffles together and leave walker p
+      // with token p's, and the next tokens' arithmetic does not wait for them
+      int tt = 0;
+      for (; tt + SCAN_P <= cnt; tt += SCAN_P) {
+        float t[SCAN_P];
 #pragma unroll
-          for (int i = 0; i < R / 4; ++i) kk[i] = kn[i], qq[i] = qn[i];
-          a = an, vj = vn;
+        for (int u = 0; u < SCAN_P; ++u) t[u] = step(tt + u);
+        if (OUT) {
+          const bool hi2 = part & 2, hi1 = part & 1;
+          const float s0 = (hi2 ? t[2] : t[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? t[0] : t[2], 2);
+          const float s1 = (hi2 ? t[3] : t[1]) + __shfl_xor_sync(0xffffffffu, hi2 ? t[1] : t[3], 2);
+          const float total = (hi1 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, hi1 ? s0 : s1, 1);
+          if (col < p.V) out[(size_t)(tt + part) * p.ld_o] = total;
+        }
+      }
+      for (; tt < cnt; ++tt) {
+        float total = step(tt);
+        if (OUT) {
+          total += __shfl_xor_sync(0xffffffffu, total, 2);
+          total += __shfl_xor_sync(0xffffffffu, total, 1);
+          if (part == 0 && col < p.V) out[(size_t)tt * p.ld_o] = total;
         }
       }
     }
     __syncthreads();
   }
+  pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
   if (helper) {
     cp_async_wait_group<0>();
-  } else if (p.write) {
+  } else if (MODE == SCAN_CLOSE || (p.write && seg == last)) {
+    float* to = MODE == SCAN_CLOSE ? kept + (seg + 1) * per_segment : st;
 #pragma unroll
     for (int i = 0; i < R; ++i) {
       const int n = part * R + i;
-      if (n < p.N && col < p.V) st[(size_t)n * p.V + col] = S[i];
+      if (n < p.N && col < p.V) to[(size_t)n * p.V + col] = i % 2 == 0 ? low_of(S[i / 2]) : high_of(S[i / 2]);
     }
+    if (MODE == SCAN_CLOSE && blockIdx.x == 0 && tid == 0) decays[(size_t)(seg + 1) * p.H] = decayed;
   }
 }
 
@@ -367,13 +432,21 @@ __global__ void __launch_bounds__(kThreads) gated_norm_kernel(T* __restrict__ ou
   }
 }
 
-template <int R>
-int launch_scan(const ScanParams& p, int requests, int vs, cudaStream_t stream) {
+template <int R, int MODE>
+int launch_scan_as(const ScanParams& p, int requests, int vs, cudaStream_t stream) {
   const size_t smem = (size_t)3 * SCAN_CT * (2 * SCAN_P * (R + 4) + vs + 4) * sizeof(float);
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(decay_scan_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid((p.V + vs - 1) / vs, p.H, requests);
-  return (int)lab_launch(decay_scan_kernel<R>, grid, dim3(2 * SCAN_P * vs), smem, stream, p);
+    cudaFuncSetAttribute(decay_scan_kernel<R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
+  dim3 grid((p.V + vs - 1) / vs, p.H, requests * segments);
+  return (int)lab_launch(decay_scan_kernel<R, MODE>, grid, dim3(2 * SCAN_P * vs), smem, stream, p);
+}
+
+template <int R>
+int launch_scan(const ScanParams& p, int requests, int vs, cudaStream_t stream) {
+  if (p.segments <= 1) return launch_scan_as<R, SCAN_WHOLE>(p, requests, vs, stream);
+  const int e = launch_scan_as<R, SCAN_CLOSE>(p, requests, vs, stream);
+  return e != 0 ? e : launch_scan_as<R, SCAN_OUTPUT>(p, requests, vs, stream);
 }
 
 }  // namespace
@@ -381,18 +454,23 @@ int launch_scan(const ScanParams& p, int requests, int vs, cudaStream_t stream) 
 // Largest key size the recurrence kernel is built for.
 LAB_EXPORT int lab_decay_scan_max_keys() { return SCAN_P * 64; }
 
-// vs: columns of the state a CTA takes (8, 16 or 32).
+// vs: columns of the state a CTA takes (8, 16 or 32).  segments > 1: every request's rows are cut into at most that many;
+// `states` [requests, segments, H, N, V] and `decays` [requests, segments, H] are scratch.
 LAB_EXPORT int lab_decay_scan(float* out, int ld_o, const float* q, const float* k, int ld_qk, const float* v, int ld_v,
                               const float* a_tok, const float* s_tok, int ld_a, const float* a_head, float* state,
                               const int* q_start, const int* state_slot, int requests, int n_slots, int H, int G, int N,
-                              int V, int act, int write, int vs, cudaStream_t stream) {
+                              int V, int act, int write, int vs, int segments, float* states, float* decays,
+                              cudaStream_t stream) {
   if (requests <= 0) return 0;
+  if (segments > 1 && (states == nullptr || decays == nullptr || (long long)requests * segments > 65535))
+    return (int)cudaErrorInvalidValue;
   if (H <= 0 || G <= 0 || H % G || N <= 0 || V <= 0 || (vs != 8 && vs != 16 && vs != 32)) return (int)cudaErrorInvalidValue;
   if (a_tok == nullptr && a_head == nullptr) return (int)cudaErrorInvalidValue;
   ScanParams p;
   p.out = out; p.ld_o = ld_o; p.q = q; p.k = k; p.ld_qk = ld_qk; p.v = v; p.ld_v = ld_v; p.a_tok = a_tok;
   p.s_tok = s_tok; p.ld_a = ld_a; p.a_head = a_head; p.state = state; p.q_start = q_start; p.state_slot = state_slot;
   p.n_slots = n_slots; p.H = H; p.G = G; p.N = N; p.V = V; p.act = act; p.write = write;
+  p.segments = segments; p.states = states; p.decays = decays;
   // 16-byte copies: every row of q, k and v, and every head's and slice's start in it, on a 16-byte boundary
   p.vec = N % 4 == 0 && V % 4 == 0 && ld_qk % 4 == 0 && ld_v % 4 == 0 &&
           ((((uintptr_t)q) | ((uintptr_t)k) | ((uintptr_t)v)) & 15) == 0;

@@ -52,17 +52,18 @@ __global__ void __launch_bounds__(kThreads) memory_gates_kernel(float* __restric
   }
 }
 
-// One warp per (request, head) walks the request's rows 32 at a time: every lane loads one row's gates, all lanes
-// follow the chain m <- max(f + m, i) through the 32 rows (the same operations in the same order as a walk row
-// by row, so a row's m does not depend on how the sequence was cut), each lane keeps the m before and after its
-// own row and forms that row's two exponentials.
+// One warp per (request, head) takes the request's rows 256 at a time, eight neighbouring ones a lane.  Rows f, i take m
+// to max(f + m, i), and so do several rows together, with the sum of their f and an i of their own: every lane forms
+// that of its rows, a scan over the lanes gives each lane the m before its rows, and it walks them, forming each row's
+// two exponentials.  What bounds it is latency (a chain through every row, 32 rows a step, took 51 us for 2,048 rows),
+// so the next 256 rows' gates are loaded before this step's arithmetic.  Any m near the running maximum gives the same
+// result: both exponentials and the floor of the denominator go by the m that is kept.
 // decay[t, h] and scale[t, h] leave as rows of [tokens, 2, H] (over the gates).
 __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __restrict__ gates, float* __restrict__ m_out,
                                                                     float* __restrict__ m_state,
                                                                     const int* __restrict__ q_start,
                                                                     const int* __restrict__ state_slot, int requests,
                                                                     int n_slots, int H, int write) {
-  __shared__ __align__(16) float chunk_gates[kThreads / 32][64];      // per warp: 32 forget gates, then 32 input gates
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -75,56 +76,47 @@ __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __res
     if (lane == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
     return;
   }
-  // Lanes beyond the request's rows hold (f, i) = (0, -inf), which leaves m as it is: every chunk walks all 32
-  // lanes, so the chain unrolls and its shuffles are issued ahead of it.  Rows come in groups of kAhead chunks:
-  // the next group's gates are loaded before the current group's chains, which hides the loads' latency.
-  constexpr int kAhead = 4;
-  float* mine = chunk_gates[warp];
+  // Rows beyond the request's hold (f, i) = (0, -inf), which leaves m as it is.
+  constexpr int kRows = 8;
   float m = m_state[(size_t)slot * H + h];
-  float gi[kAhead], gf[kAhead], gi_next[kAhead], gf_next[kAhead];
-  auto load = [&](int first, float (&to_i)[kAhead], float (&to_f)[kAhead]) {
+  float gi[kRows], gf[kRows], gi_next[kRows], gf_next[kRows];
+  auto load = [&](int first, float (&to_i)[kRows], float (&to_f)[kRows]) {
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) {
-      const int row = first + k * 32 + lane;
+    for (int k = 0; k < kRows; ++k) {
+      const int row = first + lane * kRows + k;
       const bool in = row < n;
       to_i[k] = in ? gates[(size_t)(t0 + row) * 2 * H + h] : -INFINITY;
       to_f[k] = in ? gates[(size_t)(t0 + row) * 2 * H + H + h] : 0.f;
     }
   };
   load(0, gi, gf);
-  for (int c = 0; c < n; c += kAhead * 32) {
-    load(c + kAhead * 32, gi_next, gf_next);
+  for (int c = 0; c < n; c += 32 * kRows) {
+    load(c + 32 * kRows, gi_next, gf_next);
+    float f_all = 0.f, i_all = -INFINITY;      // the lane's rows together, then the rows of all lanes up to it
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) {
-      // the chunk's gates go through shared memory: every lane reads all 32 pairs, four at a time, ahead of the
-      // chain (shuffles would put their latency on it)
-      __syncwarp();
-      mine[lane] = gf[k];
-      mine[32 + lane] = gi[k];
-      __syncwarp();
-      float carried_mine = 0.f, m_mine = 0.f;
+    for (int k = 0; k < kRows; ++k) f_all += gf[k], i_all = fmaxf(i_all + gf[k], gi[k]);
 #pragma unroll
-      for (int j4 = 0; j4 < 8; ++j4) {
-        const float4 f4 = reinterpret_cast<const float4*>(mine)[j4];
-        const float4 i4 = reinterpret_cast<const float4*>(mine + 32)[j4];
-        const float fs[4] = {f4.x, f4.y, f4.z, f4.w}, is[4] = {i4.x, i4.y, i4.z, i4.w};
+    for (int o = 1; o < 32; o <<= 1) {
+      const float f_left = __shfl_up_sync(0xffffffffu, f_all, o), i_left = __shfl_up_sync(0xffffffffu, i_all, o);
+      if (lane >= o) i_all = fmaxf(i_left + f_all, i_all), f_all += f_left;
+    }
+    const float f_before = __shfl_up_sync(0xffffffffu, f_all, 1), i_before = __shfl_up_sync(0xffffffffu, i_all, 1);
+    float mine = lane == 0 ? m : fmaxf(f_before + m, i_before);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float carried = fs[e] + m;
-          m = fmaxf(carried, is[e]);
-          if (4 * j4 + e == lane) carried_mine = carried, m_mine = m;
-        }
-      }
-      const int row = c + k * 32 + lane;
+    for (int k = 0; k < kRows; ++k) {
+      const int row = c + lane * kRows + k;
+      const float carried = gf[k] + mine;
+      mine = fmaxf(carried, gi[k]);
       if (row < n) {
         float* g = gates + (size_t)(t0 + row) * 2 * H;
-        g[h] = expf(carried_mine - m_mine);       // decay of the state
-        g[H + h] = expf(gi[k] - m_mine);          // scale of the new key
-        m_out[(size_t)(t0 + row) * H + h] = m_mine;
+        g[h] = expf(carried - mine);           // decay of the state
+        g[H + h] = expf(gi[k] - mine);         // scale of the new key
+        m_out[(size_t)(t0 + row) * H + h] = mine;
       }
     }
+    m = __shfl_sync(0xffffffffu, mine, 31);
 #pragma unroll
-    for (int k = 0; k < kAhead; ++k) gi[k] = gi_next[k], gf[k] = gf_next[k];
+    for (int k = 0; k < kRows; ++k) gi[k] = gi_next[k], gf[k] = gf_next[k];
   }
   if (write && lane == 0) m_state[(size_t)slot * H + h] = m;
 }

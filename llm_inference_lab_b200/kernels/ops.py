@@ -1479,6 +1479,18 @@ def decay_scan_supported(keys: int) -> bool:
     return 1 <= keys <= 256
 
 
+def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) -> int:
+    """Into how many segments `decay_scan` cuts a request's rows, `ctas` CTAs walking the step in one piece; a
+    multiprocessor holds four or five of up to 64 key channels, three of more.  Segments cost most of the walk's work
+    once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it: 84 CTAs and 1,000
+    tokens 283 us in one piece, 193 in 4, 180 in 8; 42 CTAs and 2,048 tokens 487, 217 in 8, 219 in 16; 42 and 300 tokens
+    123, 72 in 8; 168 CTAs and 500 tokens 171, 181 in 2, 168 in 4; 336 and 250 tokens 129, 160 in 2."""
+    if ctas >= sm_count():
+        return 1
+    room = (9 * sm_count() // 2 if keys <= 64 else 3 * sm_count()) // max(1, ctas)
+    return max(1, min(longest // 32, room, 16, 65535 // max(1, requests)))
+
+
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, ctx, heads: int, groups: int,
                keys: int, vdim: int, a_head: torch.Tensor | None = None, a_tok: torch.Tensor | None = None,
                s_tok: torch.Tensor | None = None, silu: bool = False, write: bool = True) -> torch.Tensor:
@@ -1514,10 +1526,16 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     else:
         vs = 32 if pairs * -(-vdim // 32) >= sm_count() else (16 if pairs * -(-vdim // 16) >= sm_count() else 8)
     vs = min(vs, max(8, 1 << (vdim - 1).bit_length()))
+    segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
+    states = decays = None
+    if segments > 1:
+        states = torch.empty((ctx.n_requests, segments, heads, keys, vdim), dtype=torch.float32, device=v.device)
+        decays = torch.empty((ctx.n_requests, segments, heads), dtype=torch.float32, device=v.device)
     _check(lib("linear_state").lab_decay_scan(
         _ptr(out), out.stride(0), _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(a_tok), _ptr(s_tok), ld_a,
         _ptr(a_head), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), ctx.n_requests, state.shape[0], heads, groups,
-        keys, vdim, int(silu), int(write), vs, _stream()), "decay_scan")
+        keys, vdim, int(silu), int(write), vs, segments, _ptr(states), _ptr(decays), _stream()), "decay_scan",
+        2 if segments > 1 else 1)
     return out
 
 

@@ -57,3 +57,62 @@ def test_selective_scan_segments(channels, N, segments, monkeypatch):
         at += length
     # 32-bit roundings, a few units of 2^-24 a token where the state's memory is long (150 tokens) and sums of up to 256
     assert off(out, want) < 2e-5 and off(state, W) < 2e-5
+
+
+@pytest.mark.parametrize("segments", [1, 2, 3, 5, 9])
+@pytest.mark.parametrize("heads,groups,keys,vdim,per_token,silu", [(4, 2, 64, 68, True, False), (3, 3, 16, 20, False, True),
+                                                                   (2, 1, 50, 33, True, False), (2, 2, 128, 128, True, False),
+                                                                   (1, 1, 200, 8, False, False)])
+def test_decay_scan_segments(heads, groups, keys, vdim, per_token, silu, segments, monkeypatch):
+    monkeypatch.setattr(ops(), "decay_scan_segments", lambda *a: segments)
+    g = torch.Generator(device=DEV).manual_seed(keys + vdim)
+    rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
+    T = sum(Q_LENS)
+    qk, v = rand(T, 2 * groups * keys), rand(T, heads * vdim)
+    gates = torch.stack([torch.exp(-torch.rand(T, heads, device=DEV, generator=g) * 0.2), rand(T, heads)], dim=1)
+    fixed = 1.0 - torch.rand(heads, device=DEV, generator=g) * 0.1
+    state = rand(6, heads, keys, vdim)
+    start, ctx = state.clone(), context(Q_LENS, SLOTS)
+    how = dict(a_tok=gates[:, 0], s_tok=gates[:, 1]) if per_token else dict(a_head=fixed)
+    for write in (False, True):
+        out = ops().decay_scan(qk[:, : groups * keys], qk[:, groups * keys:], v, state, ctx, heads, groups, keys, vdim, silu=silu,
+                               write=write, **how)
+        assert write or torch.equal(state, start)
+    ops().take_device_errors()
+    n = lambda t: t.double().cpu().numpy()  # noqa: E731
+    act = (lambda z: z / (1 + np.exp(-z))) if silu else (lambda z: z)
+    Q, K = (act(n(t)).reshape(T, groups, keys).repeat(heads // groups, axis=1) for t in (qk[:, : groups * keys], qk[:, groups * keys:]))
+    V, W = act(n(v)).reshape(T, heads, vdim), n(start)
+    a, s = (n(gates[:, 0]), n(gates[:, 1])) if per_token else (np.tile(n(fixed), (T, 1)), np.ones((T, heads)))
+    want, at = np.zeros((T, heads, vdim)), 0
+    for length, slot in zip(Q_LENS, SLOTS):
+        for t in range(at, at + length) if slot >= 0 else ():
+            W[slot] = a[t][:, None, None] * W[slot] + (s[t][:, None] * K[t])[:, :, None] * V[t][:, None, :]
+            want[t] = (W[slot] * Q[t][:, :, None]).sum(1)
+        at += length
+    live = T - Q_LENS[-1]      # (a row of padding leaves nothing)
+    # 32-bit roundings over a memory of ten tokens or so and sums of up to 200; SiLU's exponential is off by 2^-21
+    assert off(out[:live], want.reshape(T, -1)[:live]) < 2e-5 and off(state, W) < 2e-5
+
+
+@pytest.mark.parametrize("heads", [1, 5, 14])
+def test_running_maximum_of_any_length(heads):
+    g = torch.Generator(device=DEV).manual_seed(heads)
+    lens, slots = [1, 7, 8, 255, 256, 257, 700, 2], [3, 0, 7, 5, 1, 6, 2, -1]
+    T, ctx = sum(lens), context(lens, slots)
+    gates = torch.randn(T, 2, heads, device=DEV, generator=g) * 3
+    gates[:, 1] = -torch.nn.functional.softplus(gates[:, 1])
+    m_state = torch.randn(8, heads, device=DEV, generator=g)
+    log_i, log_f, M = (t.double().cpu().numpy() for t in (gates[:, 0], gates[:, 1], m_state))
+    m = ops().memory_stabilize(gates, m_state, ctx)
+    got, at = [t.double().cpu().numpy() for t in (m, gates[:, 0], gates[:, 1])], 0
+    for length, slot in zip(lens, slots):
+        for t in range(at, at + length) if slot >= 0 else ():
+            top = np.maximum(log_f[t] + M[slot], log_i[t])
+            # up to 700 roundings of sums of a few tens
+            assert np.abs(got[0][t] - top).max() < 1e-3
+            assert np.abs(got[1][t] - np.exp(log_f[t] + M[slot] - top)).max() < 1e-3
+            assert np.abs(got[2][t] - np.exp(log_i[t] - top)).max() < 1e-3
+            M[slot] = top
+        at += length
+    assert np.abs(m_state.double().cpu().numpy() - M).max() < 1e-3
