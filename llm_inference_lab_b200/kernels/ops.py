@@ -628,6 +628,27 @@ def _pick_prefill_tiles(T: int, n_out: int, K: int, allow_partial: bool) -> tupl
     return "tc", 128, 1
 
 
+def _pair_splits(T: int, n_out: int, K: int) -> int:
+    """K splits of a product whose consumer sums partial products, on pairs of SMs (tiles of 224 columns); 0: no such
+    split.  For long K (64 k-tiles and more a split) whose tiles fill less than the 74 pairs, while three fifths of them get
+    work: 7B down projection (3584 x 18944) at 136 tokens 41.6 us in 4 splits against 46.3 for split 128-wide tiles,
+    300 tokens 59.7 in 2 (68.0), 512 tokens 65.3 in 2 (78.4), 700 tokens 83.6 in 1 (109.3); with 70 k-tiles a split and
+    56 tiles (1.5B, 1,024 tokens) 35.5 against 36.3."""
+    tiles, k_tiles, pairs = -(-T // 256) * (-(-n_out // 224)), -(-K // 64), sm_count() // 2
+    splits = min(pairs // max(1, tiles), k_tiles // 64)
+    return splits if splits >= 1 and 5 * tiles * splits >= 3 * pairs else 0
+
+
+def _gated_on_pairs(T: int, inter: int) -> bool:
+    """Whether a gated product runs on pairs of SMs (256 tokens x 128 features per tile, gate rows in one CTA and up rows
+    in the other) or on tiles of 128 tokens.  Pairs win once their tiles fill most of the 74 pairs, 6 to 12 % at the
+    0.5B, 1.5B and 7B layer sizes (2,048 tokens: 31.7 against 33.7, 76 against 85, 349 against 385 us), unless the
+    smaller tiles take fewer rounds: 76 pair tiles are two rounds, 114 small ones are one (0.5B, 300 tokens: 15.7 against
+    12.3 us; 7B, 300 tokens, four rounds against three: 93 against 86)."""
+    pairs, tiles = -(-T // 256) * (-(-inter // 128)), -(-T // 128) * (-(-inter // 128))
+    return pairs >= 64 and -(-pairs // (sm_count() // 2)) <= -(-tiles // sm_count())
+
+
 def _tc_operands(x, w) -> bool:
     """Whether TMA can describe the operands: rows of 16-byte multiples that start on 16-byte
     boundaries.  Widths that are no multiple of 8 go to the plain kernel instead."""
@@ -664,12 +685,19 @@ def linear(x, w, bias=None, out_f32=False, allow_partial=False, out=None, act=No
         return gemm_plain(x, w, bias, out_f32=out_f32, out=out, gelu=gelu)
     T = x.shape[0]
     if T > 128:
-        kind, bn, splits = _pick_prefill_tiles(T, w.shape[0], x.shape[1],
-                                               allow_partial and bias is None and out is None)
-        if kind == "pair":
+        partial = allow_partial and bias is None and out is None
+        pair_splits = _pair_splits(T, w.shape[0], x.shape[1]) if partial else 0
+        if pair_splits > 1:
+            return gemm_tc2(x, w, None, splits=pair_splits)
+        kind, bn, splits = _pick_prefill_tiles(T, w.shape[0], x.shape[1], partial)
+        if kind == "pair" or pair_splits:
             return gemm_tc2(x, w, bias, out_f32=out_f32, out=out, gelu=gelu)
         if splits > 1:
-            return gemm_tc(x, w, None, swap=False, bn=bn, splits=splits)
+            # features on the M side: the partial products leave in fewer, longer runs (0.5B down projection at 300
+            # tokens 13.9 against 15.9 us, at 512 14.5 against 16.3; 1.5B at 300 tokens 18.4 against 20.3)
+            return gemm_tc(x, w, None, swap=True, bn=128, splits=splits)
+        if kind == "tc" and bn == 128 and 2 * (-(-T // 128)) * (-(-w.shape[0] // 128)) <= sm_count():
+            bn = 64      # too few tiles for half of the SMs: twice as many (896 x 896 at 300 tokens 6.3 against 7.4 us)
         return gemm_tc(x, w, bias, out_f32=out_f32, swap=False, bn=bn, out=out, gelu=gelu)
     splits = _pick_splits(T, w.shape[0], x.shape[1]) if allow_partial and out is None else 1
     if splits > 1:
@@ -683,11 +711,7 @@ def linear_gated(x, w_gate_up, limit: float = 0.0, act: str = "silu"):
     g' * sigmoid(1.702 g') * (u' + 1)."""
     if x.dtype == torch.float32 or _force_plain or not _tc_operands(x, w_gate_up):
         return gemm_plain(x, w_gate_up, None, gated=True, gate_limit=limit, gate_act=act)
-    # Pairs of SMs (256 tokens x 128 features per tile, gate rows in one CTA and up rows in the other)
-    # once their tiles fill most of the 74 pairs: measured 6 to 12 % faster from there on at the 0.5B,
-    # 1.5B and 7B layer sizes (2,048 tokens: 31.7 against 33.7, 76 against 85, 349 against 385 us).
-    T, inter = x.shape[0], w_gate_up.shape[0] // 2
-    if -(-T // 256) * (-(-inter // 128)) >= 64:
+    if _gated_on_pairs(x.shape[0], w_gate_up.shape[0] // 2):
         return gemm_tc2(x, w_gate_up, None, gated=True, gate_limit=limit, gate_act=act)
     return gemm_tc(x, w_gate_up, None, gated=True, gate_limit=limit, gate_act=act)
 

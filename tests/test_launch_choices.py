@@ -69,3 +69,14 @@ def test_delta_walk_shapes_are_what_the_kernel_takes():
         assert cols == 1 or keys <= 128
     assert ops.delta_walk_shape(14, 64, 64, 2048) == (16, 1) and ops.delta_walk_shape(56, 64, 64, 512) == (32, 1)
     assert ops.delta_walk_shape(128, 128, 128, 512) == (64, 2) and ops.delta_walk_shape(14, 64, 64, 1) == (32, 2)
+
+
+def test_pair_splits_and_gated_tiles_cover_the_cases_they_were_measured_on():
+    assert [ops._pair_splits(T, 3584, 18944) for T in (136, 300, 512, 700, 1024)] == [4, 2, 2, 1, 1]
+    assert ops._pair_splits(1024, 1536, 8960) == 2 and ops._pair_splits(300, 1536, 8960) == 0
+    assert ops._pair_splits(2048, 896, 4864) == 0 and ops._pair_splits(300, 896, 896) == 0
+    for T, n_out, K in itertools.product((129, 256, 1000, 2048, 8192), (8, 896, 1152, 9728), (64, 896, 4864, 18944)):
+        s = ops._pair_splits(T, n_out, K)
+        assert s == 0 or -(-K // 64) // s >= 64 and -(-T // 256) * -(-n_out // 224) * s <= ops.sm_count() // 2
+    assert ops._gated_on_pairs(2048, 4864) and ops._gated_on_pairs(300, 8960) and ops._gated_on_pairs(411, 4864)
+    assert not ops._gated_on_pairs(300, 4864) and not ops._gated_on_pairs(300, 18944) and not ops._gated_on_pairs(130, 4864)
