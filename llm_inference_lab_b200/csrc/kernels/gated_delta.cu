@@ -24,7 +24,14 @@
 //
 // which is the recurrence with its sums regrouped: eight independent products with the old state, a substitution of
 // four steps on numbers, one update, instead of four dependent rounds.  Products of decays are formed as products,
-// never as quotients, so strong decays lose nothing.  Blocks lie on multiples of four rows of the packed batch and end
+// never as quotients, so strong decays lose nothing.
+//
+// A long portion may be cut into segments of rows that are walked side by side.  What a segment makes of its opening
+// state S is M S + L with a matrix M [key channel, key channel] of its own and the closing state L that it has from
+// zeros, so a first launch walks every segment but the last for L (the first one from the request's state) and for M,
+// the closing state of the identity with no values; delta_fold forms the opening states one after the other, and the
+// walk takes every segment again from its own.  Everything stays 32-bit; the errors against 64-bit are those of the
+// walk in one piece.  Blocks lie on multiples of four rows of the packed batch and end
 // at a request's border; a row that is missing from a block has rate 0 and decay 1.
 //
 // T says how weights are stored and how the last result is rounded.
@@ -230,7 +237,21 @@ struct WalkParams {
   const float* proj;
   float* kept;           // [slots, keep, channels]
   int ld, keep, channels;
+  int segments;          // a request's rows are cut into at most that many segments of whole chunks
+  float* states;         // [requests, segments, H, D, V]: 0, a copy of the request's state; i, the closing state of segment
+                         // i - 1 (from zeros, of segment 0 from the request's state), then i's opening state
+  float* moves;          // [requests, segments, H, D, D]: what segment i - 1 makes of its opening state (from i = 2 on)
 };
+// What a launch does: everything in one piece, the segments' closing states and moves, or the outputs.
+enum { WALK_WHOLE, WALK_CLOSE, WALK_OUTPUT };
+
+// The rows of segment `seg` of a request's rows [t0, t1), on chunks of the packed batch, and the number of its last one.
+__device__ __forceinline__ int segment_rows(int& t0, int& t1, int seg, int segments) {
+  const int base = t0 / CT * CT, n = t1 - base, len = ((n + segments - 1) / segments + CT - 1) / CT * CT;
+  t0 = max(t0, base + seg * len);
+  t1 = min(t1, base + (seg + 1) * len);
+  return (n - 1) / len;
+}
 
 // grid (slices of V, heads, requests).  Walkers (the first PARTS * Vs / NC threads): thread (j, part) keeps rows
 // part * R .. part * R + R - 1 of NC neighbouring columns of the state in registers, as pairs of rows for packed
@@ -239,20 +260,25 @@ struct WalkParams {
 // by two levels of shuffles, the queries' by an exchange that leaves thread p the sums of row p, whose output it
 // forms and writes.  Helpers copy chunks of 16 rows two ahead (three buffers, one barrier of the CTA a chunk) and form
 // the coefficients of the next chunk's blocks.
-template <int R, int NC>
+template <int R, int NC, int MODE>
 __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
   extern __shared__ __align__(16) float smem[];
   constexpr int RS = R + 4;                      // floats between two threads' shares of a row's keys
   constexpr int NP = key_floats(R), REC = record_floats(R);
-  pdl_trigger();
-  const int walkers = PARTS * Vs / NC;
-  const int h = blockIdx.y, r = blockIdx.z, g = h / (p.H / p.G);
+  constexpr bool OUT = MODE != WALK_CLOSE;
+  const int walkers = PARTS * Vs / NC, segments = MODE == WALK_WHOLE ? 1 : MODE == WALK_CLOSE ? p.segments - 1 : p.segments;
+  const int h = blockIdx.y, r = blockIdx.z / segments, seg = blockIdx.z % segments, g = h / (p.H / p.G);
   const bool helper = (int)threadIdx.x >= walkers;
   const int tid = helper ? threadIdx.x - walkers : threadIdx.x;      // index within the walkers or the helpers
-  const int t0 = p.q_start[r], t1 = p.q_start[r + 1];
+  const int all0 = p.q_start[r], all1 = p.q_start[r + 1];            // the request's rows, and this CTA's
+  int t0 = all0, t1 = all1, last = 0;
+  if (MODE != WALK_WHOLE && all1 > all0) last = segment_rows(t0, t1, seg, p.segments);
   const int slot = p.state_slot[r];
-  if (t1 <= t0 || slot == -1) {      // nothing to do, or rows of padding (their output is never read)
-    pdl_wait();
+  // slices beyond the values' walk the identity; of the first segment, whose state is known, and the last nobody asks
+  const int slices = (p.V + Vs - 1) / Vs;
+  const bool move = MODE == WALK_CLOSE && (int)blockIdx.x >= slices;
+  if (t1 <= t0 || slot == -1 || (MODE == WALK_CLOSE && (seg >= last || (move && seg == 0)))) {
+    pdl_wait();      // nothing to do, or rows of padding (their output is never read)
     return;
   }
   if (slot < 0 || slot >= p.n_slots) {
@@ -267,7 +293,11 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
 
   const int base_row = t0 / BLK * BLK;           // blocks lie on multiples of BLK rows of the batch
   const int n_chunks = (t1 - base_row + CT - 1) / CT;
-  const int col0 = blockIdx.x * Vs, v_cols = min(Vs, p.V - col0);
+  const int V = move ? p.D : p.V, col0 = (blockIdx.x - (move ? slices : 0)) * Vs, v_cols = move ? 0 : min(Vs, V - col0);
+  if (move) {      // no values
+    for (int i = threadIdx.x; i < 3 * CT * Vs; i += blockDim.x) smem[i / (CT * Vs) * buf_floats + off_v + i % (CT * Vs)] = 0.f;
+    __syncthreads();
+  }
   auto buffer = [&](int chunk) { return smem + (chunk % 3) * buf_floats; };
 
   // ---- helpers' pieces ----
@@ -326,7 +356,19 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
   const int j0 = tid / PARTS * NC, part = tid % PARTS;      // a walker's first column in the slice, its rows
   pair_t S[NC][R / 2];
   float* st = p.state + ((size_t)slot * p.H + h) * p.D * p.V + col0 + j0;
-  auto in_state = [&](int n, int c) { return n < p.D && col0 + j0 + c < p.V; };
+  const size_t per_segment = (size_t)p.H * p.D * V;      // where the segments' states (or moves) of this head lie
+  float* kept_states = MODE == WALK_WHOLE ? nullptr : (move ? p.moves : p.states) + (size_t)r * p.segments * per_segment +
+                                                          (size_t)h * p.D * V + col0 + j0;
+  auto in_state = [&](int n, int c) { return n < p.D && col0 + j0 + c < V; };
+  auto opening = [&](int n, int c) {
+    if (!in_state(n, c)) return 0.f;
+    if (move) return n == col0 + j0 + c ? 1.f : 0.f;
+    const size_t at = (size_t)n * V + c;
+    if (MODE == WALK_WHOLE || (MODE == WALK_OUTPUT && last == 0)) return st[at];
+    if (MODE == WALK_OUTPUT) return kept_states[seg * per_segment + at];
+    // (the last segment's CTAs of the walk write the request's state while others still open theirs)
+    return seg == 0 ? kept_states[at] = st[at] : 0.f;
+  };
   if (helper) {
     issue(0);
     cp_async_commit_group();
@@ -340,7 +382,7 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
       const int n = part * R + 2 * i;
 #pragma unroll
       for (int c = 0; c < NC; ++c)
-        S[c][i] = pair_of(in_state(n, c) ? st[(size_t)n * p.V + c] : 0.f, in_state(n + 1, c) ? st[(size_t)(n + 1) * p.V + c] : 0.f);
+        S[c][i] = pair_of(opening(n, c), opening(n + 1, c));
     }
   }
   __syncthreads();
@@ -352,16 +394,16 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
       if (ch + 1 < n_chunks) {
         cp_async_wait_group<1>();                // all but the copies just started: chunk ch + 1 is here
         coefficients(ch + 1);
-      } else if (p.keep > 0 && p.write) {
+      } else if (OUT && seg == last && p.keep > 0 && p.write) {
         // meanwhile: the request's last inputs replace the kept ones, channels shared out over the request's CTAs.  A
         // thread walks the kept rows of a channel oldest first: what it overwrites it has already moved.
         float* kept = p.kept + (size_t)slot * p.keep * p.channels;
-        const int n = t1 - t0, cta = blockIdx.y * gridDim.x + blockIdx.x, ctas = gridDim.x * gridDim.y;
+        const int n = all1 - all0, cta = blockIdx.y * gridDim.x + blockIdx.x, ctas = gridDim.x * gridDim.y;
         for (int c = cta * HELPERS + tid; c < p.channels; c += ctas * HELPERS)
           for (int i = 0; i < p.keep; ++i) {
             const int s = n - p.keep + i;        // the step's row that becomes kept row i
             kept[(size_t)i * p.channels + c] =
-                s >= 0 ? p.proj[(size_t)(t0 + s) * p.ld + c] : kept[(size_t)(i + n) * p.channels + c];
+                s >= 0 ? p.proj[(size_t)(all0 + s) * p.ld + c] : kept[(size_t)(i + n) * p.channels + c];
           }
       }
     } else {
@@ -384,13 +426,18 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
 #pragma unroll
           for (int i = 0; i < BLK; ++i) {
             const ulonglong2 k4 = reinterpret_cast<const ulonglong2*>(tok + i * REC + part * RS)[x];
-            const ulonglong2 q4 = reinterpret_cast<const ulonglong2*>(tok + i * REC + NP + part * RS)[x];
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
               kacc[i][c] = pair_fma(k4.x, S[c][2 * x], kacc[i][c]);
-              qacc[i][c] = pair_fma(q4.x, S[c][2 * x], qacc[i][c]);
               kacc[i][c] = pair_fma(k4.y, S[c][2 * x + 1], kacc[i][c]);
-              qacc[i][c] = pair_fma(q4.y, S[c][2 * x + 1], qacc[i][c]);
+            }
+            if (OUT) {
+              const ulonglong2 q4 = reinterpret_cast<const ulonglong2*>(tok + i * REC + NP + part * RS)[x];
+#pragma unroll
+              for (int c = 0; c < NC; ++c) {
+                qacc[i][c] = pair_fma(q4.x, S[c][2 * x], qacc[i][c]);
+                qacc[i][c] = pair_fma(q4.y, S[c][2 * x + 1], qacc[i][c]);
+              }
             }
             if (R > 16) asm volatile("" ::: "memory");      // loads stay near their use: registers
           }
@@ -408,10 +455,13 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
 #pragma unroll
           for (int i = 0; i < BLK; ++i) ks[i] += __shfl_xor_sync(0xffffffffu, ks[i], 2);
           // thread p of the column's four is left with row p's sum of the queries
-          const bool hi2 = part & 2, hi1 = part & 1;
-          const float a0 = (hi2 ? qs[2] : qs[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? qs[0] : qs[2], 2);
-          const float a1 = (hi2 ? qs[3] : qs[1]) + __shfl_xor_sync(0xffffffffu, hi2 ? qs[1] : qs[3], 2);
-          const float qp = (hi1 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi1 ? a0 : a1, 1);
+          float qp = 0.f;
+          if (OUT) {
+            const bool hi2 = part & 2, hi1 = part & 1;
+            const float a0 = (hi2 ? qs[2] : qs[0]) + __shfl_xor_sync(0xffffffffu, hi2 ? qs[0] : qs[2], 2);
+            const float a1 = (hi2 ? qs[3] : qs[1]) + __shfl_xor_sync(0xffffffffu, hi2 ? qs[1] : qs[3], 2);
+            qp = (hi1 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi1 ? a0 : a1, 1);
+          }
           const float* vc = base + off_v + blk * BLK * Vs + j0 + c;
           u[0][c] = fmaf(rate.x, vc[0], -rg.x * ks[0]);
           u[1][c] = fmaf(-s1.x, u[0][c], fmaf(rate.y, vc[Vs], -rg.y * ks[1]));
@@ -421,7 +471,7 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
           o[c] = fmaf(g_part, qp, fmaf(out_w.x, u[0][c], fmaf(out_w.y, u[1][c], fmaf(out_w.z, u[2][c], out_w.w * u[3][c]))));
         }
         const int row = rows + part;
-        if (row >= t0 && row < t1) {
+        if (OUT && row >= t0 && row < t1) {
           float* dst = p.out + ((size_t)row * p.H + h) * p.V + col0 + j0;
 #pragma unroll
           for (int c = 0; c < NC; ++c)
@@ -453,9 +503,11 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
     }
     __syncthreads();
   }
+  pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
   if (helper) {
     cp_async_wait_group<0>();
-  } else if (p.write) {
+  } else if (MODE == WALK_CLOSE || (p.write && seg == last)) {
+    float* to = MODE == WALK_CLOSE ? kept_states + (seg + 1) * per_segment : st;
 #pragma unroll
     for (int i = 0; i < R / 2; ++i) {
       const int n = part * R + 2 * i;
@@ -463,11 +515,78 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
       for (int c = 0; c < NC; ++c) {
         float lo, hi;
         pair_split(S[c][i], lo, hi);
-        if (in_state(n, c)) st[(size_t)n * p.V + c] = lo;
-        if (in_state(n + 1, c)) st[(size_t)(n + 1) * p.V + c] = hi;
+        if (in_state(n, c)) to[(size_t)n * V + c] = lo;
+        if (in_state(n + 1, c)) to[(size_t)(n + 1) * V + c] = hi;
       }
     }
   }
+}
+
+// ---- the segments' opening states ---------------------------------------------------------------
+// grid (slices of FOLD_V columns, heads, requests): S_i <- M_i S_{i-1} + L_i for i = 2 .. the request's last segment, in
+// place of L_i.  The columns of S stay in shared memory, M passes through it in panels of FOLD_ROWS rows, the next panel
+// on its way in registers; a thread forms four entries of a column.  A chain of small products, bound by latency.
+constexpr int FOLD_V = 16, FOLD_ROWS = 64;
+template <int PRE>      // entries of a panel a thread brings: FOLD_ROWS D / 256, rounded up
+__global__ void __launch_bounds__(256) delta_fold_kernel(WalkParams p) {
+  extern __shared__ __align__(16) float smem[];
+  const int D = p.D, h = blockIdx.y, r = blockIdx.z, tid = threadIdx.x;
+  pdl_wait();
+  int t0 = p.q_start[r], t1 = p.q_start[r + 1];
+  const int slot = p.state_slot[r];
+  if (t1 <= t0 || slot < 0 || slot >= p.n_slots) return;
+  const int last = segment_rows(t0, t1, 0, p.segments);
+  if (last < 2) return;
+  float* now = smem;                            // [D][FOLD_V]
+  float* next = smem + D * FOLD_V;
+  float* panel = next + D * FOLD_V;             // [FOLD_ROWS][D + 4]
+  const int col = blockIdx.x * FOLD_V + tid % FOLD_V, lane_row = tid / FOLD_V, ld = D + 4;
+  const size_t per_state = (size_t)p.H * D * p.V, per_move = (size_t)p.H * D * D;
+  float* states = p.states + (size_t)r * p.segments * per_state + (size_t)h * D * p.V;
+  const float* moves = p.moves + (size_t)r * p.segments * per_move + (size_t)h * D * D;
+  for (int n = lane_row; n < D; n += 256 / FOLD_V) now[n * FOLD_V + tid % FOLD_V] = col < p.V ? states[per_state + (size_t)n * p.V + col] : 0.f;
+  const int panels = (D + FOLD_ROWS - 1) / FOLD_ROWS, steps = (last - 1) * panels;
+  float pre[PRE];
+  auto load = [&](int step) {
+    const float* from = moves + (size_t)(2 + step / panels) * per_move + (size_t)(step % panels) * FOLD_ROWS * D;
+    const int count = min(FOLD_ROWS, D - step % panels * FOLD_ROWS) * D;
+#pragma unroll
+    for (int i = 0; i < PRE; ++i) pre[i] = tid + 256 * i < count ? from[tid + 256 * i] : 0.f;
+  };
+  load(0);
+  for (int step = 0; step < steps; ++step) {
+    const int seg = 2 + step / panels, row0 = step % panels * FOLD_ROWS;
+    __syncthreads();      // the panel before has been read, `now` is whole
+#pragma unroll
+    for (int i = 0; i < PRE; ++i)
+      if (tid + 256 * i < FOLD_ROWS * D) panel[(tid + 256 * i) / D * ld + (tid + 256 * i) % D] = pre[i];
+    __syncthreads();
+    if (step + 1 < steps) load(step + 1);
+    constexpr int ROWS = FOLD_ROWS / (256 / FOLD_V);      // rows a thread forms: lane_row + 16 i
+    float acc[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const int n = row0 + lane_row + 16 * i;
+      acc[i] = n < D && col < p.V ? states[(size_t)seg * per_state + (size_t)n * p.V + col] : 0.f;
+    }
+    for (int m = 0; m < D; ++m) {
+      const float v = now[m * FOLD_V + tid % FOLD_V];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) acc[i] = fmaf(panel[(lane_row + 16 * i) * ld + m], v, acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const int n = row0 + lane_row + 16 * i;
+      if (n >= D) continue;
+      next[n * FOLD_V + tid % FOLD_V] = acc[i];
+      if (col < p.V) states[(size_t)seg * per_state + (size_t)n * p.V + col] = acc[i];
+    }
+    if (step % panels == panels - 1) {
+      float* t = now;
+      now = next, next = t;
+    }
+  }
+  pdl_trigger();
 }
 
 // ---- norm and gate ------------------------------------------------------------------------------
@@ -518,14 +637,33 @@ void launch_prepare(const PrepareParams& p, dim3 grid, size_t smem, const void* 
   lab_launch(kernel, grid, dim3(kThreads), smem, stream, (const T*)taps_w, (const T*)a_log, (const T*)dt_bias, p);
 }
 
-template <int R, int NC>
-int launch_walk(const WalkParams& p, int requests, int vs, cudaStream_t stream) {
+template <int R, int NC, int MODE>
+int launch_walk_as(const WalkParams& p, int requests, int vs, cudaStream_t stream) {
   const size_t smem = (size_t)3 * (CT * (record_floats(R) + vs + 2) + (CT / BLK) * COEF) * sizeof(float);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
   if (smem > 48 * 1024)
-    cudaFuncSetAttribute(delta_walk_kernel<R, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  dim3 grid((p.V + vs - 1) / vs, p.H, requests);
-  return (int)lab_launch(delta_walk_kernel<R, NC>, grid, dim3(PARTS * vs / NC + HELPERS), smem, stream, p, vs);
+    cudaFuncSetAttribute(delta_walk_kernel<R, NC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const int segments = MODE == WALK_WHOLE ? 1 : MODE == WALK_CLOSE ? p.segments - 1 : p.segments;
+  dim3 grid((p.V + vs - 1) / vs + (MODE == WALK_CLOSE && p.segments > 2 ? (p.D + vs - 1) / vs : 0), p.H, requests * segments);
+  return (int)lab_launch(delta_walk_kernel<R, NC, MODE>, grid, dim3(PARTS * vs / NC + HELPERS), smem, stream, p, vs);
+}
+
+template <int PRE>
+int launch_fold_as(const WalkParams& p, int requests, cudaStream_t stream) {
+  const int smem = (2 * p.D * FOLD_V + FOLD_ROWS * (p.D + 4)) * (int)sizeof(float);
+  const cudaError_t e = cudaFuncSetAttribute(delta_fold_kernel<PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return (int)e;
+  return (int)lab_launch(delta_fold_kernel<PRE>, dim3((p.V + FOLD_V - 1) / FOLD_V, p.H, requests), dim3(256), smem, stream, p);
+}
+
+template <int R, int NC>
+int launch_walk(const WalkParams& p, int requests, int vs, cudaStream_t stream) {
+  if (p.segments <= 1) return launch_walk_as<R, NC, WALK_WHOLE>(p, requests, vs, stream);
+  int e = launch_walk_as<R, NC, WALK_CLOSE>(p, requests, vs, stream);
+  if (e == 0 && p.segments > 2)
+    e = p.D <= 64 ? launch_fold_as<16>(p, requests, stream)
+                  : p.D <= 128 ? launch_fold_as<32>(p, requests, stream) : launch_fold_as<64>(p, requests, stream);
+  return e != 0 ? e : launch_walk_as<R, NC, WALK_OUTPUT>(p, requests, vs, stream);
 }
 
 template <int R>
@@ -563,11 +701,16 @@ LAB_EXPORT int lab_delta_prepare(float* rec, float* v, float* decay, float* rate
 // vs: columns of the state a CTA takes (a multiple of 8 * cols, at most 32 * cols); cols: columns a thread takes (1, or
 // up to 128 key channels 2).
 // kept (with proj, ld, keep, channels): the inputs that replace a request's kept ones; null: none.
+// segments > 1: every request's rows are cut into at most that many; `states` [requests, segments, H, D, V] and, for more
+// than two, `moves` [requests, segments, H, D, D] are scratch.
 LAB_EXPORT int lab_delta_walk(float* out, const float* rec, const float* v, const float* decay, const float* rate,
                               float* state, const int* q_start, const int* state_slot, int tokens, int requests,
                               int n_slots, int H, int G, int D, int V, const float* proj, int ld, float* kept, int keep,
-                              int channels, int write, int vs, int cols, cudaStream_t stream) {
+                              int channels, int write, int vs, int cols, int segments, float* states, float* moves,
+                              cudaStream_t stream) {
   if (requests <= 0 || tokens <= 0) return 0;
+  if (segments > 1 && (states == nullptr || (segments > 2 && moves == nullptr) || (long long)requests * segments > 65535))
+    return (int)cudaErrorInvalidValue;
   if (H <= 0 || G <= 0 || H % G || D <= 0 || V <= 0 || (cols != 1 && cols != 2) || vs <= 0 || vs % (8 * cols) ||
       PARTS * vs / cols + HELPERS > 256 || (((uintptr_t)rec) & 15))
     return (int)cudaErrorInvalidValue;
@@ -575,6 +718,7 @@ LAB_EXPORT int lab_delta_walk(float* out, const float* rec, const float* v, cons
   p.out = out; p.rec = rec; p.v = v; p.decay = decay; p.rate = rate; p.tokens = tokens; p.state = state;
   p.q_start = q_start; p.state_slot = state_slot; p.n_slots = n_slots; p.H = H; p.G = G; p.D = D; p.V = V;
   p.write = write; p.proj = proj; p.kept = kept; p.ld = ld; p.keep = kept != nullptr ? keep : 0; p.channels = channels;
+  p.segments = segments; p.states = states; p.moves = moves;
   // 16-byte copies: every row of v, and every head's and slice's start in it, on a 16-byte boundary
   p.vec = V % 4 == 0 && (((uintptr_t)v) & 15) == 0;
   switch (share_of(D)) {

@@ -1120,12 +1120,37 @@ def delta_walk(rec: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, rate: to
         assert kept.dtype == torch.float32 and kept.is_contiguous() and kept.shape[0] == state.shape[0]
         assert proj.dtype == torch.float32 and proj.stride(1) == 1 and proj.shape[0] == tokens and proj.shape[1] >= channels
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=v.device)
-    vs, cols = shape if shape is not None else delta_walk_shape(ctx.n_requests * heads, keys, vdim, ctx.max_q_len)
+    pairs = ctx.n_requests * heads
+    segments = delta_walk_segments(pairs, keys, vdim, ctx.max_q_len) if shape is None else 1
+    vs, cols = shape if shape is not None else delta_walk_shape(pairs, keys, vdim, ctx.max_q_len)
+    if segments > 1:
+        vs, cols = (min(64, -(-vdim // 16) * 16), 2) if keys <= 128 else (min(vs, 32), 1)
+    states = moves = None
+    if segments > 1:
+        states = torch.empty((ctx.n_requests, segments, heads, keys, vdim), dtype=torch.float32, device=v.device)
+    if segments > 2:
+        moves = torch.empty((ctx.n_requests, segments, heads, keys, keys), dtype=torch.float32, device=v.device)
     _check(lib("gated_delta").lab_delta_walk(
         _ptr(out), _ptr(rec), _ptr(v), _ptr(decay), _ptr(rate), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), tokens,
         ctx.n_requests, state.shape[0], heads, groups, keys, vdim, _ptr(proj if keep else None), proj.stride(0) if keep else 0,
-        _ptr(kept if keep else None), keep, channels, int(write), vs, cols, _stream()), "delta_walk")
+        _ptr(kept if keep else None), keep, channels, int(write), vs, cols, segments, _ptr(states),
+        _ptr(moves), _stream()), "delta_walk", min(segments, 3))
     return out
+
+
+def delta_walk_segments(pairs: int, keys: int, vdim: int, longest: int) -> int:
+    """Into how many segments `delta_walk` cuts a request's rows, walked by CTAs of 64 columns, two a thread.  The launch
+    for the closing states has slices for the identity's columns beside the values' (but for the first segment), and
+    after it the opening states follow one by one, so segments pay over long portions while both launches find an SM per
+    CTA.  Measured with the mixer around it, 64 x 64 states: 14 pairs and 2,048 tokens 363 us in one piece, 237 in 4, 201
+    in 6, 213 in 8; 28 pairs and 700 tokens 155, 128 in 4, 137 in 5; 56 pairs and 500 tokens 188, 154 in 2, 188 in 3; 112
+    pairs and 250 tokens 116, 142 in 2; 14 pairs and 300 tokens 72, 71 in 4.  128 x 128: 12 pairs and 2,048 tokens 603,
+    412 in 4; 24 pairs and 300 tokens 116, 139 in 2."""
+    if longest < 400 or keys > 128:
+        return 1
+    values, moves = -(-vdim // 64), -(-keys // 64)
+    segments = 1 + (sm_count() + pairs * moves) // (pairs * (values + moves))
+    return max(1, min(segments, sm_count() // max(1, pairs * values)))
 
 
 def delta_walk_shape(pairs: int, keys: int, vdim: int, max_q_len: int) -> tuple[int, int]:

@@ -116,3 +116,46 @@ def test_running_maximum_of_any_length(heads):
             M[slot] = top
         at += length
     assert np.abs(m_state.double().cpu().numpy() - M).max() < 1e-3
+
+
+@pytest.mark.parametrize("segments", [1, 2, 3, 5, 9])
+@pytest.mark.parametrize("heads,groups,keys,vdim", [(4, 2, 64, 64), (3, 1, 20, 36), (2, 2, 128, 100), (1, 1, 200, 24), (2, 1, 16, 130)])
+def test_delta_walk_segments(heads, groups, keys, vdim, segments, monkeypatch):
+    monkeypatch.setattr(ops(), "delta_walk_segments", lambda *a: segments)
+    g = torch.Generator(device=DEV).manual_seed(keys + vdim)
+    rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
+    T, taps, H, G = sum(Q_LENS), 4, heads, groups
+    gd, hv = G * keys, H * vdim
+    proj = rand(T, 2 * gd + hv + 2 * H)
+    conv, a_log, bias = rand(2 * gd + hv, taps) * 0.5, rand(H), rand(H) - 2
+    state, kept = rand(6, H, keys, vdim), rand(6, taps - 1, 2 * gd + hv)
+    start, kept_start, ctx = state.clone(), kept.clone(), context(Q_LENS, SLOTS)
+    for write in (False, True):
+        operands = ops().delta_prepare(proj, 2 * gd + hv, 2 * gd + hv + H, taps, H, G, keys, vdim, conv, a_log, bias, kept, ctx,
+                                       keys ** -0.5, 1e-6)
+        out = ops().delta_walk(*operands, state, ctx, H, G, keys, vdim, write=write, proj=proj, kept=kept)
+        assert write or torch.equal(state, start) and torch.equal(kept, kept_start)
+    ops().take_device_errors()
+    n = lambda t: t.double().cpu().numpy()  # noqa: E731
+    P, W, want, at = n(proj), n(start), np.zeros((T, H, vdim)), 0
+    silu = lambda z: z / (1 + np.exp(-z))  # noqa: E731
+    for length, slot in zip(Q_LENS, SLOTS):
+        if slot < 0:
+            continue
+        full = np.concatenate([n(kept_start)[slot], P[at: at + length, : 2 * gd + hv]])
+        assert np.array_equal(n(kept)[slot], full[-(taps - 1):])
+        u = silu(sum(full[j: j + length] * n(conv)[:, j] for j in range(taps)))
+        q, k = (u[:, i * gd: (i + 1) * gd].reshape(length, G, keys) for i in (0, 1))
+        q, k = (m / np.sqrt((m * m).sum(-1, keepdims=True) + 1e-6) for m in (q, k))
+        q, k, v = q.repeat(H // G, 1) * keys ** -0.5, k.repeat(H // G, 1), u[:, 2 * gd:].reshape(length, H, vdim)
+        rate = 1 / (1 + np.exp(-P[at: at + length, 2 * gd + hv: 2 * gd + hv + H]))
+        decay = np.exp(-np.exp(n(a_log)) * np.log1p(np.exp(P[at: at + length, 2 * gd + hv + H:] + n(bias))))
+        for t in range(length):
+            S = decay[t][:, None, None] * W[slot]
+            new = rate[t][:, None] * (v[t] - (S * k[t][:, :, None]).sum(1))
+            W[slot] = S + k[t][:, :, None] * new[:, None, :]
+            want[at + t] = (W[slot] * q[t][:, :, None]).sum(1)
+        at += length
+    live = T - Q_LENS[-1]
+    # 32-bit roundings over the state's memory (decays near 0.9) and sums of up to 200
+    assert off(out[:live], want.reshape(T, -1)[:live]) < 2e-5 and off(state, W) < 2e-5
