@@ -19,8 +19,12 @@
 // log2(G) shuffles.  (Blocks interleaved over the threads, without padding, are as free of conflicts and
 // measured slower: 0.90 against 0.75 ms for 2,048 tokens of one request.)  What bounds the walk is the chain of dependent
 // instructions one warp has per token (measured with the kernel's own clock: 540 cycles a token with
-// 4 threads a column and 16 rows each), and a head's columns are shared out over D / CS CTAs so that
-// no scheduler holds more than one such chain.  Tokens are taken in chunks:
+// 4 threads a column and 16 rows each, an entry an instruction, and every token's loads in front of its arithmetic;
+// now two rows an instruction, and a vector's share of the next token is asked for as soon as this token's is used),
+// and a head's columns are shared out over D / CS CTAs so that
+// no scheduler holds more than one such chain.  (Measured with the mixer around it, 14 heads of 64: one request of 2,048
+// tokens 517 us against 632 in the earlier form, 300 tokens 98 against 120, three of 500 201 against 218.)
+// Tokens are taken in chunks:
 // a chunk's records are brought to shared memory by cp.async into the buffer that is not being walked.
 // Three kernels: a first one, parallel over tokens, forms what does not depend on the state (decays,
 // rates, unit keys); the walk; a third, parallel over tokens, divides each head's raw output by its root
@@ -92,17 +96,38 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// A thread's SL values of one vector of D values in shared memory.
-__device__ __forceinline__ void load_rows(float (&dst)[SL], const float* vec, int g) {
+// two 32-bit numbers an instruction, each rounded as by itself
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float low_of(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high_of(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+constexpr int SP = (SL + 1) / 2;      // pairs of rows a thread keeps (an odd last row beside a zero)
+
+// A thread's SL values of one vector of D values in shared memory, in pairs.
+__device__ __forceinline__ void load_rows(f32x2 (&dst)[SP], const float* vec, int g) {
   if constexpr (VEC) {
 #pragma unroll
     for (int q = 0; q < SL / 4; ++q) {
-      const float4 t = reinterpret_cast<const float4*>(vec + g * SLP)[q];
-      dst[4 * q] = t.x, dst[4 * q + 1] = t.y, dst[4 * q + 2] = t.z, dst[4 * q + 3] = t.w;
+      const ulonglong2 t = reinterpret_cast<const ulonglong2*>(vec + g * SLP)[q];
+      dst[2 * q] = t.x, dst[2 * q + 1] = t.y;
     }
   } else {
 #pragma unroll
-    for (int ii = 0; ii < SL; ++ii) dst[ii] = vec[g * SLP + ii];
+    for (int ii = 0; ii < SP; ++ii) dst[ii] = pair_of(vec[g * SLP + 2 * ii], 2 * ii + 1 < SL ? vec[g * SLP + 2 * ii + 1] : 0.f);
   }
 }
 
@@ -111,7 +136,6 @@ __global__ void __launch_bounds__(NT) delta_rule_kernel(DeltaParams p) {
   extern __shared__ __align__(16) uint8_t delta_smem[];
   static_assert(REC % 4 == 0 && (!VEC || (SLP % 4 == 0 && RL % 4 == 0)), "16-byte loads");
   DeltaShared& sh = *reinterpret_cast<DeltaShared*>(delta_smem);
-  pdl_trigger();
   pdl_wait();
   const int h = blockIdx.x, req = blockIdx.y;
   const int tid = threadIdx.x;
@@ -130,9 +154,11 @@ __global__ void __launch_bounds__(NT) delta_rule_kernel(DeltaParams p) {
     return;
   }
   float* S_g = p.state + ((size_t)slot * p.heads + h) * D * D;
-  float S[SL];
+  f32x2 S[SP];
 #pragma unroll
-  for (int ii = 0; ii < SL; ++ii) S[ii] = live ? S_g[(size_t)row_of(g, ii) * D + j] : 0.f;
+  for (int ii = 0; ii < SP; ++ii)
+    S[ii] = pair_of(live ? S_g[(size_t)row_of(g, 2 * ii) * D + j] : 0.f,
+                    live && 2 * ii + 1 < SL ? S_g[(size_t)row_of(g, 2 * ii + 1) * D + j] : 0.f);
   const int ld_out = p.heads * D;
   const float* records = p.rec + (size_t)h * p.tokens * REC;
 
@@ -153,44 +179,62 @@ __global__ void __launch_bounds__(NT) delta_rule_kernel(DeltaParams p) {
     __syncthreads();       // the chunk has landed for everyone, and the other buffer's readers are done
     if (t0 + CH < row1) fetch(t0 + CH, buf ^ 1);
     // ---- the recurrence, token by token ---------------------------------------------------
-    for (int tok = 0; tok < n; ++tok) {
-      // All of the token's values are asked for at once; what does not wait for the sums over the column
-      // (w * S + k * v_j) is formed beside them, so that one multiply-add follows the shuffles.
-      float u[SL], rw_[SL], w[SL], au[SL], kk[SL];
-      const float* rec = sh.rec[buf][tok];
+    // What does not wait for the sums over the column (w * S + k * v_j) is formed beside them, so that one
+    // multiply-add follows the shuffles; the next token's values are asked for where this token's are used up.
+    // (With more than 16 rows a thread the registers do not allow it: a token's values are asked for in front.)
+    constexpr bool AHEAD = SL <= 16;
+    f32x2 u[SP], rw_[SP], w[SP], au[SP], kk[SP];
+    float vj, alpha, beta;
+    auto load_all = [&](const float* rec) {
       load_rows(u, rec, g);
       load_rows(rw_, rec + RL, g);
       load_rows(w, rec + 2 * RL, g);
-      load_rows(au, rec + 3 * RL, g);
       load_rows(kk, rec + 4 * RL, g);
-      const float vj = live ? rec[OFF_V + j] : 0.f;
-      const float alpha = rec[OFF_AB], beta = rec[OFF_AB + 1];
-      float sa0 = 0.f, sa1 = 0.f, rw0 = 0.f, rw1 = 0.f;
+      load_rows(au, rec + 3 * RL, g);
+      vj = live ? rec[OFF_V + j] : 0.f, alpha = rec[OFF_AB], beta = rec[OFF_AB + 1];
+    };
+    if (AHEAD) load_all(sh.rec[buf][0]);
+    for (int tok = 0; tok < n; ++tok) {
+      if (!AHEAD) load_all(sh.rec[buf][tok]);
+      const float* rec = sh.rec[buf][min(tok + 1, n - 1)];
+      const float v_now = vj, alpha_now = alpha, beta_now = beta;
+      constexpr int NA = AHEAD ? 2 : 1;      // sums side by side (more of them cost more in additions than they hide)
+      f32x2 s2[2] = {0ull, 0ull}, r2[2] = {0ull, 0ull};      // zeros
 #pragma unroll
-      for (int ii = 0; ii < SL; ii += 2) {
-        sa0 = fmaf(u[ii], S[ii], sa0);
-        rw0 = fmaf(rw_[ii], S[ii], rw0);
-        if (ii + 1 < SL) {
-          sa1 = fmaf(u[ii + 1], S[ii + 1], sa1);
-          rw1 = fmaf(rw_[ii + 1], S[ii + 1], rw1);
-        }
+      for (int ii = 0; ii < SP; ++ii) {
+        s2[ii % NA] = fma2(u[ii], S[ii], s2[ii % NA]);
+        r2[ii % NA] = fma2(rw_[ii], S[ii], r2[ii % NA]);
       }
-      float sa = sa0 + sa1, rw = rw0 + rw1;
+      if (AHEAD) {
+        load_rows(u, rec, g);
+        load_rows(rw_, rec + RL, g);
+        vj = live ? rec[OFF_V + j] : 0.f, alpha = rec[OFF_AB], beta = rec[OFF_AB + 1];
+      }
+      float sa = low_of(s2[0]) + high_of(s2[0]), rw = low_of(r2[0]) + high_of(r2[0]);
+      if (NA == 2) sa += low_of(s2[1]) + high_of(s2[1]), rw += low_of(r2[1]) + high_of(r2[1]);
+      const f32x2 vv = pair_of(v_now, v_now);
 #pragma unroll
-      for (int ii = 0; ii < SL; ++ii) S[ii] = fmaf(kk[ii], vj, w[ii] * S[ii]);
+      for (int ii = 0; ii < SP; ++ii) S[ii] = AHEAD ? fma2(kk[ii], vv, mul2(w[ii], S[ii])) : fma2(w[ii], S[ii], mul2(kk[ii], vv));
+      if (AHEAD) {
+        load_rows(w, rec + 2 * RL, g);
+        load_rows(kk, rec + 4 * RL, g);
+      }
 #pragma unroll
       for (int o = 1; o < G; o <<= 1) {
         sa += __shfl_xor_sync(0xffffffffu, sa, o);
         rw += __shfl_xor_sync(0xffffffffu, rw, o);
       }
+      const f32x2 minus_sa = pair_of(-sa, -sa);
 #pragma unroll
-      for (int ii = 0; ii < SL; ++ii) S[ii] = fmaf(-au[ii], sa, S[ii]);
-      if (live && g == 0) p.out[(size_t)(t0 + tok) * ld_out + h * D + j] = fmaf(beta, vj, fmaf(-alpha, sa, rw));
+      for (int ii = 0; ii < SP; ++ii) S[ii] = fma2(au[ii], minus_sa, S[ii]);
+      if (AHEAD) load_rows(au, rec + 3 * RL, g);
+      if (live && g == 0) p.out[(size_t)(t0 + tok) * ld_out + h * D + j] = fmaf(beta_now, v_now, fmaf(-alpha_now, sa, rw));
     }
   }
+  pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
   if (p.write && live) {
 #pragma unroll
-    for (int ii = 0; ii < SL; ++ii) S_g[(size_t)row_of(g, ii) * D + j] = S[ii];
+    for (int ii = 0; ii < SL; ++ii) S_g[(size_t)row_of(g, ii) * D + j] = ii % 2 == 0 ? low_of(S[ii / 2]) : high_of(S[ii / 2]);
   }
 }
 
@@ -204,7 +248,6 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(float* __restrict__ 
                                                             int ld, const float* __restrict__ d, int ld_d,
                                                             const T* __restrict__ d_bias, const T* __restrict__ a_bias,
                                                             int heads, float decay_rate) {
-  pdl_trigger();
   pdl_wait();
   const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int h = blockIdx.y * 8 + warp; h < heads; h += 8 * gridDim.y) {
@@ -229,6 +272,7 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(float* __restrict__ 
     be = warp_sum(be);
     if (lane == 0) dst[OFF_AB] = al, dst[OFF_AB + 1] = be;
   }
+  pdl_trigger();      // (not earlier: the walk's few, long blocks would settle unevenly where these leave room first)
 }
 
 // Each head's raw output divided by its root mean square, times a plain weight and sigmoid(gate),

@@ -124,7 +124,6 @@ template <typename T, int TAPS>
 __global__ void __launch_bounds__(kThreads) delta_prepare_kernel(const T* __restrict__ taps_w, const T* __restrict__ a_log,
                                                                  const T* __restrict__ dt_bias, PrepareParams p) {
   extern __shared__ float keys[];      // [8][D]: the rows' unit keys (q and k units)
-  pdl_trigger();
   pdl_wait();
   constexpr int kPerLane = 8;          // heads of up to 256 key channels
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, unit = blockIdx.y;
@@ -218,6 +217,7 @@ __global__ void __launch_bounds__(kThreads) delta_prepare_kernel(const T* __rest
       p.rate[(size_t)h * p.tokens + t] = padding ? 0.f : sigmoid_f(p.proj[(size_t)t * p.ld + p.b_at + h]);
     }
   }
+  pdl_trigger();      // (not earlier: the walk's few, long blocks would settle unevenly where these leave room first)
 }
 
 // ---- the walk -----------------------------------------------------------------------------------
