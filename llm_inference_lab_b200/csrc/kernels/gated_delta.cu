@@ -42,6 +42,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int PARTS = 4;        // threads that share one column of the state
 constexpr int BLK = 4;          // rows of a block
+constexpr int LONG_WALK = 256;  // rows from which the next kernel is let in at the walk's end only
 constexpr int CT = 16;          // rows staged per chunk
 constexpr int HELPERS = 64;     // threads that copy chunks ahead and form the blocks' coefficients
 constexpr int DOTS = 8;         // q . k_0..3, k . k_0..2 of a row's block, one unused
@@ -273,6 +274,7 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
   const int all0 = p.q_start[r], all1 = p.q_start[r + 1];            // the request's rows, and this CTA's
   int t0 = all0, t1 = all1, last = 0;
   if (MODE != WALK_WHOLE && all1 > all0) last = segment_rows(t0, t1, seg, p.segments);
+  if (MODE == WALK_WHOLE && t1 - t0 < LONG_WALK) pdl_trigger();
   const int slot = p.state_slot[r];
   // slices beyond the values' walk the identity; of the first segment, whose state is known, and the last nobody asks
   const int slices = (p.V + Vs - 1) / Vs;

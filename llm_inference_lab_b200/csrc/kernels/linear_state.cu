@@ -27,6 +27,7 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int SCAN_P = 4;     // threads that share one column of the state
 constexpr int SCAN_CT = 16;   // tokens staged per chunk
+constexpr int LONG_WALK = 256;      // tokens from which the next kernel is let in at the walk's end only
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
 // SiLU by the hardware's 2^x and reciprocal approximations (relative error about 2^-21, as the attention
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
     t0 += seg * len;
     n_tok = MODE == SCAN_CLOSE && seg >= last ? 0 : min(len, n_tok - seg * len);
   }
+  if (MODE == SCAN_WHOLE && n_tok < LONG_WALK) pdl_trigger();
   if (n_tok <= 0 || slot == -1) {      // nothing to do, or rows of padding (their output is never read)
     pdl_wait();
     return;

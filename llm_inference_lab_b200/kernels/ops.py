@@ -1125,16 +1125,13 @@ def delta_walk(rec: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, rate: to
     vs, cols = shape if shape is not None else delta_walk_shape(pairs, keys, vdim, ctx.max_q_len)
     if segments > 1:
         vs, cols = (min(64, -(-vdim // 16) * 16), 2) if keys <= 128 else (min(vs, 32), 1)
-    states = moves = None
-    if segments > 1:
-        states = torch.empty((ctx.n_requests, segments, heads, keys, vdim), dtype=torch.float32, device=v.device)
-    if segments > 2:
-        moves = torch.empty((ctx.n_requests, segments, heads, keys, keys), dtype=torch.float32, device=v.device)
+    scratch, (states, moves) = _segment_scratch(segments, v.device, pairs * segments * keys * vdim,
+                                                pairs * segments * keys * keys if segments > 2 else 0)
     _check(lib("gated_delta").lab_delta_walk(
         _ptr(out), _ptr(rec), _ptr(v), _ptr(decay), _ptr(rate), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), tokens,
         ctx.n_requests, state.shape[0], heads, groups, keys, vdim, _ptr(proj if keep else None), proj.stride(0) if keep else 0,
-        _ptr(kept if keep else None), keep, channels, int(write), vs, cols, segments, _ptr(states),
-        _ptr(moves), _stream()), "delta_walk", min(segments, 3))
+        _ptr(kept if keep else None), keep, channels, int(write), vs, cols, segments, states,
+        moves, _stream()), "delta_walk", min(segments, 3))
     return out
 
 
@@ -1145,8 +1142,9 @@ def delta_walk_segments(pairs: int, keys: int, vdim: int, longest: int) -> int:
     CTA.  Measured with the mixer around it, 64 x 64 states: 14 pairs and 2,048 tokens 363 us in one piece, 237 in 4, 201
     in 6, 213 in 8; 28 pairs and 700 tokens 155, 128 in 4, 137 in 5; 56 pairs and 500 tokens 188, 154 in 2, 188 in 3; 112
     pairs and 250 tokens 116, 142 in 2; 14 pairs and 300 tokens 72, 71 in 4.  128 x 128: 12 pairs and 2,048 tokens 603,
-    412 in 4; 24 pairs and 300 tokens 116, 139 in 2."""
-    if longest < 400 or keys > 128:
+    412 in 4; 24 pairs and 300 tokens 116, 139 in 2.  One request's mixer launched kernel by kernel is bound by the host up to
+    600 tokens (420: 86 us in one piece, 102 in segments)."""
+    if longest < (600 if pairs < 42 else 400) or keys > 128:
         return 1
     values, moves = -(-vdim // 64), -(-keys // 64)
     segments = 1 + (sm_count() + pairs * moves) // (pairs * (values + moves))
@@ -1524,6 +1522,16 @@ def map_difference(attn: torch.Tensor, heads: int, vdim: int, head: int, lam: fl
 # ----------------------------------------------------------------------------------------
 # Recurrent mixers with a scalar decay (csrc/kernels/linear_state.cu).
 # ----------------------------------------------------------------------------------------
+def _segment_scratch(segments: int, device, *floats: int):
+    """(a buffer or None, pointers to its parts): 32-bit scratch of the recurrences that are walked in segments, in one
+    allocation; null pointers for a walk in one piece."""
+    if segments <= 1:
+        return None, tuple(ctypes.c_void_p(0) for _ in floats)
+    buf = torch.empty((sum(floats),), dtype=torch.float32, device=device)
+    at = [sum(floats[:i]) for i in range(len(floats))]
+    return buf, tuple(ctypes.c_void_p(buf.data_ptr() + 4 * a) for a in at)
+
+
 def decay_scan_supported(keys: int) -> bool:
     return 1 <= keys <= 256
 
@@ -1533,8 +1541,10 @@ def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) 
     multiprocessor holds four or five of up to 64 key channels, three of more.  Segments cost most of the walk's work
     once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it: 84 CTAs and 1,000
     tokens 283 us in one piece, 193 in 4, 180 in 8; 42 CTAs and 2,048 tokens 487, 217 in 8, 219 in 16; 42 and 300 tokens
-    123, 72 in 8; 168 CTAs and 500 tokens 171, 181 in 2, 168 in 4; 336 and 250 tokens 129, 160 in 2."""
-    if ctas >= sm_count():
+    123, 72 in 8; 168 CTAs and 500 tokens 171, 181 in 2, 168 in 4; 336 and 250 tokens 129, 160 in 2.  Below 450 tokens the
+    mixer launched kernel by kernel is bound by the host, which a second launch costs about 10 us (270 tokens: 95 us in one
+    piece, 109 in segments)."""
+    if ctas >= sm_count() or longest < 450:
         return 1
     room = (9 * sm_count() // 2 if keys <= 64 else 3 * sm_count()) // max(1, ctas)
     return max(1, min(longest // 32, room, 16, 65535 // max(1, requests)))
@@ -1576,14 +1586,11 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
         vs = 32 if pairs * -(-vdim // 32) >= sm_count() else (16 if pairs * -(-vdim // 16) >= sm_count() else 8)
     vs = min(vs, max(8, 1 << (vdim - 1).bit_length()))
     segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
-    states = decays = None
-    if segments > 1:
-        states = torch.empty((ctx.n_requests, segments, heads, keys, vdim), dtype=torch.float32, device=v.device)
-        decays = torch.empty((ctx.n_requests, segments, heads), dtype=torch.float32, device=v.device)
+    scratch, (states, decays) = _segment_scratch(segments, v.device, pairs * segments * keys * vdim, pairs * segments)
     _check(lib("linear_state").lab_decay_scan(
         _ptr(out), out.stride(0), _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(a_tok), _ptr(s_tok), ld_a,
         _ptr(a_head), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), ctx.n_requests, state.shape[0], heads, groups,
-        keys, vdim, int(silu), int(write), vs, segments, _ptr(states), _ptr(decays), _stream()), "decay_scan",
+        keys, vdim, int(silu), int(write), vs, segments, states, decays, _stream()), "decay_scan",
         2 if segments > 1 else 1)
     return out
 
@@ -1709,7 +1716,10 @@ def scan_segments(ctas: int, longest: int) -> int:
     multiprocessor holding four.  Segments cost a second launch and most of the walk's work once more, so they pay while
     they bring idle multiprocessors to work: measured with its mixer, 56 CTAs and 2,048 tokens 684 us in one piece, 327
     in 4, 238 in 8, 223 in 12; 112 CTAs and 700 tokens 259, 189 in 4, 171 in 6, 181 in 8; 224 CTAs and 500 tokens 247, 233
-    in 2; 448 CTAs and 250 tokens 175, 196 in 2.  Segments of 32 tokens (a chunk) still pay: 128 tokens 118, 100 in 4."""
+    in 2; 448 CTAs and 250 tokens 175, 196 in 2.  Below 320 tokens the mixer launched kernel by kernel is bound by the
+    host, which a second launch costs about 10 us."""
+    if longest < 320:
+        return 1
     return max(1, min(longest // 32, 9 * sm_count() // (2 * max(1, ctas)), 32))
 
 
@@ -1731,15 +1741,13 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
         raise KernelError(f"selective_scan: a state of {N} entries a channel exceeds {SELECTIVE_SCAN_MAX_STATE}")
     out = torch.empty((tokens, channels), dtype=a_log.dtype, device=x.device)
     segments = scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
-    states = sums = None
-    if segments > 1:
-        states = torch.empty((ctx.n_requests, segments, channels, N), dtype=torch.float32, device=x.device)
-        sums = torch.empty((ctx.n_requests, segments, channels), dtype=torch.float32, device=x.device)
+    scratch, (states, sums) = _segment_scratch(segments, x.device, ctx.n_requests * segments * channels * N,
+                                               ctx.n_requests * segments * channels)
     _check(lib("selective_scan").lab_selective_scan(
         _ptr(out), out.stride(0), _ptr(x), x.stride(0), _ptr(dt_pre), dt_pre.stride(0), _ptr(bc), bc.stride(0), b_at,
         c_at, _ptr(z), z.stride(0), _ptr(a_log), _ptr(skip), _ptr(dt_bias), _ptr(state), _ptr(ctx.q_start),
-        _ptr(ctx.state_slot), ctx.n_requests, channels, N, state.shape[0], int(write), segments, _ptr(states),
-        _ptr(sums), dtype_code(a_log.dtype), _stream()), "selective_scan", 2 if segments > 1 else 1)
+        _ptr(ctx.state_slot), ctx.n_requests, channels, N, state.shape[0], int(write), segments, states, sums,
+        dtype_code(a_log.dtype), _stream()), "selective_scan", 2 if segments > 1 else 1)
     return out
 
 
