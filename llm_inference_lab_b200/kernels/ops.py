@@ -1125,8 +1125,10 @@ def delta_walk(rec: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, rate: to
     vs, cols = shape if shape is not None else delta_walk_shape(pairs, keys, vdim, ctx.max_q_len)
     if segments > 1:
         vs, cols = (min(64, -(-vdim // 16) * 16), 2) if keys <= 128 else (min(vs, 32), 1)
-    scratch, (states, moves) = _segment_scratch(segments, v.device, pairs * segments * keys * vdim,
-                                                pairs * segments * keys * keys if segments > 2 else 0)
+    states = moves = None
+    if segments > 1:
+        scratch, (states, moves) = _segment_scratch(v.device, pairs * segments * keys * vdim,
+                                                    pairs * segments * keys * keys if segments > 2 else 0)
     _check(lib("gated_delta").lab_delta_walk(
         _ptr(out), _ptr(rec), _ptr(v), _ptr(decay), _ptr(rate), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), tokens,
         ctx.n_requests, state.shape[0], heads, groups, keys, vdim, _ptr(proj if keep else None), proj.stride(0) if keep else 0,
@@ -1522,11 +1524,9 @@ def map_difference(attn: torch.Tensor, heads: int, vdim: int, head: int, lam: fl
 # ----------------------------------------------------------------------------------------
 # Recurrent mixers with a scalar decay (csrc/kernels/linear_state.cu).
 # ----------------------------------------------------------------------------------------
-def _segment_scratch(segments: int, device, *floats: int):
-    """(a buffer or None, pointers to its parts): 32-bit scratch of the recurrences that are walked in segments, in one
-    allocation; null pointers for a walk in one piece."""
-    if segments <= 1:
-        return None, tuple(ctypes.c_void_p(0) for _ in floats)
+def _segment_scratch(device, *floats: int):
+    """(a buffer, pointers to its parts): 32-bit scratch of the recurrences that are walked in segments, in one
+    allocation."""
     buf = torch.empty((sum(floats),), dtype=torch.float32, device=device)
     at = [sum(floats[:i]) for i in range(len(floats))]
     return buf, tuple(ctypes.c_void_p(buf.data_ptr() + 4 * a) for a in at)
@@ -1586,7 +1586,9 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
         vs = 32 if pairs * -(-vdim // 32) >= sm_count() else (16 if pairs * -(-vdim // 16) >= sm_count() else 8)
     vs = min(vs, max(8, 1 << (vdim - 1).bit_length()))
     segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
-    scratch, (states, decays) = _segment_scratch(segments, v.device, pairs * segments * keys * vdim, pairs * segments)
+    states = decays = None
+    if segments > 1:
+        scratch, (states, decays) = _segment_scratch(v.device, pairs * segments * keys * vdim, pairs * segments)
     _check(lib("linear_state").lab_decay_scan(
         _ptr(out), out.stride(0), _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(a_tok), _ptr(s_tok), ld_a,
         _ptr(a_head), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), ctx.n_requests, state.shape[0], heads, groups,
@@ -1741,8 +1743,10 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
         raise KernelError(f"selective_scan: a state of {N} entries a channel exceeds {SELECTIVE_SCAN_MAX_STATE}")
     out = torch.empty((tokens, channels), dtype=a_log.dtype, device=x.device)
     segments = scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
-    scratch, (states, sums) = _segment_scratch(segments, x.device, ctx.n_requests * segments * channels * N,
-                                               ctx.n_requests * segments * channels)
+    states = sums = None
+    if segments > 1:
+        scratch, (states, sums) = _segment_scratch(x.device, ctx.n_requests * segments * channels * N,
+                                                   ctx.n_requests * segments * channels)
     _check(lib("selective_scan").lab_selective_scan(
         _ptr(out), out.stride(0), _ptr(x), x.stride(0), _ptr(dt_pre), dt_pre.stride(0), _ptr(bc), bc.stride(0), b_at,
         c_at, _ptr(z), z.stride(0), _ptr(a_log), _ptr(skip), _ptr(dt_bias), _ptr(state), _ptr(ctx.q_start),
