@@ -194,31 +194,25 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-// exp of two numbers that are not positive, to the hardware's 2^x (relative error about 2^-22): x log2(e) is cut into the
-// nearest integer and a rest of at most a half, the rest formed from log2(e) in two pieces (the range reduction of Cody
-// and Waite), so that a slow decay, whose error comes with the same sign at every token and adds up over the state's
-// memory, is off by no more than a fast one.  Below -86 the result stays at exp(-86), 4e-38.
-__device__ __forceinline__ f32x2 exp2_of(f32x2 x) {
-  const float magic = 12582912.f;      // 1.5 * 2^23: adding it rounds to an integer, which is left in the low bits
-  x = pair_of(fmaxf(low_of(x), -86.f), fmaxf(high_of(x), -86.f));
-  const f32x2 hi = pair_of(1.44269502f, 1.44269502f), lo = pair_of(1.92596299e-8f, 1.92596299e-8f);
-  const f32x2 t = fma2(x, hi, pair_of(magic, magic));
-  const f32x2 minus_j = fma2(t, pair_of(-1.f, -1.f), pair_of(magic, magic));
-  const f32x2 rest = fma2(x, lo, fma2(x, hi, minus_j));
-  return pair_of(__uint_as_float(__float_as_uint(fast_exp2(low_of(rest))) + ((uint32_t)t << 23)),
-                 __uint_as_float(__float_as_uint(fast_exp2(high_of(rest))) + ((uint32_t)(t >> 32) << 23)));
-}
+// The library's exponential: a slow decay's error comes with the same sign at every token and adds up over the state's
+// memory, so a form that is off by more is none.  (One by a range reduction and a polynomial, two entries an instruction,
+// took the mixer 242 us for 2,048 tokens, this one 222.)
+__device__ __forceinline__ f32x2 exp_of(f32x2 x) { return pair_of(expf(low_of(x)), expf(high_of(x))); }
+
+// The first `n` of two entries, zeros for the others.
+__device__ __forceinline__ f32x2 first_of(f32x2 v, int n) { return n >= 2 ? v : n == 1 ? v & 0xffffffffull : 0ull; }
 
 // Floats of one chunk's inputs as they arrive: dt_pre, x, z [WT][channels] each, then B and C [WT][N4] each, N4 the
 // state's entries in whole quads.
 __host__ __device__ inline int scan_chunk_floats(int wc, int n4) { return 3 * WT * wc + 2 * WT * n4; }
 
 // Lane l of a channel's WL holds the quads l, l + WL, ... of its state, R entries in all.  What bounds the walk, once
-// there are CTAs enough, is the issue of instructions: an entry and token takes eight, most of them for two entries at
-// once; a token of a CTA also takes its step sizes, gates and copies.  Measured on a B200, 1,792 channels of 16 entries:
-// 8 requests of 250 tokens 69 us (102 with eight lanes a channel, an entry an instruction and expf); one of 2,048
-// 114 us in eleven segments (344 in one piece of that form).
-template <typename T, int WL, int R, int MODE>
+// there are CTAs enough, is the issue of instructions: most of an entry's and token's are its exponential's, the others
+// take two entries each; a token of a CTA also takes its step sizes, gates and copies.  Measured on a B200, inputs from
+// memory, 1,792 channels of 16 entries: 8 requests of 250 tokens 84 us (115 with eight lanes a channel and an entry an
+// instruction); one of 2,048 131 us in eleven segments (352 in one piece of that form).  QUADS: the state is whole quads; else the entries that fill
+// the last one are kept at zero (an infinite step would leave no numbers there).
+template <typename T, int WL, int R, int MODE, bool QUADS>
 __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict__ out, const T* __restrict__ a_log,
                                                                   const T* __restrict__ skip,
                                                                   const T* __restrict__ dt_bias, ScanParams p) {
@@ -255,7 +249,7 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
     if (tid == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
     return;
   }
-  if (N != n4) {      // the last quad's missing entries of B and C are zeros, which no copy touches
+  if (!QUADS) {      // the last quad's missing entries of B and C are zeros, which no copy touches
     for (int i = tid; i < 2 * chunk_floats; i += WTHREADS) s_in[i] = 0.f;
     __syncthreads();
   }
@@ -362,8 +356,9 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
         if (Q * WL * 4 > 16 && e >= n4) break;
         if (Q * WL * 4 == 16 && e >= n4) continue;
         const ulonglong2 bq = *reinterpret_cast<const ulonglong2*>(b_b + tt * n4 + e);
-        S2[2 * q] = fma2(exp2_of(mul2(dt2, A2[2 * q])), S2[2 * q], mul2(dx2, bq.x));
-        S2[2 * q + 1] = fma2(exp2_of(mul2(dt2, A2[2 * q + 1])), S2[2 * q + 1], mul2(dx2, bq.y));
+        S2[2 * q] = fma2(exp_of(mul2(dt2, A2[2 * q])), S2[2 * q], mul2(dx2, bq.x));
+        S2[2 * q + 1] = fma2(exp_of(mul2(dt2, A2[2 * q + 1])), S2[2 * q + 1], mul2(dx2, bq.y));
+        if (!QUADS) S2[2 * q] = first_of(S2[2 * q], N - e), S2[2 * q + 1] = first_of(S2[2 * q + 1], N - e - 2);
         if (MODE != SCAN_CLOSE) {
           const ulonglong2 cq = *reinterpret_cast<const ulonglong2*>(b_c + tt * n4 + e);
           acc = fma2(S2[2 * q], cq.x, acc);
@@ -407,33 +402,39 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
   }
 }
 
-template <typename T, int WL, int R, int MODE>
+template <typename T, int WL, int R, int MODE, bool QUADS>
 int launch_scan_as(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
                    cudaStream_t stream) {
   constexpr int WC = WTHREADS / WL;
   const size_t smem = sizeof(float) * ((size_t)2 * scan_chunk_floats(WC, (p.N + 3) & ~3) + WT * WC + WT * WTHREADS);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, WL, R, MODE>,
+    cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, WL, R, MODE, QUADS>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
   const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
-  return (int)lab_launch(selective_scan_kernel<T, WL, R, MODE>, dim3((p.channels + WC - 1) / WC, requests, segments),
+  return (int)lab_launch(selective_scan_kernel<T, WL, R, MODE, QUADS>, dim3((p.channels + WC - 1) / WC, requests, segments),
                          dim3(WTHREADS), smem, stream, (T*)out, (const T*)a_log, (const T*)skip, (const T*)dt_bias, p);
 }
 
-template <typename T, int WL, int R>
+template <typename T, int WL, int R, bool QUADS = true>
 int launch_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
                 cudaStream_t stream) {
-  if (p.segments <= 1) return launch_scan_as<T, WL, R, SCAN_WHOLE>(out, a_log, skip, dt_bias, p, requests, stream);
-  const int e = launch_scan_as<T, WL, R, SCAN_CLOSE>(out, a_log, skip, dt_bias, p, requests, stream);
-  return e != 0 ? e : launch_scan_as<T, WL, R, SCAN_OUTPUT>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (p.segments <= 1) return launch_scan_as<T, WL, R, SCAN_WHOLE, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
+  const int e = launch_scan_as<T, WL, R, SCAN_CLOSE, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
+  return e != 0 ? e : launch_scan_as<T, WL, R, SCAN_OUTPUT, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
 }
 
 // Four lanes a channel up to 64 entries; eight beyond, where a lane's registers would not hold a quarter.
 template <typename T>
 int pick_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
               cudaStream_t stream) {
+  if (p.N % 4 != 0) {
+    if (p.N <= 16) return launch_scan<T, 4, 4, false>(out, a_log, skip, dt_bias, p, requests, stream);
+    if (p.N <= 64) return launch_scan<T, 4, 16, false>(out, a_log, skip, dt_bias, p, requests, stream);
+    if (p.N <= SCAN_MAX_STATE) return launch_scan<T, 8, 32, false>(out, a_log, skip, dt_bias, p, requests, stream);
+    return (int)cudaErrorInvalidValue;
+  }
   if (p.N <= 16) return launch_scan<T, 4, 4>(out, a_log, skip, dt_bias, p, requests, stream);
   if (p.N <= 32) return launch_scan<T, 4, 8>(out, a_log, skip, dt_bias, p, requests, stream);
   if (p.N <= 64) return launch_scan<T, 4, 16>(out, a_log, skip, dt_bias, p, requests, stream);
