@@ -57,7 +57,8 @@ __global__ void __launch_bounds__(kThreads) memory_gates_kernel(float* __restric
 // that of its rows, a scan over the lanes gives each lane the m before its rows, and it walks them, forming each row's
 // two exponentials.  What bounds it is latency (a chain through every row, 32 rows a step, took 51 us for 2,048 rows),
 // so the next 256 rows' gates are loaded before this step's arithmetic.  Any m near the running maximum gives the same
-// result: both exponentials and the floor of the denominator go by the m that is kept.
+// result: both exponentials and the floor of the denominator go by the m that is kept, a lane's first decay by the one
+// that the lane before it ends with (the scan's m before its rows may differ from that by roundings).
 // decay[t, h] and scale[t, h] leave as rows of [tokens, 2, H] (over the gates).
 __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __restrict__ gates, float* __restrict__ m_out,
                                                                     float* __restrict__ m_state,
@@ -101,20 +102,24 @@ __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __res
       if (lane >= o) i_all = fmaxf(i_left + f_all, i_all), f_all += f_left;
     }
     const float f_before = __shfl_up_sync(0xffffffffu, f_all, 1), i_before = __shfl_up_sync(0xffffffffu, i_all, 1);
-    float mine = lane == 0 ? m : fmaxf(f_before + m, i_before);
+    float mine = lane == 0 ? m : fmaxf(f_before + m, i_before), first = 0.f;      // first: m after the lane's first row
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
       const int row = c + lane * kRows + k;
       const float carried = gf[k] + mine;
       mine = fmaxf(carried, gi[k]);
+      if (k == 0) first = mine;
       if (row < n) {
         float* g = gates + (size_t)(t0 + row) * 2 * H;
-        g[h] = expf(carried - mine);           // decay of the state
-        g[H + h] = expf(gi[k] - mine);         // scale of the new key
+        if (k > 0) g[h] = expf(carried - mine);      // decay of the state
+        g[H + h] = expf(gi[k] - mine);               // scale of the new key
         m_out[(size_t)(t0 + row) * H + h] = mine;
       }
     }
-    m = __shfl_sync(0xffffffffu, mine, 31);
+    const float left = __shfl_up_sync(0xffffffffu, mine, 1);
+    if (c + lane * kRows < n)
+      gates[(size_t)(t0 + c + lane * kRows) * 2 * H + h] = expf(gf[0] + (lane == 0 ? m : left) - first);
+    m = __shfl_sync(0xffffffffu, mine, min(31, (n - 1 - c) / kRows));      // after the last of these rows
 #pragma unroll
     for (int k = 0; k < kRows; ++k) gi[k] = gi_next[k], gf[k] = gf_next[k];
   }

@@ -159,3 +159,24 @@ def test_delta_walk_segments(heads, groups, keys, vdim, segments, monkeypatch):
     live = T - Q_LENS[-1]
     # 32-bit roundings over the state's memory (decays near 0.9) and sums of up to 200
     assert off(out[:live], want.reshape(T, -1)[:live]) < 2e-5 and off(state, W) < 2e-5
+
+
+def test_decays_go_by_the_running_maximum_that_is_kept():
+    g = torch.Generator(device=DEV).manual_seed(11)
+    lens, slots, heads = [9, 700, 1, 256], [1, 0, 3, 2], 3
+    T, ctx = sum(lens), context(lens, slots)
+    log_i = torch.randn(T, heads, device=DEV, generator=g) * 3 + torch.tensor([0.0, 4900.0, 5100.0], device=DEV)
+    log_f = -torch.rand(T, heads, device=DEV, generator=g)
+    gates, m_state = torch.stack([log_i, log_f], dim=1), torch.full((4, heads), 5000.0, device=DEV)
+    m = ops().memory_stabilize(gates, m_state, ctx).cpu().numpy()
+    decay, scale = (gates[:, i].cpu().numpy() for i in (0, 1))
+    log_i, log_f, at = log_i.cpu().numpy(), log_f.cpu().numpy(), 0
+    for length, slot in zip(lens, slots):
+        before = np.concatenate([np.full((1, heads), 5000.0, dtype=np.float32), m[at: at + length - 1]])
+        now = m[at: at + length]
+        carried = log_f[at: at + length] + before      # 32-bit, as the kernel forms it
+        # the exponentials' arguments are differences of 32-bit numbers: what is left is the exponentials' own rounding
+        assert np.abs(decay[at: at + length] - np.exp((carried - now).astype(np.float64))).max() < 1e-6
+        assert np.abs(scale[at: at + length] - np.exp((log_i[at: at + length] - now).astype(np.float64))).max() < 1e-6
+        assert np.array_equal(m_state[slot].cpu().numpy(), now[-1])
+        at += length
