@@ -59,12 +59,14 @@ __global__ void __launch_bounds__(kThreads) memory_gates_kernel(float* __restric
 // so the next 256 rows' gates are loaded before this step's arithmetic.  Any m near the running maximum gives the same
 // result: both exponentials and the floor of the denominator go by the m that is kept, a lane's first decay by the one
 // that the lane before it ends with (the scan's m before its rows may differ from that by roundings).
+// in_order: the chain itself, a lane's rows after the other's, so that a row's m does not depend on how the sequence was
+// cut into steps; 2,048 rows take about 12 us longer.
 // decay[t, h] and scale[t, h] leave as rows of [tokens, 2, H] (over the gates).
 __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __restrict__ gates, float* __restrict__ m_out,
                                                                     float* __restrict__ m_state,
                                                                     const int* __restrict__ q_start,
                                                                     const int* __restrict__ state_slot, int requests,
-                                                                    int n_slots, int H, int write) {
+                                                                    int n_slots, int H, int write, int in_order) {
   pdl_trigger();
   pdl_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -93,16 +95,28 @@ __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __res
   load(0, gi, gf);
   for (int c = 0; c < n; c += 32 * kRows) {
     load(c + 32 * kRows, gi_next, gf_next);
-    float f_all = 0.f, i_all = -INFINITY;      // the lane's rows together, then the rows of all lanes up to it
+    const float m_step = m;
+    float mine = m, first = 0.f;      // m before the lane's rows; after its first row
+    if (in_order) {
+      for (int l = 0; l < 32 && c + l * kRows < n; ++l) {
+        if (lane >= l) mine = m;
+        float walked = m;
 #pragma unroll
-    for (int k = 0; k < kRows; ++k) f_all += gf[k], i_all = fmaxf(i_all + gf[k], gi[k]);
+        for (int k = 0; k < kRows; ++k) walked = fmaxf(gf[k] + walked, gi[k]);
+        m = __shfl_sync(0xffffffffu, walked, l);
+      }
+    } else {
+      float f_all = 0.f, i_all = -INFINITY;      // the lane's rows together, then the rows of all lanes up to it
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float f_left = __shfl_up_sync(0xffffffffu, f_all, o), i_left = __shfl_up_sync(0xffffffffu, i_all, o);
-      if (lane >= o) i_all = fmaxf(i_left + f_all, i_all), f_all += f_left;
+      for (int k = 0; k < kRows; ++k) f_all += gf[k], i_all = fmaxf(i_all + gf[k], gi[k]);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float f_left = __shfl_up_sync(0xffffffffu, f_all, o), i_left = __shfl_up_sync(0xffffffffu, i_all, o);
+        if (lane >= o) i_all = fmaxf(i_left + f_all, i_all), f_all += f_left;
+      }
+      const float f_before = __shfl_up_sync(0xffffffffu, f_all, 1), i_before = __shfl_up_sync(0xffffffffu, i_all, 1);
+      if (lane > 0) mine = fmaxf(f_before + m, i_before);
     }
-    const float f_before = __shfl_up_sync(0xffffffffu, f_all, 1), i_before = __shfl_up_sync(0xffffffffu, i_all, 1);
-    float mine = lane == 0 ? m : fmaxf(f_before + m, i_before), first = 0.f;      // first: m after the lane's first row
 #pragma unroll
     for (int k = 0; k < kRows; ++k) {
       const int row = c + lane * kRows + k;
@@ -118,8 +132,8 @@ __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __res
     }
     const float left = __shfl_up_sync(0xffffffffu, mine, 1);
     if (c + lane * kRows < n)
-      gates[(size_t)(t0 + c + lane * kRows) * 2 * H + h] = expf(gf[0] + (lane == 0 ? m : left) - first);
-    m = __shfl_sync(0xffffffffu, mine, min(31, (n - 1 - c) / kRows));      // after the last of these rows
+      gates[(size_t)(t0 + c + lane * kRows) * 2 * H + h] = expf(gf[0] + (lane == 0 ? m_step : left) - first);
+    if (!in_order) m = __shfl_sync(0xffffffffu, mine, min(31, (n - 1 - c) / kRows));      // after the last of these rows
 #pragma unroll
     for (int k = 0; k < kRows; ++k) gi[k] = gi_next[k], gf[k] = gf_next[k];
   }
@@ -183,11 +197,11 @@ LAB_EXPORT int lab_memory_gates(float* gates, float* v_out, const float* proj, i
 
 // gates [tokens, 2, H]: in, the log gates; out, the decay and the key's scale of every row.  m_out [tokens, H].
 LAB_EXPORT int lab_memory_stabilize(float* gates, float* m_out, float* m_state, const int* q_start, const int* state_slot,
-                                    int requests, int n_slots, int H, int write, cudaStream_t stream) {
+                                    int requests, int n_slots, int H, int write, int in_order, cudaStream_t stream) {
   if (requests <= 0) return 0;
   const int warps = kThreads / 32;
   lab_launch(memory_stabilize_kernel, dim3((requests * H + warps - 1) / warps), dim3(kThreads), 0, stream, gates, m_out,
-             m_state, q_start, state_slot, requests, n_slots, H, write);
+             m_state, q_start, state_slot, requests, n_slots, H, write, in_order);
   LAB_LAUNCH_CHECK();
 }
 

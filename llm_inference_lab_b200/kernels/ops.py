@@ -1552,12 +1552,14 @@ def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, ctx, heads: int, groups: int,
                keys: int, vdim: int, a_head: torch.Tensor | None = None, a_tok: torch.Tensor | None = None,
-               s_tok: torch.Tensor | None = None, silu: bool = False, write: bool = True) -> torch.Tensor:
+               s_tok: torch.Tensor | None = None, silu: bool = False, write: bool = True,
+               in_order: bool = False) -> torch.Tensor:
     """Per request and head, over the step's rows in order: S <- a S + (s k) v^T, o = S^T q, with S
     [keys, vdim] read from and (with `write`) left in `state` [slots, heads, keys, vdim].  q and k are 32-bit
     column slices [tokens, groups * keys] of one tensor (same row stride), v [tokens, heads * vdim]; `a_head`
     [heads] a fixed decay per head, or `a_tok`/`s_tok` [tokens, heads] per token; `silu`: q, k and v pass a
-    SiLU first.  Returns o [tokens, heads * vdim] in 32-bit."""
+    SiLU first.  `in_order`: a request's rows are walked in one piece, so that a position's bits depend neither on the
+    cut nor on the other requests of the step.  Returns o [tokens, heads * vdim] in 32-bit."""
     _on_gpu(q, k, v, state, a_head, a_tok, s_tok)
     tokens = v.shape[0]
     for t in (q, k, v):
@@ -1585,7 +1587,7 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     else:
         vs = 32 if pairs * -(-vdim // 32) >= sm_count() else (16 if pairs * -(-vdim // 16) >= sm_count() else 8)
     vs = min(vs, max(8, 1 << (vdim - 1).bit_length()))
-    segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
+    segments = 1 if in_order else decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
     states = decays = None
     if segments > 1:
         scratch, (states, decays) = _segment_scratch(v.device, pairs * segments * keys * vdim, pairs * segments)
@@ -1727,11 +1729,12 @@ def scan_segments(ctas: int, longest: int) -> int:
 
 def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int, z: torch.Tensor,
                    a_log: torch.Tensor, skip: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor, ctx,
-                   write: bool = True) -> torch.Tensor:
+                   write: bool = True, in_order: bool = False) -> torch.Tensor:
     """The walk of a state-space mixer with a decay per channel and state entry: 32-bit x, dt_pre, z
     [tokens, channels] (rows may be strided), B and C [tokens, N] at columns b_at and c_at of `bc`; a_log
-    [channels, N], skip and dt_bias [channels] in the storage type; state [slots, channels, N] 32-bit.  Returns
-    (sum_n S C + skip x) * silu(z) rounded to the storage type."""
+    [channels, N], skip and dt_bias [channels] in the storage type; state [slots, channels, N] 32-bit.  `in_order`: a
+    request's rows are walked in one piece, so that a position's bits depend neither on the cut nor on the other requests
+    of the step.  Returns (sum_n S C + skip x) * silu(z) rounded to the storage type."""
     _on_gpu(x, dt_pre, bc, z, a_log, skip, dt_bias, state)
     tokens, channels = x.shape
     N = a_log.shape[1]
@@ -1742,7 +1745,7 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
     if N > SELECTIVE_SCAN_MAX_STATE:
         raise KernelError(f"selective_scan: a state of {N} entries a channel exceeds {SELECTIVE_SCAN_MAX_STATE}")
     out = torch.empty((tokens, channels), dtype=a_log.dtype, device=x.device)
-    segments = scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
+    segments = 1 if in_order else scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
     states = sums = None
     if segments > 1:
         scratch, (states, sums) = _segment_scratch(x.device, ctx.n_requests * segments * channels * N,
@@ -2143,10 +2146,12 @@ def memory_gates(proj: torch.Tensor, v_at: int, i_at: int, f_at: int, b_i: torch
     return gates, values
 
 
-def memory_stabilize(gates: torch.Tensor, m_state: torch.Tensor, ctx, write: bool = True) -> torch.Tensor:
+def memory_stabilize(gates: torch.Tensor, m_state: torch.Tensor, ctx, write: bool = True,
+                     in_order: bool = False) -> torch.Tensor:
     """Walks every request's rows in order: m <- max(f + m, i) from the request's slot of `m_state` [slots, heads];
     `gates` [tokens, 2, heads] become the state's decay exp(f + m_before - m) and the key's scale exp(i - m) of each
-    row; returns m of every row [tokens, heads].  With `write` the last m goes back to the slot."""
+    row; returns m of every row [tokens, heads].  With `write` the last m goes back to the slot.  `in_order`: m is formed
+    row after row, so that its roundings do not depend on the cut."""
     _on_gpu(gates, m_state)
     tokens, _, heads = gates.shape
     assert gates.dtype == torch.float32 and gates.is_contiguous()
@@ -2154,7 +2159,7 @@ def memory_stabilize(gates: torch.Tensor, m_state: torch.Tensor, ctx, write: boo
     m = torch.empty((tokens, heads), dtype=torch.float32, device=gates.device)
     _check(lib("matrix_memory").lab_memory_stabilize(
         _ptr(gates), _ptr(m), _ptr(m_state), _ptr(ctx.q_start), _ptr(ctx.state_slot), ctx.n_requests, m_state.shape[0],
-        heads, int(write), _stream()), "memory_stabilize")
+        heads, int(write), int(in_order), _stream()), "memory_stabilize")
     return m
 
 

@@ -54,7 +54,8 @@ class DecayLinearAttention(Mixer):
         if proj is None:
             proj = ops.linear(x, self.w_in, None, out_f32=True)
         o = ops.decay_scan(proj[:, :hd], proj[:, hd: 2 * hd], proj[:, 2 * hd: 2 * hd + hv], cache.state, ctx, self.heads,
-                           self.heads, self.dim, self.vdim, a_head=self.decay, silu=True, write=cache.write)
+                           self.heads, self.dim, self.vdim, a_head=self.decay, silu=True, write=cache.write,
+                           in_order=self.dtype == torch.float32)
         return ops.gated_norm(o, proj[:, 2 * hd + hv:], self.norm_weight, self.eps, mult=mult, out=out)
 
     def forward(self, x, ctx, cache):
@@ -126,7 +127,8 @@ class StateSpaceMixer(Mixer):
                                           write=cache.write)
         xs = conv[:, :inner]
         y = ops.decay_scan(conv[:, inner + gn:], conv[:, inner: inner + gn], xs, state.state, ctx, self.heads,
-                           self.groups, self.state, self.vdim, a_tok=decay, s_tok=dt, write=cache.write)
+                           self.groups, self.state, self.vdim, a_tok=decay, s_tok=dt, write=cache.write,
+                           in_order=self.dtype == torch.float32)
         return ops.gated_norm(y, proj[:, :inner], self.norm_weight, self.eps, parts=self.parts, gate_first=True,
                               skip=self.skip, x=xs, head_size=self.vdim, mult=mult, out=out)
 

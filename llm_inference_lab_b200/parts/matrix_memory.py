@@ -68,9 +68,10 @@ class MatrixMemory(Mixer):
         memory, top = cache.part(0), cache.part(1)
         gates, values = ops.memory_gates(proj, 2 * hd, 2 * hd + 2 * hv, 2 * hd + 2 * hv + H, self.b_i, self.b_f, H,
                                          self.vdim, self.cap)
-        m = ops.memory_stabilize(gates, top.state, ctx, write=cache.write)
+        in_order = self.dtype == torch.float32
+        m = ops.memory_stabilize(gates, top.state, ctx, write=cache.write, in_order=in_order)
         o = ops.decay_scan(proj[:, :hd], proj[:, hd: 2 * hd], values, memory.state, ctx, H, H, self.dim, self.vpad,
-                           a_tok=gates[:, 0, :], s_tok=gates[:, 1, :], write=cache.write)
+                           a_tok=gates[:, 0, :], s_tok=gates[:, 1, :], write=cache.write, in_order=in_order)
         return ops.memory_finish(o, m, proj[:, 2 * hd + hv: 2 * hd + 2 * hv], self.norm_weight, ctx, H, self.vdim,
                                  self.dim ** -0.5, self.floor, self.eps, mult=mult, out=out)
 

@@ -70,7 +70,7 @@ class SelectiveScanMixer(Mixer):
             bc, b_at = ops.linear(xt, self.w_x_bc, None, out_f32=True), 0
         dt_pre = ops.linear(dt_low, self.w_dt, None, out_f32=True)
         y = ops.selective_scan(x32, dt_pre, bc, b_at, b_at + N, proj[:, inner:], self.a_log, self.skip, self.dt_bias,
-                               state.state, ctx, write=cache.write)
+                               state.state, ctx, write=cache.write, in_order=self.dtype == torch.float32)
         return ops.linear(y, self.w_o, None, out_f32=True, allow_partial=True)
 
 
