@@ -132,8 +132,10 @@ __global__ void __launch_bounds__(WARPS * 32) attention_plain_kernel(
 // values come to its own buffers by cp.async, the next chunk's keys while the values of this one are used and the other
 // way round.  A warp takes 8 rows: scores with a key per lane (the row's query as broadcasts, two products an
 // instruction: sums of even and odd entries apart), the weights left in shared memory, then the weighted sum with two
-// neighbouring entries of the head per lane.  A row's own arithmetic is the same in every tile and batch; rows of other
-// requests in the tile take a pass of their own.
+// neighbouring entries of the head per lane.  A row's own arithmetic is the same in every tile and batch.  With the
+// requests' first rows (`q_start`) no tile holds rows of two requests: a CTA finds its request by a scan over their
+// numbers of tiles, and single tokens beside a prompt's portion are walked side by side.  Without, rows of another request
+// in the tile take a pass of their own, after the first.
 //
 // What bounds it: multiply-adds and loads from shared memory, about even with 8 rows to a warp.  The other kernel's block
 // per (row, head) reads a row's keys and values once per head and row.  Measured on a B200, 32-bit, 14 query and 2 kv
@@ -173,9 +175,10 @@ struct RowsParams {
   const int* row_req;
   const int* row_pos;
   const int* block_table;
+  const int* q_start;      // [requests + 1], or null
   const float* sinks;
   const float* dist_bias;
-  int out_stride, q_stride, max_blocks, tokens, n_q, n_kv, d, page_size, num_pages, window, keep_first, sink, bias_len,
+  int requests, out_stride, q_stride, max_blocks, tokens, n_q, n_kv, d, page_size, num_pages, window, keep_first, sink, bias_len,
       out_f32, tile_tokens, head_tiles;      // tokens of a tile; tiles that share a token's heads
   float scale, softcap;
 };
@@ -198,14 +201,37 @@ __global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsPa
   const int tid = threadIdx.x, lane = tid & 31, part = tid / (32 * WPG), warp = (tid >> 5) % WPG;
   const int kvh = blockIdx.y, group = p.n_q / p.n_kv;
   const int tile = gridDim.x - 1 - blockIdx.x;      // the last rows see the most keys: they go first
-  const int t0 = tile / p.head_tiles * p.tile_tokens, h0 = tile % p.head_tiles * R;
-  const int heads = min(R, group - h0);             // of a token in this tile
+  int t0 = tile / p.head_tiles * p.tile_tokens, t_end = p.tokens;
+  const int h0 = tile % p.head_tiles * R, heads = min(R, group - h0);      // of a token in this tile
+  pdl_wait();
+  if (p.q_start != nullptr) {
+    int left = tile / p.head_tiles;      // tiles of tokens before this one, of requests that have not been passed
+    t0 = t_end;
+    for (int q0 = 0; q0 < p.requests; q0 += 32) {      // (the same in every warp)
+      const int q = q0 + lane, first = q < p.requests ? p.q_start[q] : 0, rows = q < p.requests ? p.q_start[q + 1] - first : 0;
+      const int tiles = (rows + p.tile_tokens - 1) / p.tile_tokens;
+      int upto = tiles;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const unsigned there = __ballot_sync(0xffffffffu, upto > left);
+      if (there != 0u) {
+        const int at = __ffs(there) - 1;
+        t0 = __shfl_sync(0xffffffffu, first + (left - (upto - tiles)) * p.tile_tokens, at);
+        t_end = min(t_end, __shfl_sync(0xffffffffu, first + rows, at));
+        break;
+      }
+      left -= __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (t0 >= t_end) return;      // a tile more than there are
+  }
   auto token_of = [&](int r) { return t0 + r / heads; };
   auto head_of = [&](int r) { return kvh * group + h0 + r % heads; };
-  pdl_wait();
   for (int r = tid; r < R; r += NT) {
     const int t = token_of(r);
-    const bool has = r < heads * p.tile_tokens && t < p.tokens;
+    const bool has = r < heads * p.tile_tokens && t < t_end;
     s_req[r] = has ? p.row_req[t] : -1;
     s_pos[r] = has ? p.row_pos[t] : -1;
   }
@@ -409,7 +435,10 @@ int launch_rows(RowsParams p, cudaStream_t stream) {
   const cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<T, D, PARTS, WPG>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return (int)e;
-  const long long tiles = ((long long)p.tokens + p.tile_tokens - 1) / p.tile_tokens * p.head_tiles;
+  if (p.tile_tokens == 1) p.q_start = nullptr;
+  // with the requests' borders: every request may end in a tile that is not full
+  const long long more = p.q_start != nullptr ? (long long)p.requests * (p.tile_tokens - 1) : p.tile_tokens - 1;
+  const long long tiles = (p.tokens + more) / p.tile_tokens * p.head_tiles;
   return (int)lab_launch(attention_rows_kernel<T, D, PARTS, WPG>, dim3((unsigned)tiles, p.n_kv), dim3(PARTS * 32 * WPG),
                          smem, stream, p);
 }
@@ -432,19 +461,20 @@ int pick_rows(RowsParams p, bool single, cudaStream_t stream) {
 }
 }  // namespace
 
-// `single`: no request brings more than one row (rows of one token then make up a tile).
+// `single`: no request brings more than one row (rows of one token then make up a tile).  q_start: the requests' first
+// rows, and the number of all rows behind them, or null; then no tile takes rows of two requests.
 LAB_EXPORT int lab_attention_plain(void* out, int out_stride, const void* q, int q_stride, const void* cache_k,
                                    const void* cache_v, const int* row_req, const int* row_pos, const int* block_table,
                                    int max_blocks, int tokens, int n_q, int n_kv, int d, int page_size, int num_pages,
                                    int window, float scale, int keep_first, int sink, const float* sinks,
                                    const float* dist_bias, int bias_len, float softcap, int out_f32, int single,
-                                   int dtype, cudaStream_t stream) {
+                                   const int* q_start, int requests, int dtype, cudaStream_t stream) {
   if (tokens <= 0) return 0;
   if (d > 32 * MAX_DPL || d <= 0 || n_q % n_kv || (dist_bias != nullptr && bias_len < 1)) return (int)cudaErrorInvalidValue;
   if (sinks != nullptr) sink = 1;
   if (d % (dtype == LAB_F32 ? 4 : 8) == 0 && (((uintptr_t)cache_k | (uintptr_t)cache_v) & 15) == 0 && n_kv <= 65535) {
-    const RowsParams p{out, q, cache_k, cache_v, row_req, row_pos, block_table, sinks, dist_bias, out_stride, q_stride,
-                       max_blocks, tokens, n_q, n_kv, d, page_size, num_pages, window, keep_first, sink, bias_len,
+    const RowsParams p{out, q, cache_k, cache_v, row_req, row_pos, block_table, requests > 1 ? q_start : nullptr, sinks,
+                       dist_bias, requests, out_stride, q_stride, max_blocks, tokens, n_q, n_kv, d, page_size, num_pages, window, keep_first, sink, bias_len,
                        out_f32, 1, 1, scale, softcap};
     return dtype == LAB_F32 ? pick_rows<float>(p, single != 0, stream) : pick_rows<__nv_bfloat16>(p, single != 0, stream);
   }

@@ -317,14 +317,16 @@ def attention_plain(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tenso
                     window: int, scale: float, out: torch.Tensor | None = None, keep_first: int = 0,
                     sink_one: bool = False, sink: torch.Tensor | None = None,
                     dist_bias: torch.Tensor | None = None, softcap: float = 0.0, out_f32: bool = False,
-                    single: bool = False) -> torch.Tensor:
+                    single: bool = False, q_start: torch.Tensor | None = None, requests: int = 0) -> torch.Tensor:
     """Attention of every row over its request's pages; q may be a column slice of the fused projection.
     `keep_first`: with a window, the first that many positions stay visible; `sink_one`: one more in the
     softmax's denominator; `sink` [n_q] 32-bit: exp(sink[h]) more instead; `dist_bias` [n_q, L] 32-bit: added to
     the scaled score by distance query - key, distances from L - 1 on sharing the last entry; `softcap` c > 0: the
     scaled score s becomes c * tanh(s / c), before the bias.  `out_f32`: the result is 32-bit, not rounded to q's type.
-    `single`: no request brings more than one row (a choice of tiles only: the result is the same)."""
-    _on_gpu(q, cache_k, cache_v, row_req, row_pos, block_table, sink, dist_bias)
+    `single`: no request brings more than one row; `q_start` [requests + 1]: the requests' first rows, all rows in their
+    order (both a choice of tiles only: the result is the same)."""
+    _on_gpu(q, cache_k, cache_v, row_req, row_pos, block_table, sink, dist_bias, q_start)
+    assert q_start is None or (q_start.dtype == torch.int32 and q_start.numel() > requests and q_start.is_contiguous())
     assert sink is None or (sink.dtype == torch.float32 and sink.numel() >= n_q and sink.is_contiguous())
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.dim() == 2 and
                                  dist_bias.shape[0] == n_q and dist_bias.is_contiguous())
@@ -340,7 +342,7 @@ def attention_plain(q: torch.Tensor, cache_k: torch.Tensor, cache_v: torch.Tenso
         _ptr(block_table), block_table.shape[1], tokens, n_q, n_kv, head_dim, page_size, num_pages, window,
         ctypes.c_float(scale), int(keep_first), int(bool(sink_one) or sink is not None), _ptr(sink), _ptr(dist_bias),
         dist_bias.shape[1] if dist_bias is not None else 0, ctypes.c_float(softcap), int(bool(out_f32)),
-        int(bool(single)), dtype_code(q.dtype), _stream()), "attention_plain")
+        int(bool(single)), _ptr(q_start), requests, dtype_code(q.dtype), _stream()), "attention_plain")
     return out
 
 
@@ -861,7 +863,8 @@ def attention(q, cache_k, cache_v, ctx, group, n_q, n_kv, head_dim, window, scal
                             sink=sink if sink is not None else (_zero_sinks(q.device, n_q) if sink_one else None))
     return attention_plain(q, cache_k, cache_v, ctx.row_req, ctx.row_pos, group.block_table, n_q, n_kv, head_dim,
                            window, scale, keep_first=keep_first, sink_one=sink_one, sink=sink, dist_bias=dist_bias,
-                           softcap=softcap, out_f32=out_f32, single=ctx.max_q_len == 1)
+                           softcap=softcap, out_f32=out_f32, single=ctx.max_q_len == 1, q_start=ctx.q_start,
+                           requests=ctx.n_requests)
 
 
 _zero_sink_cache: dict = {}

@@ -1,5 +1,7 @@
 """The plain kernels at the edges of their tiles: every variant a size picks, against 64-bit, and rows that do not
 depend on the batch they come in."""
+from types import SimpleNamespace
+
 import numpy as np
 import pytest
 import torch
@@ -122,3 +124,53 @@ def test_attention_rows_keep_infinities_and_nans_to_the_rows_that_see_them():
     assert bool(heads[:, :2, 5].isnan().all()) and bool((heads[:, :2, 9] == float("inf")).all())
     assert not bool(heads[:, 2:].any())      # a denominator that is no positive number leaves zeros, as the other kernel does
     assert torch.equal(heads[:, :2, 10:], before[:, :2, 10:])
+
+
+def step_of(requests):
+    """(rows' requests, rows' positions, the requests' first rows and the number of all) of requests (held, new)"""
+    t = lambda a: torch.from_numpy(np.asarray(a, dtype=np.int32)).to(DEV)  # noqa: E731
+    return (t(np.concatenate([np.full(new, r) for r, (_, new) in enumerate(requests)])),
+            t(np.concatenate([np.arange(n - new, n) for n, new in requests])), t(np.cumsum([0] + [new for _, new in requests])))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_q,n_kv,d,requests", [
+    (2, 2, 64, [(40, 1)] * 3 + [(90, 33)] + [(70, 1)] * 17 + [(20, 16)] + [(65, 2)] * 15),      # tiles of 8 tokens; 37 requests
+    (16, 16, 64, [(40, 5)] * 60 + [(130, 70)]),                                                  # of 16
+    (6, 3, 128, [(33, 1), (300, 300), (31, 1), (64, 64)]),                                       # of 8 and 4
+    (7, 1, 64, [(50, 1), (80, 80), (90, 1)]), (20, 2, 32, [(50, 3), (30, 1), (90, 2)])])         # of one token
+def test_requests_in_tiles_of_their_own_change_no_bit(n_q, n_kv, d, requests, dtype):
+    rng = np.random.default_rng(n_q * d)
+    ck, cv, bt, _ = paged(rng, [n for n, _ in requests], n_kv, d, 16, dtype)
+    req, pos, q_start = step_of(requests)
+    q = torch.from_numpy(rng.standard_normal((len(pos), n_q * d)).astype(np.float32)).to(DEV).to(dtype)
+    run = lambda **k: ops().attention_plain(q, ck, cv, req, pos, bt, n_q, n_kv, d, 0, d ** -0.5, **k)  # noqa: E731
+    together = run()
+    assert torch.equal(run(out=torch.full_like(together, float("nan")), q_start=q_start, requests=len(requests)), together)
+    ops().take_device_errors()
+
+
+@pytest.mark.parametrize("n_q,n_kv", [(8, 8), (16, 8)])
+def test_single_tokens_beside_a_portion_do_not_wait_for_one_another(n_q, n_kv):
+    rng, d = np.random.default_rng(1), 64
+    singles, portion = [(3000, 1)] * 16, [(64, 64)]
+    ck, cv, bt, _ = paged(rng, [n for n, _ in singles + portion], n_kv, d, 16, torch.float32)
+
+    def time_of(requests):
+        req, pos, q_start = step_of(requests)
+        q = torch.randn(len(pos), n_q * d, device=DEV)
+        ctx = SimpleNamespace(row_req=req, row_pos=pos, q_start=q_start, n_requests=len(requests), max_q_len=max(n for _, n in requests),
+                              q_lens=[n for _, n in requests])
+        run = lambda: ops().attention(q, ck, cv, ctx, SimpleNamespace(block_table=bt), n_q, n_kv, d, 0, 0.125)  # noqa: E731
+        times = []
+        for _ in range(8):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            run()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    # one after another the sixteen would take many times what they take as a step of their own
+    assert time_of(singles + portion) <= 2.5 * time_of(singles) + time_of(portion)
