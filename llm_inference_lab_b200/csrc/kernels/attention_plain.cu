@@ -432,8 +432,8 @@ __global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsPa
 template <typename T, int D, int PARTS, int WPG>
 int launch_rows(RowsParams p, cudaStream_t stream) {
   const int smem = rows_smem<T>(p.d, PARTS, WPG);
-  const cudaError_t e = cudaFuncSetAttribute(attention_rows_kernel<T, D, PARTS, WPG>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)attention_rows_kernel<T, D, PARTS, WPG>, smem);
   if (e != cudaSuccess) return (int)e;
   if (p.tile_tokens == 1) p.q_start = nullptr;
   // with the requests' borders: every request may end in a tile that is not full

@@ -11,6 +11,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #define LAB_EXPORT extern "C" __attribute__((visibility("default")))
 
 enum LabDtype : int { LAB_F32 = 0, LAB_BF16 = 1 };
@@ -222,6 +225,27 @@ static inline cudaError_t lab_launch(void (*kernel)(KArgs...), dim3 grid, dim3 b
   cfg.attrs = attr;
   cfg.numAttrs = g_lab_pdl ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Lets a kernel take `bytes` of dynamic shared memory.  The driver is asked once per kernel, device and largest size:
+// `granted`, one per kernel (a static of its launcher), remembers what was asked for, and smaller launches need no more.
+struct LabShared {
+  static constexpr int kDevices = 16;      // (beyond: asked at every launch)
+  std::atomic<int> bytes[kDevices] = {};
+};
+static inline cudaError_t lab_allow_shared(LabShared& granted, const void* kernel, size_t bytes) {
+  if (bytes <= 48 * 1024) return cudaSuccess;
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const bool kept = device < LabShared::kDevices;
+  if (kept && granted.bytes[device].load(std::memory_order_acquire) >= (int)bytes) return cudaSuccess;
+  static std::mutex asking;      // a smaller size must not be set after a larger one
+  std::lock_guard<std::mutex> lock(asking);
+  if (kept && granted.bytes[device].load(std::memory_order_acquire) >= (int)bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  if (e == cudaSuccess && kept) granted.bytes[device].store((int)bytes, std::memory_order_release);
+  return e;
 }
 
 // Reads the error word of this library and clears it.  Synchronises the device.

@@ -643,8 +643,9 @@ template <int R, int NC, int MODE>
 int launch_walk_as(const WalkParams& p, int requests, int vs, cudaStream_t stream) {
   const size_t smem = (size_t)3 * (CT * (record_floats(R) + vs + 2) + (CT / BLK) * COEF) * sizeof(float);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(delta_walk_kernel<R, NC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)delta_walk_kernel<R, NC, MODE>, smem);
+  if (e != cudaSuccess) return (int)e;
   const int segments = MODE == WALK_WHOLE ? 1 : MODE == WALK_CLOSE ? p.segments - 1 : p.segments;
   dim3 grid((p.V + vs - 1) / vs + (MODE == WALK_CLOSE && p.segments > 2 ? (p.D + vs - 1) / vs : 0), p.H, requests * segments);
   return (int)lab_launch(delta_walk_kernel<R, NC, MODE>, grid, dim3(PARTS * vs / NC + HELPERS), smem, stream, p, vs);
@@ -653,7 +654,8 @@ int launch_walk_as(const WalkParams& p, int requests, int vs, cudaStream_t strea
 template <int PRE>
 int launch_fold_as(const WalkParams& p, int requests, cudaStream_t stream) {
   const int smem = (2 * p.D * FOLD_V + FOLD_ROWS * (p.D + 4)) * (int)sizeof(float);
-  const cudaError_t e = cudaFuncSetAttribute(delta_fold_kernel<PRE>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)delta_fold_kernel<PRE>, smem);
   if (e != cudaSuccess) return (int)e;
   return (int)lab_launch(delta_fold_kernel<PRE>, dim3((p.V + FOLD_V - 1) / FOLD_V, p.H, requests), dim3(256), smem, stream, p);
 }

@@ -576,11 +576,9 @@ int launch_few_rows_as(void* out, const void* x, const void* w, const void* bias
                        int act, float gate_limit, cudaStream_t stream) {
   constexpr int cols = 8 * (4 / WR);
   const size_t smem = sizeof(float) * FR_STAGES * ((GATED ? 2 : 1) * cols + WR * MR) * (STAGE_K + 4);
-  if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_few_rows_kernel<GATED, MR, WR>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)gemm_few_rows_kernel<GATED, MR, WR>, smem);
+  if (e != cudaSuccess) return (int)e;
   return (int)lab_launch(gemm_few_rows_kernel<GATED, MR, WR>, dim3((N + cols - 1) / cols), dim3(128), smem, stream,
                          (float*)out, (const float*)x, (const float*)w, (const float*)bias, M, N, K, ldx, ldo, act,
                          gate_limit);
@@ -606,7 +604,8 @@ int launch_tile(void* out, const void* x, const void* w, const void* bias, int M
   using Shape = TileShape<T, MI>;
   constexpr int cols = GATED ? Shape::COLS / 2 : Shape::COLS;
   const auto kernel = gemm_plain_kernel<T, OutT, GATED, MI, VEC>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Shape::BYTES);
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)kernel, Shape::BYTES);
   if (e != cudaSuccess) return (int)e;
   constexpr int most = 65534 * Shape::ROWS;      // rows of a launch: the grid's limit, whole tiles of groups
   for (int m0 = 0; m0 < M; m0 += most) {

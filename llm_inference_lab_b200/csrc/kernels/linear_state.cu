@@ -437,8 +437,9 @@ __global__ void __launch_bounds__(kThreads) gated_norm_kernel(T* __restrict__ ou
 template <int R, int MODE>
 int launch_scan_as(const ScanParams& p, int requests, int vs, cudaStream_t stream) {
   const size_t smem = (size_t)3 * SCAN_CT * (2 * SCAN_P * (R + 4) + vs + 4) * sizeof(float);
-  if (smem > 48 * 1024)
-    cudaFuncSetAttribute(decay_scan_kernel<R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)decay_scan_kernel<R, MODE>, smem);
+  if (e != cudaSuccess) return (int)e;
   const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
   dim3 grid((p.V + vs - 1) / vs, p.H, requests * segments);
   return (int)lab_launch(decay_scan_kernel<R, MODE>, grid, dim3(2 * SCAN_P * vs), smem, stream, p);

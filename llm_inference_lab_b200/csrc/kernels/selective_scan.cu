@@ -408,11 +408,9 @@ int launch_scan_as(void* out, const void* a_log, const void* skip, const void* d
                    cudaStream_t stream) {
   constexpr int WC = WTHREADS / WL;
   const size_t smem = sizeof(float) * ((size_t)2 * scan_chunk_floats(WC, (p.N + 3) & ~3) + WT * WC + WT * WTHREADS);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(selective_scan_kernel<T, WL, R, MODE, QUADS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)selective_scan_kernel<T, WL, R, MODE, QUADS>, smem);
+  if (e != cudaSuccess) return (int)e;
   const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
   return (int)lab_launch(selective_scan_kernel<T, WL, R, MODE, QUADS>, dim3((p.channels + WC - 1) / WC, requests, segments),
                          dim3(WTHREADS), smem, stream, (T*)out, (const T*)a_log, (const T*)skip, (const T*)dt_bias, p);
