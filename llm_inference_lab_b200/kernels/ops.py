@@ -8,6 +8,7 @@ raises.  Tensors are torch tensors on the GPU; a kernel never allocates.
 from __future__ import annotations
 
 import ctypes
+import functools
 import threading
 
 import torch
@@ -95,8 +96,11 @@ def current_stream() -> "torch.cuda.Stream":
     return obj
 
 
+_NULL = ctypes.c_void_p(0)
+
+
 def _ptr(t) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+    return _NULL if t is None else ctypes.c_void_p(t.data_ptr())
 
 
 class _Counter:
@@ -641,6 +645,7 @@ def _pair_splits(T: int, n_out: int, K: int) -> int:
     return splits if splits >= 1 and 5 * tiles * splits >= 3 * pairs else 0
 
 
+@functools.lru_cache(maxsize=4096)
 def _gated_on_pairs(T: int, inter: int) -> bool:
     """Whether a gated product runs on pairs of SMs (256 tokens x 128 features per tile, gate rows in one CTA and up rows
     in the other) or on tiles of 128 tokens.  Pairs win once their tiles fill most of the 74 pairs, 6 to 12 % at the
@@ -649,6 +654,26 @@ def _gated_on_pairs(T: int, inter: int) -> bool:
     12.3 us; 7B, 300 tokens, four rounds against three: 93 against 86)."""
     pairs, tiles = -(-T // 256) * (-(-inter // 128)), -(-T // 128) * (-(-inter // 128))
     return pairs >= 64 and -(-pairs // (sm_count() // 2)) <= -(-tiles // sm_count())
+
+
+@functools.lru_cache(maxsize=4096)
+def _prefill_plan(T: int, n_out: int, K: int, partial: bool) -> tuple[str, int, int]:
+    """(kernel, N tile, K splits) of a product of more than 128 tokens whose consumer may sum partial products
+    (`partial`): "pair" and "tc" as in `_pick_prefill_tiles`, "swap" with features on the 128-row side.  Kept by the
+    sizes: a step's products are the same from layer to layer."""
+    pair_splits = _pair_splits(T, n_out, K) if partial else 0
+    if pair_splits > 1:
+        return "pair", 224, pair_splits
+    kind, bn, splits = _pick_prefill_tiles(T, n_out, K, partial)
+    if kind == "pair" or pair_splits:
+        return "pair", 256, 1
+    if splits > 1:
+        # features on the M side: the partial products leave in fewer, longer runs (0.5B down projection at 300
+        # tokens 13.9 against 15.9 us, at 512 14.5 against 16.3; 1.5B at 300 tokens 18.4 against 20.3)
+        return "swap", 128, splits
+    if bn == 128 and 2 * (-(-T // 128)) * (-(-n_out // 128)) <= sm_count():
+        bn = 64      # too few tiles for half of the SMs: twice as many (896 x 896 at 300 tokens 6.3 against 7.4 us)
+    return "tc", bn, 1
 
 
 def _tc_operands(x, w) -> bool:
@@ -687,19 +712,11 @@ def linear(x, w, bias=None, out_f32=False, allow_partial=False, out=None, act=No
         return gemm_plain(x, w, bias, out_f32=out_f32, out=out, gelu=gelu)
     T = x.shape[0]
     if T > 128:
-        partial = allow_partial and bias is None and out is None
-        pair_splits = _pair_splits(T, w.shape[0], x.shape[1]) if partial else 0
-        if pair_splits > 1:
-            return gemm_tc2(x, w, None, splits=pair_splits)
-        kind, bn, splits = _pick_prefill_tiles(T, w.shape[0], x.shape[1], partial)
-        if kind == "pair" or pair_splits:
-            return gemm_tc2(x, w, bias, out_f32=out_f32, out=out, gelu=gelu)
+        kind, bn, splits = _prefill_plan(T, w.shape[0], x.shape[1], allow_partial and bias is None and out is None)
+        if kind == "pair":
+            return gemm_tc2(x, w, None, splits=splits) if splits > 1 else gemm_tc2(x, w, bias, out_f32=out_f32, out=out, gelu=gelu)
         if splits > 1:
-            # features on the M side: the partial products leave in fewer, longer runs (0.5B down projection at 300
-            # tokens 13.9 against 15.9 us, at 512 14.5 against 16.3; 1.5B at 300 tokens 18.4 against 20.3)
-            return gemm_tc(x, w, None, swap=True, bn=128, splits=splits)
-        if kind == "tc" and bn == 128 and 2 * (-(-T // 128)) * (-(-w.shape[0] // 128)) <= sm_count():
-            bn = 64      # too few tiles for half of the SMs: twice as many (896 x 896 at 300 tokens 6.3 against 7.4 us)
+            return gemm_tc(x, w, None, swap=True, bn=bn, splits=splits)
         return gemm_tc(x, w, bias, out_f32=out_f32, swap=False, bn=bn, out=out, gelu=gelu)
     splits = _pick_splits(T, w.shape[0], x.shape[1]) if allow_partial and out is None else 1
     if splits > 1:
