@@ -452,7 +452,7 @@ int pick_rows(RowsParams p, bool single, cudaStream_t stream) {
     p.head_tiles = (group + rows - 1) / rows;
     return ((long long)p.tokens + p.tile_tokens - 1) / p.tile_tokens * p.head_tiles * p.n_kv;
   };
-  const bool wide = shape(2 * RW) >= 2 * 148;
+  const bool wide = shape(2 * RW) >= 2 * lab_sm_count();
   if (!wide) shape(RW);
   if (p.d == 64) return wide ? launch_rows<T, 64, 4, 2>(p, stream) : launch_rows<T, 64, 4, 1>(p, stream);
   if (p.d == 128) return wide ? launch_rows<T, 128, 4, 2>(p, stream) : launch_rows<T, 128, 4, 1>(p, stream);

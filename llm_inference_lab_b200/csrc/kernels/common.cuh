@@ -227,6 +227,19 @@ static inline cudaError_t lab_launch(void (*kernel)(KArgs...), dim3 grid, dim3 b
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
+// Streaming multiprocessors of the current device (148, a B200's, where it cannot be asked).
+static inline int lab_sm_count() {
+  static std::atomic<int> count{0};
+  int n = count.load(std::memory_order_relaxed);
+  if (n == 0) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess)
+      n = 148;
+    count.store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
 // Lets a kernel take `bytes` of dynamic shared memory.  The driver is asked once per kernel, device and largest size:
 // `granted`, one per kernel (a static of its launcher), remembers what was asked for, and smaller launches need no more.
 struct LabShared {

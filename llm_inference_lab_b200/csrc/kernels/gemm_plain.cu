@@ -627,8 +627,8 @@ int launch_tile(void* out, const void* x, const void* w, const void* bias, int M
 // multiprocessor has one, 0.57 where it has four).  517 x 896 x 4864: 155 us in tiles of 32, 176 of 16; 517 x 1152 x 896:
 // 47 and 43; 100 x 896 x 4864: 93 and 74.
 static inline bool flat_tiles(long long M, long long N, int batch) {
-  const long long columns = (N + 63) / 64 * batch;
-  return ((M + 15) / 16 * columns + 147) / 148 * 54 < ((M + 31) / 32 * columns + 147) / 148 * 100;
+  const long long columns = (N + 63) / 64 * batch, sms = lab_sm_count();
+  return ((M + 15) / 16 * columns + sms - 1) / sms * 54 < ((M + 31) / 32 * columns + sms - 1) / sms * 100;
 }
 
 template <typename T, typename OutT>
