@@ -247,7 +247,7 @@ struct LabShared {
   std::atomic<int> bytes[kDevices] = {};
 };
 static inline cudaError_t lab_allow_shared(LabShared& granted, const void* kernel, size_t bytes) {
-  if (bytes <= 48 * 1024) return cudaSuccess;
+  if (bytes <= 40 * 1024) return cudaSuccess;      // (48 KB without asking, a kernel's static shared memory among them)
   int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return e;
