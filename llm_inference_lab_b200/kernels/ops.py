@@ -646,14 +646,17 @@ def _pair_splits(T: int, n_out: int, K: int) -> int:
 
 
 @functools.lru_cache(maxsize=4096)
-def _gated_on_pairs(T: int, inter: int) -> bool:
+def _gated_on_pairs(T: int, inter: int, K: int = 2048) -> bool:
     """Whether a gated product runs on pairs of SMs (256 tokens x 128 features per tile, gate rows in one CTA and up rows
-    in the other) or on tiles of 128 tokens.  Pairs win once their tiles fill most of the 74 pairs, 6 to 12 % at the
-    0.5B, 1.5B and 7B layer sizes (2,048 tokens: 31.7 against 33.7, 76 against 85, 349 against 385 us), unless the
-    smaller tiles take fewer rounds: 76 pair tiles are two rounds, 114 small ones are one (0.5B, 300 tokens: 15.7 against
-    12.3 us; 7B, 300 tokens, four rounds against three: 93 against 86)."""
+    in the other) or on tiles of 128 tokens: the kind whose rounds take less time, once pairs fill most of the 74 pairs of
+    SMs.  A round of pairs takes 0.83 to 0.93 of one of small tiles where K is 1,536 or 3,584 (here 0.9), so it may be one
+    more of eleven (us, weights from memory: 7B 2,176 tokens 392 in 18 rounds against 445 in 17, 1.5B 2,432 tokens 93 in 10
+    against 99 in 9) but not two of one (0.5B 300 tokens 22.5 against 20.5; 7B 300 tokens 96 in 4 against 91 in 3).  With
+    K 896 the fixed part of a tile counts for more and a round takes as long either way: the fewer rounds (2,432 tokens 48
+    in 6 against 42 in 5; 411 tokens 22.5 in 2 against 24.6 in 2)."""
     pairs, tiles = -(-T // 256) * (-(-inter // 128)), -(-T // 128) * (-(-inter // 128))
-    return pairs >= 64 and -(-pairs // (sm_count() // 2)) <= -(-tiles // sm_count())
+    cost = 0.9 if K >= 1280 else 1.0
+    return pairs >= 64 and -(-pairs // (sm_count() // 2)) * cost <= -(-tiles // sm_count())
 
 
 @functools.lru_cache(maxsize=4096)
@@ -730,7 +733,7 @@ def linear_gated(x, w_gate_up, limit: float = 0.0, act: str = "silu"):
     g' * sigmoid(1.702 g') * (u' + 1)."""
     if x.dtype == torch.float32 or _force_plain or not _tc_operands(x, w_gate_up):
         return gemm_plain(x, w_gate_up, None, gated=True, gate_limit=limit, gate_act=act)
-    if _gated_on_pairs(x.shape[0], w_gate_up.shape[0] // 2):
+    if _gated_on_pairs(x.shape[0], w_gate_up.shape[0] // 2, x.shape[1]):
         return gemm_tc2(x, w_gate_up, None, gated=True, gate_limit=limit, gate_act=act)
     return gemm_tc(x, w_gate_up, None, gated=True, gate_limit=limit, gate_act=act)
 

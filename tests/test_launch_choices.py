@@ -90,3 +90,17 @@ def test_segments_of_recurrences_cover_the_cases_they_were_measured_on():
     assert ops.scan_segments(56, 319) == 1 and ops.scan_segments(1, 5000) == 32
     assert ops.decay_scan_segments(84, 1000, 2) == 7 and ops.decay_scan_segments(168, 500, 4) == 1
     assert ops.decay_scan_segments(42, 449, 1) == 1 and ops.decay_scan_segments(60, 2048, 1, 128) == 7
+
+
+def test_gated_products_take_the_kind_of_tile_whose_rounds_take_less_time():
+    """By the measured costs of a round (pairs of SMs 0.9 of the small tiles' where K is long, the same where it is short),
+    for every number of tokens."""
+    for K, inter, cost in ((896, 4864, 1.0), (1536, 8960, 0.9), (3584, 18944, 0.9)):
+        for T in range(129, 16385):
+            pairs, small = -(-T // 256) * (inter // 128), -(-T // 128) * (inter // 128)
+            if pairs >= 64:
+                assert ops._gated_on_pairs(T, inter, K) == (cost * -(-pairs // 74) <= -(-small // 148)), (K, T)
+    # seen to be faster on pairs, in one round more than the small tiles take
+    assert all(ops._gated_on_pairs(T, 18944, 3584) for T in (1408, 1664, 2176, 2432, 4224))
+    assert all(ops._gated_on_pairs(T, 8960, 1536) for T in (2432, 2944, 4224))
+    assert not any(ops._gated_on_pairs(T, 4864, 896) for T in (300, 1408, 2432, 2944, 9856))
