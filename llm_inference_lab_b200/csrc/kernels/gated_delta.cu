@@ -44,6 +44,7 @@ constexpr int PARTS = 4;        // threads that share one column of the state
 constexpr int BLK = 4;          // rows of a block
 constexpr int LONG_WALK = 256;  // rows from which the next kernel is let in at the walk's end only
 constexpr int CT = 16;          // rows staged per chunk
+constexpr int SEGMENT_SHARE = 32;      // rows of a column a thread keeps where segments are built: up to 128 key channels
 constexpr int HELPERS = 64;     // threads that copy chunks ahead and form the blocks' coefficients
 constexpr int DOTS = 8;         // q . k_0..3, k . k_0..2 of a row's block, one unused
 // coefficients of a block: rates, rates times G, three rows of the substitution, four of the outputs, g_3j, G
@@ -663,11 +664,12 @@ int launch_fold_as(const WalkParams& p, int requests, cudaStream_t stream) {
 template <int R, int NC>
 int launch_walk(const WalkParams& p, int requests, int vs, cudaStream_t stream) {
   if (p.segments <= 1) return launch_walk_as<R, NC, WALK_WHOLE>(p, requests, vs, stream);
-  int e = launch_walk_as<R, NC, WALK_CLOSE>(p, requests, vs, stream);
-  if (e == 0 && p.segments > 2)
-    e = p.D <= 64 ? launch_fold_as<16>(p, requests, stream)
-                  : p.D <= 128 ? launch_fold_as<32>(p, requests, stream) : launch_fold_as<64>(p, requests, stream);
-  return e != 0 ? e : launch_walk_as<R, NC, WALK_OUTPUT>(p, requests, vs, stream);
+  if constexpr (NC == 2 && R <= SEGMENT_SHARE) {
+    int e = launch_walk_as<R, NC, WALK_CLOSE>(p, requests, vs, stream);
+    if (e == 0 && p.segments > 2) e = p.D <= 64 ? launch_fold_as<16>(p, requests, stream) : launch_fold_as<32>(p, requests, stream);
+    return e != 0 ? e : launch_walk_as<R, NC, WALK_OUTPUT>(p, requests, vs, stream);
+  }
+  return (int)cudaErrorInvalidValue;
 }
 
 template <int R>
@@ -705,7 +707,7 @@ LAB_EXPORT int lab_delta_prepare(float* rec, float* v, float* decay, float* rate
 // vs: columns of the state a CTA takes (a multiple of 8 * cols, at most 32 * cols); cols: columns a thread takes (1, or
 // up to 128 key channels 2).
 // kept (with proj, ld, keep, channels): the inputs that replace a request's kept ones; null: none.
-// segments > 1: every request's rows are cut into at most that many; `states` [requests, segments, H, D, V] and, for more
+// segments > 1 (up to 128 key channels, two columns a thread): every request's rows are cut into at most that many; `states` [requests, segments, H, D, V] and, for more
 // than two, `moves` [requests, segments, H, D, D] are scratch.
 LAB_EXPORT int lab_delta_walk(float* out, const float* rec, const float* v, const float* decay, const float* rate,
                               float* state, const int* q_start, const int* state_slot, int tokens, int requests,

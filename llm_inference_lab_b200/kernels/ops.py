@@ -1144,10 +1144,10 @@ def delta_walk(rec: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, rate: to
         assert proj.dtype == torch.float32 and proj.stride(1) == 1 and proj.shape[0] == tokens and proj.shape[1] >= channels
     out = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=v.device)
     pairs = ctx.n_requests * heads
-    segments = delta_walk_segments(pairs, keys, vdim, ctx.max_q_len) if shape is None else 1
+    segments = delta_walk_segments(pairs, keys, vdim, ctx.max_q_len) if shape is None and keys <= 128 else 1
     vs, cols = shape if shape is not None else delta_walk_shape(pairs, keys, vdim, ctx.max_q_len)
     if segments > 1:
-        vs, cols = (min(64, -(-vdim // 16) * 16), 2) if keys <= 128 else (min(vs, 32), 1)
+        vs, cols = min(64, -(-vdim // 16) * 16), 2
     states = moves = None
     if segments > 1:
         scratch, (states, moves) = _segment_scratch(v.device, pairs * segments * keys * vdim,
@@ -1167,7 +1167,7 @@ def delta_walk_segments(pairs: int, keys: int, vdim: int, longest: int) -> int:
     CTA.  Measured with the mixer around it, 64 x 64 states: 14 pairs and 2,048 tokens 363 us in one piece, 237 in 4, 201
     in 6, 213 in 8; 28 pairs and 700 tokens 155, 128 in 4, 137 in 5; 56 pairs and 500 tokens 188, 154 in 2, 188 in 3; 112
     pairs and 250 tokens 116, 142 in 2; 14 pairs and 300 tokens 72, 71 in 4.  128 x 128: 12 pairs and 2,048 tokens 603,
-    412 in 4; 24 pairs and 300 tokens 116, 139 in 2.  One request's mixer launched kernel by kernel is bound by the host up to
+    412 in 4; 24 pairs and 300 tokens 116, 139 in 2.  Beyond 128 key channels the walk is built in one piece only.  One request's mixer launched kernel by kernel is bound by the host up to
     600 tokens (420: 86 us in one piece, 102 in segments)."""
     if longest < (600 if pairs < 42 else 400) or keys > 128:
         return 1

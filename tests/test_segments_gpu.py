@@ -119,6 +119,7 @@ def test_running_maximum_of_any_length(heads):
 
 
 @pytest.mark.parametrize("segments", [1, 2, 3, 5, 9])
+# (200 key channels: in one piece whatever the rule says)
 @pytest.mark.parametrize("heads,groups,keys,vdim", [(4, 2, 64, 64), (3, 1, 20, 36), (2, 2, 128, 100), (1, 1, 200, 24), (2, 1, 16, 130)])
 def test_delta_walk_segments(heads, groups, keys, vdim, segments, monkeypatch):
     monkeypatch.setattr(ops(), "delta_walk_segments", lambda *a: segments)
