@@ -174,3 +174,92 @@ def test_single_tokens_beside_a_portion_do_not_wait_for_one_another(n_q, n_kv):
 
     # one after another the sixteen would take many times what they take as a step of their own
     assert time_of(singles + portion) <= 2.5 * time_of(singles) + time_of(portion)
+
+
+# tiles of sixteen rows (taken once they fill the multiprocessors twice): every build of them, heads in one tile and in two
+WIDE = [
+    (16, 8, 128, [(200, 200), (130, 110), (33, 1)]),
+    (12, 4, 96, [(300, 280), (120, 119), (40, 1)]),
+    (8, 8, 40, [(500, 480), (150, 130), (10, 1)]),
+    (8, 8, 200, [(400, 400), (330, 219), (64, 1)]),
+    (40, 2, 256, [(90, 70), (60, 20), (33, 1)]),
+    (34, 2, 64, [(90, 70), (60, 20), (33, 1)]),
+]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n_q,n_kv,d,requests", WIDE)
+def test_attention_in_tiles_of_sixteen_rows(n_q, n_kv, d, requests, dtype):
+    group, T = n_q // n_kv, sum(new for _, new in requests)
+    assert -(-T // max(1, 16 // group)) * -(-group // 16) * n_kv >= 2 * ops().sm_count()
+    rng = np.random.default_rng(d)
+    ck, cv, bt, held = paged(rng, [n for n, _ in requests], n_kv, d, 16, dtype)
+    req, pos, q_start = step_of(requests)
+    q = torch.from_numpy(rng.standard_normal((T, n_q * d)).astype(np.float32)).to(DEV).to(dtype)
+    run = lambda q, req, pos, **k: ops().attention_plain(q, ck, cv, req, pos, bt, n_q, n_kv, d, 0, d ** -0.5, **k)  # noqa: E731
+    full = run(q, req, pos, q_start=q_start, requests=len(requests))
+    ops().take_device_errors()
+    at, want = 0, []
+    for (n, new), (k, v) in zip(requests, held):
+        k, v = (torch.from_numpy(a).to(DEV).to(dtype).double().repeat_interleave(group, 1) for a in (k, v))
+        scores = torch.einsum("qhd,khd->hqk", q[at: at + new].double().view(new, n_q, d), k) * d ** -0.5
+        ahead = torch.arange(n, device=DEV)[None, :] > torch.arange(n - new, n, device=DEV)[:, None]
+        want.append(torch.einsum("hqk,khd->qhd", torch.softmax(scores.masked_fill(ahead, -torch.inf), -1), v).reshape(new, -1))
+        at += new
+    want = torch.cat(want)
+    assert float((full.double() - want).norm() / want.norm()) < (2e-6 if dtype == torch.float32 else 4e-3)
+    for i in (0, T // 3, T // 2, T - 2, T - 1):      # a row alone, in a tile of eight
+        assert torch.equal(run(q[i: i + 1], req[i: i + 1], pos[i: i + 1], single=True)[0], full[i])
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_product_of_more_rows_than_a_grid_has_tiles(gated):
+    M, N, K = 65534 * 32 + 45, 3, 4
+    g = torch.Generator(device=DEV).manual_seed(0)
+    x, w = torch.randn(M, K, device=DEV, generator=g), torch.randn(2 * N if gated else N, K, device=DEV, generator=g)
+    full = ops().gemm_plain(x, w, gated=gated)
+    for a, b in ((0, 500), (65534 * 32 - 300, 65534 * 32), (65534 * 32 - 33, M), (65534 * 32, M)):
+        assert torch.equal(full[a:b], ops().gemm_plain(x[a:b], w, gated=gated))
+    want = x @ w.T
+    if gated:
+        want = torch.nn.functional.silu(want[:, :N]) * want[:, N:]
+    assert torch.allclose(full, want, rtol=1e-4, atol=1e-5)      # (every row is there, to 32-bit roundings)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_convolution_of_many_rows(dtype):
+    """From 1,500,000 entries on a thread takes eight rows: bit for bit what a thread a row gives, at requests' borders inside
+    an eight, with the inputs kept from earlier steps, rows of padding and a last eight that is not full."""
+    lens, slots, taps, channels = [1, 2, 3, 8, 5, 700, 16, 1, 400, 4, 300, 1], [7, 0, 2, 9, 1, 3, -1, 4, 8, -1, 5, 6], 4, 1100
+    g, T = torch.Generator(device=DEV).manual_seed(4), sum(lens)
+    assert T * channels >= 1500000 > T * (channels // 4) and T % 8
+    t = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    ctx = SimpleNamespace(row_req=t(np.repeat(np.arange(len(lens)), lens).tolist()), q_start=t([0] + np.cumsum(lens).tolist()),
+                          state_slot=t(slots), n_requests=len(lens), n_tokens=T, max_q_len=max(lens))
+    proj = torch.randn(T, channels + 24, device=DEV, generator=g)
+    w, b = (torch.randn(channels, taps, device=DEV, generator=g) * 0.5).to(dtype), torch.randn(channels, device=DEV, generator=g).to(dtype)
+    kept = torch.randn(10, taps - 1, channels, device=DEV, generator=g)
+    many = kept.clone()
+    out, rounded = ops().conv_silu(proj, 8, channels, taps, w, b, many, ctx)
+    part = channels // 4
+    for c in range(0, channels, part):
+        few = kept[:, :, c: c + part].contiguous()
+        small, small_rounded = ops().conv_silu(proj, 8 + c, part, taps, w[c: c + part].contiguous(), b[c: c + part].contiguous(), few, ctx)
+        assert torch.equal(out[:, c: c + part], small) and torch.equal(rounded[:, c: c + part], small_rounded)
+        assert torch.equal(many[:, :, c: c + part], few)
+    ops().take_device_errors()
+    at = 0
+    for n, slot in zip(lens, slots):
+        if slot < 0:
+            assert not bool(out[at: at + n].any()) and not bool(rounded[at: at + n].any())
+        else:
+            u = torch.cat([kept[slot], proj[at: at + n, 8: 8 + channels]]).double()
+            want = torch.nn.functional.silu(sum(u[j: j + n] * w[:, j].double() for j in range(taps)) + b.double())
+            # five roundings of sums of a few units, and the exponential's
+            assert float((out[at: at + n].double() - want).abs().max()) < 1e-5
+            assert torch.equal(many[slot].double(), u[-(taps - 1):])
+        at += n
+    ctx.state_slot = t([10] + slots[1:])
+    ops().conv_silu(proj, 8, channels, taps, w, b, many.clone(), ctx)
+    with pytest.raises(ops().KernelError):
+        ops().take_device_errors()
