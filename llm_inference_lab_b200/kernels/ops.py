@@ -1173,7 +1173,8 @@ def delta_walk_segments(pairs: int, keys: int, vdim: int, longest: int) -> int:
         return 1
     values, moves = -(-vdim // 64), -(-keys // 64)
     segments = 1 + (sm_count() + pairs * moves) // (pairs * (values + moves))
-    return max(1, min(segments, sm_count() // max(1, pairs * values)))
+    segments = min(segments, sm_count() // max(1, pairs * values))
+    return segments if segments > 2 else 1
 
 
 def delta_walk_shape(pairs: int, keys: int, vdim: int, max_q_len: int) -> tuple[int, int]:

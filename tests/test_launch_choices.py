@@ -84,7 +84,7 @@ def test_pair_splits_and_gated_tiles_cover_the_cases_they_were_measured_on():
 
 def test_segments_of_recurrences_cover_the_cases_they_were_measured_on():
     walk = ops.delta_walk_segments
-    assert [walk(14, 64, 64, 2048), walk(28, 64, 64, 700), walk(56, 64, 64, 500), walk(112, 64, 64, 500)] == [6, 4, 2, 1]
+    assert [walk(14, 64, 64, 2048), walk(28, 64, 64, 700), walk(56, 64, 64, 500), walk(112, 64, 64, 500)] == [6, 4, 1, 1]
     assert walk(12, 128, 128, 2048) == 4 and walk(14, 64, 64, 300) == 1 and walk(14, 256, 64, 2048) == 1
     assert ops.scan_segments(56, 2048) == 11 and ops.scan_segments(112, 700) == 5 and ops.scan_segments(448, 250) == 1
     assert ops.scan_segments(56, 319) == 1 and ops.scan_segments(1, 5000) == 32
