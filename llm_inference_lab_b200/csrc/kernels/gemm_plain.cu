@@ -8,8 +8,10 @@
 // The sum over k is taken in four parts: blocks of 16 k's go to the parts in turn, a part
 // runs over its blocks in ascending order, even and odd k's apart, with one fused
 // multiply-add per term; a part is even + odd, the parts are added as (0 + 1) + (2 + 3).
-// Every kernel and tile of the product takes it so, whatever the number of rows: an output
-// element does not depend on how the rows were batched.  Formulas:
+// The kernel for few rows and the tiles take it so, whatever the number of rows: an output
+// element does not depend on how the rows were batched.  (Two kernels for few rows take lanes
+// over k and a shuffle tree: a batch of heads of up to 16 rows, and grouped rows of a decode
+// step.  Their elements differ from the tiles' by 32-bit roundings.)  Formulas:
 // rust/engine/src/runner/model/qwen2/kernels.rs:156-178, 393-418 (linear, bias in 32-bit,
 // one rounding), 422-448 (gate/up with the SiLU product), 1469-1486 (SiLU).
 #include <type_traits>
@@ -61,8 +63,8 @@ __device__ __forceinline__ Quad load_quad(const __nv_bfloat16* p) {
 // keeps MI rows, 4 apart, by 8 columns, 8 apart.
 //
 // What bounds it: multiply-adds, of which a warp's 8 x 8 products a lane reach half of the units' rate (37 of 74
-// TFLOP/s, the pipe 52 % busy, loads from shared memory at 48 % of their rate; larger tiles a lane or a CTA, one
-// multiply-add an instruction, or more warps a multiprocessor did not pass that).  The four warps are what spreads an
+// TFLOP/s, the pipe 51 % busy, six warps a multiprocessor that wait for their own results; larger tiles a lane or a CTA,
+// one multiply-add an instruction, or more warps a multiprocessor did not pass that).  The four warps are what spreads an
 // output of few tiles over the multiprocessors' four schedulers.  Operands lie in shared memory as they lie in memory,
 // row by row, rows an odd number of 16-byte units apart (no bank conflicts), and come by cp.async through a ring of
 // STAGES stages of 64 k's: copies in flight cost no registers and are waited for in their order.  VEC: rows are whole
@@ -260,8 +262,8 @@ __global__ void __launch_bounds__(PARTS * 32) gemm_plain_kernel(
 
 // Per-head products for few tokens (a decode step): out[t, h, n] = sum_k w[h, n, k] * x[t, h, k].  A warp
 // forms one output column for every token: it reads the weight row once, lanes over k, and finishes each
-// token's sum with a shuffle tree; the tokens' inputs of the head wait in shared memory.  The 64 x 64 tiles
-// above walk K in steps of 16 behind a barrier each, which costs a memory latency per step.
+// token's sum with a shuffle tree; the tokens' inputs of the head wait in shared memory.  The tiles above walk K in
+// stages of 64 behind a barrier each, for 16 rows or more.
 constexpr int HF_TOKENS = 16;
 template <typename T, typename OutT>
 __global__ void __launch_bounds__(256) gemm_heads_few_kernel(OutT* __restrict__ out, const T* __restrict__ x,
@@ -301,8 +303,8 @@ int launch_heads_few(void* out, const void* x, const void* w, int M, int N, int 
                          head_x, head_o);
 }
 
-// Grouped rows for few rows (a decode step's pairs of token and expert): the tiles above would walk K in steps
-// of 16 behind a barrier each for a handful of live rows.  Here a CTA takes one tile of the layout and 16 (gated)
+// Grouped rows for few rows (a decode step's pairs of token and expert): the tiles above would walk K in stages
+// of 64 behind a barrier each for a handful of live rows.  Here a CTA takes one tile of the layout and 16 (gated)
 // or 32 output columns; a warp reads its four weight rows once, 16 bytes a lane where the rows allow it, for up
 // to GF_ROWS live rows of the tile, whose inputs wait in shared memory in 32-bit; each row's sums close with a
 // shuffle tree.  More live rows take further passes.  Rows whose source is -1 stay unwritten.

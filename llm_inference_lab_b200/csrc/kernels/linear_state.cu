@@ -98,9 +98,8 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
 // Walkers (the first SCAN_P * Vs threads): thread (j, part) keeps rows part * R .. part * R + R - 1 of column
 // slice * Vs + j of the state in registers (R a multiple of 4: the rows' keys and queries come from shared
 // memory four at a time; the four threads' shares of a token's keys lie R + 4 floats apart, which spreads
-// their 16-byte loads over the banks).  A token costs a walker 3 R / 2 instructions on two rows each behind R / 2 loads; the four
-// walkers of a column add their shares of the output by two shuffles.  The next token's keys, queries and
-// value are loaded before the current token's arithmetic (up to R = 16; beyond, registers do not allow it).
+// their 16-byte loads over the banks).  A token costs a walker 3 R / 2 instructions on two rows each behind R / 2 loads;
+// the four walkers of a column add their shares of four tokens' outputs by three shuffles together.
 // The walk of a segment is one dependent chain: its time is the number of tokens times that step, whatever the number
 // of CTAs, so nothing else may sit on it.  (A launch for the closing states forms no outputs: no queries, two thirds
 // of the instructions.)

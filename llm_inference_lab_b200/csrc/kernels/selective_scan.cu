@@ -210,8 +210,9 @@ __host__ __device__ inline int scan_chunk_floats(int wc, int n4) { return 3 * WT
 // there are CTAs enough, is the issue of instructions: most of an entry's and token's are its exponential's, the others
 // take two entries each; a token of a CTA also takes its step sizes, gates and copies.  Measured on a B200, inputs from
 // memory, 1,792 channels of 16 entries: 8 requests of 250 tokens 84 us (115 with eight lanes a channel and an entry an
-// instruction); one of 2,048 131 us in eleven segments (352 in one piece of that form).  QUADS: the state is whole quads; else the entries that fill
-// the last one are kept at zero (an infinite step would leave no numbers there).
+// instruction); one of 2,048 131 us in eleven segments (352 in one piece of that form), issuing in two cycles of three.
+// QUADS: the state is whole quads; else the entries that fill the last one are kept at zero (an infinite step would leave
+// no numbers there).
 template <typename T, int WL, int R, int MODE, bool QUADS>
 __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict__ out, const T* __restrict__ a_log,
                                                                   const T* __restrict__ skip,
