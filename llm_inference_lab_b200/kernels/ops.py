@@ -1164,17 +1164,18 @@ def delta_walk_segments(pairs: int, keys: int, vdim: int, longest: int) -> int:
     """Into how many segments `delta_walk` cuts a request's rows, walked by CTAs of 64 columns, two a thread.  The launch
     for the closing states has slices for the identity's columns beside the values' (but for the first segment), and
     after it the opening states follow one by one, so segments pay over long portions while both launches find an SM per
-    CTA.  Measured with the mixer around it, 64 x 64 states: 14 pairs and 2,048 tokens 363 us in one piece, 237 in 4, 201
-    in 6, 213 in 8; 28 pairs and 700 tokens 155, 128 in 4, 137 in 5; 56 pairs and 500 tokens 188, 154 in 2, 188 in 3; 112
-    pairs and 250 tokens 116, 142 in 2; 14 pairs and 300 tokens 72, 71 in 4.  128 x 128: 12 pairs and 2,048 tokens 603,
-    412 in 4; 24 pairs and 300 tokens 116, 139 in 2.  Beyond 128 key channels the walk is built in one piece only.  One request's mixer launched kernel by kernel is bound by the host up to
-    600 tokens (420: 86 us in one piece, 102 in segments)."""
+    CTA, and two never do.  Measured with the mixer around it (us, from a graph), 64 x 64 states: 14 pairs and 2,048 tokens
+    302 in one piece, 242 in 4, 207 in 6, 219 in 8; 700 tokens 117, 109 in 4, 104 in 6; 420 tokens 80, 84 in 4; 28 pairs and
+    700 tokens 136, 131 in 4; 420 tokens 94, 98 in 4; 42 pairs (three requests of those 14 heads) and 420 tokens 113, 112
+    in 3; 56 pairs and 500 tokens 150, 162 in 2; 112 pairs and 250 tokens 119, 150 in 2.  128 x 128: 12 pairs and 2,048
+    tokens 450, 481 in 3, 420 in 4, 433 in 6; 24 pairs and 700 tokens 244, 250 in 3; 300 tokens 119, 144 in 3.  Beyond 128
+    key channels the walk is built in one piece only."""
     if longest < (600 if pairs < 42 else 400) or keys > 128:
         return 1
     values, moves = -(-vdim // 64), -(-keys // 64)
     segments = 1 + (sm_count() + pairs * moves) // (pairs * (values + moves))
     segments = min(segments, sm_count() // max(1, pairs * values))
-    return segments if segments > 2 else 1
+    return segments if segments > (2 if keys <= 64 else 3) else 1
 
 
 def delta_walk_shape(pairs: int, keys: int, vdim: int, max_q_len: int) -> tuple[int, int]:
@@ -1563,11 +1564,12 @@ def decay_scan_supported(keys: int) -> bool:
 def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) -> int:
     """Into how many segments `decay_scan` cuts a request's rows, `ctas` CTAs walking the step in one piece; a
     multiprocessor holds four or five of up to 64 key channels, three of more.  Segments cost most of the walk's work
-    once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it: 84 CTAs and 1,000
-    tokens 283 us in one piece, 193 in 4, 180 in 8; 42 CTAs and 2,048 tokens 487, 217 in 8, 219 in 16; 42 and 300 tokens
-    123, 72 in 8; 168 CTAs and 500 tokens 171, 181 in 2, 168 in 4; 336 and 250 tokens 129, 160 in 2.  Below 450 tokens the
-    mixer launched kernel by kernel is bound by the host, which a second launch costs about 10 us (270 tokens: 95 us in one
-    piece, 109 in segments)."""
+    once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it (us, from a graph): 42
+    CTAs and 2,048 tokens 418 in one piece, 288 in 4, 236 in 8, 239 in 15; 460 tokens 113, 82 in 8; 84 CTAs and 1,000 tokens
+    236, 201 in 4, 198 in 8; 420 tokens 113, 105 in 4; 168 CTAs and 500 tokens 182, 186 in 2, 176 in 4; 336 and 250 tokens
+    137, 169 in 2.  Below 450 tokens they would still save the device time (42 CTAs and 300 tokens 84, 67 in 8), but there
+    the mixer launched kernel by kernel, as prompts of such models are, is bound by the host, which a second launch and its
+    scratch cost 8 us (94 us in one piece, 101 in segments)."""
     if ctas >= sm_count() or longest < 450:
         return 1
     room = (9 * sm_count() // 2 if keys <= 64 else 3 * sm_count()) // max(1, ctas)
@@ -1742,10 +1744,12 @@ def conv_silu(proj: torch.Tensor, conv_at: int, channels: int, taps: int, w: tor
 def scan_segments(ctas: int, longest: int) -> int:
     """Into how many segments `selective_scan` cuts a request's rows, `ctas` CTAs walking the step in one piece and a
     multiprocessor holding four.  Segments cost a second launch and most of the walk's work once more, so they pay while
-    they bring idle multiprocessors to work: measured with its mixer, 56 CTAs and 2,048 tokens 684 us in one piece, 327
-    in 4, 238 in 8, 223 in 12; 112 CTAs and 700 tokens 259, 189 in 4, 171 in 6, 181 in 8; 224 CTAs and 500 tokens 247, 233
-    in 2; 448 CTAs and 250 tokens 175, 196 in 2.  Below 320 tokens the mixer launched kernel by kernel is bound by the
-    host, which a second launch costs about 10 us."""
+    they bring idle multiprocessors to work: measured with its mixer (us, from a graph), 56 CTAs and 2,048 tokens 690 in one
+    piece, 327 in 4, 239 in 8, 222 in 11, 226 in 16; 700 tokens 214, 158 in 4, 123 in 8; 112 CTAs and 420 tokens 195, 139 in
+    4, 128 in 6; 224 CTAs and 500 tokens 246, 235 in 2, 209 in 6; 448 CTAs and 250 tokens 173, 196 in 2.  Below 320 tokens
+    they would still save the device time (319 tokens 114, 91 in 8; 130 tokens 76, 71 in 8), but there the mixer launched
+    kernel by kernel, as prompts of such models are, is bound by the host, which a second launch and its scratch cost 8 us
+    (130 tokens 99 us in one piece, 107 in segments)."""
     if longest < 320:
         return 1
     return max(1, min(longest // 32, 9 * sm_count() // (2 * max(1, ctas)), 32))
