@@ -195,6 +195,29 @@ __device__ __forceinline__ float4 sum_splits4(const float* __restrict__ p, int s
   return t;
 }
 
+// ---- two 32-bit numbers an instruction, each rounded as by itself ---------------------------
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float low_of(f32x2 v) { return __uint_as_float((uint32_t)v); }
+__device__ __forceinline__ float high_of(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ void fma_pair(f32x2& d, f32x2 a, f32x2 b) {      // d += a b
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
 #define LAB_LAUNCH_CHECK() return (int)cudaGetLastError()
 
 // ---- programmatic dependent launch --------------------------------------------------------

@@ -96,25 +96,6 @@ __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
-// two 32-bit numbers an instruction, each rounded as by itself
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float low_of(f32x2 v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float high_of(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 constexpr int SP = (SL + 1) / 2;      // pairs of rows a thread keeps (an odd last row beside a zero)
 
 // A thread's SL values of one vector of D values in shared memory, in pairs.

@@ -40,12 +40,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 struct Quad {
   unsigned long long lo, hi;
 };
-__device__ __forceinline__ void fma_pair(unsigned long long& d, unsigned long long a, unsigned long long b) {
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
-}
-__device__ __forceinline__ float sum_of_pair(unsigned long long d) {
-  return __uint_as_float((uint32_t)d) + __uint_as_float((uint32_t)(d >> 32));
-}
+__device__ __forceinline__ float sum_of_pair(f32x2 d) { return low_of(d) + high_of(d); }
 __device__ __forceinline__ Quad load_quad(const float* p) {
   const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
   return {v.x, v.y};

@@ -175,25 +175,6 @@ __device__ __forceinline__ void cp_async_f32x4(float* dst, const float* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// ---- two 32-bit numbers an instruction, each rounded as by itself -------------------------------------
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float low_of(f32x2 v) { return __uint_as_float((uint32_t)v); }
-__device__ __forceinline__ float high_of(f32x2 v) { return __uint_as_float((uint32_t)(v >> 32)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 // The library's exponential: a slow decay's error comes with the same sign at every token and adds up over the state's
 // memory, so a form that is off by more is none.  (One by a range reduction and a polynomial, two entries an instruction,
 // took the mixer 242 us for 2,048 tokens, this one 222.)
