@@ -190,8 +190,8 @@ __host__ __device__ inline int scan_chunk_floats(int wc, int n4) { return 3 * WT
 // Lane l of a channel's WL holds the quads l, l + WL, ... of its state, R entries in all.  What bounds the walk, once
 // there are CTAs enough, is the issue of instructions: most of an entry's and token's are its exponential's, the others
 // take two entries each; a token of a CTA also takes its step sizes, gates and copies.  Measured on a B200, inputs from
-// memory, 1,792 channels of 16 entries: 8 requests of 250 tokens 84 us (115 with eight lanes a channel and an entry an
-// instruction); one of 2,048 131 us in eleven segments (352 in one piece of that form), issuing in two cycles of three.
+// memory, 1,792 channels of 16 entries: 8 requests of 250 tokens 82 us (115 with eight lanes a channel and an entry an
+// instruction); one of 2,048 129 us in eleven segments (352 in one piece of that form), issuing in two cycles of three.
 // QUADS: the state is whole quads; else the entries that fill the last one are kept at zero (an infinite step would leave
 // no numbers there).
 template <typename T, int WL, int R, int MODE, bool QUADS>
@@ -326,9 +326,9 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
       if (MODE == SCAN_CLOSE) dt_sum += dt;
     }
     __syncthreads();
-    // the walk: nothing but the state's own update passes from token to token (in one piece with few entries a lane four
-    // tokens in flight: 8 requests of 2,048 tokens 600 us, 625 by two; one 370, 383; no gain elsewhere)
-#pragma unroll (MODE == SCAN_WHOLE && R == 4 ? 4 : 2)
+    // the walk: nothing but the state's own update passes from token to token (with few entries a lane four tokens in flight:
+    // one request of 2,048 tokens in segments 129 us, 131 by two; in one piece 370, 383; 8 requests 598, 625; no gain with more)
+#pragma unroll (R == 4 ? 4 : 2)
     for (int tt = 0; tt < nt; ++tt) {
       const float dt = b_dt[tt * WC + ch], dx = s_dx[tt * WC + ch];
       const f32x2 dt2 = pair_of(dt, dt), dx2 = pair_of(dx, dx);
