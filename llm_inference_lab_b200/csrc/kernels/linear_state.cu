@@ -90,7 +90,7 @@ enum { SCAN_WHOLE, SCAN_CLOSE, SCAN_OUTPUT };
 // where the operands' addresses allow it: `vec`), and start the copies of chunk c + 2 into the buffer the
 // walkers left one chunk ago.  Three buffers, one barrier of the whole CTA per chunk.
 template <int R, int MODE>
-__global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
+__device__ __forceinline__ void decay_scan(const ScanParams& p) {
   extern __shared__ __align__(16) float smem[];
   constexpr int RS = R + 4;                      // floats between two threads' shares of a token's keys
   constexpr int NP = SCAN_P * RS;                // floats of a token's keys (or queries) in shared memory
@@ -301,6 +301,19 @@ __global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
   }
 }
 
+template <int R, int MODE>
+__global__ void __launch_bounds__(256) decay_scan_kernel(ScanParams p) {
+  decay_scan<R, MODE>(p);
+}
+// More than 64 key channels in one piece: registers for as many CTAs as shared memory allows, three a multiprocessor up to
+// 128 channels, two beyond, for steps that have so many (a long walk of few CTAs is shorter with all the registers it wants).
+// Measured, 12 heads of 128 x 128: 64 single tokens 49 us against 55 with two CTAs a multiprocessor, eight requests of 250
+// 150 against 168; one of 300 (48 CTAs) 88 with all its registers, 98 without.
+template <int R>
+__global__ void __launch_bounds__(256, R <= 32 ? 3 : 2) decay_scan_dense_kernel(ScanParams p) {
+  decay_scan<R, SCAN_WHOLE>(p);
+}
+
 // ---- state-space mixer: convolution, step sizes, decays ---------------------------------------
 struct SsmParams {
   const float* proj;     // [tokens, ld]
@@ -417,12 +430,20 @@ __global__ void __launch_bounds__(kThreads) gated_norm_kernel(T* __restrict__ ou
 template <int R, int MODE>
 int launch_scan_as(const ScanParams& p, int requests, int vs, cudaStream_t stream) {
   const size_t smem = (size_t)3 * SCAN_CT * (2 * SCAN_P * (R + 4) + vs + 4) * sizeof(float);
+  const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
+  const dim3 grid((p.V + vs - 1) / vs, p.H, requests * segments), block(2 * SCAN_P * vs);
+  if constexpr (MODE == SCAN_WHOLE && R > 16) {
+    if ((long long)grid.x * grid.y * grid.z > (R <= 32 ? 2 : 1) * lab_sm_count()) {
+      static LabShared granted;
+      const cudaError_t e = lab_allow_shared(granted, (const void*)decay_scan_dense_kernel<R>, smem);
+      if (e != cudaSuccess) return (int)e;
+      return (int)lab_launch(decay_scan_dense_kernel<R>, grid, block, smem, stream, p);
+    }
+  }
   static LabShared granted;
   const cudaError_t e = lab_allow_shared(granted, (const void*)decay_scan_kernel<R, MODE>, smem);
   if (e != cudaSuccess) return (int)e;
-  const int segments = MODE == SCAN_WHOLE ? 1 : MODE == SCAN_CLOSE ? p.segments - 1 : p.segments;
-  dim3 grid((p.V + vs - 1) / vs, p.H, requests * segments);
-  return (int)lab_launch(decay_scan_kernel<R, MODE>, grid, dim3(2 * SCAN_P * vs), smem, stream, p);
+  return (int)lab_launch(decay_scan_kernel<R, MODE>, grid, block, smem, stream, p);
 }
 
 template <int R>

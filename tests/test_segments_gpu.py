@@ -181,3 +181,28 @@ def test_decays_go_by_the_running_maximum_that_is_kept():
         assert np.abs(scale[at: at + length] - np.exp((log_i[at: at + length] - now).astype(np.float64))).max() < 1e-6
         assert np.array_equal(m_state[slot].cpu().numpy(), now[-1])
         at += length
+
+
+@pytest.mark.parametrize("heads,keys,vdim", [(12, 128, 128), (9, 100, 68), (7, 256, 96), (14, 64, 64)])
+def test_decay_scan_of_many_requests_has_the_bits_of_one(heads, keys, vdim):
+    """Steps of many CTAs of more than 64 key channels run a build with fewer registers."""
+    g = torch.Generator(device=DEV).manual_seed(keys)
+    rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
+    lens = [1] * 12 + [17, 40, 3, 16, 1, 33]
+    T, slots = sum(lens), list(np.random.default_rng(keys).permutation(len(lens)))
+    qk, v, state = rand(T, 2 * heads * keys), rand(T, heads * vdim), rand(len(lens), heads, keys, vdim)
+    decay, scale = torch.exp(-torch.rand(T, heads, device=DEV, generator=g) * 0.2), rand(T, heads)
+    gates = torch.stack([decay, scale], dim=1)
+
+    def walk(a, b, lens, slots, state):
+        return ops().decay_scan(qk[a:b, : heads * keys], qk[a:b, heads * keys:], v[a:b], state, context(lens, slots), heads, heads, keys,
+                                vdim, a_tok=gates[a:b, 0], s_tok=gates[a:b, 1], in_order=True)
+
+    together, at = state.clone(), 0
+    out = walk(0, T, lens, slots, together)
+    ops().take_device_errors()
+    assert len(lens) * heads * -(-vdim // 32) > 2 * ops().sm_count() or keys <= 64
+    for n, slot in zip(lens, slots):
+        alone = state.clone()
+        assert torch.equal(walk(at, at + n, [n], [slot], alone), out[at: at + n]) and torch.equal(alone[slot], together[slot])
+        at += n
