@@ -275,8 +275,8 @@ __global__ void __launch_bounds__(256) delta_walk_kernel(WalkParams p, int Vs) {
   const int all0 = p.q_start[r], all1 = p.q_start[r + 1];            // the request's rows, and this CTA's
   int t0 = all0, t1 = all1, last = 0;
   if (MODE != WALK_WHOLE && all1 > all0) last = segment_rows(t0, t1, seg, p.segments);
+  const int slot = p.state_slot[r];      // (asked for before anything waits for the rows)
   if (MODE == WALK_WHOLE && t1 - t0 < LONG_WALK) pdl_trigger();
-  const int slot = p.state_slot[r];
   // slices beyond the values' walk the identity; of the first segment, whose state is known, and the last nobody asks
   const int slices = (p.V + Vs - 1) / Vs;
   const bool move = MODE == WALK_CLOSE && (int)blockIdx.x >= slices;
