@@ -59,8 +59,7 @@ namespace {
 constexpr int BM = 128;  // rows of the M-side tile (UMMA M)
 constexpr int BK = 64;   // bf16 elements per k-tile: 128 bytes, one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 192;
-constexpr int SMEM_BUDGET = 200 * 1024;
+constexpr int SMEM_BUDGET = 200 * 1024, SMEM_MOST = 220 * 1024;      // (with the epilogue's rows)
 
 enum Mode : int { PLAIN = 0, GATED_SILU = 1, QKV_ROPE = 2, PICK = 3 };
 
@@ -197,12 +196,19 @@ struct Shape {
   static constexpr int EXCHANGE_BYTES = ((MODE == GATED_SILU || MODE == PICK) && SWAP) ? ((TM * (BN + 1) * 4 + 1023) / 1024) * 1024 : 0;
   static_assert(MODE != PICK || SWAP, "the picking head runs with the vocabulary on the 128-row side");
   static_assert(MODE != QKV_ROPE || !SWAP, "the q/k/v epilogue runs with tokens on the 128-row side");
-  static constexpr int STAGES_RAW = (SMEM_BUDGET - EXCHANGE_BYTES) / STAGE_BYTES;
+  static constexpr int ROWS_BYTES = !SWAP && MODE != QKV_ROPE ? 8 * STAGE_ROWS_BYTES : 0;      // where the epilogue's rows are put in order
+  static constexpr int STAGES_RAW = (ROWS_BYTES ? SMEM_MOST - ROWS_BYTES : SMEM_BUDGET - EXCHANGE_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
   static constexpr int ACC_COLS = BN < 32 ? 32 : BN;
   static constexpr int ACC_BUFS = 2 * ACC_COLS <= 512 ? 2 : 1;  // accumulators in tensor memory
   static constexpr int TMEM_COLS = ACC_BUFS * ACC_COLS;         // a power of two >= 32
-  static constexpr int SMEM = STAGES * STAGE_BYTES + EXCHANGE_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + EXCHANGE_BYTES + 1024 /*align*/ + 512 /*barriers*/ + ROWS_BYTES;
+  // Epilogue warps: a tile of many columns is shared by two warps per quarter of the lanes, which take its groups of
+  // columns in turn (gated 2,048 x 4,864 x 896 in tiles of 256 columns 32.6 us, 32.9 with four; the narrow tiles' gain is in
+  // the rows below).
+  static constexpr int EPI_WARPS = SWAP && (MODE != PLAIN || BN <= 32) ? 4 : 8;
+  static constexpr int SHARES = EPI_WARPS / 4;
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
   static_assert(STAGES >= 2, "the tile does not leave room for a pipeline");
   static_assert((2 * STAGES + 4) * 8 + 8 <= 512, "the barriers outgrow their 512 bytes");
 };
@@ -211,7 +217,7 @@ struct Shape {
 // the M side fastest, so CTAs that run at the same time share the N-side operand in L2.
 // Two accumulators in tensor memory let the epilogue of one tile run beside the MMAs of the next.
 template <int MODE, int BN, bool SWAP, typename OutT>
-__global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
+__global__ void __launch_bounds__(Shape<MODE, BN, SWAP>::THREADS) gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a,
                                                           const __grid_constant__ CUtensorMap map_b, Params p) {
   using S = Shape<MODE, BN, SWAP>;
   constexpr int TM = BM;
@@ -225,6 +231,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
   uint64_t* acc_empty = acc_full + 2;           // [ACC_BUFS]
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  uint8_t* rows_stage = (uint8_t*)full + 512;      // (normal orientation) of an epilogue warp
 
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -239,7 +246,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 4);  // one arrival per epilogue warp
+      mbar_init(&acc_empty[a], S::EPI_WARPS);  // one arrival per epilogue warp
     }
     *abort_flag = 0;
     mbar_init_fence();
@@ -374,8 +381,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
       }
     }
   } else {
-    // ---- epilogue: warps 2..5, each reads its quarter of the 128 accumulator lanes ----
-    const int quarter = warp & 3;
+    // ---- epilogue: warps 2.., each reads its quarter of the 128 accumulator lanes, its share of the columns ----
+    const int quarter = warp & 3, share = (warp - 2) >> 2;
     constexpr int QROWS = TM / 4;            // tile rows in a quarter: one per lane
     pdl_wait();  // the output may still be read by an earlier kernel until it has completed
     int local = -1;
@@ -415,11 +422,12 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
           if (head >= n_heads) break;  // same for the whole warp
 #pragma unroll 1
           for (int g = 0; g < groups; ++g) {
+            if ((hh * groups + g) % S::SHARES != share) continue;
             uint32_t rlo[32], rhi[32];
             tmem_ld32_issue(lane_addr + hh * d + g * 32, rlo);
             tmem_ld32_issue(lane_addr + hh * d + d / 2 + g * 32, rhi);
             tmem_wait();
-            if (g == groups - 1 && ((hh + 1) * d >= BN || head + 1 >= n_heads)) release();
+            if (hh * groups + g + S::SHARES >= min(BN / d, n_heads - n0 / d) * groups) release();
             if (m < p.m_rows) qkv_store_row(p, m, head, g * 32, rlo, rhi);
           }
         }
@@ -490,6 +498,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
         asm volatile("bar.sync 1, 128;" ::: "memory");  // the buffer is free for the next tile
       } else if constexpr (!SWAP) {
         // thread = token row m; columns = output features, 32 at a time
+        uint8_t* stage = rows_stage + (warp - 2) * STAGE_ROWS_BYTES;
         constexpr int OUT_COLS = GATED ? BN / 2 : BN;
         static_assert(OUT_COLS % 32 == 0, "normal orientation works on 32 output columns at a time");
         const int nbase = (n0 / N_ROWS) * OUT_COLS;
@@ -501,7 +510,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
           }
         }
 #pragma unroll 1
-        for (int c = 0; c < OUT_COLS / 32 && go; ++c) {
+        for (int c = share; c < OUT_COLS / 32 && go; c += S::SHARES) {
           uint32_t r[32];
           float v[32];
           if (n_kt > 0) {
@@ -521,11 +530,18 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = 0.f;
           }
-          if (c == OUT_COLS / 32 - 1) release();
+          if (c + S::SHARES >= OUT_COLS / 32) release();
           const int n = nbase + c * 32;
-          if (m >= p.m_rows || n >= p.n_rows) continue;
+          if (n >= p.n_rows) continue;
+          const int rows = min(32, p.m_rows - (m - lane));      // of the warp
           if (partial) {
-            float* dst = (float*)p.out + split * p.split_stride + (size_t)m * p.ld_out + n;
+            float* to = (float*)p.out + split * p.split_stride + (size_t)(m - lane) * p.ld_out + n;
+            if (n + 32 <= p.n_rows && rows_on_16(to, p.ld_out)) {
+              store_columns_32(stage, v, to, p.ld_out, rows, lane);
+              continue;
+            }
+            if (lane >= rows) continue;
+            float* dst = to + (size_t)lane * p.ld_out;
             if (n + 32 <= p.n_rows && (((uintptr_t)dst) & 15) == 0) {
 #pragma unroll
               for (int j = 0; j < 8; ++j)
@@ -559,7 +575,13 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
 #pragma unroll
               for (int j = 0; j < 32; ++j) v[j] = lab_act(v[j], p.gelu);
             }
-            OutT* dst = (OutT*)p.out + (size_t)m * p.ld_out + n;
+            OutT* to = (OutT*)p.out + (size_t)(m - lane) * p.ld_out + n;
+            if (n + 32 <= p.n_rows && rows_on_16(to, p.ld_out)) {
+              store_columns_32(stage, v, to, p.ld_out, rows, lane);
+              continue;
+            }
+            if (lane >= rows) continue;
+            OutT* dst = to + (size_t)lane * p.ld_out;
             if (n + 32 <= p.n_rows && (((uintptr_t)dst) & 15) == 0) {
               if (sizeof(OutT) == 2) {
 #pragma unroll
@@ -617,9 +639,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
       } else {
         // thread = output feature m; columns = tokens
         const float b = (p.bias && !partial && m < p.m_rows) ? __bfloat162float(p.bias[m]) : 0.f;
-        int c = 0;
 #pragma unroll 1
-        for (; c < BN / 16 && go; ++c) {
+        for (int c = share; c < BN / 16 && go; c += S::SHARES) {
           const int t = n0 + c * 16;
           if (t >= p.n_rows) break;  // same for the whole warp
           float v[16];
@@ -627,7 +648,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc_kernel(const __grid_constant_
           else
 #pragma unroll
             for (int j = 0; j < 16; ++j) v[j] = 0.f;
-          if (c == BN / 16 - 1 || t + 16 >= p.n_rows) release();
+          if (c + S::SHARES >= BN / 16 || t + 16 * S::SHARES >= p.n_rows) release();
           if (m >= p.m_rows) continue;
           if (partial) {
             float* dst = (float*)p.out + split * p.split_stride + m;
@@ -665,7 +686,7 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const Params& p, dim3 g
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  return (int)lab_launch(kern, grid, dim3(THREADS), (size_t)S::SMEM, stream, ma, mb, p);
+  return (int)lab_launch(kern, grid, dim3(S::THREADS), (size_t)S::SMEM, stream, ma, mb, p);
 }
 
 template <int MODE, bool SWAP, typename OutT>

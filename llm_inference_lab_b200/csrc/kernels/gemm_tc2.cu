@@ -16,7 +16,7 @@
 //
 // Per CTA: warp 0 loads (TMA; both CTAs' copies complete on the leader's barrier), warp 1 of the
 // leader issues the MMAs (the whole warp walks the loop, an elected lane issues) and commits to
-// the barriers of both CTAs (tcgen05.commit with multicast), warps 2-5 of each CTA read their
+// the barriers of both CTAs (tcgen05.commit with multicast), warps 2-9 of each CTA read their
 // accumulator back and store.  CTAs are persistent: a pair walks the tiles, with two accumulators
 // in tensor memory, so the epilogue of one tile runs beside the MMAs of the next.  No load uses
 // cluster multicast.  Every wait is bounded: when one runs out the kernel records an error code
@@ -32,7 +32,11 @@ namespace {
 constexpr int BM = 128;   // token rows per CTA (the pair's MMA has M = 256)
 constexpr int BK = 64;    // bf16 elements per k-tile: 128 bytes, one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 192;
+// Epilogue warps: two per quarter of the lanes, which take groups of 32 columns in turn.  A gated tile's epilogue was longer
+// than its MMAs with one (us, weights from memory: 2,048 x 4,864 x 896 29.3, with one per quarter 35.9; 700 tokens 15.4 and 19.1;
+// 300 x 8,960 x 1,536 22.4 and 23.7).
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int A_BYTES = BM * BK * 2;
 constexpr int ACC_BUFS = 2;
 constexpr int ACC_STRIDE = 256;                   // columns of tensor memory between the two accumulators
@@ -46,7 +50,7 @@ struct Tile {
   static constexpr int B_BYTES = (BN / 2) * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int STAGES = 192 * 1024 / STAGE_BYTES > 8 ? 8 : 192 * 1024 / STAGE_BYTES;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 512 /*barriers*/;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 512 /*barriers*/ + EPI_WARPS * STAGE_ROWS_BYTES;
   // Instruction descriptor: bf16 x bf16 -> f32, both operands K-major, M = 256 over the pair, N = BN.
   static constexpr uint32_t IDESC =
       (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
@@ -117,6 +121,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
   uint64_t* acc_empty = acc_full + ACC_BUFS;    // [ACC_BUFS], used in the leader only
   uint32_t* tmem_slot = (uint32_t*)(acc_empty + ACC_BUFS);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+  uint8_t* rows_stage = tiles + STAGES * STAGE_BYTES + 512;      // of an epilogue warp
 
   pdl_trigger();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -133,7 +138,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
     }
     for (int a = 0; a < ACC_BUFS; ++a) {
       mbar_init(&acc_full[a], 1);   // one commit, sent to both CTAs
-      mbar_init(&acc_empty[a], 8);  // the four epilogue warps of each CTA
+      mbar_init(&acc_empty[a], 2 * EPI_WARPS);  // the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     mbar_init_fence();
@@ -225,8 +230,10 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
       }
     }
   } else {
-    // ---- epilogue: warps 2..5, each reads its quarter of this CTA's 128 accumulator lanes ----
-    const int quarter = warp & 3;
+    // ---- epilogue: warps 2.., each reads its quarter of this CTA's 128 accumulator lanes, its share of the columns ----
+    constexpr int SHARES = EPI_WARPS / 4;
+    const int quarter = warp & 3, share = (warp - 2) >> 2;
+    uint8_t* stage = rows_stage + (warp - 2) * STAGE_ROWS_BYTES;
     pdl_wait();  // the output may still be read by an earlier kernel until it has completed
     int local = 0;
     for (int tile = pair; tile < total_tiles; tile += n_pairs, ++local) {
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
       constexpr int CHUNKS = (OUT_COLS + 31) / 32;
       const int n_end = min(p.n_out, n0 + OUT_COLS);
 #pragma unroll 1
-      for (int c = 0; c < CHUNKS && go; ++c) {
+      for (int c = share; c < CHUNKS && go; c += SHARES) {
         uint32_t r[32];
         float v[32];
         if (n_kt > 0) {
@@ -272,10 +279,17 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = 0.f;
         }
-        if (c == CHUNKS - 1) release();
+        if (c + SHARES >= CHUNKS) release();
         const int n = n0 + c * 32;
-        if (m >= p.tokens || n >= n_end) continue;
+        if (n >= n_end) continue;
+        const int rows = min(32, p.tokens - (m - lane));      // of the warp
         if (partial) {
+          float* to = (float*)p.out + split * p.split_stride + (size_t)(m - lane) * p.ld_out + n;
+          if (n + 32 <= n_end && rows_on_16(to, p.ld_out)) {
+            store_columns_32(stage, v, to, p.ld_out, rows, lane);
+            continue;
+          }
+          if (lane >= rows) continue;
           float* dst = (float*)p.out + split * p.split_stride + (size_t)m * p.ld_out + n;
           const bool aligned = (((uintptr_t)dst) & 15) == 0;
 #pragma unroll
@@ -298,7 +312,13 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = lab_act(v[j], p.gelu);
           }
-          OutT* dst = (OutT*)p.out + (size_t)m * p.ld_out + n;
+          OutT* to = (OutT*)p.out + (size_t)(m - lane) * p.ld_out + n;
+          if (n + 32 <= n_end && rows_on_16(to, p.ld_out)) {
+            store_columns_32(stage, v, to, p.ld_out, rows, lane);
+            continue;
+          }
+          if (lane >= rows) continue;
+          OutT* dst = to + (size_t)lane * p.ld_out;
           const bool aligned = (((uintptr_t)dst) & 15) == 0;
           constexpr int PER = 16 / (int)sizeof(OutT);   // elements of a 16-byte store
 #pragma unroll
