@@ -121,11 +121,13 @@ __global__ void add_rmsnorm_kernel(T* __restrict__ y, T* __restrict__ x, const T
 }
 
 // The same for bfloat16 rows whose width is a multiple of 8, for steps with many rows: a thread owns chunks of 8 elements
-// (16-byte loads and stores), CHUNKS at most, and keeps them in registers.  LANES threads a row: a warp, which needs no
-// barrier, or a CTA where the registers of a warp would not hold the row.  The CTAs of a launch are no more than find room
-// beside the product before (each takes several rows), so that the product after is let in while they still wait and its
-// set-up and first weights are not in the way.  48 of them in a step of 2,048 rows of 896: the step 2.70 ms, 2.96 with a CTA a
-// row (2,048 CTAs of which a part waits for the others' end, and with them the next kernel).
+// (16-byte loads and stores), CHUNKS at most, and keeps them in registers.  LANES threads a row: a CTA, so that a row's loads
+// are all under way at once, or, with more rows than CTAs find room beside the product before, a warp, which takes several
+// rows where it has to: the product after is then let in while the CTAs still wait, and its set-up and first weights are not
+// in the way.  48 of them in a step of 2,048 rows of 896: the step 2.70 ms, 2.96 with a CTA a row (2,048 CTAs of which a part
+// waits for the others' end, and with them the next kernel).  Steps of 150, 300 and 700 rows with a CTA a row 1,407, 1,432
+// and 1,899 us (1,511, 1,547 and 1,990 by the former build, whose threads kept room for 8,192 entries a row); with a warp a
+// row one of them took a seventh longer: the loads of the product's partial sums follow one another.
 constexpr int NORM_VEC_THREADS = 128;
 constexpr int NORM_VEC_MAX_CHUNKS = 8;  // per thread: widths up to 128 * 8 * 8 = 8192
 
@@ -172,9 +174,10 @@ __global__ void __launch_bounds__(NORM_VEC_THREADS, CHUNKS <= 4 ? 6 : 4) add_rms
       }
       if (partial) {
         float p[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        const float* from = partial + base + c * 8;
+#pragma unroll 2
         for (int s = 0; s < splits; ++s) {  // ascending split order, as the scalar kernel
-          const float4 a = *reinterpret_cast<const float4*>(partial + s * split_stride + base + c * 8);
-          const float4 b = *reinterpret_cast<const float4*>(partial + s * split_stride + base + c * 8 + 4);
+          const float4 a = load4(from + s * split_stride), b = load4(from + s * split_stride + 4);
           p[0] += a.x; p[1] += a.y; p[2] += a.z; p[3] += a.w;
           p[4] += b.x; p[5] += b.y; p[6] += b.z; p[7] += b.w;
         }
@@ -225,11 +228,14 @@ LAB_EXPORT int lab_add_rmsnorm(void* y, void* x, const void* delta, const float*
   if (dtype == LAB_BF16 && n_out_rows > 64 && hidden % 8 == 0 && aligned &&
       hidden <= NORM_VEC_THREADS * NORM_VEC_MAX_CHUNKS * 8 && (split_stride % 4) == 0)
   {
-    const auto kernel = hidden <= 1024 ? add_rmsnorm_vec_kernel<32, 4>
-                        : hidden <= 2048 ? add_rmsnorm_vec_kernel<32, 8>
+    const int most = 4 * lab_sm_count();
+    const bool warps = n_out_rows > most && hidden <= 2048;
+    const auto kernel = warps ? (hidden <= 1024 ? add_rmsnorm_vec_kernel<32, 4> : add_rmsnorm_vec_kernel<32, 8>)
+                        : hidden <= 1024 ? add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 1>
+                        : hidden <= 2048 ? add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 2>
                         : hidden <= 4096 ? add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 4>
                                          : add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 8>;
-    const int tiles = hidden <= 2048 ? (n_out_rows + 3) / 4 : n_out_rows, most = 4 * lab_sm_count();
+    const int tiles = warps ? (n_out_rows + 3) / 4 : n_out_rows;
     return (int)lab_launch(kernel, dim3(tiles < most ? tiles : most), dim3(NORM_VEC_THREADS), 0, stream,
                            (__nv_bfloat16*)y, (__nv_bfloat16*)x, (const __nv_bfloat16*)delta, partial, splits,
                            (size_t)split_stride, (const __nv_bfloat16*)w, rows, n_out_rows, n_in_rows, hidden, eps);
