@@ -300,6 +300,8 @@ __global__ void __launch_bounds__(Shape<MODE, BN, SWAP>::THREADS) gemm_tc_kernel
         else tma_load_2d(a_dst, &map_a, &full[s], kx, m0);
       };
       int it = 0;  // stages filled so far, over all tiles
+      int s = 0;   // the next stage and its phase, counted on: divisions would sit on every stage's chain
+      uint32_t ph = 1;
       bool first_tile = true, alive = true;
       if (p.tile_group != nullptr) pdl_wait();
       for (int tile = blockIdx.x; tile < total_tiles && alive; tile += gridDim.x) {
@@ -317,16 +319,17 @@ __global__ void __launch_bounds__(Shape<MODE, BN, SWAP>::THREADS) gemm_tc_kernel
           pdl_wait();
           for (int j = 0; j < ahead; ++j) load_activations(j, (kt0 + j) * BK, m0, n0);
           it = ahead;
+          s = ahead % S::STAGES;
+          if (ahead == S::STAGES) ph ^= 1;
           first_tile = false;
         }
         for (; i < n_kt; ++i, ++it) {
-          const int s = it % S::STAGES;
-          const uint32_t ph = (it / S::STAGES) & 1;
-          if (!mbar_wait(&empty[s], ph ^ 1, abort_flag)) { alive = false; break; }
+          if (!mbar_wait(&empty[s], ph, abort_flag)) { alive = false; break; }
           mbar_expect_tx(&full[s], S::STAGE_BYTES);
           const int kx = (kt0 + i) * BK;
           load_weights(s, kx, m0, n0, wb);
           load_activations(s, kx, m0, n0);
+          if (++s == S::STAGES) s = 0, ph ^= 1;
         }
       }
       if (first_tile) pdl_wait();
@@ -347,7 +350,8 @@ __global__ void __launch_bounds__(Shape<MODE, BN, SWAP>::THREADS) gemm_tc_kernel
       auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
         return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
       };
-      int it = 0, local = 0;  // local: tiles this CTA has worked on (skipped ones do not count)
+      int s = 0, local = 0;  // local: tiles this CTA has worked on (skipped ones do not count)
+      uint32_t ph = 0;
       bool ok = true;
       if (p.tile_group != nullptr) pdl_wait();
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -361,9 +365,7 @@ __global__ void __launch_bounds__(Shape<MODE, BN, SWAP>::THREADS) gemm_tc_kernel
         if (!ok) break;
         tc_fence_after();
         const uint32_t acc_addr = tmem_base + buf * S::ACC_COLS;
-        for (int i = 0; i < n_kt; ++i, ++it) {
-          const int s = it % S::STAGES;
-          const uint32_t ph = (it / S::STAGES) & 1;
+        for (int i = 0; i < n_kt; ++i) {
           ok = wait_all(&full[s], ph);
           if (!ok) break;
           tc_fence_after();
@@ -375,6 +377,7 @@ __global__ void __launch_bounds__(Shape<MODE, BN, SWAP>::THREADS) gemm_tc_kernel
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma_bf16(acc_addr, desc_a + 2 * k, desc_b + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
           umma_commit(&empty[s]);  // the stage may be refilled once these MMAs have read it
+          if (++s == S::STAGES) s = 0, ph ^= 1;
         }
         umma_commit(&acc_full[buf]);  // the accumulator is complete once every MMA has retired
         ++local;

@@ -173,7 +173,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
     if (lane == 0) {
       // ---- producer: this CTA's token rows and its half of the weight rows ----
       pdl_wait();
-      int it = 0;
+      int s = 0;                 // (stages and phases are counted on: divisions would sit on every stage's chain)
+      uint32_t ph = 1;
       bool alive = true;
       for (int tile = pair; tile < total_tiles && alive; tile += n_pairs) {
         int m0, n0, kt0, n_kt, split;
@@ -181,16 +182,15 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
         const int a_row = m0 + (int)rank * BM;
         // gated: the leader holds the gate rows, its peer the up rows of the same features
         const int b_row = GATED ? (leader ? n0 : p.up_offset + n0) : n0 + (int)rank * (BN / 2);
-        for (int i = 0; i < n_kt; ++i, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!mbar_wait<true>(&empty[s], ph ^ 1, abort_flag)) { alive = false; break; }
+        for (int i = 0; i < n_kt; ++i) {
+          if (!mbar_wait<true>(&empty[s], ph, abort_flag)) { alive = false; break; }
           if (leader) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
           const uint32_t bar = map_to_rank(smem_u32(&full[s]), 0);
           uint8_t* a_dst = tiles + s * STAGE_BYTES;
           const int kx = (kt0 + i) * BK;
           tma_load_2d_pair(a_dst, &map_a, bar, kx, a_row);
           tma_load_2d_pair(a_dst + A_BYTES, &map_b, bar, kx, b_row);
+          if (++s == STAGES) s = 0, ph ^= 1;
         }
       }
     }
@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
       auto wait_all = [&](uint64_t* bar, uint32_t parity) -> bool {
         return __all_sync(0xffffffffu, mbar_wait<true>(bar, parity, abort_flag));
       };
-      int it = 0, local = 0;
+      int s = 0, local = 0;
+      uint32_t ph = 0;
       bool ok = true;
       for (int tile = pair; tile < total_tiles && ok; tile += n_pairs, ++local) {
         int m0, n0, kt0, n_kt, split;
@@ -212,9 +213,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
         if (!ok) break;
         tc_fence_after();
         const uint32_t acc_addr = tmem_base + buf * ACC_STRIDE;
-        for (int i = 0; i < n_kt; ++i, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
+        for (int i = 0; i < n_kt; ++i) {
           ok = wait_all(&full[s], ph);
           if (!ok) break;
           tc_fence_after();
@@ -225,6 +224,7 @@ __global__ void __launch_bounds__(THREADS) gemm_tc2_kernel(const __grid_constant
           for (int k = 0; k < BK / UMMA_K; ++k)
             umma_bf16_pair(acc_addr, desc_a + 2 * k, desc_b + 2 * k, IDESC, (i > 0 || k > 0) ? 1u : 0u);
           umma_commit_pair(&empty[s], 3);  // both CTAs may refill the stage once these MMAs have read it
+          if (++s == STAGES) s = 0, ph ^= 1;
         }
         umma_commit_pair(&acc_full[buf], 3);  // the accumulators of both CTAs are complete
       }
