@@ -30,7 +30,9 @@
 // rates, unit keys); the walk; a third, parallel over tokens, divides each head's raw output by its root
 // mean square and applies weight and gate.  A step of one token per request (decode) is the same three
 // kernels with a chunk of one.
-#include "common.cuh"
+#include <type_traits>
+
+#include "tcgen05.cuh"
 
 #ifndef LAB_HEAD_DIM
 #define LAB_HEAD_DIM 64
@@ -256,6 +258,318 @@ __global__ void __launch_bounds__(256) delta_prepare_kernel(float* __restrict__ 
   pdl_trigger();      // (not earlier: the walk's few, long blocks would settle unevenly where these leave room first)
 }
 
+// ---- portions of a prompt: four tokens in one go ---------------------------------------------------
+// Within a block of tokens 0..3 let P_i be the product of the decays up to token i, R_ij that of the decays after token j
+// up to token i, and p_i = u_i^T S the old state's part that token i removes.  With the state S before the block
+//
+//   p_i = (P_{i-1} u_i)^T S + sum_{j<i} (u_i . R_{i-1,j} k_j) v_j - (u_i . R_{i-1,j} a_j u_j) p_j
+//   o_i = (P_i r_i)^T S     + sum_{j<=i} (r_i . R_ij k_j) v_j     - (r_i . R_ij a_j u_j) p_j
+//   S  <- P_3 S + sum_j (R_3j k_j) v_j^T - (R_3j a_j u_j) p_j^T
+//
+// which is the recurrence with its sums regrouped: eight independent sums over a column of S, four steps on numbers, one
+// update, where there were four dependent rounds.  Products of decays are formed as products, never as quotients, so
+// strong decays lose nothing.  A request's blocks start at its first row; rows beyond its last have decay 1 and zeros.
+// 32-bit storage keeps the walk token by token: a result must not depend on where a portion starts.
+constexpr int BLK = 4;
+constexpr int B_DOTS = 8, B_KEYS = 8, B_GONE = 12, B_DECAY = 16, B_VECTORS = 17;      // P u, P r; R k; -R a u; P_3
+constexpr int N_PAIR = BLK * (BLK - 1) / 2, N_TRI = BLK * (BLK + 1) / 2;              // j < i and j <= i
+// coefficients: u . R k and -u . R a u of the pairs j < i, then a row of r . R k and one of -r . R a u a token (zeros
+// beyond j = i)
+constexpr int C_UK = 0, C_UA = N_PAIR, C_RK = 2 * N_PAIR, C_RA = C_RK + BLK * BLK, N_COEF = C_RA + BLK * BLK;
+static_assert(2 * (N_PAIR + N_TRI) == 32 && N_COEF % 4 == 0, "a lane a sum");
+// Eight rows of two columns a thread, so that a whole block's share of the record fits its registers and is asked for a
+// block ahead: GB threads a pair of columns.
+constexpr bool BLOCKS_BUILT = D == 32 || D == 64 || D == 128 || D == 256;
+constexpr int SLB = 8, GB = BLOCKS_BUILT ? D / SLB : 4, SLBP = SLB + 4, RLB = GB * SLBP;      // (padded as above)
+constexpr int AT_V = B_VECTORS * RLB, AT_C = AT_V + BLK * D, BREC = AT_C + N_COEF;             // floats of a record
+constexpr int BCHUNK = BREC * 4 * 8 <= 64 * 1024 ? 4 : 2;                                      // blocks of a chunk
+constexpr int NCOL = 2, BCOLS = 16, BTHREADS = BCOLS / NCOL * GB;
+constexpr size_t BSMEM = sizeof(float) * 2 * BCHUNK * BREC + 32;      // two chunks, their barriers, the abort flag
+
+// The place of a request's first block among the records of a head: there are no more than tokens / 4 + requests.
+__host__ __device__ __forceinline__ int first_block(int row0, int request) { return row0 / BLK + request; }
+
+// One warp per (block, head): everything of the recurrence that does not depend on the state.  Bound by its writes.
+template <typename T>
+__global__ void __launch_bounds__(256) delta_prepare_blocks_kernel(float* __restrict__ records, int n_records,
+                                                                   const float* __restrict__ r, const float* __restrict__ k,
+                                                                   const float* __restrict__ v, const float* __restrict__ a,
+                                                                   int ld, const float* __restrict__ d, int ld_d,
+                                                                   const T* __restrict__ d_bias, const T* __restrict__ a_bias,
+                                                                   const int* __restrict__ q_start, int requests, int heads,
+                                                                   float decay_rate) {
+  pdl_wait();
+  const int lane = threadIdx.x & 31, h = blockIdx.y * 8 + (threadIdx.x >> 5), at = blockIdx.x;
+  // the last request whose blocks start at or before this record
+  int req = 0;
+  for (int r0 = 0; r0 < requests; r0 += 32) {
+    const bool before = r0 + lane < requests && first_block(q_start[min(r0 + lane, requests - 1)], r0 + lane) <= at;
+    const unsigned all = __ballot_sync(0xffffffffu, before);
+    if (all == 0u) break;
+    req = r0 + 31 - __clz((int)all);
+  }
+  const int row0 = q_start[req], t0 = row0 + BLK * (at - first_block(row0, req)), n = min(BLK, q_start[req + 1] - t0);
+  if (n > 0 && h < heads) {
+    float inv[BLK];
+#pragma unroll
+    for (int t = 0; t < BLK; ++t) {
+      float ss = 0.f;
+      for (int i = lane; i < D; i += 32) {
+        const float kk = t < n ? k[(size_t)(t0 + t) * ld + h * D + i] : 0.f;
+        ss = fmaf(kk, kk, ss);
+      }
+      inv[t] = 1.0f / sqrtf(warp_sum(ss) + 1e-6f);
+    }
+    float c[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) c[i] = 0.f;
+    float* dst = records + ((size_t)h * n_records + at) * BREC;
+    for (int i = lane; i < D; i += 32) {
+      const int ch = h * D + i, ir = (i / SLB) * SLBP + i % SLB;
+      float w[BLK], u[BLK], au[BLK], kk[BLK], rr[BLK];
+#pragma unroll
+      for (int t = 0; t < BLK; ++t) {
+        w[t] = 1.f, u[t] = au[t] = kk[t] = rr[t] = 0.f;
+        float vv = 0.f;
+        if (t < n) {
+          const size_t from = (size_t)(t0 + t) * ld + ch;
+          kk[t] = k[from], rr[t] = r[from], vv = v[from];
+          w[t] = expf(-decay_rate * sigmoidf_(d[(size_t)(t0 + t) * ld_d + ch] + to_f32(d_bias[ch])));
+          u[t] = kk[t] * inv[t];
+          au[t] = -(sigmoidf_(a[from] + to_f32(a_bias[ch])) * u[t]);
+        }
+        dst[AT_V + t * D + i] = vv;
+      }
+      float before = 1.f;      // the product of the decays up to the token before
+#pragma unroll
+      for (int t = 0; t < BLK; ++t) {
+        dst[t * RLB + ir] = before * u[t];
+        before *= w[t];
+        dst[(BLK + t) * RLB + ir] = before * rr[t];
+      }
+      dst[B_DECAY * RLB + ir] = before;
+      // R_{i-1,j} k_j and -R_{i-1,j} a_j u_j for all j < i, then R_3j's; token by token
+      float rk[BLK], ra[BLK];
+      int pair = 0, tri = 0;
+#pragma unroll
+      for (int t = 0; t < BLK; ++t) {
+#pragma unroll
+        for (int j = 0; j < t; ++j, ++pair) {
+          c[pair] = fmaf(u[t], rk[j], c[pair]);
+          c[N_PAIR + pair] = fmaf(u[t], ra[j], c[N_PAIR + pair]);
+        }
+        rk[t] = kk[t], ra[t] = au[t];
+#pragma unroll
+        for (int j = 0; j <= t; ++j, ++tri) {
+          if (j < t) rk[j] *= w[t], ra[j] *= w[t];
+          c[2 * N_PAIR + tri] = fmaf(rr[t], rk[j], c[2 * N_PAIR + tri]);
+          c[2 * N_PAIR + N_TRI + tri] = fmaf(rr[t], ra[j], c[2 * N_PAIR + N_TRI + tri]);
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < BLK; ++t) dst[(B_KEYS + t) * RLB + ir] = rk[t], dst[(B_GONE + t) * RLB + ir] = ra[t];
+    }
+    // 32 sums over the lanes, one of them left in each lane
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool upper = (lane & o) != 0;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const float mine = upper ? c[i + o] : c[i], theirs = upper ? c[i] : c[i + o];
+        c[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, o);
+      }
+    }
+    float* coef = dst + AT_C;
+    if (lane < 2 * N_PAIR) {
+      coef[lane] = c[0];
+      // (the twelve places beyond the diagonals)
+      const int pair = lane % N_PAIR, i = pair < 3 ? 0 : pair < 5 ? 1 : 2, j = pair < 3 ? pair + 1 : pair < 5 ? pair - 1 : 3;
+      coef[(lane < N_PAIR ? C_RK : C_RA) + BLK * i + j] = 0.f;
+    } else {
+      const int tri = (lane - 2 * N_PAIR) % N_TRI, i = tri < 1 ? 0 : tri < 3 ? 1 : tri < 6 ? 2 : 3;
+      coef[(lane < 2 * N_PAIR + N_TRI ? C_RK : C_RA) + BLK * i + tri - i * (i + 1) / 2] = c[0];
+    }
+  }
+  pdl_trigger();      // (not earlier: see delta_prepare_kernel)
+}
+
+// A thread's eight rows of one vector of a record, in pairs.
+__device__ __forceinline__ void load_share(f32x2 (&dst)[SLB / 2], const float* share, int vector) {
+#pragma unroll
+  for (int q = 0; q < SLB / 4; ++q) {
+    const ulonglong2 t = reinterpret_cast<const ulonglong2*>(share + vector * RLB)[q];
+    dst[2 * q] = t.x, dst[2 * q + 1] = t.y;
+  }
+}
+
+__global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, int n_records) {
+  extern __shared__ __align__(16) float blocks_smem[];
+  pdl_wait();
+  const int h = blockIdx.x, req = blockIdx.y, tid = threadIdx.x;
+  const int j = blockIdx.z * BCOLS + tid / GB * NCOL, g = tid % GB;      // this thread's first column of S, its share of the rows
+  const int row0 = p.q_start[req], rows = p.q_start[req + 1] - row0;
+  const int slot = p.state_slot[req];
+  if (slot == -1) {      // rows of padding: zeros out, no state
+    if (g == 0)
+      for (int t = row0; t < row0 + rows; ++t)
+        *reinterpret_cast<float2*>(p.out + (size_t)t * p.heads * D + h * D + j) = make_float2(0.f, 0.f);
+    return;
+  }
+  if (slot < 0 || slot >= p.n_slots) {
+    if (tid == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
+    return;
+  }
+  const int blocks = (rows + BLK - 1) / BLK;
+  if (blocks == 0) return;
+  const float* records = p.rec + ((size_t)h * n_records + first_block(row0, req)) * BREC;
+  // Chunks come by bulk copies, which cost the walk one thread's instruction (copies of 16 bytes by all threads held its
+  // own loads up: 1,400 of a chunk's 6,500 cycles).
+  uint64_t* here = reinterpret_cast<uint64_t*>(blocks_smem + 2 * BCHUNK * BREC);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(here + 2);
+  if (tid == 0) {
+    mbar_init(&here[0], 1), mbar_init(&here[1], 1);
+    *abort_flag = 0;
+    mbar_init_fence();
+  }
+  __syncthreads();
+  auto fetch = [&](int b0) {      // one thread; a chunk, where there is one
+    if (b0 >= blocks) return;
+    const uint32_t bytes = min(BCHUNK, blocks - b0) * BREC * 4;
+    uint64_t* bar = &here[b0 / BCHUNK % 2];
+    mbar_expect_tx(bar, bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     smem_u32(blocks_smem + b0 / BCHUNK % 2 * BCHUNK * BREC)),
+                 "l"(records + (size_t)b0 * BREC), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+  };
+  auto landed = [&](int b0) { return mbar_wait(&here[b0 / BCHUNK % 2], b0 / BCHUNK / 2 & 1, abort_flag); };
+  if (tid == 0) fetch(0), fetch(BCHUNK);
+  float* S_g = p.state + ((size_t)slot * p.heads + h) * D * D + (size_t)(g * SLB) * D + j;
+  f32x2 S[NCOL][SLB / 2];
+#pragma unroll
+  for (int i = 0; i < SLB / 2; ++i) {
+    const float2 lo = *reinterpret_cast<const float2*>(S_g + (size_t)(2 * i) * D);
+    const float2 hi = *reinterpret_cast<const float2*>(S_g + (size_t)(2 * i + 1) * D);
+    S[0][i] = pair_of(lo.x, hi.x), S[1][i] = pair_of(lo.y, hi.y);
+  }
+  float* out = p.out + (size_t)row0 * p.heads * D + h * D + j;
+  if (!landed(0)) return;
+  const int o_row = g % BLK;      // the token whose output this thread forms (threads g < BLK write)
+  // vectors of the block at hand; as soon as one is used up its place takes the next block's
+  f32x2 dots[B_DOTS][SLB / 2], keys[BLK][SLB / 2], gone_by[BLK][SLB / 2], decay[SLB / 2];
+  const float* share = blocks_smem + g * SLBP;
+#pragma unroll
+  for (int i = 0; i < B_DOTS; ++i) load_share(dots[i], share, i);
+#pragma unroll
+  for (int i = 0; i < BLK; ++i) load_share(keys[i], share, B_KEYS + i), load_share(gone_by[i], share, B_GONE + i);
+  load_share(decay, share, B_DECAY);
+  for (int b = 0; b < blocks; ++b) {
+    const float* rec = blocks_smem + (b / BCHUNK % 2 * BCHUNK + b % BCHUNK) * BREC;
+    float v[NCOL][BLK], uk[2 * N_PAIR];
+#pragma unroll
+    for (int i = 0; i < BLK; ++i) {
+      const float2 vv = *reinterpret_cast<const float2*>(rec + AT_V + i * D + j);
+      v[0][i] = vv.x, v[1][i] = vv.y;
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * N_PAIR / 4; ++i) {
+      const float4 f = *reinterpret_cast<const float4*>(rec + AT_C + 4 * i);
+      uk[4 * i] = f.x, uk[4 * i + 1] = f.y, uk[4 * i + 2] = f.z, uk[4 * i + 3] = f.w;
+    }
+    const float4 rk = *reinterpret_cast<const float4*>(rec + AT_C + C_RK + BLK * o_row);
+    const float4 ra = *reinterpret_cast<const float4*>(rec + AT_C + C_RA + BLK * o_row);
+    f32x2 s2[NCOL][B_DOTS];
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c)
+#pragma unroll
+      for (int i = 0; i < B_DOTS; ++i) s2[c][i] = mul2(dots[i][0], S[c][0]);
+#pragma unroll
+    for (int q = 1; q < SLB / 2; ++q)
+#pragma unroll
+      for (int c = 0; c < NCOL; ++c)
+#pragma unroll
+        for (int i = 0; i < B_DOTS; ++i) fma_pair(s2[c][i], dots[i][q], S[c][q]);
+    // the next block (after the last one this one again, for nothing), in the other buffer where a chunk ends
+    const int nb = min(b + 1, blocks - 1);
+    if (nb % BCHUNK == 0 && nb > b) {
+      if (!landed(nb)) break;
+      __syncthreads();       // nobody reads this chunk any more
+      if (tid == 0) fetch(nb + BCHUNK);
+    }
+    share = blocks_smem + (nb / BCHUNK % 2 * BCHUNK + nb % BCHUNK) * BREC + g * SLBP;
+    float t[NCOL][B_DOTS], mine[NCOL];
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c)
+#pragma unroll
+      for (int i = 0; i < B_DOTS; ++i) t[c][i] = low_of(s2[c][i]) + high_of(s2[c][i]);
+    // every thread of a column needs what is removed; a token's output is formed by one (its sums are passed on alone)
+#pragma unroll
+    for (int o = 1; o < GB; o <<= 1)
+#pragma unroll
+      for (int c = 0; c < NCOL; ++c)
+#pragma unroll
+        for (int i = 0; i < BLK; ++i) t[c][i] += __shfl_xor_sync(0xffffffffu, t[c][i], o);
+#pragma unroll
+    for (int i = 0; i < B_DOTS; ++i) load_share(dots[i], share, i);
+    const bool hi2 = g & 2, hi1 = g & 1;
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c) {
+      const float a0 = (hi2 ? t[c][6] : t[c][4]) + __shfl_xor_sync(0xffffffffu, hi2 ? t[c][4] : t[c][6], 2);
+      const float a1 = (hi2 ? t[c][7] : t[c][5]) + __shfl_xor_sync(0xffffffffu, hi2 ? t[c][5] : t[c][7], 2);
+      mine[c] = (hi1 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, hi1 ? a0 : a1, 1);
+#pragma unroll
+      for (int o = 4; o < GB; o <<= 1) mine[c] += __shfl_xor_sync(0xffffffffu, mine[c], o);
+    }
+    // what does not wait for the sums
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c)
+#pragma unroll
+      for (int q = 0; q < SLB / 2; ++q) {
+        S[c][q] = mul2(decay[q], S[c][q]);
+#pragma unroll
+        for (int i = 0; i < BLK; ++i) fma_pair(S[c][q], keys[i][q], pair_of(v[c][i], v[c][i]));
+      }
+    load_share(decay, share, B_DECAY);
+#pragma unroll
+    for (int i = 0; i < BLK; ++i) load_share(keys[i], share, B_KEYS + i);
+    float result[NCOL];
+#pragma unroll
+    for (int c = 0; c < NCOL; ++c) {
+      float gone[BLK];
+      int pair = 0;
+#pragma unroll
+      for (int i = 0; i < BLK; ++i) {
+        float known = 0.f;
+#pragma unroll
+        for (int jj = 0; jj < i; ++jj) known = fmaf(uk[C_UK + pair + jj], v[c][jj], known);
+        gone[i] = t[c][i] + known;
+#pragma unroll
+        for (int jj = 0; jj < i; ++jj) gone[i] = fmaf(uk[C_UA + pair + jj], gone[jj], gone[i]);
+        pair += i;
+      }
+#pragma unroll
+      for (int q = 0; q < SLB / 2; ++q)
+#pragma unroll
+        for (int i = 0; i < BLK; ++i) fma_pair(S[c][q], gone_by[i][q], pair_of(gone[i], gone[i]));
+      const float held = fmaf(rk.w, v[c][3], fmaf(rk.z, v[c][2], fmaf(rk.y, v[c][1], rk.x * v[c][0])));
+      const float lost = fmaf(ra.w, gone[3], fmaf(ra.z, gone[2], fmaf(ra.y, gone[1], ra.x * gone[0])));
+      result[c] = mine[c] + (held + lost);
+    }
+#pragma unroll
+    for (int i = 0; i < BLK; ++i) load_share(gone_by[i], share, B_GONE + i);
+    const int row = b * BLK + o_row;
+    if (g < BLK && row < rows) *reinterpret_cast<float2*>(out + (size_t)row * p.heads * D) = make_float2(result[0], result[1]);
+  }
+  pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
+  if (p.write) {
+#pragma unroll
+    for (int i = 0; i < SLB / 2; ++i) {
+      *reinterpret_cast<float2*>(S_g + (size_t)(2 * i) * D) = make_float2(low_of(S[0][i]), low_of(S[1][i]));
+      *reinterpret_cast<float2*>(S_g + (size_t)(2 * i + 1) * D) = make_float2(high_of(S[0][i]), high_of(S[1][i]));
+    }
+  }
+}
+
 // Each head's raw output divided by its root mean square, times a plain weight and sigmoid(gate),
 // rounded to T: one CTA per token, a warp per head at a time.
 template <typename T>
@@ -292,47 +606,71 @@ __global__ void __launch_bounds__(256) tanh_cast_kernel(T* __restrict__ out, con
 
 LAB_EXPORT int lab_delta_rule_head_dim() { return D; }
 
-// scratch: floats for the heads' raw outputs and the records
-LAB_EXPORT long long lab_delta_rule_scratch(int tokens, int heads) {
-  return (long long)tokens * heads * (D + REC) + REC;
+namespace {
+// Raw outputs lie first in the scratch, the records behind them on a boundary of 16 bytes.
+inline float* records_of(float* scratch, int tokens, int heads) { return scratch + ((size_t)tokens * heads * D + 3) / 4 * 4; }
+
+template <typename T>
+int launch_blocks(const DeltaParams& p, const float* r, const float* k, const float* v, const float* a, int ld, const float* d,
+                  int ld_d, const T* d_bias, const T* a_bias, int requests, float decay_rate, cudaStream_t stream) {
+  static LabShared granted;
+  const cudaError_t e = lab_allow_shared(granted, (const void*)delta_blocks_kernel, BSMEM);
+  if (e != cudaSuccess) return (int)e;
+  const int n_records = p.tokens / BLK + requests;
+  lab_launch(delta_prepare_blocks_kernel<T>, dim3(n_records, (p.heads + 7) / 8), dim3(256), 0, stream, (float*)p.rec, n_records,
+             r, k, v, a, ld, d, ld_d, d_bias, a_bias, p.q_start, requests, p.heads, decay_rate);
+  return (int)lab_launch(delta_blocks_kernel, dim3(p.heads, requests, D / BCOLS), dim3(BTHREADS), BSMEM, stream, p, n_records);
 }
 
+template <typename T>
+int launch_delta_rule(DeltaParams p, void* out, const float* r, const float* k, const float* v, const float* g, const float* a,
+                      int ld, const float* d, int ld_d, const T* d_bias, const T* a_bias, const T* norm_w, int requests,
+                      int blocks, float eps, float decay_rate, cudaStream_t stream) {
+  // the kernels that are parallel over tokens: a warp per (token, head); with few tokens the heads spread over CTAs as well
+  const dim3 per_token(p.tokens, p.tokens >= 512 ? 1 : (p.heads + 7) / 8);
+  int e = (int)cudaErrorInvalidValue;
+  if (blocks != 0) {
+    if constexpr (BLOCKS_BUILT && !std::is_same_v<T, float>)
+      e = launch_blocks<T>(p, r, k, v, a, ld, d, ld_d, d_bias, a_bias, requests, decay_rate, stream);
+  } else {
+    static LabShared granted;
+    e = (int)lab_allow_shared(granted, (const void*)delta_rule_kernel<T>, sizeof(DeltaShared));
+    if (e != 0) return e;
+    lab_launch(delta_prepare_kernel<T>, per_token, dim3(256), 0, stream, (float*)p.rec, p.tokens, r, k, v, a, ld, d, ld_d,
+               d_bias, a_bias, p.heads, decay_rate);
+    e = (int)lab_launch(delta_rule_kernel<T>, dim3(p.heads, requests, NS), dim3(NT), sizeof(DeltaShared), stream, p);
+  }
+  if (e != 0) return e;
+  return (int)lab_launch(delta_finish_kernel<T>, per_token, dim3(256), 0, stream, (T*)out, (const float*)p.out, g, ld, norm_w,
+                         p.heads, eps);
+}
+}  // namespace
+
+// Whether the walk by blocks of four tokens is built for this head size.
+LAB_EXPORT int lab_delta_rule_blocks() { return BLOCKS_BUILT; }
+
+// Floats of scratch: the heads' raw outputs and the records.  blocks: as lab_delta_rule takes it.
+LAB_EXPORT long long lab_delta_rule_scratch(int tokens, int heads, int requests, int blocks) {
+  const long long records = blocks != 0 ? ((long long)tokens / BLK + requests) * BREC : (long long)tokens * REC;
+  return (long long)tokens * heads * D + 4 + heads * records;
+}
+
+// blocks: 0, a token at a time; 1 (16-bit storage, where lab_delta_rule_blocks), four at a time.
 LAB_EXPORT int lab_delta_rule(void* out, float* scratch, const float* r, const float* k, const float* v,
                               const float* g, const float* a, int ld, const float* d, int ld_d, const void* d_bias,
                               const void* a_bias, const void* norm_w, float* state, const int* q_start,
                               const int* state_slot, int tokens, int n_requests, int heads, int n_slots, int write,
-                              float eps, float decay_rate, int dtype, cudaStream_t stream) {
+                              int blocks, float eps, float decay_rate, int dtype, cudaStream_t stream) {
   if (n_requests <= 0 || heads <= 0 || tokens <= 0) return 0;
-  float* raw = scratch;
-  float* records = raw + (size_t)tokens * heads * D;      // tokens * heads * D is a multiple of 4 floats or not:
-  records += (4 - ((size_t)tokens * heads * D) % 4) % 4;  // records start on 16 bytes (one spare record is asked for)
   DeltaParams p;
-  p.out = raw; p.rec = records; p.tokens = tokens; p.state = state; p.q_start = q_start;
+  p.out = scratch; p.rec = records_of(scratch, tokens, heads); p.tokens = tokens; p.state = state; p.q_start = q_start;
   p.state_slot = state_slot; p.heads = heads; p.n_slots = n_slots; p.write = write;
-  const size_t smem = sizeof(DeltaShared);
-  const dim3 grid(heads, n_requests, NS);
-  // the two kernels that are parallel over tokens: a warp per (token, head); with few tokens the heads
-  // spread over CTAs as well
-  const dim3 per_token(tokens, tokens >= 512 ? 1 : (heads + 7) / 8);
-  cudaError_t e;
-  if (dtype == LAB_F32) {
-    e = cudaFuncSetAttribute(delta_rule_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    lab_launch(delta_prepare_kernel<float>, per_token, dim3(256), 0, stream, records, tokens, r, k, v, a, ld, d,
-               ld_d, (const float*)d_bias, (const float*)a_bias, heads, decay_rate);
-    lab_launch(delta_rule_kernel<float>, grid, dim3(NT), smem, stream, p);
-    lab_launch(delta_finish_kernel<float>, per_token, dim3(256), 0, stream, (float*)out, (const float*)raw, g, ld,
-               (const float*)norm_w, heads, eps);
-  } else {
-    e = cudaFuncSetAttribute(delta_rule_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    lab_launch(delta_prepare_kernel<__nv_bfloat16>, per_token, dim3(256), 0, stream, records, tokens, r, k, v, a,
-               ld, d, ld_d, (const __nv_bfloat16*)d_bias, (const __nv_bfloat16*)a_bias, heads, decay_rate);
-    lab_launch(delta_rule_kernel<__nv_bfloat16>, grid, dim3(NT), smem, stream, p);
-    lab_launch(delta_finish_kernel<__nv_bfloat16>, per_token, dim3(256), 0, stream, (__nv_bfloat16*)out,
-               (const float*)raw, g, ld, (const __nv_bfloat16*)norm_w, heads, eps);
-  }
-  LAB_LAUNCH_CHECK();
+  if (dtype == LAB_F32)
+    return launch_delta_rule<float>(p, out, r, k, v, g, a, ld, d, ld_d, (const float*)d_bias, (const float*)a_bias,
+                                    (const float*)norm_w, n_requests, blocks, eps, decay_rate, stream);
+  return launch_delta_rule<__nv_bfloat16>(p, out, r, k, v, g, a, ld, d, ld_d, (const __nv_bfloat16*)d_bias,
+                                          (const __nv_bfloat16*)a_bias, (const __nv_bfloat16*)norm_w, n_requests, blocks, eps,
+                                          decay_rate, stream);
 }
 
 LAB_EXPORT int lab_tanh_cast(void* out, const float* x, long long tokens, int n, int ld, int dtype,
