@@ -8,14 +8,16 @@
 // everything here is 32-bit, the output is rounded once for the output projection.
 //
 // Kernels: the causal convolution of x with the request's last inputs kept between steps (+ SiLU), and
-// the walk.  The walk is sequential in tokens; a CTA takes some channels of one request, WL lanes a channel,
+// the walk, of which there are three: states of up to 16 entries an entry a lane, in one piece; steps of single
+// tokens of such states; larger states a share of the entries a lane, in segments.  The walk is sequential in
+// tokens; a CTA takes some channels of one request, WL lanes a channel,
 // each lane a share of the state's entries in registers.  A chunk of tokens waits in shared memory while the
 // next one arrives there (cp.async); step sizes are formed once per channel and token before the chunk is
 // walked.  From token to token passes only the state's own update: every lane leaves its share of the sum
 // over the state in shared memory, and the sums, the skip term and the gate are formed after the chunk, a
 // thread per channel and token.
 //
-// A long portion is cut into segments of tokens that are walked side by side, in two launches: the first walks every
+// A long portion of larger states is cut into segments of tokens that are walked side by side, in two launches: the first walks every
 // segment but the last from zeros (the first one from the request's state) for its closing state and the sum of its
 // step sizes, the second takes every segment again from its opening state, which follows from the segments before it
 // (S <- exp(A sum dt) S + S_segment), and leaves the outputs.  Everything stays 32-bit; the errors against 64-bit are
@@ -155,7 +157,8 @@ struct ScanParams {
   const int* q_start;
   const int* state_slot;
   int ld_x, ld_dt, ld_bc, ld_z, b_at, c_at, channels, N, n_slots, write, ld_out;
-  int vec;               // rows of all inputs may be copied 16 bytes at a time
+  int vec;               // rows of all inputs (small states: of dt_pre, x and z) may be copied 16 bytes at a time
+  int vec_bc, vec_out, vec_state;      // small states: B's and C's, the output's, the state's
   int segments;          // a request's rows are cut into at most that many segments of whole chunks
   float* states;         // [requests, segments, channels, N]: 0, a copy of the request's state; i, the state at the end
                          // of segment i - 1 (from zeros, of segment 0 from the request's state)
@@ -190,7 +193,7 @@ __host__ __device__ inline int scan_chunk_floats(int wc, int n4) { return 3 * WT
 // Lane l of a channel's WL holds the quads l, l + WL, ... of its state, R entries in all.  What bounds the walk, once
 // there are CTAs enough, is the issue of instructions: most of an entry's and token's are its exponential's, the others
 // take two entries each; a token of a CTA also takes its step sizes, gates and copies.  Measured on a B200, inputs from
-// memory, 1,792 channels of 16 entries: 8 requests of 250 tokens 82 us (115 with eight lanes a channel and an entry an
+// memory, 1,792 channels of 16 entries, before those had a walk of their own: 8 requests of 250 tokens 82 us (115 with eight lanes a channel and an entry an
 // instruction); one of 2,048 129 us in eleven segments (352 in one piece of that form), issuing in two cycles of three.
 // QUADS: the state is whole quads; else the entries that fill the last one are kept at zero (an infinite step would leave
 // no numbers there).
@@ -326,9 +329,8 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
       if (MODE == SCAN_CLOSE) dt_sum += dt;
     }
     __syncthreads();
-    // the walk: nothing but the state's own update passes from token to token (with few entries a lane four tokens in flight:
-    // one request of 2,048 tokens in segments 129 us, 131 by two; in one piece 370, 383; 8 requests 598, 625; no gain with more)
-#pragma unroll (R == 4 ? 4 : 2)
+    // the walk: nothing but the state's own update passes from token to token
+#pragma unroll 2
     for (int tt = 0; tt < nt; ++tt) {
       const float dt = b_dt[tt * WC + ch], dx = s_dx[tt * WC + ch];
       const f32x2 dt2 = pair_of(dt, dt), dx2 = pair_of(dx, dx);
@@ -336,8 +338,7 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int e = (q * WL + l) * 4;
-        if (Q * WL * 4 > 16 && e >= n4) break;
-        if (Q * WL * 4 == 16 && e >= n4) continue;
+        if (e >= n4) break;
         const ulonglong2 bq = *reinterpret_cast<const ulonglong2*>(b_b + tt * n4 + e);
         S2[2 * q] = fma2(exp_of(mul2(dt2, A2[2 * q])), S2[2 * q], mul2(dx2, bq.x));
         S2[2 * q + 1] = fma2(exp_of(mul2(dt2, A2[2 * q + 1])), S2[2 * q + 1], mul2(dx2, bq.y));
@@ -385,6 +386,304 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
   }
 }
 
+// ---- the walk of states of up to 16 entries ----------------------------------------------------------
+// A lane an entry: LN lanes a channel, 32 / LN channels a warp.  A warp forms its channels' step sizes for a chunk of WTS
+// tokens, walks it, and forms its channels' outputs; only the chunk's inputs, brought by cp.async, are shared by the CTA's
+// warps, so they meet once a chunk.  Inputs lie so that a lane reads four tokens at a time; every lane leaves its
+// share of the sum over the state in shared memory.  A request's rows are walked in one piece, whatever their number: a
+// channel's numbers depend on neither the cut nor the batch.
+// What bounds it: the issue of instructions, most of them the exponential's, by the few warps that a request's channels make
+// (six a multiprocessor for 1,792 channels of 16; they issue in two cycles of five).  The mixer around it (us, from a graph)
+// against four entries a lane, in segments from 320 tokens on: 1,792 channels, one request of 2,048 tokens 212 (220), of 700
+// 110 (121), of 319 75 (113), eight of 250 157 (172); 3,072 channels, 1,500 tokens 219 (257).
+constexpr int SMALL_STATE = 16;
+struct ScanTile {      // floats of shared memory
+  int in, chunk, dt, part, out, total;
+  __host__ __device__ ScanTile(int wc, int ln, int wts, int warps) {
+    chunk = 3 * wts * wc + 2 * wts * ln;            // dt_pre, x, z [wts][wc], then B and C [wts][ln]
+    in = 0;
+    dt = 2 * chunk;                                 // step sizes and step size times x, [wc][wts + 4] each
+    part = dt + 2 * wc * (wts + 4);                 // [warp][wts][36]
+    out = part + warps * wts * 36;                  // two chunks of [wts][wc]
+    total = out + 2 * wts * wc;
+  }
+};
+
+template <typename T, int LN, int WARPS, int WTS, bool WHOLE_LANES>
+__global__ void __launch_bounds__(32 * WARPS) selective_walk_kernel(T* __restrict__ out, const T* __restrict__ a_log,
+                                                                    const T* __restrict__ skip,
+                                                                    const T* __restrict__ dt_bias, ScanParams p) {
+  constexpr int THREADS = 32 * WARPS, CPW = 32 / LN, WC = WARPS * CPW, LD = WTS + 4, SL = 36;
+  static_assert(WTS % 4 == 0, "four tokens at a time");
+  extern __shared__ __align__(16) float smem[];
+  const ScanTile tile(WC, LN, WTS, WARPS);
+  pdl_wait();
+  const int r = blockIdx.y, c0 = blockIdx.x * WC, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int first = p.q_start[r], n = p.q_start[r + 1] - first, slot = p.state_slot[r];
+  if (n < LONG_WALK) pdl_trigger();
+  if (n <= 0) return;
+  if (slot == -1) {       // rows of padding leave zeros
+    for (int i = tid; i < n * WC; i += THREADS)
+      if (c0 + i % WC < p.channels) out[(size_t)(first + i / WC) * p.ld_out + c0 + i % WC] = from_f32<T>(0.f);
+    return;
+  }
+  if (slot < 0 || slot >= p.n_slots) {
+    if (tid == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
+    return;
+  }
+  const int N = WHOLE_LANES ? LN : p.N;
+  // a chunk's inputs set out for shared memory; channels and entries beyond the last read nothing and stay unused
+  auto fetch = [&](int t0, float* buf) {
+    const int nt = min(WTS, n - t0);
+    const size_t row0 = (size_t)(first + t0);
+    float *b_x = buf + WTS * WC, *b_z = b_x + WTS * WC, *b_b = b_z + WTS * WC, *b_c = b_b + WTS * LN;
+    if (p.vec) {
+      for (int i = tid; i < nt * (WC / 4); i += THREADS) {
+        const int cc = c0 + 4 * (i % (WC / 4));
+        if (cc >= p.channels) continue;
+        const size_t row = row0 + i / (WC / 4);
+        cp_async_f32x4(buf + 4 * i, p.dt_pre + row * p.ld_dt + cc);
+        cp_async_f32x4(b_x + 4 * i, p.x + row * p.ld_x + cc);
+        cp_async_f32x4(b_z + 4 * i, p.z + row * p.ld_z + cc);
+      }
+    } else {
+      for (int i = tid; i < nt * WC; i += THREADS) {
+        const int cc = c0 + i % WC;
+        if (cc >= p.channels) continue;
+        const size_t row = row0 + i / WC;
+        cp_async_f32(buf + i, p.dt_pre + row * p.ld_dt + cc);
+        cp_async_f32(b_x + i, p.x + row * p.ld_x + cc);
+        cp_async_f32(b_z + i, p.z + row * p.ld_z + cc);
+      }
+    }
+    if (p.vec_bc) {
+      for (int i = tid; i < nt * (N / 4); i += THREADS) {
+        const int e = 4 * (i % (N / 4)), t = i / (N / 4);
+        const float* row = p.bc + (row0 + t) * p.ld_bc + e;
+        cp_async_f32x4(b_b + t * LN + e, row + p.b_at);
+        cp_async_f32x4(b_c + t * LN + e, row + p.c_at);
+      }
+      return;
+    }
+    for (int i = tid; i < nt * N; i += THREADS) {
+      const int e = i % N, t = i / N;
+      const float* row = p.bc + (row0 + t) * p.ld_bc + e;
+      cp_async_f32(b_b + t * LN + e, row + p.b_at);
+      cp_async_f32(b_c + t * LN + e, row + p.c_at);
+    }
+  };
+  fetch(0, smem);
+  const int ch = lane / LN, e = lane % LN, mine = warp * CPW + ch, c = c0 + mine;      // this lane's channel and entry
+  const bool has = c < p.channels && e < N;
+  const float A = has ? -expf(to_f32(a_log[(size_t)c * N + e])) : 0.f;
+  float* st = p.state + ((size_t)slot * p.channels + (has ? c : 0)) * N + e;
+  float S = has ? *st : 0.f;
+  // what the tokens' terms take: lane l is at token l / CPW (+ 32 / CPW, ...) of channel l % CPW of the warp's
+  const int tc = lane % CPW, of = warp * CPW + tc;
+  const bool term = c0 + of < p.channels;
+  const float bias = term ? to_f32(dt_bias[c0 + of]) : 0.f, D = term ? to_f32(skip[c0 + of]) : 0.f;
+  float *s_dt = smem + tile.dt, *s_dx = s_dt + WC * LD, *s_part = smem + tile.part + warp * WTS * SL;
+  T* s_out = reinterpret_cast<T*>(smem + tile.out);
+  // outputs of a chunk, row by row
+  auto leave = [&](int t0, int which) {
+    const int nt = min(WTS, n - t0);
+    const T* from = s_out + which * WTS * WC;
+    constexpr int UNIT = 16 / (int)sizeof(T), PER = WC / UNIT;
+    if (PER > 0 && p.vec_out) {
+      for (int i = tid; i < nt * PER; i += THREADS) {
+        const int cc = c0 + UNIT * (i % (PER > 0 ? PER : 1)), t = i / (PER > 0 ? PER : 1);
+        if (cc < p.channels)
+          *reinterpret_cast<uint4*>(out + (size_t)(first + t0 + t) * p.ld_out + cc) = *reinterpret_cast<const uint4*>(from + UNIT * i);
+      }
+      return;
+    }
+    for (int i = tid; i < nt * WC; i += THREADS)
+      if (c0 + i % WC < p.channels) out[(size_t)(first + t0 + i / WC) * p.ld_out + c0 + i % WC] = from[i];
+  };
+  int which = 0;
+  for (int t0 = 0; t0 < n; t0 += WTS, which ^= 1) {
+    const int nt = min(WTS, n - t0);
+    const float* buf = smem + which * tile.chunk;
+    const float *b_x = buf + WTS * WC, *b_z = b_x + WTS * WC, *b_b = b_z + WTS * WC, *b_c = b_b + WTS * LN;
+    cp_async_wait_all();
+    __syncthreads();       // the chunk is here, every warp is done with the one before
+    if (t0 + WTS < n) fetch(t0 + WTS, smem + (which ^ 1) * tile.chunk);
+    if (t0 > 0) leave(t0 - WTS, which ^ 1);
+#pragma unroll
+    for (int i = 0; i < (CPW * WTS + 31) / 32; ++i) {
+      const int t = min((lane + 32 * i) / CPW, WTS - 1);      // (a chunk of few tokens: several lanes form the last one's)
+      const float dt = term ? softplus_f(buf[t * WC + of] + bias) : 0.f;      // (tokens beyond the last: never read)
+      s_dt[of * LD + t] = dt;
+      s_dx[of * LD + t] = dt * b_x[t * WC + of];
+    }
+    __syncwarp();
+    const float *my_dt = s_dt + mine * LD, *my_dx = s_dx + mine * LD, *my_b = b_b + e, *my_c = b_c + e;
+    auto token = [&](float decay, float dx, float b) {
+      S = fmaf(decay, S, dx * b);
+      if (!WHOLE_LANES) S = has ? S : 0.f;      // (an infinite step would leave no number)
+    };
+    // LOT tokens at a time: only the state's own update passes from one to the next
+    constexpr int LOT = 8;
+    int t = 0;
+    for (; t + LOT <= nt; t += LOT) {
+      float dt[LOT], dx[LOT], b[LOT], cc[LOT];
+#pragma unroll
+      for (int i = 0; i < LOT; i += 4) {
+        const float4 q = load4(my_dt + t + i), x = load4(my_dx + t + i);
+        dt[i] = q.x, dt[i + 1] = q.y, dt[i + 2] = q.z, dt[i + 3] = q.w;
+        dx[i] = x.x, dx[i + 1] = x.y, dx[i + 2] = x.z, dx[i + 3] = x.w;
+      }
+#pragma unroll
+      for (int i = 0; i < LOT; ++i) b[i] = my_b[(t + i) * LN], cc[i] = my_c[(t + i) * LN];
+#pragma unroll
+      for (int i = 0; i < LOT; ++i) dt[i] = expf(dt[i] * A);
+#pragma unroll
+      for (int i = 0; i < LOT; ++i) {
+        token(dt[i], dx[i], b[i]);
+        cc[i] = WHOLE_LANES || has ? S * cc[i] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < LOT; ++i) s_part[(t + i) * SL + lane] = cc[i];
+    }
+    for (; t < nt; ++t) {
+      token(expf(my_dt[t] * A), my_dx[t], my_b[t * LN]);
+      s_part[t * SL + lane] = WHOLE_LANES || has ? S * my_c[t * LN] : 0.f;
+    }
+    __syncwarp();
+    // the sum over the lanes (in their order), the skip term and the gate
+#pragma unroll
+    for (int i = 0; i < (CPW * WTS + 31) / 32; ++i) {
+      const int t = (lane + 32 * i) / CPW;
+      if (!term || t >= nt) continue;
+      const float* from = s_part + t * SL + tc * LN;
+      float4 sum = load4(from);
+#pragma unroll
+      for (int q = 1; q < LN / 4; ++q) {
+        const float4 v = load4(from + 4 * q);
+        sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+      }
+      const float acc = (sum.x + sum.z) + (sum.y + sum.w);
+      s_out[which * WTS * WC + t * WC + of] = from_f32<T>(fmaf(D, b_x[t * WC + of], acc) * silu_f(b_z[t * WC + of]));
+    }
+    __syncwarp();
+  }
+  pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
+  __syncthreads();
+  leave((n - 1) / WTS * WTS, which ^ 1);
+  if (has && p.write) *st = S;
+}
+
+// A step of single tokens: a thread four entries of a channel, QL threads a channel, everything straight from memory.  The
+// same sums in the same order as the walk's.  Bound by the state's way from and to memory.
+template <typename T, int QL>
+__global__ void __launch_bounds__(kThreads) selective_step_kernel(T* __restrict__ out, const T* __restrict__ a_log,
+                                                                  const T* __restrict__ skip, const T* __restrict__ dt_bias,
+                                                                  ScanParams p) {
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, q = lane % QL, r = blockIdx.y;
+  const int c = (int)((blockIdx.x * (unsigned)kThreads + threadIdx.x) / QL), N = p.N;
+  const bool live = c < p.channels;
+  float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (live) {      // (weights do not depend on the kernels before)
+    const T* from = a_log + (size_t)c * N + 4 * q;
+    if (4 * q < N) A.x = -expf(to_f32(from[0]));
+    if (4 * q + 1 < N) A.y = -expf(to_f32(from[1]));
+    if (4 * q + 2 < N) A.z = -expf(to_f32(from[2]));
+    if (4 * q + 3 < N) A.w = -expf(to_f32(from[3]));
+  }
+  const float bias = live ? to_f32(dt_bias[c]) : 0.f, D = live ? to_f32(skip[c]) : 0.f;
+  pdl_wait();
+  const int t = p.q_start[r], slot = p.state_slot[r];
+  if (p.q_start[r + 1] == t) return;
+  if (slot == -1) {       // a row of padding leaves zeros
+    if (live && q == 0) out[(size_t)t * p.ld_out + c] = from_f32<T>(0.f);
+    return;
+  }
+  if (slot < 0 || slot >= p.n_slots) {
+    if (threadIdx.x == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
+    return;
+  }
+  float4 S = make_float4(0.f, 0.f, 0.f, 0.f), b = S, cc = S;
+  float* st = p.state + ((size_t)slot * p.channels + (live ? c : 0)) * N + 4 * q;
+  const float *row_b = p.bc + (size_t)t * p.ld_bc + p.b_at + 4 * q, *row_c = p.bc + (size_t)t * p.ld_bc + p.c_at + 4 * q;
+  auto four = [&](float4& v, const float* from) {
+    if (4 * q < N) v.x = from[0];
+    if (4 * q + 1 < N) v.y = from[1];
+    if (4 * q + 2 < N) v.z = from[2];
+    if (4 * q + 3 < N) v.w = from[3];
+  };
+  if (live && p.vec_state) {
+    if (4 * q < N) S = load4(st);
+  } else if (live) {
+    four(S, st);
+  }
+  if (p.vec_bc) {
+    if (4 * q < N) b = load4(row_b), cc = load4(row_c);
+  } else {
+    four(b, row_b), four(cc, row_c);
+  }
+  const float x = live ? p.x[(size_t)t * p.ld_x + c] : 0.f, z = live ? p.z[(size_t)t * p.ld_z + c] : 0.f;
+  const float dt = live ? softplus_f(p.dt_pre[(size_t)t * p.ld_dt + c] + bias) : 0.f, dx = dt * x;
+  auto step = [&](float& s, float a, float bb, float c4, int e) {
+    s = fmaf(expf(dt * a), s, dx * bb);
+    if (4 * q + e >= N) s = 0.f;
+    return 4 * q + e < N ? s * c4 : 0.f;
+  };
+  const float4 part = make_float4(step(S.x, A.x, b.x, cc.x, 0), step(S.y, A.y, b.y, cc.y, 1), step(S.z, A.z, b.z, cc.z, 2),
+                                  step(S.w, A.w, b.w, cc.w, 3));
+  float4 sum;
+#pragma unroll
+  for (int i = 0; i < QL; ++i) {
+    const int from = lane - q + i;
+    const float px = __shfl_sync(0xffffffffu, part.x, from), py = __shfl_sync(0xffffffffu, part.y, from);
+    const float pz = __shfl_sync(0xffffffffu, part.z, from), pw = __shfl_sync(0xffffffffu, part.w, from);
+    if (i == 0) sum = make_float4(px, py, pz, pw);
+    else sum.x += px, sum.y += py, sum.z += pz, sum.w += pw;
+  }
+  if (!live) return;
+  if (q == 0) out[(size_t)t * p.ld_out + c] = from_f32<T>(fmaf(D, x, (sum.x + sum.z) + (sum.y + sum.w)) * silu_f(z));
+  if (!p.write) return;
+  if (p.vec_state) {
+    if (4 * q < N) store4(st, S);
+    return;
+  }
+  if (4 * q < N) st[0] = S.x;
+  if (4 * q + 1 < N) st[1] = S.y;
+  if (4 * q + 2 < N) st[2] = S.z;
+  if (4 * q + 3 < N) st[3] = S.w;
+}
+
+template <typename T, int LN, int WARPS, int WTS>
+int launch_walk_as(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
+                   cudaStream_t stream) {
+  constexpr int WC = WARPS * (32 / LN);
+  const long long ctas = (long long)((p.channels + WC - 1) / WC) * requests, sms = lab_sm_count();
+  size_t smem = sizeof(float) * ScanTile(WC, LN, WTS, WARPS).total;
+  // A long walk of few CTAs: no more of them a multiprocessor than need be, wherever the kernel before leaves room first
+  // (2,048 tokens by 1,792 channels of 16, with the mixer around it, 214 us; 331 where five may settle on one).
+  if (WTS == 32 && ctas <= 3 * sms) {
+    const size_t each = (size_t)(226 * 1024) / (size_t)((ctas + sms - 1) / sms) - 1024;
+    if (each > smem) smem = each / 128 * 128;
+  }
+  const bool whole = p.N == LN;
+  const auto kernel = whole ? selective_walk_kernel<T, LN, WARPS, WTS, true> : selective_walk_kernel<T, LN, WARPS, WTS, false>;
+  static LabShared granted[2];
+  const cudaError_t e = lab_allow_shared(granted[whole], (const void*)kernel, smem);
+  if (e != cudaSuccess) return (int)e;
+  return (int)lab_launch(kernel, dim3((p.channels + WC - 1) / WC, requests), dim3(32 * WARPS), smem, stream, (T*)out,
+                         (const T*)a_log, (const T*)skip, (const T*)dt_bias, p);
+}
+
+template <typename T, int LN>
+int launch_walk(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
+                int longest, cudaStream_t stream) {
+  if (longest == 1)
+    return (int)lab_launch(selective_step_kernel<T, LN / 4>, dim3((p.channels * (LN / 4) + kThreads - 1) / kThreads, requests),
+                           dim3(kThreads), 0, stream, (T*)out, (const T*)a_log, (const T*)skip, (const T*)dt_bias, p);
+  if (longest <= 8) return launch_walk_as<T, LN, 8, 8>(out, a_log, skip, dt_bias, p, requests, stream);
+  return launch_walk_as<T, LN, 4, 32>(out, a_log, skip, dt_bias, p, requests, stream);
+}
+
 template <typename T, int WL, int R, int MODE, bool QUADS>
 int launch_scan_as(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
                    cudaStream_t stream) {
@@ -409,14 +708,15 @@ int launch_scan(void* out, const void* a_log, const void* skip, const void* dt_b
 // Four lanes a channel up to 64 entries; eight beyond, where a lane's registers would not hold a quarter.
 template <typename T>
 int pick_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
-              cudaStream_t stream) {
+              int longest, cudaStream_t stream) {
+  if (p.N <= 4) return launch_walk<T, 4>(out, a_log, skip, dt_bias, p, requests, longest, stream);
+  if (p.N <= 8) return launch_walk<T, 8>(out, a_log, skip, dt_bias, p, requests, longest, stream);
+  if (p.N <= SMALL_STATE) return launch_walk<T, 16>(out, a_log, skip, dt_bias, p, requests, longest, stream);
   if (p.N % 4 != 0) {
-    if (p.N <= 16) return launch_scan<T, 4, 4, false>(out, a_log, skip, dt_bias, p, requests, stream);
     if (p.N <= 64) return launch_scan<T, 4, 16, false>(out, a_log, skip, dt_bias, p, requests, stream);
     if (p.N <= SCAN_MAX_STATE) return launch_scan<T, 8, 32, false>(out, a_log, skip, dt_bias, p, requests, stream);
     return (int)cudaErrorInvalidValue;
   }
-  if (p.N <= 16) return launch_scan<T, 4, 4>(out, a_log, skip, dt_bias, p, requests, stream);
   if (p.N <= 32) return launch_scan<T, 4, 8>(out, a_log, skip, dt_bias, p, requests, stream);
   if (p.N <= 64) return launch_scan<T, 4, 16>(out, a_log, skip, dt_bias, p, requests, stream);
   if (p.N <= 128) return launch_scan<T, 8, 16>(out, a_log, skip, dt_bias, p, requests, stream);
@@ -424,6 +724,9 @@ int pick_scan(void* out, const void* a_log, const void* skip, const void* dt_bia
   return (int)cudaErrorInvalidValue;
 }
 }  // namespace
+
+// The largest state that is walked an entry a lane, in one piece.
+LAB_EXPORT int lab_selective_scan_small_state() { return SMALL_STATE; }
 
 // The largest state (entries per channel) the walk takes.
 LAB_EXPORT int lab_selective_scan_max_state() { return SCAN_MAX_STATE; }
@@ -467,8 +770,8 @@ LAB_EXPORT int lab_selective_scan(void* out, int ld_out, const float* x, int ld_
                                   const float* bc, int ld_bc, int b_at, int c_at, const float* z, int ld_z,
                                   const void* a_log, const void* skip, const void* dt_bias, float* state,
                                   const int* q_start, const int* state_slot, int requests, int channels, int N,
-                                  int n_slots, int write, int segments, float* states, float* sums, int dtype,
-                                  cudaStream_t stream) {
+                                  int n_slots, int write, int longest, int segments, float* states, float* sums,
+                                  int dtype, cudaStream_t stream) {
   if (requests <= 0) return 0;
   if (channels <= 0 || N <= 0 || N > SCAN_MAX_STATE) return (int)cudaErrorInvalidValue;
   if (segments > 65535 || (segments > 1 && (states == nullptr || sums == nullptr))) return (int)cudaErrorInvalidValue;
@@ -477,9 +780,13 @@ LAB_EXPORT int lab_selective_scan(void* out, int ld_out, const float* x, int ld_
   p.ld_x = ld_x; p.ld_dt = ld_dt; p.ld_bc = ld_bc; p.ld_z = ld_z; p.b_at = b_at; p.c_at = c_at; p.channels = channels;
   p.N = N; p.n_slots = n_slots; p.write = write; p.ld_out = ld_out;
   p.segments = segments; p.states = states; p.sums = sums;
-  p.vec = ((ld_x | ld_dt | ld_bc | ld_z | b_at | c_at | channels | N) & 3) == 0 &&
-          ((((uintptr_t)x) | ((uintptr_t)dt_pre) | ((uintptr_t)bc) | ((uintptr_t)z)) & 15) == 0;
+  p.vec = ((ld_x | ld_dt | ld_z | channels) & 3) == 0 && ((((uintptr_t)x) | ((uintptr_t)dt_pre) | ((uintptr_t)z)) & 15) == 0;
+  p.vec_bc = ((ld_bc | b_at | c_at | N) & 3) == 0 && (((uintptr_t)bc) & 15) == 0;
+  p.vec_state = N % 4 == 0 && (((uintptr_t)state) & 15) == 0;
+  const int unit = dtype == LAB_F32 ? 4 : 8;
+  p.vec_out = channels % unit == 0 && ld_out % unit == 0 && (((uintptr_t)out) & 15) == 0;
+  if (N > SMALL_STATE) p.vec = p.vec && p.vec_bc;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
-  if (dtype == LAB_F32) return pick_scan<float>(out, a_log, skip, dt_bias, p, requests, stream);
-  return pick_scan<__nv_bfloat16>(out, a_log, skip, dt_bias, p, requests, stream);
+  if (dtype == LAB_F32) return pick_scan<float>(out, a_log, skip, dt_bias, p, requests, longest, stream);
+  return pick_scan<__nv_bfloat16>(out, a_log, skip, dt_bias, p, requests, longest, stream);
 }

@@ -1733,6 +1733,7 @@ def rope_pairs_store(proj: torch.Tensor, bias, positions: torch.Tensor, inv_freq
 # Selective scan (csrc/kernels/selective_scan.cu).
 # ----------------------------------------------------------------------------------------
 SELECTIVE_SCAN_MAX_STATE = 256
+SELECTIVE_SCAN_SMALL_STATE = 16      # up to here an entry a lane, in one piece
 
 
 def conv_silu(proj: torch.Tensor, conv_at: int, channels: int, taps: int, w: torch.Tensor, b: torch.Tensor,
@@ -1755,9 +1756,10 @@ def conv_silu(proj: torch.Tensor, conv_at: int, channels: int, taps: int, w: tor
 
 
 def scan_segments(ctas: int, longest: int) -> int:
-    """Into how many segments `selective_scan` cuts a request's rows, `ctas` CTAs walking the step in one piece and a
-    multiprocessor holding four.  Segments cost a second launch and most of the walk's work once more, so they pay while
-    they bring idle multiprocessors to work: measured with its mixer (us, from a graph), 56 CTAs and 2,048 tokens 690 in one
+    """Into how many segments `selective_scan` cuts a request's rows of states of more than 16 entries (smaller ones are
+    walked in one piece), `ctas` CTAs walking the step in one piece and a multiprocessor holding four.  Segments cost a second
+    launch and most of the walk's work once more, so they pay while they bring idle multiprocessors to work: measured with its
+    mixer (us, from a graph, states of 16 entries walked by the kernel for larger ones), 56 CTAs and 2,048 tokens 690 in one
     piece, 327 in 4, 239 in 8, 222 in 11, 226 in 16; 700 tokens 214, 158 in 4, 123 in 8; 112 CTAs and 420 tokens 195, 139 in
     4, 128 in 6; 224 CTAs and 500 tokens 246, 235 in 2, 209 in 6; 448 CTAs and 250 tokens 173, 196 in 2.  Below 320 tokens
     they would still save the device time (319 tokens 114, 91 in 8; 130 tokens 76, 71 in 8), but there the mixer launched
@@ -1786,7 +1788,9 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
     if N > SELECTIVE_SCAN_MAX_STATE:
         raise KernelError(f"selective_scan: a state of {N} entries a channel exceeds {SELECTIVE_SCAN_MAX_STATE}")
     out = torch.empty((tokens, channels), dtype=a_log.dtype, device=x.device)
-    segments = 1 if in_order else scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
+    segments = 1
+    if not in_order and N > SELECTIVE_SCAN_SMALL_STATE:
+        segments = scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
     states = sums = None
     if segments > 1:
         scratch, (states, sums) = _segment_scratch(x.device, ctx.n_requests * segments * channels * N,
@@ -1794,7 +1798,7 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
     _check(lib("selective_scan").lab_selective_scan(
         _ptr(out), out.stride(0), _ptr(x), x.stride(0), _ptr(dt_pre), dt_pre.stride(0), _ptr(bc), bc.stride(0), b_at,
         c_at, _ptr(z), z.stride(0), _ptr(a_log), _ptr(skip), _ptr(dt_bias), _ptr(state), _ptr(ctx.q_start),
-        _ptr(ctx.state_slot), ctx.n_requests, channels, N, state.shape[0], int(write), segments, states, sums,
+        _ptr(ctx.state_slot), ctx.n_requests, channels, N, state.shape[0], int(write), ctx.max_q_len, segments, states, sums,
         dtype_code(a_log.dtype), _stream()), "selective_scan", 2 if segments > 1 else 1)
     return out
 
