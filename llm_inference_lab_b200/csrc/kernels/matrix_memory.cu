@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kThreads) memory_stabilize_kernel(float* __res
                                                                     const int* __restrict__ state_slot, int requests,
                                                                     int n_slots, int H, int write, int in_order) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pair = blockIdx.x * (kThreads / 32) + warp;
+  const int pair = blockIdx.x * (blockDim.x / 32) + warp;
   if (pair >= requests * H) return;
   const int r = pair / H, h = pair - r * H;
   const int t0 = q_start[r], n = q_start[r + 1] - t0, slot = state_slot[r];
@@ -203,8 +203,10 @@ LAB_EXPORT int lab_memory_gates(float* gates, float* v_out, const float* proj, i
 LAB_EXPORT int lab_memory_stabilize(float* gates, float* m_out, float* m_state, const int* q_start, const int* state_slot,
                                     int requests, int n_slots, int H, int write, int in_order, cudaStream_t stream) {
   if (requests <= 0) return 0;
-  const int warps = kThreads / 32;
-  lab_launch(memory_stabilize_kernel, dim3((requests * H + warps - 1) / warps), dim3(kThreads), 0, stream, gates, m_out,
+  // A warp's loads and stores touch a sector a lane each, so eight warps of a CTA wait for one another's; a CTA a warp while
+  // there are few of them (28 of 1,000 rows 32 us in CTAs of eight, 7 so).
+  const int warps = requests * H <= 4 * lab_sm_count() ? 1 : kThreads / 32;
+  lab_launch(memory_stabilize_kernel, dim3((requests * H + warps - 1) / warps), dim3(32 * warps), 0, stream, gates, m_out,
              m_state, q_start, state_slot, requests, n_slots, H, write, in_order);
   LAB_LAUNCH_CHECK();
 }
