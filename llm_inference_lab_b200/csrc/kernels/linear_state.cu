@@ -20,7 +20,7 @@
 //                     rounded to T for the output projection
 //
 // T says how weights are stored and how the last result is rounded.
-#include "common.cuh"
+#include "chunks.cuh"
 
 namespace {
 
@@ -30,10 +30,6 @@ constexpr int SCAN_CT = 16;   // tokens staged per chunk
 constexpr int LONG_WALK = 256;      // tokens from which the next kernel is let in at the walk's end only
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + expf(-z)); }
-// SiLU by the hardware's 2^x and reciprocal approximations (relative error about 2^-21, as the attention
-// kernels' softmax has it): a few instructions instead of the seventy of the exact exponential and division,
-// which the recurrence's helpers would otherwise spend longer on than its walkers on their chunk.
-__device__ __forceinline__ float silu_quick(float z) { return __fdividef(z, 1.0f + fast_exp2(-1.4426950408889634f * z)); }
 __device__ __forceinline__ float sigmoid_f(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float softplus_f(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 
@@ -314,6 +310,114 @@ __global__ void __launch_bounds__(256, R <= 32 ? 3 : 2) decay_scan_dense_kernel(
   decay_scan<R, SCAN_WHOLE>(p);
 }
 
+// ---- portions of a prompt: chunks of rows side by side ------------------------------------------
+// The recurrence with its sums regrouped into products of small matrices: a first kernel forms every chunk's own contribution
+// to the state, a second one runs through a request's chunks and leaves the state before each, a third one forms the outputs
+// (chunks.cuh).  A chunk's contribution is sum_j g_63,j s_j k_j v_j^T.  Measured, two requests of 1,000 rows, 14 heads of
+// 64 x 68 (us): 15, 5 and 36, against 84 and 36 of the walk's two launches in 7 segments.  The products on the tensor cores as
+// sums of two TF32 values (mma.sync) took as long, 14 and 43, with two to three times the error.
+
+// grid (places of chunks, heads, slices of N of 64 x slices of V of Vs): sum_j g_63,j s_j k_j v_j^T in place `at` of
+// p.states [places, H, N, V]; the product of the chunk's decays in p.decays [places, H].
+template <bool VEC>
+__global__ void __launch_bounds__(CHUNK_THREADS) chunk_close_kernel(ScanParams p, int requests, int Vs, int slices) {
+  __shared__ __align__(16) float ks[CHUNK * 64], vs[CHUNK * WIDE], weight[CHUNK];
+  pdl_wait();
+  const int at = blockIdx.x, h = blockIdx.y, g = h / (p.H / p.G), tid = threadIdx.x;
+  const int n0 = blockIdx.z / slices * 64, col0 = blockIdx.z % slices * Vs, cols = min(Vs, p.V - col0), keys = min(64, p.N - n0);
+  int row0, rows;
+  chunk_rows(p.q_start, p.state_slot, requests, p.n_slots, at, row0, rows);
+  if (rows == 0) return;
+  const int quads = (cols + 3) / 4;
+  if (tid < 32) {      // two rows a lane: the product of the decays after each
+    float a[2], s[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = 2 * tid + i;
+      a[i] = t >= rows ? 1.f : p.a_tok != nullptr ? p.a_tok[(size_t)(row0 + t) * p.ld_a + h] : p.a_head[h];
+      s[i] = t >= rows ? 0.f : p.s_tok != nullptr ? p.s_tok[(size_t)(row0 + t) * p.ld_a + h] : 1.f;
+    }
+    float after = a[0] * a[1];      // of this lane's rows and those behind
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float right = __shfl_down_sync(0xffffffffu, after, o);
+      if (tid + o < 32) after *= right;
+    }
+    const float behind = __shfl_down_sync(0xffffffffu, after, 1), w1 = tid < 31 ? behind : 1.f;
+    weight[2 * tid] = a[1] * w1 * s[0], weight[2 * tid + 1] = w1 * s[1];
+    if (tid == 0 && blockIdx.z == 0) p.decays[(size_t)at * p.H + h] = after;
+  }
+  const float4 zeros = make_float4(0.f, 0.f, 0.f, 0.f);
+  const Divider by_c(quads);
+  copy_quads(CHUNK * 16, [&](int e) {
+    return e / 16 < rows ? row4<VEC>(p.k + (size_t)(row0 + e / 16) * p.ld_qk + g * p.N + n0, 4 * (e % 16), keys) : zeros;
+  }, [&](int e, float4 z) { store4(ks + 4 * e, act4(z, p.act)); });
+  __syncthreads();      // the weights
+  copy_quads(CHUNK * quads, [&](int e) {
+    return by_c.over(e) < rows ? row4<VEC>(p.v + (size_t)(row0 + by_c.over(e)) * p.ld_v + h * p.V + col0, 4 * by_c.rest(e), cols) : zeros;
+  }, [&](int e, float4 z) {
+    const float w = weight[by_c.over(e)];
+    z = act4(z, p.act);
+    store4(vs + by_c.over(e) * WIDE + 4 * by_c.rest(e), make_float4(z.x * w, z.y * w, z.z * w, z.w * w));
+  });
+  __syncthreads();
+  const int n = by_c.over(tid) * 8, c = by_c.rest(tid) * 4;
+  if (n >= keys) return;
+  Tile acc;
+  acc.clear();
+  for (int t0 = 0; t0 < CHUNK; t0 += RUN) {
+    Tile part;
+    part.clear();
+#pragma unroll 4
+    for (int t = t0; t < t0 + RUN; ++t) part.step(ks + t * 64 + n, ks + t * 64 + n + 4, vs + t * WIDE + c);
+    acc.add(part);
+  }
+  float* dst = p.states + (((size_t)at * p.H + h) * p.N + n0 + n) * p.V + col0 + c;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (n + i >= keys) break;
+    if (VEC) store4(dst + (size_t)i * p.V, make_float4(acc.get(i, 0), acc.get(i, 1), acc.get(i, 2), acc.get(i, 3)));
+    else
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < cols) dst[(size_t)i * p.V + j] = acc.get(i, j);
+  }
+}
+
+// grid (blocks of N V entries, heads, requests): an entry of the state a thread, through the request's chunks in order; what a
+// chunk contributes makes way for the state before it.
+__global__ void __launch_bounds__(256) chunk_open_kernel(ScanParams p) {
+  pdl_wait();
+  const int h = blockIdx.y, r = blockIdx.z, e = blockIdx.x * 256 + threadIdx.x, first = p.q_start[r], rows = p.q_start[r + 1] - first;
+  const int slot = p.state_slot[r], NV = p.N * p.V;
+  if (rows <= 0 || slot == -1 || e >= NV) return;
+  if (slot < 0 || slot >= p.n_slots) {
+    if (e == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
+    return;
+  }
+  float* state = p.state + ((size_t)slot * p.H + h) * NV + e;
+  const int chunks = (rows + CHUNK - 1) / CHUNK;
+  const size_t at = (size_t)first_chunk(first, r) * p.H + h, next = p.H;
+  float* own = p.states + at * NV + e;
+  const float* decay = p.decays + at;
+  float S = *state;
+  constexpr int AHEAD = 8;
+  float l[AHEAD], a[AHEAD];
+  for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (c0 + i < chunks) l[i] = own[(c0 + i) * next * NV], a[i] = decay[(c0 + i) * next];
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i)
+      if (c0 + i < chunks) {
+        own[(c0 + i) * next * NV] = S;
+        S = fmaf(a[i], S, l[i]);
+      }
+  }
+  if (p.write) *state = S;
+  pdl_trigger();
+}
+
 // ---- state-space mixer: convolution, step sizes, decays ---------------------------------------
 struct SsmParams {
   const float* proj;     // [tokens, ld]
@@ -449,22 +553,45 @@ int launch_scan_as(const ScanParams& p, int requests, int vs, cudaStream_t strea
 template <int R>
 int launch_scan(const ScanParams& p, int requests, int vs, cudaStream_t stream) {
   if (p.segments <= 1) return launch_scan_as<R, SCAN_WHOLE>(p, requests, vs, stream);
-  const int e = launch_scan_as<R, SCAN_CLOSE>(p, requests, vs, stream);
-  return e != 0 ? e : launch_scan_as<R, SCAN_OUTPUT>(p, requests, vs, stream);
+  if constexpr (R > 32) {      // (fewer key channels go in chunks)
+    const int e = launch_scan_as<R, SCAN_CLOSE>(p, requests, vs, stream);
+    return e != 0 ? e : launch_scan_as<R, SCAN_OUTPUT>(p, requests, vs, stream);
+  }
+  return (int)cudaErrorInvalidValue;
+}
+
+// Three launches: see "portions of a prompt".
+int launch_chunks(const ScanParams& p, int requests, int tokens, cudaStream_t stream) {
+  const int Vs = chunk_slice(p.V), slices = (p.V + Vs - 1) / Vs;
+  cudaError_t e = lab_launch(p.vec ? chunk_close_kernel<true> : chunk_close_kernel<false>,
+                             dim3(first_chunk(tokens, requests), p.H, (p.N + 63) / 64 * slices), dim3(CHUNK_THREADS), 0, stream, p, requests, Vs, slices);
+  if (e != cudaSuccess) return (int)e;
+  e = lab_launch(chunk_open_kernel, dim3((p.N * p.V + 255) / 256, p.H, requests), dim3(256), 0, stream, p);
+  if (e != cudaSuccess) return (int)e;
+  ChunkParams c;
+  c.out = p.out; c.ld_o = p.ld_o; c.q = p.q; c.k = p.k; c.ld_qk = p.ld_qk; 
+  c.v = p.v; c.ld_v = p.ld_v; c.a = p.a_tok != nullptr ? p.a_tok : p.a_head; c.a_row = p.a_tok != nullptr ? p.ld_a : 0; c.a_head = 1;
+  c.s = p.s_tok; c.states = p.states; c.q_start = p.q_start; c.state_slot = p.state_slot; c.requests = requests;
+  c.n_slots = p.n_slots; c.H = p.H; c.G = p.G; c.N = p.N; c.V = p.V; c.act = p.act; c.vec = p.vec;
+  return launch_chunk_outputs(c, tokens, stream);
 }
 
 }  // namespace
+
+// Places of chunks (states of N x V and a decay per place and head) that `lab_decay_scan` wants for a step in chunks.
+LAB_EXPORT int lab_decay_scan_places(int tokens, int requests) { return first_chunk(tokens, requests); }
 
 // Largest key size the recurrence kernel is built for.
 LAB_EXPORT int lab_decay_scan_max_keys() { return SCAN_P * 64; }
 
 // vs: columns of the state a CTA takes (8, 16 or 32).  segments > 1: every request's rows are cut into at most that many;
-// `states` [requests, segments, H, N, V] and `decays` [requests, segments, H] are scratch.
+// `states` [requests, segments, H, N, V] and `decays` [requests, segments, H] are scratch.  chunk_tokens > 0 (up to 128 key
+// channels): the step's rows, which are taken in chunks side by side; the scratch is then [places, H, N, V] and [places, H].
 LAB_EXPORT int lab_decay_scan(float* out, int ld_o, const float* q, const float* k, int ld_qk, const float* v, int ld_v,
                               const float* a_tok, const float* s_tok, int ld_a, const float* a_head, float* state,
                               const int* q_start, const int* state_slot, int requests, int n_slots, int H, int G, int N,
-                              int V, int act, int write, int vs, int segments, float* states, float* decays,
-                              cudaStream_t stream) {
+                              int V, int act, int write, int vs, int segments, int chunk_tokens, float* states,
+                              float* decays, cudaStream_t stream) {
   if (requests <= 0) return 0;
   if (segments > 1 && (states == nullptr || decays == nullptr || (long long)requests * segments > 65535))
     return (int)cudaErrorInvalidValue;
@@ -478,6 +605,10 @@ LAB_EXPORT int lab_decay_scan(float* out, int ld_o, const float* q, const float*
   // 16-byte copies: every row of q, k and v, and every head's and slice's start in it, on a 16-byte boundary
   p.vec = N % 4 == 0 && V % 4 == 0 && ld_qk % 4 == 0 && ld_v % 4 == 0 &&
           ((((uintptr_t)q) | ((uintptr_t)k) | ((uintptr_t)v)) & 15) == 0;
+  if (chunk_tokens > 0) {
+    if (states == nullptr || decays == nullptr || N > 128 || requests > 65535 || H > 65535) return (int)cudaErrorInvalidValue;
+    return launch_chunks(p, requests, chunk_tokens, stream);
+  }
   if (N <= SCAN_P * 4) return launch_scan<4>(p, requests, vs, stream);
   if (N <= SCAN_P * 8) return launch_scan<8>(p, requests, vs, stream);
   if (N <= SCAN_P * 16) return launch_scan<16>(p, requests, vs, stream);

@@ -1574,10 +1574,21 @@ def decay_scan_supported(keys: int) -> bool:
     return 1 <= keys <= 256
 
 
+def decay_scan_chunks(ctas: int, keys: int, longest: int) -> bool:
+    """Whether `decay_scan` takes a step's rows in chunks of 64 side by side (three launches), `ctas` CTAs walking the step in
+    one piece.  Measured with the matrix memory around it, 14 heads of 64 x 68 (us, kernel by kernel, chunks / walk, the walk
+    of 450 rows on in segments): two requests of 1,000 rows 126 / 202, one of 2,048 137 / 241, eight of 250 118 / 135; 12 heads
+    of 128 x 132: one of 1,500 187 / 376, four of 300 170 / 182.  Shorter portions save device time (from a graph one of 420
+    rows 59 / 104, 200 56 / 66, 100 64 / 68, 64 55 / 45), but there the mixer launched kernel by kernel is bound by the
+    host, which two more launches and the scratch cost 12 us (420 rows 108 / 105, 200 108 / 96)."""
+    return keys <= 128 and (longest >= 450 or (longest >= 200 and ctas >= sm_count()))
+
+
 def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) -> int:
-    """Into how many segments `decay_scan` cuts a request's rows, `ctas` CTAs walking the step in one piece; a
-    multiprocessor holds four or five of up to 64 key channels, three of more.  Segments cost most of the walk's work
-    once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it (us, from a graph): 42
+    """Into how many segments `decay_scan` cuts a request's rows of more than 128 key channels (fewer go in chunks), `ctas`
+    CTAs walking the step in one piece; a multiprocessor holds three.  Segments cost most of the walk's work
+    once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it (us, from a graph,
+    states of 64 key channels, which went this way): 42
     CTAs and 2,048 tokens 418 in one piece, 288 in 4, 236 in 8, 239 in 15; 460 tokens 113, 82 in 8; 84 CTAs and 1,000 tokens
     236, 201 in 4, 198 in 8; 420 tokens 113, 105 in 4; 168 CTAs and 500 tokens 182, 186 in 2, 176 in 4; 336 and 250 tokens
     137, 169 in 2.  Below 450 tokens they would still save the device time (42 CTAs and 300 tokens 84, 67 in 8), but there
@@ -1626,15 +1637,21 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     else:
         vs = 32 if pairs * -(-vdim // 32) >= sm_count() else (16 if pairs * -(-vdim // 16) >= sm_count() else 8)
     vs = min(vs, max(8, 1 << (vdim - 1).bit_length()))
-    segments = 1 if in_order else decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
+    segments, chunk_tokens, launches = 1, 0, 1
     states = decays = None
-    if segments > 1:
-        scratch, (states, decays) = _segment_scratch(v.device, pairs * segments * keys * vdim, pairs * segments)
+    if not in_order and decay_scan_chunks(pairs * -(-vdim // vs), keys, ctx.max_q_len):
+        places = lib("linear_state").lab_decay_scan_places(tokens, ctx.n_requests)
+        scratch, (states, decays) = _segment_scratch(v.device, places * heads * keys * vdim, places * heads)
+        chunk_tokens, launches = tokens, 3
+    elif not in_order and keys > 128:
+        segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
+        if segments > 1:
+            scratch, (states, decays) = _segment_scratch(v.device, pairs * segments * keys * vdim, pairs * segments)
+            launches = 2
     _check(lib("linear_state").lab_decay_scan(
         _ptr(out), out.stride(0), _ptr(q), _ptr(k), q.stride(0), _ptr(v), v.stride(0), _ptr(a_tok), _ptr(s_tok), ld_a,
         _ptr(a_head), _ptr(state), _ptr(ctx.q_start), _ptr(ctx.state_slot), ctx.n_requests, state.shape[0], heads, groups,
-        keys, vdim, int(silu), int(write), vs, segments, states, decays, _stream()), "decay_scan",
-        2 if segments > 1 else 1)
+        keys, vdim, int(silu), int(write), vs, segments, chunk_tokens, states, decays, _stream()), "decay_scan", launches)
     return out
 
 
