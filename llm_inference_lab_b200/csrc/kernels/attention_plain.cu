@@ -19,6 +19,8 @@
 // exp(sinks[h]) instead), and `dist_bias` [n_q, bias_len]: a number per head and distance query - key that is
 // added to the scaled score, distances from bias_len - 1 on sharing the last entry.  `softcap` c > 0: the scaled score
 // s becomes c * tanh(s / c) first.  `out_f32`: the output is 32-bit whatever T is.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace {
@@ -127,21 +129,22 @@ __global__ void __launch_bounds__(WARPS * 32) attention_plain_kernel(
 }
 
 // ---- tiles of query rows ------------------------------------------------------------------------
-// A CTA takes 8 WPG rows: neighbouring tokens with the query heads that share one kv head (or some of them, where they
+// A CTA takes 4 RQ WPG rows: neighbouring tokens with the query heads that share one kv head (or some of them, where they
 // are more than the tile).  PARTS groups of WPG warps: chunk c of 32 keys goes to group c mod PARTS, whose keys and
 // values come to its own buffers by cp.async, the next chunk's keys while the values of this one are used and the other
-// way round.  A warp takes 8 rows: scores with a key per lane (the row's query as broadcasts, two products an
-// instruction: sums of even and odd entries apart), the weights left in shared memory, then the weighted sum with two
-// neighbouring entries of the head per lane.  A row's own arithmetic is the same in every tile and batch.  With the
+// way round.  A warp takes 4 RQ rows.  For the scores a lane has four of the rows and every KG-th key of the chunk (two
+// products an instruction: sums of even and odd entries apart); the weights are left in shared memory; for the weighted sum it
+// has four rows and every KG-th quad of the head's entries.  A row's own arithmetic is the same in every tile and batch.  With the
 // requests' first rows (`q_start`) no tile holds rows of two requests: a CTA finds its request by a scan over their
 // numbers of tiles, and single tokens beside a prompt's portion are walked side by side.  Without, rows of another request
 // in the tile take a pass of their own, after the first.
 //
-// What bounds it: multiply-adds and loads from shared memory, about even with 8 rows to a warp.  The other kernel's block
-// per (row, head) reads a row's keys and values once per head and row.  Measured on a B200, 32-bit, 14 query and 2 kv
-// heads of 64 (the other kernel in brackets): a prompt of 517 53 us (560), 8 single tokens after 520 36 us (57), one after
-// 3,000 155 us (296), where a row's chain of chunks bounds it; 12 and 2 heads of 128, 300 rows after 500 174 us (1,330).
-constexpr int RW = 8;      // rows a warp takes
+// What bounds it: the multiply-adds (a quarter of the time of 2,000 rows) and what goes around them, the loads of their operands
+// from shared memory, exponentials and hand-overs; a lane with one row and key (or entry pair) of eight loaded twice as much and
+// looked at every value for infinities.  The other kernel's block per (row, head) reads a row's keys and values once per head
+// and row.  Measured on a B200, 32-bit, 14 query and 2 kv heads of 64 (us; the former lanes, then the other kernel in brackets):
+// a prompt of 517 43 (54, 560), two of 1,000 208 (299), 8 single tokens after 520 27 (36, 57), where a row's chain of chunks
+// bounds it; 12 and 2 heads of 128, 300 rows after 500 131 (177, 1,330).
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool has) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(has ? 16 : 0)
@@ -174,18 +177,21 @@ struct RowsParams {
 };
 
 template <typename T> __host__ __device__ constexpr int rows_ld(int d) { return d + 16 / (int)sizeof(T); }
-template <typename T> static int rows_smem(int d, int parts, int wpg) {
-  return 4 * RW * wpg * d + (int)sizeof(T) * parts * 2 * 32 * rows_ld<T>(d) + 4 * parts * wpg * 32 * RW;
+template <typename T> static int rows_smem(int d, int parts, int wpg, int rw) {
+  return 4 * rw * wpg * d + (int)sizeof(T) * parts * 2 * 32 * rows_ld<T>(d) + 4 * parts * wpg * 32 * (rw + 4);
 }
 
-template <typename T, int D, int PARTS, int WPG>
-__global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsParams p) {
+template <typename T, int D, int PARTS, int WPG, int RQ>
+__global__ void __launch_bounds__(PARTS * 32 * WPG, D == 64 || (D == 128 && RQ == 2) ? 16 / (PARTS * WPG) : 1) attention_rows_kernel(RowsParams p) {
   extern __shared__ __align__(16) char ap_smem[];
-  constexpr int R = RW * WPG, NT = PARTS * 32 * WPG, DP = D ? (D + 63) / 64 : 4;
+  constexpr int RW = 4 * RQ, R = RW * WPG, NT = PARTS * 32 * WPG;
+  constexpr int KG = 32 / RQ, KPL = 32 / KG;                        // key groups, a lane's keys of a chunk
+  constexpr int DP = ((D ? D : 256) + 4 * KG - 1) / (4 * KG);       // a lane's quads of a head's entries
+  constexpr int WLD = RW + 4;                                       // floats between two keys' weights
   const int d = D ? D : p.d, ld = rows_ld<T>(d);
   float* qs = reinterpret_cast<float*>(ap_smem);                                       // [R][d]
   T* kv = reinterpret_cast<T*>(ap_smem + 4 * R * d);                                   // [PARTS][keys, values][32][ld]
-  float* weights = reinterpret_cast<float*>(kv + PARTS * 2 * 32 * ld);                 // [PARTS][WPG][32][RW]
+  float* weights = reinterpret_cast<float*>(kv + PARTS * 2 * 32 * ld);                 // [PARTS][WPG][32][WLD]
   __shared__ int s_req[R], s_pos[R];
   pdl_trigger();
   const int tid = threadIdx.x, lane = tid & 31, part = tid / (32 * WPG), warp = (tid >> 5) % WPG;
@@ -234,8 +240,9 @@ __global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsPa
 
   T* keys = kv + (size_t)part * 2 * 32 * ld;
   T* values = keys + 32 * ld;
-  float* mine = weights + (part * WPG + warp) * 32 * RW;
-  const float* qw = qs + warp * RW * d;
+  float* mine = weights + (part * WPG + warp) * 32 * WLD;
+  const int rq = lane / KG, kg = lane % KG;      // this lane's rows 4 rq .. of the warp's, its group
+  const float* qw = qs + (warp * RW + 4 * rq) * d;
   auto group_sync = [&]() {      // the warps of this group
     if (WPG == 1) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(1 + part), "r"(32 * WPG) : "memory");
@@ -287,110 +294,158 @@ __global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsPa
       cp_async_commit();
     };
 
-    float m[RW], l[RW];
-    unsigned long long acc[RW][DP];
+    float m[4], l[4][KPL];
+    unsigned long long acc[4][DP][2];
+    // An infinity or NaN among the values counts for the rows that give it a weight only.  The first pass does not look; if a
+    // sum is not finite in the end, a second one leaves terms of weight zero out (finite ones add nothing either way).
+    for (bool guarded = false;; guarded = true) {
 #pragma unroll
-    for (int i = 0; i < RW; ++i) {
-      m[i] = -INFINITY, l[i] = 0.f;
+      for (int i = 0; i < 4; ++i) {
+        m[i] = -INFINITY;
 #pragma unroll
-      for (int u = 0; u < DP; ++u) acc[i][u] = 0ull;
-    }
-    int c = settle(part);
-    long long base = place(c);
-    fetch(keys, p.cache_k, base, c <= last);
-    fetch(values, p.cache_v, base, c <= last);
-    while (c <= last) {
-      const int cn = settle(c + PARTS);
-      const long long base_n = place(cn);
-      cp_async_wait<1>();
-      group_sync();
-      // scores of the warp's rows with key 32 c + lane
-      unsigned long long dot[RW];
+        for (int k = 0; k < KPL; ++k) l[i][k] = 0.f;
 #pragma unroll
-      for (int i = 0; i < RW; ++i) dot[i] = 0ull;
-      const T* kr = keys + lane * ld;
-#pragma unroll 4
-      for (int e = 0; e < d; e += 4) {
-        const float4 kq = load4(kr + e);
-        const unsigned long long k_lo = pair_of(kq.x, kq.y), k_hi = pair_of(kq.z, kq.w);
-        ulonglong2 qv[RW];
-#pragma unroll
-        for (int i = 0; i < RW; ++i) qv[i] = *reinterpret_cast<const ulonglong2*>(qw + i * d + e);
-#pragma unroll
-        for (int i = 0; i < RW; ++i) fma_pair(dot[i], qv[i].x, k_lo);
-#pragma unroll
-        for (int i = 0; i < RW; ++i) fma_pair(dot[i], qv[i].y, k_hi);
+        for (int u = 0; u < DP; ++u) acc[i][u][0] = acc[i][u][1] = 0ull;
       }
-      group_sync();
-      fetch(keys, p.cache_k, base_n, cn <= last);      // the keys' buffer is free
-      const int j = c * 32 + lane;
+      int c = settle(part);
+      long long base = place(c);
+      fetch(keys, p.cache_k, base, c <= last);
+      fetch(values, p.cache_v, base, c <= last);
+      while (c <= last) {
+        const int cn = settle(c + PARTS);
+        const long long base_n = place(cn);
+        cp_async_wait<1>();
+        group_sync();
+        const unsigned there = __ballot_sync(0xffffffffu, base >= 0);      // the chunk's keys that may be read
+        // scores of the lane's rows with its keys; sums of even and odd entries apart
+        unsigned long long dot[4][KPL];
 #pragma unroll
-      for (int i = 0; i < RW; ++i) {
-        const int r = warp * RW + i, pos = s_pos[r];
-        const int first = lab_first_key(pos, p.window);
-        const int kept = p.window > 0 && p.keep_first > 0 ? min(p.keep_first, first) : 0;
-        float s = -INFINITY;
-        if (r >= r0 && r < r1 && base >= 0 && j <= pos && (j >= first || j < kept)) {
-          s = (low_of(dot[i]) + high_of(dot[i])) * p.scale;
-          if (p.softcap > 0.f) s = p.softcap * tanhf(s / p.softcap);
-          if (p.dist_bias != nullptr) s += p.dist_bias[(size_t)head_of(r) * p.bias_len + min(pos - j, p.bias_len - 1)];
-        }
-        const float m_new = fmaxf(m[i], warp_max(s));
-        float pj = 0.f;
-        if (m_new != -INFINITY) {      // (else no readable key so far)
-          pj = s == -INFINITY ? 0.f : expf(s - m_new);
-          const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
-          l[i] = l[i] * corr + pj;
-          const unsigned long long cc = pair_of(corr, corr);
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int u = 0; u < DP; ++u) asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][u]) : "l"(cc));
-          m[i] = m_new;
-        }
-        mine[lane * RW + i] = pj;
-      }
-      cp_async_wait<1>();
-      group_sync();
-      // the weighted sum: a key's weights of all rows, its entries 2 lane, 2 lane + 1 (and 64 further on)
-#pragma unroll 4
-      for (int jj = 0; jj < 32; ++jj) {
-        const float4 w0 = load4(mine + jj * RW), w1 = load4(mine + jj * RW + 4);
-        const float w[RW] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          for (int k = 0; k < KPL; ++k) dot[i][k] = 0ull;
+        const T* kr = keys + kg * ld;
+#pragma unroll 2
+        for (int e = 0; e < d; e += 4) {
+          unsigned long long k_lo[KPL], k_hi[KPL];
 #pragma unroll
-        for (int u = 0; u < DP; ++u) {
-          const int e = 2 * lane + 64 * u;
-          if (D % 64 != 0 || D == 0) {
-            if (e >= d) break;
+          for (int k = 0; k < KPL; ++k) {
+            const float4 kq = load4(kr + k * KG * ld + e);
+            k_lo[k] = pair_of(kq.x, kq.y), k_hi[k] = pair_of(kq.z, kq.w);
           }
-          const float2 v = load2(values + jj * ld + e);
-          const unsigned long long vv = pair_of(v.x, v.y);
-          if (v.x * 0.f + v.y * 0.f == 0.f) {
 #pragma unroll
-            for (int i = 0; i < RW; ++i) fma_pair(acc[i][u], pair_of(w[i], w[i]), vv);
-          } else {      // an infinity or NaN counts for the rows that give it a weight only
+          for (int i = 0; i < 4; ++i) {
+            const ulonglong2 qv = *reinterpret_cast<const ulonglong2*>(qw + i * d + e);
 #pragma unroll
-            for (int i = 0; i < RW; ++i)
-              if (w[i] != 0.f) fma_pair(acc[i][u], pair_of(w[i], w[i]), vv);
+            for (int k = 0; k < KPL; ++k) fma_pair(dot[i][k], qv.x, k_lo[k]);
+#pragma unroll
+            for (int k = 0; k < KPL; ++k) fma_pair(dot[i][k], qv.y, k_hi[k]);
           }
         }
-      }
-      group_sync();
-      fetch(values, p.cache_v, base_n, cn <= last);
-      c = cn;
-      base = base_n;
-    }
-    cp_async_wait<0>();
-    __syncthreads();      // every buffer has been read: the parts' results take their place
-    float* results = reinterpret_cast<float*>(kv);      // [PARTS][R][d + 2]
+        group_sync();
+        fetch(keys, p.cache_k, base_n, cn <= last);      // the keys' buffer is free
+        float w[KPL][4];
 #pragma unroll
-    for (int i = 0; i < RW; ++i) {
-      float* to = results + (part * R + warp * RW + i) * (d + 2);
-      const float all = warp_sum(l[i]);
-      if (lane == 0) to[d] = m[i], to[d + 1] = all;
+        for (int i = 0; i < 4; ++i) {
+          const int r = warp * RW + 4 * rq + i, pos = s_pos[r];
+          const int first = lab_first_key(pos, p.window);
+          const int kept = p.window > 0 && p.keep_first > 0 ? min(p.keep_first, first) : 0;
+          float s[KPL], top = -INFINITY;
+#pragma unroll
+          for (int k = 0; k < KPL; ++k) {
+            const int key = kg + KG * k, j = c * 32 + key;
+            s[k] = -INFINITY;
+            if (r >= r0 && r < r1 && (there >> key & 1u) != 0u && j <= pos && (j >= first || j < kept)) {
+              s[k] = (low_of(dot[i][k]) + high_of(dot[i][k])) * p.scale;
+              if (p.softcap > 0.f) s[k] = p.softcap * tanhf(s[k] / p.softcap);
+              if (p.dist_bias != nullptr) s[k] += p.dist_bias[(size_t)head_of(r) * p.bias_len + min(pos - j, p.bias_len - 1)];
+            }
+            top = fmaxf(top, s[k]);
+          }
+#pragma unroll
+          for (int o = KG / 2; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+          const float m_new = fmaxf(m[i], top);
+#pragma unroll
+          for (int k = 0; k < KPL; ++k) w[k][i] = 0.f;
+          if (m_new != -INFINITY) {      // (else no readable key so far)
+            const float corr = m[i] == -INFINITY ? 0.f : expf(m[i] - m_new);
+#pragma unroll
+            for (int k = 0; k < KPL; ++k) {
+              w[k][i] = s[k] == -INFINITY ? 0.f : expf(s[k] - m_new);
+              l[i][k] = l[i][k] * corr + w[k][i];
+            }
+            const unsigned long long cc = pair_of(corr, corr);
+#pragma unroll
+            for (int u = 0; u < DP; ++u) {
+              asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][u][0]) : "l"(cc));
+              asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(acc[i][u][1]) : "l"(cc));
+            }
+            m[i] = m_new;
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < KPL; ++k) store4(mine + (kg + KG * k) * WLD + 4 * rq, make_float4(w[k][0], w[k][1], w[k][2], w[k][3]));
+        cp_async_wait<1>();
+        group_sync();
+        // the weighted sum: a key's weights of the lane's rows, its quads kg, kg + KG, .. of the entries
+        auto weighted = [&](auto guard) {
+#pragma unroll 4
+          for (int jj = 0; jj < 32; ++jj) {
+            const float4 w4 = load4(mine + jj * WLD + 4 * rq);
+            const float wt[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int u = 0; u < DP; ++u) {
+              const int e = 4 * (kg + KG * u);
+              if (D % (4 * KG) != 0 || D == 0) {
+                if (e >= d) break;
+              }
+              const float4 v = load4(values + jj * ld + e);
+              const unsigned long long v_lo = pair_of(v.x, v.y), v_hi = pair_of(v.z, v.w);
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (decltype(guard)::value && wt[i] == 0.f) continue;
+                const unsigned long long ww = pair_of(wt[i], wt[i]);
+                fma_pair(acc[i][u][0], ww, v_lo);
+                fma_pair(acc[i][u][1], ww, v_hi);
+              }
+            }
+          }
+        };
+        if (guarded) weighted(std::true_type{});
+        else weighted(std::false_type{});
+        group_sync();
+        fetch(values, p.cache_v, base_n, cn <= last);
+        c = cn;
+        base = base_n;
+      }
+      bool finite = true;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int u = 0; u < DP; ++u)
+          finite &= isfinite(low_of(acc[i][u][0])) && isfinite(high_of(acc[i][u][0])) && isfinite(low_of(acc[i][u][1])) &&
+                    isfinite(high_of(acc[i][u][1]));
+      cp_async_wait<0>();
+      if (!__syncthreads_or(!finite && !guarded)) break;      // every buffer has been read
+    }
+    float* results = reinterpret_cast<float*>(kv);      // the parts' results take the buffers' place: [PARTS][R][d + 2]
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float* to = results + (part * R + warp * RW + 4 * rq + i) * (d + 2);
+      // (the order of a sum over 32 lanes with a key each: half with half)
+#pragma unroll
+      for (int o = KPL / 2; o > 0; o /= 2)
+#pragma unroll
+        for (int k = 0; k < o; ++k) l[i][k] += l[i][k + o];
+      float all = l[i][0];
+#pragma unroll
+      for (int o = KG / 2; o > 0; o >>= 1) all += __shfl_xor_sync(0xffffffffu, all, o);
+      if (kg == 0) to[d] = m[i], to[d + 1] = all;
 #pragma unroll
       for (int u = 0; u < DP; ++u) {
-        const int e = 2 * lane + 64 * u;
-        if (e < d) to[e] = low_of(acc[i][u]);
-        if (e + 1 < d) to[e + 1] = high_of(acc[i][u]);
+        const int e = 4 * (kg + KG * u);
+        if (e >= d) break;
+        to[e] = low_of(acc[i][u][0]), to[e + 1] = high_of(acc[i][u][0]);
+        to[e + 2] = low_of(acc[i][u][1]), to[e + 3] = high_of(acc[i][u][1]);
       }
     }
     __syncthreads();
@@ -419,21 +474,24 @@ __global__ void __launch_bounds__(PARTS * 32 * WPG) attention_rows_kernel(RowsPa
   }
 }
 
-template <typename T, int D, int PARTS, int WPG>
+template <typename T, int D, int PARTS, int WPG, int RQ>
 int launch_rows(RowsParams p, cudaStream_t stream) {
-  const int smem = rows_smem<T>(p.d, PARTS, WPG);
+  const int smem = rows_smem<T>(p.d, PARTS, WPG, 4 * RQ);
   static LabShared granted;
-  const cudaError_t e = lab_allow_shared(granted, (const void*)attention_rows_kernel<T, D, PARTS, WPG>, smem);
+  const cudaError_t e = lab_allow_shared(granted, (const void*)attention_rows_kernel<T, D, PARTS, WPG, RQ>, smem);
   if (e != cudaSuccess) return (int)e;
   if (p.tile_tokens == 1) p.q_start = nullptr;
   // with the requests' borders: every request may end in a tile that is not full
   const long long more = p.q_start != nullptr ? (long long)p.requests * (p.tile_tokens - 1) : p.tile_tokens - 1;
   const long long tiles = (p.tokens + more) / p.tile_tokens * p.head_tiles;
-  return (int)lab_launch(attention_rows_kernel<T, D, PARTS, WPG>, dim3((unsigned)tiles, p.n_kv), dim3(PARTS * 32 * WPG),
+  return (int)lab_launch(attention_rows_kernel<T, D, PARTS, WPG, RQ>, dim3((unsigned)tiles, p.n_kv), dim3(PARTS * 32 * WPG),
                          smem, stream, p);
 }
 
-// Sixteen rows a CTA halve what it reads, eight give twice the CTAs: sixteen once they fill every multiprocessor twice.
+// Sixteen rows a CTA halve what it reads, eight give twice the CTAs: sixteen once they fill every multiprocessor twice.  With
+// heads of 64 thirty-two, sixteen to a warp, once they fill every multiprocessor four times: fewer leave the long rows' CTAs
+// alone at the end.  Measured (us, 32 / 16 rows, 14 and 2 heads): one prompt of 1,200 143 / 162, 1,600 246 / 268, 800 85 / 84,
+// 517 59 / 43, two of 1,000 208 / 234, three of 400 85 / 81, eight of 250 120 / 127.
 template <typename T>
 int pick_rows(RowsParams p, bool single, cudaStream_t stream) {
   const int group = p.n_q / p.n_kv;
@@ -442,12 +500,13 @@ int pick_rows(RowsParams p, bool single, cudaStream_t stream) {
     p.head_tiles = (group + rows - 1) / rows;
     return ((long long)p.tokens + p.tile_tokens - 1) / p.tile_tokens * p.head_tiles * p.n_kv;
   };
-  const bool wide = shape(2 * RW) >= 2 * lab_sm_count();
-  if (!wide) shape(RW);
-  if (p.d == 64) return wide ? launch_rows<T, 64, 4, 2>(p, stream) : launch_rows<T, 64, 4, 1>(p, stream);
-  if (p.d == 128) return wide ? launch_rows<T, 128, 4, 2>(p, stream) : launch_rows<T, 128, 4, 1>(p, stream);
-  if (p.d < 128) return wide ? launch_rows<T, 0, 4, 2>(p, stream) : launch_rows<T, 0, 4, 1>(p, stream);
-  return wide ? launch_rows<T, 0, 2, 2>(p, stream) : launch_rows<T, 0, 2, 1>(p, stream);
+  if (p.d == 64 && shape(32) >= 4 * lab_sm_count()) return launch_rows<T, 64, 4, 2, 4>(p, stream);
+  const bool wide = shape(16) >= 2 * lab_sm_count();
+  if (!wide) shape(8);
+  if (p.d == 64) return wide ? launch_rows<T, 64, 4, 2, 2>(p, stream) : launch_rows<T, 64, 4, 1, 2>(p, stream);
+  if (p.d == 128) return wide ? launch_rows<T, 128, 4, 2, 2>(p, stream) : launch_rows<T, 128, 4, 1, 2>(p, stream);
+  if (p.d < 128) return wide ? launch_rows<T, 0, 4, 2, 2>(p, stream) : launch_rows<T, 0, 4, 1, 2>(p, stream);
+  return wide ? launch_rows<T, 0, 2, 2, 2>(p, stream) : launch_rows<T, 0, 2, 1, 2>(p, stream);
 }
 }  // namespace
 
