@@ -194,14 +194,29 @@ struct DcLayout {
 // memory of the CTA that merges them (remote stores do not stall, remote loads would), and after
 // one cluster barrier everyone finds all it needs at home: no scratch and no merge kernel.
 // MORE: as in the prefill kernel.
-template <bool CLUSTER, bool MORE>
+// ROT: q, k and v are still the projection's: its parts (32-bit, bias to add) or its rounded rows.  Every CTA sums and rotates
+// its own query heads, and the one whose split ends at the newest key rotates that and leaves it and its value in the cache
+// before it reads them back, all as the kernel for that would (rowwise.cu): one launch of a chain of a step's small ones less.
+// Measured: a step of eight requests and 24 layers 752 us, 797 with the launch; a layer's attention with its products of 32
+// requests of 4,096 keys, 28 and 4 heads of 128, 76 and 81.  Bound by the latency of one load (with a column and part after the
+// other, 859).
+struct Rotate {
+  const void* rows;          // [tokens, width] bfloat16, or [parts, tokens, width] floats
+  int parts, width;          // parts 0: bfloat16
+  size_t part_stride;
+  const __nv_bfloat16* bias; // [width], or null
+  const int* positions;      // [tokens]
+  const float* inv_freq;     // [D / 2]
+  const int* slots;          // [tokens]: where a row's key lies in the cache, or negative
+};
+template <bool CLUSTER, bool MORE, bool ROT>
 __global__ void __launch_bounds__(DC_THREADS) attention_decode_kernel(
     void* __restrict__ out, int out_stride, const __nv_bfloat16* __restrict__ q, int q_stride,
     __nv_bfloat16* __restrict__ cache_k, __nv_bfloat16* __restrict__ cache_v,
     const int* __restrict__ q_start, const int* __restrict__ kv_len_arr, const int* __restrict__ block_table,
     int max_blocks, int n_q, int n_kv, int page_size, int num_pages, int window, float scale_log2, int splits,
     float* __restrict__ part_acc, float* __restrict__ part_ml, int keep, const float* __restrict__ sink,
-    const float* __restrict__ dist_bias, int bias_len, float cap_log2, float arg_log2, int out_f32) {
+    const float* __restrict__ dist_bias, int bias_len, float cap_log2, float arg_log2, int out_f32, Rotate rot) {
   extern __shared__ __align__(16) uint8_t smem[];
   if constexpr (!MORE) cap_log2 = 0.f, out_f32 = 0;
   using L = DcLayout<CLUSTER>;
@@ -252,7 +267,55 @@ __global__ void __launch_bounds__(DC_THREADS) attention_decode_kernel(
     cp_async_commit();
     t_issue += DC_WARPS;
   }
-  pdl_wait();
+  constexpr int QLD = ROT ? D + 8 : 1;      // (eight rows' words of a fragment in different banks)
+  __shared__ __align__(16) __nv_bfloat16 qs_rot[ROT ? 18 * QLD : 1];      // the queries, the new key, its value
+  if constexpr (ROT) {
+    constexpr int HALF = D / 2;
+    __shared__ float2 turn[HALF];
+    const float pos = (float)rot.positions[qs];
+    for (int i = tid; i < HALF; i += DC_THREADS) {
+      float sn, cs;
+      sincosf(pos * rot.inv_freq[i], &sn, &cs);
+      turn[i] = make_float2(cs, sn);
+    }
+    const int slot = tile_lo < tile_hi && tile_hi == total_tiles ? rot.slots[qs] : -1;
+    __syncthreads();
+    pdl_wait();
+    const int page = slot >= 0 ? slot / page_size : 0;
+    if (slot >= 0 && page >= num_pages && tid == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
+    const int heads = n_heads + (slot >= 0 && page < num_pages ? 2 : 0);
+    // four neighbouring columns a thread, summed in the parts' order, all parts asked for together
+    for (int e = tid; e < heads * (D / 4); e += DC_THREADS) {
+      const int head = e / (D / 4), i = e % (D / 4) * 4;
+      const int col = (head < n_heads ? head0 + head : head == n_heads ? n_q + kvh : n_q + n_kv + kvh) * D + i;
+      float4 v;
+      if (rot.parts == 0) {
+        v = load4(static_cast<const __nv_bfloat16*>(rot.rows) + (size_t)qs * rot.width + col);
+      } else {
+        const float* from = static_cast<const float*>(rot.rows) + (size_t)qs * rot.width + col;
+        v = sum_splits4(from, rot.parts, (long long)rot.part_stride, 0);
+        if (rot.bias != nullptr) {
+          const float4 z = load4(rot.bias + col);
+          v.x += z.x, v.y += z.y, v.z += z.z, v.w += z.w;
+        }
+      }
+      store4(qs_rot + head * QLD + i, v);
+    }
+    __syncthreads();
+    // a pair of a query head, of the new key, or of its value
+    const size_t at = (((size_t)page * n_kv + kvh) * page_size + (slot - page * page_size)) * D;
+    for (int e = tid; e < heads * HALF; e += DC_THREADS) {
+      const int head = e / HALF, i = e % HALF;
+      __nv_bfloat16 *row = qs_rot + head * QLD, *to = head < n_heads ? row : (head == n_heads ? cache_k : cache_v) + at;
+      const float lo = to_f32(row[i]), hi = to_f32(row[i + HALF]);
+      float rlo = lo, rhi = hi;
+      if (head <= n_heads) rope_rotate(lo, hi, turn[i].x, turn[i].y, rlo, rhi);
+      to[i] = from_f32<__nv_bfloat16>(rlo), to[i + HALF] = from_f32<__nv_bfloat16>(rhi);
+    }
+    __syncthreads();      // the queries; the newest key and value, before their tile's copies
+  } else {
+    pdl_wait();
+  }
   for (; staged < L::STAGES - 1; ++staged) {
     if (t_issue < tile_hi) issue(t_issue, staged);
     cp_async_commit();
@@ -262,13 +325,14 @@ __global__ void __launch_bounds__(DC_THREADS) attention_decode_kernel(
   uint32_t qf[KSTEPS][4];
   {
     // q fragments straight from global memory: row r of the A operand is query head head0 + r
-    const __nv_bfloat16* qrow = q + (size_t)qs * q_stride;
+    const __nv_bfloat16* qrow = ROT ? qs_rot : q + (size_t)qs * q_stride + (size_t)head0 * D;
+    constexpr int ld = ROT ? QLD : D;
     const int ra = lane >> 2, rb = ra + 8;
 #pragma unroll
     for (int k = 0; k < KSTEPS; ++k) {
       const int c = k * 16 + 2 * (lane & 3);
-      const uint32_t* pa = reinterpret_cast<const uint32_t*>(qrow + (size_t)(head0 + ra) * D + c);
-      const uint32_t* pb = reinterpret_cast<const uint32_t*>(qrow + (size_t)(head0 + rb) * D + c);
+      const uint32_t* pa = reinterpret_cast<const uint32_t*>(qrow + (size_t)ra * ld + c);
+      const uint32_t* pb = reinterpret_cast<const uint32_t*>(qrow + (size_t)rb * ld + c);
       qf[k][0] = ra < n_heads ? pa[0] : 0u;
       qf[k][1] = rb < n_heads ? pb[0] : 0u;
       qf[k][2] = ra < n_heads ? pa[4] : 0u;
@@ -498,7 +562,7 @@ static int decode_launch(void* out, int out_stride, const void* q, int q_stride,
                          int max_blocks, int requests, int n_q, int n_kv, int page_size, int num_pages, int window,
                          float scale, int splits, float* scratch, bool may_cluster, cudaStream_t stream,
                          int keep_first = 0, const float* sink = nullptr, const float* dist_bias = nullptr,
-                         int bias_len = 0, float softcap = 0.f, int out_f32 = 0) {
+                         int bias_len = 0, float softcap = 0.f, int out_f32 = 0, const Rotate* rotate = nullptr) {
   if (requests <= 0) return 0;
   if (dist_bias == nullptr) bias_len = 0;
   const int keep = window > 0 && keep_first > 0 ? keep_first : 0;
@@ -510,15 +574,17 @@ static int decode_launch(void* out, int out_stride, const void* q, int q_stride,
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
   if (!configured[device]) {
     cudaError_t e = cudaSuccess;
-    for (auto k : {attention_decode_kernel<false, false>, attention_decode_kernel<false, true>})
+    for (auto k : {attention_decode_kernel<false, false, false>, attention_decode_kernel<false, true, false>, attention_decode_kernel<false, false, true>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DcLayout<false>::SMEM);
-    for (auto k : {attention_decode_kernel<true, false>, attention_decode_kernel<true, true>})
+    for (auto k : {attention_decode_kernel<true, false, false>, attention_decode_kernel<true, true, false>, attention_decode_kernel<true, false, true>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DcLayout<true>::SMEM);
     if (e != cudaSuccess) return (int)e;
     configured[device] = true;
   }
   const int group = n_q / n_kv, m_tiles = (group + 15) / 16;
   const bool more = softcap > 0.f || out_f32;
+  if (rotate != nullptr && (more || m_tiles > 1)) return (int)cudaErrorInvalidValue;
+  const Rotate rot = rotate != nullptr ? *rotate : Rotate{};
   dim3 grid(splits, n_kv * m_tiles, requests);
   if (cluster) {
     cudaLaunchConfig_t cfg = {};
@@ -535,21 +601,24 @@ static int decode_launch(void* out, int out_stride, const void* q, int q_stride,
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_lab_pdl ? 2 : 1;
-    return (int)cudaLaunchKernelEx(&cfg, more ? attention_decode_kernel<true, true> : attention_decode_kernel<true, false>,
-                                   out, out_stride,
+    return (int)cudaLaunchKernelEx(&cfg, rotate != nullptr ? attention_decode_kernel<true, false, true>
+                                         : more ? attention_decode_kernel<true, true, false>
+                                                : attention_decode_kernel<true, false, false>, out, out_stride,
                                    (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)cache_k, (__nv_bfloat16*)cache_v,
                                    q_start, kv_len, block_table, max_blocks, n_q, n_kv, page_size, num_pages, window,
                                    scale * LOG2E, splits, (float*)nullptr, (float*)nullptr, keep, sink, dist_bias,
-                                   bias_len, cap_of(softcap), cap_arg(softcap, scale), out_f32);
+                                   bias_len, cap_of(softcap), cap_arg(softcap, scale), out_f32, rot);
   }
   float* part_acc = scratch;
   float* part_ml = scratch ? scratch + (size_t)requests * n_q * splits * D : nullptr;
-  cudaError_t e = lab_launch(more ? attention_decode_kernel<false, true> : attention_decode_kernel<false, false>, grid, dim3(DC_THREADS), (size_t)DcLayout<false>::SMEM, stream,
+  cudaError_t e = lab_launch(rotate != nullptr ? attention_decode_kernel<false, false, true>
+                             : more ? attention_decode_kernel<false, true, false> : attention_decode_kernel<false, false, false>,
+                             grid, dim3(DC_THREADS), (size_t)DcLayout<false>::SMEM, stream,
                              out, out_stride, (const __nv_bfloat16*)q, q_stride,
                              (__nv_bfloat16*)cache_k, (__nv_bfloat16*)cache_v, q_start, kv_len, block_table,
                              max_blocks, n_q, n_kv, page_size, num_pages, window, scale * LOG2E, splits, part_acc,
                              part_ml, keep, sink, dist_bias, bias_len, cap_of(softcap), cap_arg(softcap, scale),
-                             out_f32);
+                             out_f32, rot);
   if (e != cudaSuccess) return (int)e;
   if (splits > 1)
     e = lab_launch(attention_merge_kernel, dim3(requests, n_q), dim3(D), 0, stream, out, out_stride,
@@ -573,6 +642,26 @@ LAB_EXPORT int lab_attention_decode(void* out, int out_stride, const void* q, in
   return decode_launch(out, out_stride, q, q_stride, cache_k, cache_v, q_start, kv_len, block_table, max_blocks,
                        requests, n_q, n_kv, page_size, num_pages, window, scale, splits, scratch, cluster_merge != 0,
                        stream, keep_first, sink, dist_bias, bias_len, softcap, out_f32);
+}
+
+// A step of one row a request whose q, k and v are still to be rotated over the whole head and k and v to be stored: rows
+// [tokens, width] bfloat16 (parts 0), or [parts, tokens, width] floats that are summed, `bias` [width] added; positions and
+// slots [tokens], inv_freq [D / 2].  At most 16 query heads a kv head.
+LAB_EXPORT int lab_attention_decode_rotated(void* out, int out_stride, const void* rows, int parts, int tokens, int width,
+                                            const void* bias, const int* positions, const float* inv_freq, const int* slots,
+                                            void* cache_k, void* cache_v, const int* q_start, const int* kv_len,
+                                            const int* block_table, int max_blocks, int requests, int n_q, int n_kv,
+                                            int page_size, int num_pages, int window, float scale, int splits,
+                                            float* scratch, int cluster_merge, cudaStream_t stream) {
+  if (rows == nullptr || positions == nullptr || inv_freq == nullptr || slots == nullptr || parts < 0 ||
+      width != (n_q + 2 * n_kv) * D)
+    return (int)cudaErrorInvalidValue;
+  Rotate rot;
+  rot.rows = rows; rot.parts = parts; rot.width = width; rot.part_stride = (size_t)tokens * width;
+  rot.bias = (const __nv_bfloat16*)bias; rot.positions = positions; rot.inv_freq = inv_freq; rot.slots = slots;
+  return decode_launch(out, out_stride, nullptr, 0, cache_k, cache_v, q_start, kv_len, block_table, max_blocks, requests,
+                       n_q, n_kv, page_size, num_pages, window, scale, splits, scratch, cluster_merge != 0, stream, 0,
+                       nullptr, nullptr, 0, 0.f, 0, &rot);
 }
 
 // ----------------------------------------------------------------------------------------

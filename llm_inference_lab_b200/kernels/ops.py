@@ -837,17 +837,8 @@ def attention_tc(q, cache_k, cache_v, q_start, kv_len, pos0, block_table, n_requ
                                        bias_len, ctypes.c_float(softcap), int(bool(out_f32)), _stream()),
                "attention_prefill")
     if n_decode:
-        if splits is None:
-            span = min(max_kv_len, abs(window) + keep_first) if window else max_kv_len     # a chunk reaches as far as a window
-            splits = decode_splits(n_decode, n_kv, n_q // n_kv, span, *decode_shape(head_dim))
-        ctas = n_decode * n_kv * (-(-(n_q // n_kv) // 16)) * splits
-        in_cluster = CLUSTER_MERGE and 2 <= splits <= 8 and ctas <= sm_count()
-        if splits > 1 and not in_cluster:
-            need = n_requests * n_q * splits * (head_dim + 2)
-            if scratch is None or scratch.numel() < need:
-                scratch = torch.empty((need,), dtype=torch.float32, device=q.device)
-        else:
-            scratch = None
+        splits, in_cluster, scratch = _decode_plan(n_decode, n_requests, n_q, n_kv, head_dim, window, max_kv_len, keep_first, splits,
+                                                   scratch, q.device)
         _check(L.lab_attention_decode(_ptr(out), out.stride(0), _ptr(q), q.stride(0), _ptr(cache_k), _ptr(cache_v),
                                       _ptr(q_start), _ptr(kv_len), _ptr(block_table), block_table.shape[1],
                                       n_requests, n_q, n_kv, page_size, num_pages, window, ctypes.c_float(scale),
@@ -855,6 +846,56 @@ def attention_tc(q, cache_k, cache_v, q_start, kv_len, pos0, block_table, n_requ
                                       _ptr(dist_bias), bias_len, ctypes.c_float(softcap), int(bool(out_f32)), _stream()),
                "attention_decode",
                2 if splits > 1 and not in_cluster else 1)
+    return out
+
+
+def _decode_plan(n_decode, n_requests, n_q, n_kv, head_dim, window, max_kv_len, keep_first, splits, scratch, device):
+    """(splits, whether they merge inside their cluster, scratch or None) of the decode kernel's launch."""
+    if splits is None:
+        span = min(max_kv_len, abs(window) + keep_first) if window else max_kv_len     # a chunk reaches as far as a window
+        splits = decode_splits(n_decode, n_kv, n_q // n_kv, span, *decode_shape(head_dim))
+    ctas = n_decode * n_kv * (-(-(n_q // n_kv) // 16)) * splits
+    in_cluster = CLUSTER_MERGE and 2 <= splits <= 8 and ctas <= sm_count()
+    if splits == 1 or in_cluster:
+        return splits, in_cluster, None
+    need = n_requests * n_q * splits * (head_dim + 2)
+    if scratch is None or scratch.numel() < need:
+        scratch = torch.empty((need,), dtype=torch.float32, device=device)
+    return splits, in_cluster, scratch
+
+
+def attention_rotates(ctx, n_q: int, n_kv: int, head_dim: int, rotary_dim: int, cache_k) -> bool:
+    """Whether `attention_rotated` takes the step: one row a request, 16-bit storage, whole heads rotated, at most 16 query
+    heads a kv head."""
+    return (ctx.max_q_len == 1 and cache_k.dtype == torch.bfloat16 and not _force_plain and attention_tc_supported(head_dim)
+            and rotary_dim == head_dim and n_q // n_kv <= 16)
+
+
+def attention_rotated(qkv: torch.Tensor, bias, positions: torch.Tensor, inv_freq: torch.Tensor, slots: torch.Tensor, cache_k, cache_v,
+                      ctx, group, n_q, n_kv, head_dim, window, scale):
+    """`rope_kv_write` and `attention` of a step of one row a request (`attention_rotates`) in one kernel: `qkv` is the fused
+    projection [tokens, (n_q + 2 n_kv) * d], or its 32-bit partial products [parts, tokens, ..] with `bias` still to add."""
+    _on_gpu(qkv, positions, inv_freq, slots, cache_k, cache_v, bias)
+    width, parts = (n_q + 2 * n_kv) * head_dim, qkv.shape[0] if qkv.dim() == 3 else 0
+    tokens = qkv.shape[-2]
+    assert qkv.is_contiguous() and qkv.shape[-1] == width and qkv.dtype == (torch.float32 if parts else torch.bfloat16)
+    assert bias is None or parts
+    assert inv_freq.dtype == torch.float32 and inv_freq.numel() == head_dim // 2 and positions.numel() >= tokens
+    num_pages, kvh, page_size, d = cache_k.shape
+    assert kvh == n_kv and d == head_dim and cache_k.is_contiguous() and cache_v.is_contiguous() and cache_v.shape == cache_k.shape
+    table = group.block_table
+    assert table.dim() == 2 and table.is_contiguous() and table.shape[0] >= ctx.n_requests
+    out = torch.empty((tokens, n_q * head_dim), dtype=torch.bfloat16, device=qkv.device)
+    n_decode = sum(1 for n in ctx.q_lens if n == 1)
+    if n_decode == 0:
+        return out
+    splits, in_cluster, scratch = _decode_plan(n_decode, ctx.n_requests, n_q, n_kv, head_dim, window, ctx.max_kv_len, 0, None, None,
+                                               qkv.device)
+    _check(lib("attention_tc", {"LAB_HEAD_DIM": head_dim}).lab_attention_decode_rotated(
+        _ptr(out), out.stride(0), _ptr(qkv), parts, tokens, width, _ptr(bias), _ptr(positions), _ptr(inv_freq), _ptr(slots),
+        _ptr(cache_k), _ptr(cache_v), _ptr(ctx.q_start), _ptr(ctx.kv_len), _ptr(table), table.shape[1], ctx.n_requests, n_q, n_kv,
+        page_size, num_pages, window, ctypes.c_float(scale), splits, _ptr(scratch), 1 if in_cluster else 0, _stream()),
+        "attention_decode", 2 if splits > 1 and not in_cluster else 1)
     return out
 
 

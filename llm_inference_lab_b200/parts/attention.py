@@ -7,6 +7,7 @@ import torch
 
 from ..kernels import ops
 from .base import CacheView, Mixer, StepContext, lookup, register_part
+from .rope import Rope
 from .spec import PagedKV, PartSpec, TensorSpec
 
 
@@ -74,6 +75,13 @@ class GQAttention(Mixer):
             # the position encoding takes them: it then sums them, adds the bias and rounds once.
             partial = bool(getattr(self.position, "takes_partials", False))
             qkv = ops.linear(x, self.w_qkv, self.b_qkv, allow_partial=partial)
+            if type(self.position) is Rope and cache.write and ops.attention_rotates(ctx, self.n_q, self.n_kv, self.d,
+                                                                                     self.position.rotary_dim, cache.k):
+                # A step of single rows: the rotation and the cache write happen inside the attention's kernel.
+                attn = ops.attention_rotated(qkv, self.b_qkv if qkv.dim() == 3 else None, ctx.row_pos, self.position.inv_freq,
+                                             group.row_slot, cache.k, cache.v, ctx, group, self.n_q, self.n_kv, self.d, self.window,
+                                             self.scale)
+                return ops.linear(attn, self.w_o, self.b_o, allow_partial=self.b_o is None)
             q = self.position.rotate_and_store(qkv, ctx.row_pos, group.row_slot, cache, self.n_q, self.n_kv, self.d,
                                                bias=self.b_qkv if qkv.dim() == 3 else None, scratch=ctx.scratch)
         attn = ops.attention(q, cache.k, cache.v, ctx, group, self.n_q, self.n_kv, self.d, self.window, self.scale)
