@@ -197,9 +197,9 @@ struct DcLayout {
 // ROT: q, k and v are still the projection's: its parts (32-bit, bias to add) or its rounded rows.  Every CTA sums and rotates
 // its own query heads, and the one whose split ends at the newest key rotates that and leaves it and its value in the cache
 // before it reads them back, all as the kernel for that would (rowwise.cu): one launch of a chain of a step's small ones less.
-// Measured: a step of eight requests and 24 layers 752 us, 797 with the launch; a layer's attention with its products of 32
+// Measured: a step of eight requests and 24 layers 744 us, 797 with the launch; a layer's attention with its products of 32
 // requests of 4,096 keys, 28 and 4 heads of 128, 76 and 81.  Bound by the latency of one load (with a column and part after the
-// other, 859).
+// other 859; the new key's columns and the bias asked for in a second round 752).
 struct Rotate {
   const void* rows;          // [tokens, width] bfloat16, or [parts, tokens, width] floats
   int parts, width;          // parts 0: bfloat16
@@ -279,27 +279,52 @@ __global__ void __launch_bounds__(DC_THREADS) attention_decode_kernel(
       turn[i] = make_float2(cs, sn);
     }
     const int slot = tile_lo < tile_hi && tile_hi == total_tiles ? rot.slots[qs] : -1;
-    __syncthreads();
-    pdl_wait();
     const int page = slot >= 0 ? slot / page_size : 0;
     if (slot >= 0 && page >= num_pages && tid == 0) lab_set_error(LAB_ERR_PAGE_RANGE);
-    const int heads = n_heads + (slot >= 0 && page < num_pages ? 2 : 0);
-    // four neighbouring columns a thread, summed in the parts' order, all parts asked for together
-    for (int e = tid; e < heads * (D / 4); e += DC_THREADS) {
-      const int head = e / (D / 4), i = e % (D / 4) * 4;
-      const int col = (head < n_heads ? head0 + head : head == n_heads ? n_q + kvh : n_q + n_kv + kvh) * D + i;
-      float4 v;
+    const int heads = n_heads + (slot >= 0 && page < num_pages ? 2 : 0), places = heads * (D / 4);
+    // four neighbouring columns a thread, summed in the parts' order; the parts of its first two places asked for together
+    auto column = [&](int e) {
+      const int head = e / (D / 4);
+      return (head < n_heads ? head0 + head : head == n_heads ? n_q + kvh : n_q + n_kv + kvh) * D + e % (D / 4) * 4;
+    };
+    const float4 zeros = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool biased = rot.parts > 0 && rot.bias != nullptr, first = tid < places, second = tid + DC_THREADS < places;
+    const float4 bias1 = biased && first ? load4(rot.bias + column(tid)) : zeros;
+    const float4 bias2 = biased && second ? load4(rot.bias + column(tid + DC_THREADS)) : zeros;
+    __syncthreads();
+    pdl_wait();
+    const float* sums = static_cast<const float*>(rot.rows) + (size_t)qs * rot.width;
+    auto ask = [&](int e, float4 (&v)[8]) {
+      const int col = column(e);
       if (rot.parts == 0) {
-        v = load4(static_cast<const __nv_bfloat16*>(rot.rows) + (size_t)qs * rot.width + col);
-      } else {
-        const float* from = static_cast<const float*>(rot.rows) + (size_t)qs * rot.width + col;
-        v = sum_splits4(from, rot.parts, (long long)rot.part_stride, 0);
-        if (rot.bias != nullptr) {
-          const float4 z = load4(rot.bias + col);
-          v.x += z.x, v.y += z.y, v.z += z.z, v.w += z.w;
-        }
+        v[0] = load4(static_cast<const __nv_bfloat16*>(rot.rows) + (size_t)qs * rot.width + col);
+        return;
       }
-      store4(qs_rot + head * QLD + i, v);
+#pragma unroll
+      for (int s = 0; s < 8; ++s) v[s] = s < rot.parts ? load4(sums + s * rot.part_stride + col) : zeros;
+    };
+    auto settle = [&](int e, const float4 (&v)[8], float4 bias) {
+      float4 z = v[0];
+      if (rot.parts > 0) {
+        auto add = [&](float4 f) { z.x += f.x, z.y += f.y, z.z += f.z, z.w += f.w; };
+#pragma unroll
+        for (int s = 1; s < 8; ++s) add(v[s]);
+        for (int s = 8; s < rot.parts; ++s) add(load4(sums + s * rot.part_stride + column(e)));
+        add(bias);
+      }
+      store4(qs_rot + e / (D / 4) * QLD + e % (D / 4) * 4, z);
+    };
+    {
+      float4 v1[8], v2[8];
+      if (first) ask(tid, v1);
+      if (second) ask(tid + DC_THREADS, v2);
+      if (first) settle(tid, v1, bias1);
+      if (second) settle(tid + DC_THREADS, v2, bias2);
+    }
+    for (int e = tid + 2 * DC_THREADS; e < places; e += DC_THREADS) {
+      float4 v[8];
+      ask(e, v);
+      settle(e, v, biased ? load4(rot.bias + column(e)) : zeros);
     }
     __syncthreads();
     // a pair of a query head, of the new key, or of its value

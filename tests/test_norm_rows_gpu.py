@@ -1,0 +1,43 @@
+"""Residual add and RMS norm of bfloat16 rows, few and many, at the widths where the launch changes: against 64-bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def ops():
+    from llm_inference_lab_b200.kernels import ops as module
+    return module
+
+
+@pytest.mark.parametrize("hidden", [4, 128, 132, 896, 1026, 4096, 4100])
+@pytest.mark.parametrize("rows,parts,delta,picked", [(1, 0, False, False), (8, 9, False, False), (64, 1, True, False), (65, 3, False, True),
+                                                     (700, 2, False, False), (7, 0, True, True), (8, 0, False, True)])
+def test_add_and_norm(hidden, rows, parts, delta, picked):
+    g = torch.Generator(device=DEV).manual_seed(hidden + rows)
+    rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
+    x, w = rand(rows, hidden).bfloat16(), rand(hidden).bfloat16()
+    add, partial = rand(rows, hidden).bfloat16() if delta else None, rand(parts, rows, hidden) if parts else None
+    pick = torch.randperm(rows, device=DEV, generator=g).to(torch.int32)[: max(1, rows // 2)] if picked else None
+    before = x.clone()
+    y = ops().add_rmsnorm(x, w, 1e-6, delta=add, partial=partial, rows=pick)
+    ops().take_device_errors()
+    v = before.double() + (add.double() if delta else 0) + (partial.double().sum(0) if parts else 0)
+    if picked:
+        assert torch.equal(x, before)
+        stream = v[pick.long()]
+    else:
+        # the stream is rounded once; where 32-bit sums end on the other side of a tie, to the next value
+        assert ((x.double() - v).abs() <= 2.0 ** -8 * v.abs() + 1e-6).all()
+        stream = x.double()
+    want = stream / torch.sqrt((stream * stream).mean(1, keepdim=True) + 1e-6) * w.double()
+    # a rounding of the result, and of the stream where it is not left behind
+    assert ((y.double() - want).abs() <= (2 if picked else 1) * 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
+def test_a_row_out_of_range_is_an_error():
+    x, w = torch.zeros(3, 896, device=DEV, dtype=torch.bfloat16), torch.ones(896, device=DEV, dtype=torch.bfloat16)
+    ops().add_rmsnorm(x, w, 1e-6, rows=torch.tensor([1, 3], dtype=torch.int32, device=DEV))
+    with pytest.raises(ops().KernelError):
+        ops().take_device_errors()
