@@ -128,6 +128,22 @@ __global__ void add_rmsnorm_kernel(T* __restrict__ y, T* __restrict__ x, const T
 // waits for the others' end, and with them the next kernel).  Steps of 150, 300 and 700 rows with a CTA a row 1,407, 1,432
 // and 1,899 us (1,511, 1,547 and 1,990 by the former build, whose threads kept room for 8,192 entries a row); with a warp a
 // row one of them took a seventh longer: the loads of the product's partial sums follow one another.
+// A warp adds a row's squares up in the order of a CTA's four warps, so a row's bits do not depend on how many come with it.
+// The sum over a CTA of four warps, as block_sum forms it, of which this warp holds every warp's terms: each half of the lanes,
+// then each quarter, passes on what the other one goes on with.
+__device__ __forceinline__ float four_warps_sum(const float (&ss)[4]) {
+  const int lane = threadIdx.x & 31;
+  const bool hi = (lane & 16) != 0, hi8 = (lane & 8) != 0;
+  const float a = (hi ? ss[2] : ss[0]) + __shfl_xor_sync(0xffffffffu, hi ? ss[0] : ss[2], 16);
+  const float b = (hi ? ss[3] : ss[1]) + __shfl_xor_sync(0xffffffffu, hi ? ss[1] : ss[3], 16);
+  float t = (hi8 ? b : a) + __shfl_xor_sync(0xffffffffu, hi8 ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+#pragma unroll
+  for (int o = 16; o >= 8; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);      // (first + third) + (second + fourth)
+  return t;
+}
+
 constexpr int NORM_VEC_THREADS = 128;
 constexpr int NORM_VEC_MAX_CHUNKS = 8;  // per thread: widths up to 128 * 8 * 8 = 8192
 
@@ -152,7 +168,7 @@ __global__ void __launch_bounds__(NORM_VEC_THREADS, CHUNKS <= 4 ? 6 : 4) add_rms
     }
     const size_t base = (size_t)in_row * hidden;
     float v[CHUNKS][8];
-    float ss = 0.f;
+    float ss[PER] = {};      // of the chunks that a CTA's first warp has, its second, ..
 #pragma unroll
     for (int k = 0; k < CHUNKS; ++k) {
       const int c = mine + k * LANES;
@@ -197,10 +213,12 @@ __global__ void __launch_bounds__(NORM_VEC_THREADS, CHUNKS <= 4 ? 6 : 4) add_rms
         if (!rows) *reinterpret_cast<uint4*>(x + base + c * 8) = packed;
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += v[k][e] * v[k][e];
+      for (int e = 0; e < 8; ++e) ss[k % PER] += v[k][e] * v[k][e];
     }
-    ss = LANES == 32 ? warp_sum(ss) : block_sum(ss, scratch);
-    const float inv = rsqrtf(ss / (float)hidden + eps);
+    float total;
+    if constexpr (PER == 1) total = block_sum(ss[0], scratch);
+    else total = four_warps_sum(ss);
+    const float inv = rsqrtf(total / (float)hidden + eps);
     __nv_bfloat16* yr = y + (size_t)row * hidden;
 #pragma unroll
     for (int k = 0; k < CHUNKS; ++k) {

@@ -36,6 +36,24 @@ def test_add_and_norm(hidden, rows, parts, delta, picked):
     assert ((y.double() - want).abs() <= (2 if picked else 1) * 2.0 ** -8 * want.abs() + 1e-5).all()
 
 
+@pytest.mark.parametrize("hidden", [8, 896, 1024, 1032, 1536, 2048, 2056])
+def test_a_row_has_the_same_bits_in_every_step_of_many_rows(hidden):
+    """A CTA a row, a warp a row, a warp that takes several."""
+    most = 4 * ops().sm_count()
+    g = torch.Generator(device=DEV).manual_seed(hidden)
+    rows = 4 * most + 7
+    x, w = torch.randn(rows, hidden, device=DEV, generator=g).bfloat16(), torch.randn(hidden, device=DEV, generator=g).bfloat16()
+    delta = torch.randn(rows, hidden, device=DEV, generator=g).bfloat16()
+    few = [(x[a: a + 65].clone(), delta[a: a + 65].contiguous()) for a in range(0, rows - 65, 65)]
+    y = ops().add_rmsnorm(x, w, 1e-6, delta=delta)
+    for i, (stream, add) in enumerate(few):
+        assert torch.equal(ops().add_rmsnorm(stream, w, 1e-6, delta=add), y[65 * i: 65 * i + 65])
+        assert torch.equal(stream, x[65 * i: 65 * i + 65])
+    for n in (most, most + 1, most + 6):
+        assert torch.equal(ops().add_rmsnorm(x[:n].clone(), w, 1e-6), ops().add_rmsnorm(x.clone(), w, 1e-6)[:n])
+    ops().take_device_errors()
+
+
 def test_a_row_out_of_range_is_an_error():
     x, w = torch.zeros(3, 896, device=DEV, dtype=torch.bfloat16), torch.ones(896, device=DEV, dtype=torch.bfloat16)
     ops().add_rmsnorm(x, w, 1e-6, rows=torch.tensor([1, 3], dtype=torch.int32, device=DEV))
