@@ -551,8 +551,10 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
       for (int q = 0; q < SLB / 2; ++q)
 #pragma unroll
         for (int i = 0; i < BLK; ++i) fma_pair(S[c][q], gone_by[i][q], pair_of(gone[i], gone[i]));
-      const float held = fmaf(rk.w, v[c][3], fmaf(rk.z, v[c][2], fmaf(rk.y, v[c][1], rk.x * v[c][0])));
-      const float lost = fmaf(ra.w, gone[3], fmaf(ra.z, gone[2], fmaf(ra.y, gone[1], ra.x * gone[0])));
+      // (a later token's numbers stay out: zero times an infinity would be none)
+      auto upto = [&](int jj, float f) { return jj <= o_row ? f : 0.f; };
+      const float held = fmaf(rk.w, upto(3, v[c][3]), fmaf(rk.z, upto(2, v[c][2]), fmaf(rk.y, upto(1, v[c][1]), rk.x * v[c][0])));
+      const float lost = fmaf(ra.w, upto(3, gone[3]), fmaf(ra.z, upto(2, gone[2]), fmaf(ra.y, upto(1, gone[1]), ra.x * gone[0])));
       result[c] = mine[c] + (held + lost);
     }
 #pragma unroll

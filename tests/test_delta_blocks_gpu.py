@@ -60,3 +60,34 @@ def test_blocks_of_four_tokens(D, heads, lens):
     used = [s for s in slots if s >= 0]
     rest = [s for s in range(7) if s not in used]
     assert torch.equal(state[rest], start[rest])
+
+
+@pytest.mark.parametrize("D,heads", [(32, 1), (64, 2)])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("row", [0, 1, 2, 3, 8, 17, 22, 31])
+def test_rows_before_a_non_finite_one_are_as_they_were(D, heads, bad, row):
+    """Every place of a block, of a portion's first block and of later ones; one entry of r, k, v, the gate, the rate or the decay."""
+    T, hd = 35, heads * D
+    assert ops().delta_rule_blocks(T)
+    g = torch.Generator(device=DEV).manual_seed(row)
+    rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
+    proj, decay_pre, start = rand(T, 5 * hd), rand(T, hd), rand(1, heads, D, D)
+    bias, weight = rand(hd).bfloat16(), rand(hd).bfloat16()
+
+    def run(proj, decay_pre):
+        return ops().delta_rule(proj, decay_pre, bias, bias, weight, start.clone(), context([T], [0]), heads, D, 1e-6, 0.6)
+
+    clean = run(proj, decay_pre)
+    assert clean.isfinite().all()
+    for i in range(5):
+        spoilt = proj.clone()
+        spoilt[row, i * hd + 5] = bad
+        out = run(spoilt, decay_pre)
+        assert torch.equal(out[:row], clean[:row]), i
+        if i < 3:
+            assert not out[row, :D].isfinite().all(), i
+        assert torch.equal(out[:, D:], clean[:, D:])      # the other heads
+    spoilt = decay_pre.clone()
+    spoilt[row, 5] = bad
+    assert torch.equal(run(proj, spoilt)[:row], clean[:row])
+    ops().take_device_errors()
