@@ -120,121 +120,99 @@ __global__ void add_rmsnorm_kernel(T* __restrict__ y, T* __restrict__ x, const T
   }
 }
 
-// The same for bfloat16 rows whose width is a multiple of 8, for steps with many rows: a thread owns chunks of 8 elements
-// (16-byte loads and stores), CHUNKS at most, and keeps them in registers.  LANES threads a row: a CTA, so that a row's loads
-// are all under way at once, or, with more rows than CTAs find room beside the product before, a warp, which takes several
-// rows where it has to: the product after is then let in while the CTAs still wait, and its set-up and first weights are not
-// in the way.  48 of them in a step of 2,048 rows of 896: the step 2.70 ms, 2.96 with a CTA a row (2,048 CTAs of which a part
-// waits for the others' end, and with them the next kernel).  Steps of 150, 300 and 700 rows with a CTA a row 1,407, 1,432
-// and 1,899 us (1,511, 1,547 and 1,990 by the former build, whose threads kept room for 8,192 entries a row); with a warp a
-// row one of them took a seventh longer: the loads of the product's partial sums follow one another.
-// A warp adds a row's squares up in the order of a CTA's four warps, so a row's bits do not depend on how many come with it.
-// The sum over a CTA of four warps, as block_sum forms it, of which this warp holds every warp's terms: each half of the lanes,
-// then each quarter, passes on what the other one goes on with.
-__device__ __forceinline__ float four_warps_sum(const float (&ss)[4]) {
-  const int lane = threadIdx.x & 31;
-  const bool hi = (lane & 16) != 0, hi8 = (lane & 8) != 0;
-  const float a = (hi ? ss[2] : ss[0]) + __shfl_xor_sync(0xffffffffu, hi ? ss[0] : ss[2], 16);
-  const float b = (hi ? ss[3] : ss[1]) + __shfl_xor_sync(0xffffffffu, hi ? ss[1] : ss[3], 16);
-  float t = (hi8 ? b : a) + __shfl_xor_sync(0xffffffffu, hi8 ? a : b, 8);
-#pragma unroll
-  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-#pragma unroll
-  for (int o = 16; o >= 8; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);      // (first + third) + (second + fourth)
-  return t;
-}
-
+// The same for bfloat16 rows whose width is a multiple of 8, for steps with many rows: a CTA a row, a thread owns chunks of 8
+// elements (16-byte loads and stores), CHUNKS at most, and keeps them in registers.  Bound by the latency of a row's loads, then
+// by memory; threads keep room for no more than a row needs, so that more CTAs are resident: 2,048 rows of 896 4.2 us, 8,192 of
+// 2,048 21.7, 4,096 of 3,584 19.0 (5.4, 33.1 and 25.1 with room for 8,192 entries a row).  Whole steps of 600, 1,024, 1,600 and
+// 2,048 rows of 896 1,684, 1,821, 2,747 and 2,718 us; with a warp a row beyond four rows a multiprocessor, whose loads of the
+// product's partial sums follow one another, 1,840, 1,918, 2,847 and 2,706; with no more than four CTAs a multiprocessor, which
+// take several rows, 1,728, 1,864, 2,809 and 2,725.
 constexpr int NORM_VEC_THREADS = 128;
 constexpr int NORM_VEC_MAX_CHUNKS = 8;  // per thread: widths up to 128 * 8 * 8 = 8192
 
-template <int LANES, int CHUNKS>
+template <int CHUNKS>
 __global__ void __launch_bounds__(NORM_VEC_THREADS, CHUNKS <= 4 ? 6 : 4) add_rmsnorm_vec_kernel(
     __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ delta,
     const float* __restrict__ partial, int splits, size_t split_stride, const __nv_bfloat16* __restrict__ w,
-    const int* __restrict__ rows, int n_out_rows, int n_in_rows, int hidden, float eps) {
+    const int* __restrict__ rows, int n_in_rows, int hidden, float eps) {
   __shared__ float scratch[32];
   pdl_trigger();
   pdl_wait();
-  constexpr int PER = NORM_VEC_THREADS / LANES;      // rows of a CTA at a time
-  const int mine = threadIdx.x % LANES, chunks = hidden / 8;
-  for (int row = blockIdx.x * PER + threadIdx.x / LANES; row < n_out_rows; row += gridDim.x * PER) {
-    int in_row = row;
-    if (rows) {
-      in_row = rows[row];
-      if (in_row < 0 || in_row >= n_in_rows) {
-        if (mine == 0) lab_set_error(LAB_ERR_ROW_RANGE);
-        in_row = 0;
+  const int row = blockIdx.x, mine = threadIdx.x, chunks = hidden / 8;
+  int in_row = row;
+  if (rows) {
+    in_row = rows[row];
+    if (in_row < 0 || in_row >= n_in_rows) {
+      if (mine == 0) lab_set_error(LAB_ERR_ROW_RANGE);
+      in_row = 0;
+    }
+  }
+  const size_t base = (size_t)in_row * hidden;
+  float v[CHUNKS][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < CHUNKS; ++k) {
+    const int c = mine + k * NORM_VEC_THREADS;
+    if (c >= chunks) break;
+    const uint4 raw = *reinterpret_cast<const uint4*>(x + base + c * 8);
+    const uint4 add = delta ? *reinterpret_cast<const uint4*>(delta + base + c * 8) : make_uint4(0, 0, 0, 0);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&add);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 f = __bfloat1622float2(h[e]);
+      v[k][2 * e] = f.x;
+      v[k][2 * e + 1] = f.y;
+      if (delta) {
+        const float2 d = __bfloat1622float2(hd[e]);
+        v[k][2 * e] += d.x;
+        v[k][2 * e + 1] += d.y;
       }
     }
-    const size_t base = (size_t)in_row * hidden;
-    float v[CHUNKS][8];
-    float ss[PER] = {};      // of the chunks that a CTA's first warp has, its second, ..
-#pragma unroll
-    for (int k = 0; k < CHUNKS; ++k) {
-      const int c = mine + k * LANES;
-      if (c >= chunks) break;
-      const uint4 raw = *reinterpret_cast<const uint4*>(x + base + c * 8);
-      const uint4 add = delta ? *reinterpret_cast<const uint4*>(delta + base + c * 8) : make_uint4(0, 0, 0, 0);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
-      const __nv_bfloat162* hd = reinterpret_cast<const __nv_bfloat162*>(&add);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = __bfloat1622float2(h[e]);
-        v[k][2 * e] = f.x;
-        v[k][2 * e + 1] = f.y;
-        if (delta) {
-          const float2 d = __bfloat1622float2(hd[e]);
-          v[k][2 * e] += d.x;
-          v[k][2 * e + 1] += d.y;
-        }
-      }
-      if (partial) {
-        float p[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        const float* from = partial + base + c * 8;
+    if (partial) {
+      float p[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      const float* from = partial + base + c * 8;
 #pragma unroll 2
-        for (int s = 0; s < splits; ++s) {  // ascending split order, as the scalar kernel
-          const float4 a = load4(from + s * split_stride), b = load4(from + s * split_stride + 4);
-          p[0] += a.x; p[1] += a.y; p[2] += a.z; p[3] += a.w;
-          p[4] += b.x; p[5] += b.y; p[6] += b.z; p[7] += b.w;
-        }
-#pragma unroll
-        for (int e = 0; e < 8; ++e) v[k][e] += p[e];
-      }
-      if (delta || partial) {
-        uint4 packed;
-        __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&packed);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          hp[e] = __floats2bfloat162_rn(v[k][2 * e], v[k][2 * e + 1]);
-          const float2 f = __bfloat1622float2(hp[e]);
-          v[k][2 * e] = f.x;
-          v[k][2 * e + 1] = f.y;
-        }
-        if (!rows) *reinterpret_cast<uint4*>(x + base + c * 8) = packed;
+      for (int s = 0; s < splits; ++s) {  // ascending split order, as the scalar kernel
+        const float4 a = load4(from + s * split_stride), b = load4(from + s * split_stride + 4);
+        p[0] += a.x; p[1] += a.y; p[2] += a.z; p[3] += a.w;
+        p[4] += b.x; p[5] += b.y; p[6] += b.z; p[7] += b.w;
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss[k % PER] += v[k][e] * v[k][e];
+      for (int e = 0; e < 8; ++e) v[k][e] += p[e];
     }
-    float total;
-    if constexpr (PER == 1) total = block_sum(ss[0], scratch);
-    else total = four_warps_sum(ss);
-    const float inv = rsqrtf(total / (float)hidden + eps);
-    __nv_bfloat16* yr = y + (size_t)row * hidden;
-#pragma unroll
-    for (int k = 0; k < CHUNKS; ++k) {
-      const int c = mine + k * LANES;
-      if (c >= chunks) break;
-      const uint4 rw = *reinterpret_cast<const uint4*>(w + c * 8);
-      const __nv_bfloat162* hw = reinterpret_cast<const __nv_bfloat162*>(&rw);
+    if (delta || partial) {
       uint4 packed;
       __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const float2 fw = __bfloat1622float2(hw[e]);
-        hp[e] = __floats2bfloat162_rn(v[k][2 * e] * inv * fw.x, v[k][2 * e + 1] * inv * fw.y);
+        hp[e] = __floats2bfloat162_rn(v[k][2 * e], v[k][2 * e + 1]);
+        const float2 f = __bfloat1622float2(hp[e]);
+        v[k][2 * e] = f.x;
+        v[k][2 * e + 1] = f.y;
       }
-      *reinterpret_cast<uint4*>(yr + c * 8) = packed;
+      if (!rows) *reinterpret_cast<uint4*>(x + base + c * 8) = packed;
     }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ss += v[k][e] * v[k][e];
+  }
+  ss = block_sum(ss, scratch);
+  const float inv = rsqrtf(ss / (float)hidden + eps);
+  __nv_bfloat16* yr = y + (size_t)row * hidden;
+#pragma unroll
+  for (int k = 0; k < CHUNKS; ++k) {
+    const int c = mine + k * NORM_VEC_THREADS;
+    if (c >= chunks) break;
+    const uint4 rw = *reinterpret_cast<const uint4*>(w + c * 8);
+    const __nv_bfloat162* hw = reinterpret_cast<const __nv_bfloat162*>(&rw);
+    uint4 packed;
+    __nv_bfloat162* hp = reinterpret_cast<__nv_bfloat162*>(&packed);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 fw = __bfloat1622float2(hw[e]);
+      hp[e] = __floats2bfloat162_rn(v[k][2 * e] * inv * fw.x, v[k][2 * e + 1] * inv * fw.y);
+    }
+    *reinterpret_cast<uint4*>(yr + c * 8) = packed;
   }
 }
 
@@ -246,17 +224,13 @@ LAB_EXPORT int lab_add_rmsnorm(void* y, void* x, const void* delta, const float*
   if (dtype == LAB_BF16 && n_out_rows > 64 && hidden % 8 == 0 && aligned &&
       hidden <= NORM_VEC_THREADS * NORM_VEC_MAX_CHUNKS * 8 && (split_stride % 4) == 0)
   {
-    const int most = 4 * lab_sm_count();
-    const bool warps = n_out_rows > most && hidden <= 2048;
-    const auto kernel = warps ? (hidden <= 1024 ? add_rmsnorm_vec_kernel<32, 4> : add_rmsnorm_vec_kernel<32, 8>)
-                        : hidden <= 1024 ? add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 1>
-                        : hidden <= 2048 ? add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 2>
-                        : hidden <= 4096 ? add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 4>
-                                         : add_rmsnorm_vec_kernel<NORM_VEC_THREADS, 8>;
-    const int tiles = warps ? (n_out_rows + 3) / 4 : n_out_rows;
-    return (int)lab_launch(kernel, dim3(tiles < most ? tiles : most), dim3(NORM_VEC_THREADS), 0, stream,
-                           (__nv_bfloat16*)y, (__nv_bfloat16*)x, (const __nv_bfloat16*)delta, partial, splits,
-                           (size_t)split_stride, (const __nv_bfloat16*)w, rows, n_out_rows, n_in_rows, hidden, eps);
+    const auto kernel = hidden <= 1024   ? add_rmsnorm_vec_kernel<1>
+                        : hidden <= 2048 ? add_rmsnorm_vec_kernel<2>
+                        : hidden <= 4096 ? add_rmsnorm_vec_kernel<4>
+                                         : add_rmsnorm_vec_kernel<8>;
+    return (int)lab_launch(kernel, dim3(n_out_rows), dim3(NORM_VEC_THREADS), 0, stream, (__nv_bfloat16*)y, (__nv_bfloat16*)x,
+                           (const __nv_bfloat16*)delta, partial, splits, (size_t)split_stride, (const __nv_bfloat16*)w, rows,
+                           n_in_rows, hidden, eps);
   }
   int threads = (hidden + 31) / 32 * 32;   // one element per thread where the row allows it
   threads = threads < 128 ? 128 : (threads > 1024 ? 1024 : threads);

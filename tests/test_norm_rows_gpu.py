@@ -11,9 +11,10 @@ def ops():
     return module
 
 
-@pytest.mark.parametrize("hidden", [4, 128, 132, 896, 1026, 4096, 4100])
+@pytest.mark.parametrize("hidden", [4, 128, 132, 896, 1024, 1026, 1032, 1536, 2048, 2056, 4096, 4100, 4104, 8192, 8200])
 @pytest.mark.parametrize("rows,parts,delta,picked", [(1, 0, False, False), (8, 9, False, False), (64, 1, True, False), (65, 3, False, True),
-                                                     (700, 2, False, False), (7, 0, True, True), (8, 0, False, True)])
+                                                     (700, 2, False, False), (7, 0, True, True), (8, 0, False, True),
+                                                     (131, 0, True, False), (130, 0, False, True), (1300, 5, True, True)])
 def test_add_and_norm(hidden, rows, parts, delta, picked):
     g = torch.Generator(device=DEV).manual_seed(hidden + rows)
     rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
@@ -32,13 +33,14 @@ def test_add_and_norm(hidden, rows, parts, delta, picked):
         assert ((x.double() - v).abs() <= 2.0 ** -8 * v.abs() + 1e-6).all()
         stream = x.double()
     want = stream / torch.sqrt((stream * stream).mean(1, keepdim=True) + 1e-6) * w.double()
-    # a rounding of the result, and of the stream where it is not left behind
-    assert ((y.double() - want).abs() <= (2 if picked else 1) * 2.0 ** -8 * want.abs() + 1e-5).all()
+    # a rounding, of 2^-8 at most, of the result; where the stream is not left behind one of its entry as well, and one of the
+    # row's root mean square, which a few rounded entries may make up
+    assert ((y.double() - want).abs() <= (3 if picked else 1) * 2.0 ** -8 * want.abs() + 1e-5).all()
 
 
 @pytest.mark.parametrize("hidden", [8, 896, 1024, 1032, 1536, 2048, 2056])
 def test_a_row_has_the_same_bits_in_every_step_of_many_rows(hidden):
-    """A CTA a row, a warp a row, a warp that takes several."""
+    """Whatever their number: 65, around four a multiprocessor, around sixteen."""
     most = 4 * ops().sm_count()
     g = torch.Generator(device=DEV).manual_seed(hidden)
     rows = 4 * most + 7
