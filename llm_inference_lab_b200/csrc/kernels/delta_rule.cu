@@ -432,8 +432,10 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
     mbar_init_fence();
   }
   __syncthreads();
+  int sent = 0;                   // chunks whose copies have set out (thread 0)
   auto fetch = [&](int b0) {      // one thread; a chunk, where there is one
     if (b0 >= blocks) return;
+    ++sent;
     const uint32_t bytes = min(BCHUNK, blocks - b0) * BREC * 4;
     uint64_t* bar = &here[b0 / BCHUNK % 2];
     mbar_expect_tx(bar, bytes);
@@ -442,7 +444,13 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
                  "l"(records + (size_t)b0 * BREC), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
   };
-  auto landed = [&](int b0) { return mbar_wait(&here[b0 / BCHUNK % 2], b0 / BCHUNK / 2 & 1, abort_flag); };
+  // A chunk is here and nobody reads the one before it any more; or the wait ran out (the error word says so): the whole block
+  // then goes no further than the block at hand.
+  auto landed = [&](int b0) {
+    mbar_wait(&here[b0 / BCHUNK % 2], b0 / BCHUNK / 2 & 1, abort_flag);
+    __syncthreads();
+    return *abort_flag == 0;
+  };
   if (tid == 0) fetch(0), fetch(BCHUNK);
   float* S_g = p.state + ((size_t)slot * p.heads + h) * D * D + (size_t)(g * SLB) * D + j;
   f32x2 S[NCOL][SLB / 2];
@@ -453,7 +461,7 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
     S[0][i] = pair_of(lo.x, hi.x), S[1][i] = pair_of(lo.y, hi.y);
   }
   float* out = p.out + (size_t)row0 * p.heads * D + h * D + j;
-  if (!landed(0)) return;
+  bool alive = landed(0);
   const int o_row = g % BLK;      // the token whose output this thread forms (threads g < BLK write)
   // vectors of the block at hand; as soon as one is used up its place takes the next block's
   f32x2 dots[B_DOTS][SLB / 2], keys[BLK][SLB / 2], gone_by[BLK][SLB / 2], decay[SLB / 2];
@@ -463,7 +471,7 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
 #pragma unroll
   for (int i = 0; i < BLK; ++i) load_share(keys[i], share, B_KEYS + i), load_share(gone_by[i], share, B_GONE + i);
   load_share(decay, share, B_DECAY);
-  for (int b = 0; b < blocks; ++b) {
+  for (int b = 0; b < blocks && alive; ++b) {
     const float* rec = blocks_smem + (b / BCHUNK % 2 * BCHUNK + b % BCHUNK) * BREC;
     float v[NCOL][BLK], uk[2 * N_PAIR];
 #pragma unroll
@@ -492,8 +500,7 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
     // the next block (after the last one this one again, for nothing), in the other buffer where a chunk ends
     const int nb = min(b + 1, blocks - 1);
     if (nb % BCHUNK == 0 && nb > b) {
-      if (!landed(nb)) break;
-      __syncthreads();       // nobody reads this chunk any more
+      alive = landed(nb);
       if (tid == 0) fetch(nb + BCHUNK);
     }
     share = blocks_smem + (nb / BCHUNK % 2 * BCHUNK + nb % BCHUNK) * BREC + g * SLBP;
@@ -561,6 +568,15 @@ __global__ void __launch_bounds__(BTHREADS) delta_blocks_kernel(DeltaParams p, i
     for (int i = 0; i < BLK; ++i) load_share(gone_by[i], share, B_GONE + i);
     const int row = b * BLK + o_row;
     if (g < BLK && row < rows) *reinterpret_cast<float2*>(out + (size_t)row * p.heads * D) = make_float2(result[0], result[1]);
+  }
+  if (!alive) {      // copies in flight land before the block's shared memory goes away
+    if (tid == 0)
+      for (int c = max(0, sent - 2); c < sent; ++c) {
+        const uint64_t t0 = global_timer_ns();
+        while (!mbar_try_wait(&here[c % 2], c / 2 & 1) && global_timer_ns() - t0 < 100000000ull) {
+        }
+      }
+    return;
   }
   pdl_trigger();      // (not earlier: the next kernel's blocks would settle beside this one's and slow them down)
   if (p.write) {
