@@ -632,11 +632,12 @@ template <typename T>
 int launch_blocks(const DeltaParams& p, const float* r, const float* k, const float* v, const float* a, int ld, const float* d,
                   int ld_d, const T* d_bias, const T* a_bias, int requests, float decay_rate, cudaStream_t stream) {
   static LabShared granted;
-  const cudaError_t e = lab_allow_shared(granted, (const void*)delta_blocks_kernel, BSMEM);
+  cudaError_t e = lab_allow_shared(granted, (const void*)delta_blocks_kernel, BSMEM);
   if (e != cudaSuccess) return (int)e;
   const int n_records = p.tokens / BLK + requests;
-  lab_launch(delta_prepare_blocks_kernel<T>, dim3(n_records, (p.heads + 7) / 8), dim3(256), 0, stream, (float*)p.rec, n_records,
-             r, k, v, a, ld, d, ld_d, d_bias, a_bias, p.q_start, requests, p.heads, decay_rate);
+  e = lab_launch(delta_prepare_blocks_kernel<T>, dim3(n_records, (p.heads + 7) / 8), dim3(256), 0, stream, (float*)p.rec,
+                 n_records, r, k, v, a, ld, d, ld_d, d_bias, a_bias, p.q_start, requests, p.heads, decay_rate);
+  if (e != cudaSuccess) return (int)e;
   return (int)lab_launch(delta_blocks_kernel, dim3(p.heads, requests, D / BCOLS), dim3(BTHREADS), BSMEM, stream, p, n_records);
 }
 
@@ -654,8 +655,9 @@ int launch_delta_rule(DeltaParams p, void* out, const float* r, const float* k, 
     static LabShared granted;
     e = (int)lab_allow_shared(granted, (const void*)delta_rule_kernel<T>, sizeof(DeltaShared));
     if (e != 0) return e;
-    lab_launch(delta_prepare_kernel<T>, per_token, dim3(256), 0, stream, (float*)p.rec, p.tokens, r, k, v, a, ld, d, ld_d,
-               d_bias, a_bias, p.heads, decay_rate);
+    e = (int)lab_launch(delta_prepare_kernel<T>, per_token, dim3(256), 0, stream, (float*)p.rec, p.tokens, r, k, v, a, ld, d, ld_d,
+                        d_bias, a_bias, p.heads, decay_rate);
+    if (e != 0) return e;
     e = (int)lab_launch(delta_rule_kernel<T>, dim3(p.heads, requests, NS), dim3(NT), sizeof(DeltaShared), stream, p);
   }
   if (e != 0) return e;
