@@ -329,8 +329,9 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
       if (MODE == SCAN_CLOSE) dt_sum += dt;
     }
     __syncthreads();
-    // the walk: nothing but the state's own update passes from token to token
-#pragma unroll 2
+    // the walk: nothing but the state's own update passes from token to token (with few entries a lane four tokens in flight: one
+    // request of 2,048 tokens in segments 129 us, 131 by two; no gain with more)
+#pragma unroll (R == 4 ? 4 : 2)
     for (int tt = 0; tt < nt; ++tt) {
       const float dt = b_dt[tt * WC + ch], dx = s_dx[tt * WC + ch];
       const f32x2 dt2 = pair_of(dt, dt), dx2 = pair_of(dx, dx);
@@ -338,7 +339,8 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
 #pragma unroll
       for (int q = 0; q < Q; ++q) {
         const int e = (q * WL + l) * 4;
-        if (e >= n4) break;
+        if (Q * WL * 4 > 16 && e >= n4) break;
+        if (Q * WL * 4 == 16 && e >= n4) continue;
         const ulonglong2 bq = *reinterpret_cast<const ulonglong2*>(b_b + tt * n4 + e);
         S2[2 * q] = fma2(exp_of(mul2(dt2, A2[2 * q])), S2[2 * q], mul2(dx2, bq.x));
         S2[2 * q + 1] = fma2(exp_of(mul2(dt2, A2[2 * q + 1])), S2[2 * q + 1], mul2(dx2, bq.y));
@@ -700,7 +702,9 @@ int launch_scan_as(void* out, const void* a_log, const void* skip, const void* d
 template <typename T, int WL, int R, bool QUADS = true>
 int launch_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
                 cudaStream_t stream) {
-  if (p.segments <= 1) return launch_scan_as<T, WL, R, SCAN_WHOLE, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
+  if constexpr (R > 4) {      // (smaller states in one piece have a walk of their own)
+    if (p.segments <= 1) return launch_scan_as<T, WL, R, SCAN_WHOLE, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
+  }
   const int e = launch_scan_as<T, WL, R, SCAN_CLOSE, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
   return e != 0 ? e : launch_scan_as<T, WL, R, SCAN_OUTPUT, QUADS>(out, a_log, skip, dt_bias, p, requests, stream);
 }
@@ -709,6 +713,9 @@ int launch_scan(void* out, const void* a_log, const void* skip, const void* dt_b
 template <typename T>
 int pick_scan(void* out, const void* a_log, const void* skip, const void* dt_bias, const ScanParams& p, int requests,
               int longest, cudaStream_t stream) {
+  if (p.N <= SMALL_STATE && p.segments > 1)
+    return p.N % 4 != 0 ? launch_scan<T, 4, 4, false>(out, a_log, skip, dt_bias, p, requests, stream)
+                        : launch_scan<T, 4, 4>(out, a_log, skip, dt_bias, p, requests, stream);
   if (p.N <= 4) return launch_walk<T, 4>(out, a_log, skip, dt_bias, p, requests, longest, stream);
   if (p.N <= 8) return launch_walk<T, 8>(out, a_log, skip, dt_bias, p, requests, longest, stream);
   if (p.N <= SMALL_STATE) return launch_walk<T, 16>(out, a_log, skip, dt_bias, p, requests, longest, stream);
@@ -785,7 +792,7 @@ LAB_EXPORT int lab_selective_scan(void* out, int ld_out, const float* x, int ld_
   p.vec_state = N % 4 == 0 && (((uintptr_t)state) & 15) == 0;
   const int unit = dtype == LAB_F32 ? 4 : 8;
   p.vec_out = channels % unit == 0 && ld_out % unit == 0 && (((uintptr_t)out) & 15) == 0;
-  if (N > SMALL_STATE) p.vec = p.vec && p.vec_bc;
+  if (N > SMALL_STATE || segments > 1) p.vec = p.vec && p.vec_bc;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
   if (dtype == LAB_F32) return pick_scan<float>(out, a_log, skip, dt_bias, p, requests, longest, stream);
   return pick_scan<__nv_bfloat16>(out, a_log, skip, dt_bias, p, requests, longest, stream);

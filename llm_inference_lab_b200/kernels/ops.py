@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes
 import functools
+import math
 import threading
 
 import torch
@@ -1791,7 +1792,7 @@ def rope_pairs_store(proj: torch.Tensor, bias, positions: torch.Tensor, inv_freq
 # Selective scan (csrc/kernels/selective_scan.cu).
 # ----------------------------------------------------------------------------------------
 SELECTIVE_SCAN_MAX_STATE = 256
-SELECTIVE_SCAN_SMALL_STATE = 16      # up to here an entry a lane, in one piece
+SELECTIVE_SCAN_SMALL_STATE = 16      # up to here the walk in one piece has an entry a lane
 
 
 def conv_silu(proj: torch.Tensor, conv_at: int, channels: int, taps: int, w: torch.Tensor, b: torch.Tensor,
@@ -1814,10 +1815,10 @@ def conv_silu(proj: torch.Tensor, conv_at: int, channels: int, taps: int, w: tor
 
 
 def scan_segments(ctas: int, longest: int) -> int:
-    """Into how many segments `selective_scan` cuts a request's rows of states of more than 16 entries (smaller ones are
-    walked in one piece), `ctas` CTAs walking the step in one piece and a multiprocessor holding four.  Segments cost a second
+    """Into how many segments `selective_scan` cuts a request's rows, `ctas` CTAs of 32 channels walking the step in one piece
+    and a multiprocessor holding four (states of up to 16 entries: where `scan_segments_pay`).  Segments cost a second
     launch and most of the walk's work once more, so they pay while they bring idle multiprocessors to work: measured with its
-    mixer (us, from a graph, states of 16 entries walked by the kernel for larger ones), 56 CTAs and 2,048 tokens 690 in one
+    mixer (us, from a graph, states of 16 entries, four a lane), 56 CTAs and 2,048 tokens 690 in one
     piece, 327 in 4, 239 in 8, 222 in 11, 226 in 16; 700 tokens 214, 158 in 4, 123 in 8; 112 CTAs and 420 tokens 195, 139 in
     4, 128 in 6; 224 CTAs and 500 tokens 246, 235 in 2, 209 in 6; 448 CTAs and 250 tokens 173, 196 in 2.  Below 320 tokens
     they would still save the device time (319 tokens 114, 91 in 8; 130 tokens 76, 71 in 8), but there the mixer launched
@@ -1826,6 +1827,21 @@ def scan_segments(ctas: int, longest: int) -> int:
     if longest < 320:
         return 1
     return max(1, min(longest // 32, 9 * sm_count() // (2 * max(1, ctas)), 32))
+
+
+def scan_segments_pay(segments: int, channels: int, N: int, requests: int, longest: int) -> bool:
+    """Whether that many segments, four entries a lane, beat the walk of a state of up to 16 entries in one piece, an entry a
+    lane: the fewer channels, the longer the rows and the fewer entries, by what either takes (us).  Measured, one request
+    (from a graph, one piece / segments): 64 channels of 16 entries and 2,048 tokens 99 / 34; 512 and 2,048 100 / 46, 1,000 51 / 35,
+    500 27 / 27, 330 19 / 26; 1,024 and 2,048 100 / 74, 500 27 / 31; 1,280 and 2,048 114 / 108; 1,792 and 2,048 115 / 119, 700 42 / 51;
+    5,120 and 2,048 206 / 341; 256 and 8,192 392 / 105; four requests of 500 and 512 channels 31 / 39; 8 entries, 512
+    channels and 2,048 tokens 134 / 46, 1,792 136 / 122; 4 entries 214 / 46 and 216 / 121."""
+    lanes = 4 if N <= 4 else 8 if N <= 8 else 16
+    rounds = -(-requests * -(-channels // (128 // lanes)) // sm_count())      # CTAs of 4 warps a multiprocessor
+    token = {4: 0.1 + 0.005 * rounds, 8: 0.055 + 0.0105 * rounds, 16: max(0.0475, 0.019 + 0.0175 * rounds)}[lanes]
+    rows = -(-longest // (32 * segments)) * 32                                # of a segment
+    load = requests * -(-channels // 32) * -(-longest // rows) / (4 * sm_count())
+    return 11 + rows * (0.23 + 0.285 * min(1.0, load) + 0.1 * max(0, math.ceil(load) - 1)) < 3 + token * longest
 
 
 def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at: int, c_at: int, z: torch.Tensor,
@@ -1846,9 +1862,9 @@ def selective_scan(x: torch.Tensor, dt_pre: torch.Tensor, bc: torch.Tensor, b_at
     if N > SELECTIVE_SCAN_MAX_STATE:
         raise KernelError(f"selective_scan: a state of {N} entries a channel exceeds {SELECTIVE_SCAN_MAX_STATE}")
     out = torch.empty((tokens, channels), dtype=a_log.dtype, device=x.device)
-    segments = 1
-    if not in_order and N > SELECTIVE_SCAN_SMALL_STATE:
-        segments = scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
+    segments = 1 if in_order else scan_segments(ctx.n_requests * -(-channels // (32 if N <= 64 else 16)), ctx.max_q_len)
+    if segments > 1 and N <= SELECTIVE_SCAN_SMALL_STATE and not scan_segments_pay(segments, channels, N, ctx.n_requests, ctx.max_q_len):
+        segments = 1
     states = sums = None
     if segments > 1:
         scratch, (states, sums) = _segment_scratch(x.device, ctx.n_requests * segments * channels * N,

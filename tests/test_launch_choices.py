@@ -92,6 +92,18 @@ def test_segments_of_recurrences_cover_the_cases_they_were_measured_on():
     assert ops.decay_scan_segments(42, 449, 1) == 1 and ops.decay_scan_segments(60, 2048, 1, 128) == 7
 
 
+def test_small_states_are_walked_in_segments_where_that_was_faster():
+    """(channels, entries, requests, tokens) on either side of the line."""
+    def cut(channels, N, requests, tokens):
+        n = ops.scan_segments(requests * -(-channels // 32), tokens)
+        return n > 1 and ops.scan_segments_pay(n, channels, N, requests, tokens)
+
+    assert all(cut(*c) for c in ((64, 16, 1, 2048), (512, 16, 1, 2048), (512, 16, 1, 1000), (1024, 16, 1, 2048), (256, 16, 1, 8192),
+                                 (512, 8, 1, 2048), (1792, 8, 1, 2048), (512, 4, 1, 330), (1792, 4, 1, 2048)))
+    assert not any(cut(*c) for c in ((256, 16, 1, 319), (512, 16, 1, 330), (1024, 16, 1, 500), (1792, 16, 1, 2048), (1792, 16, 1, 700),
+                                     (5120, 16, 1, 2048), (512, 16, 4, 500), (3072, 8, 1, 2048), (5120, 4, 1, 2048), (1792, 16, 64, 400)))
+
+
 def test_gated_products_take_the_kind_of_tile_whose_rounds_take_less_time():
     """By the measured costs of a round (pairs of SMs 0.9 of the small tiles' where K is long, the same where it is short),
     for every number of tokens."""

@@ -35,6 +35,7 @@ SLOTS = [4, 0, 2, 5, 1, -1]
 @pytest.mark.parametrize("channels,N", [(40, 16), (33, 3), (36, 20), (8, 64), (20, 100), (5, 256)])
 def test_selective_scan_segments(channels, N, segments, monkeypatch):
     monkeypatch.setattr(ops(), "scan_segments", lambda ctas, longest: segments)
+    monkeypatch.setattr(ops(), "scan_segments_pay", lambda *a: True)
     g = torch.Generator(device=DEV).manual_seed(channels + N)
     rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
     T = sum(Q_LENS)
@@ -43,7 +44,9 @@ def test_selective_scan_segments(channels, N, segments, monkeypatch):
     state = rand(6, channels, N)
     start, ctx = state.clone(), context(Q_LENS, SLOTS)
     for write in (False, True):
+        before = ops().COUNTER.launches
         out = ops().selective_scan(x, dt_pre, bc, 0, N, z, a_log, skip, bias, state, ctx, write=write)
+        assert ops().COUNTER.launches - before == min(segments, 2)
         assert write or torch.equal(state, start)
     ops().take_device_errors()
     n = lambda t: t.double().cpu().numpy()  # noqa: E731
