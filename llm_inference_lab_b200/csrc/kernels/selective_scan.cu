@@ -148,6 +148,8 @@ constexpr int WTHREADS = 128;
 constexpr int SCAN_MAX_STATE = 256;
 constexpr int LONG_WALK = 256;      // tokens from which the next kernel is let in at the walk's end only
 
+// What may be moved 16 bytes at a time: rows of dt_pre, x and z; of B and C; the state's; the output's.
+enum { VEC_ROWS = 1, VEC_BC = 2, VEC_STATE = 4, VEC_OUT = 8 };
 struct ScanParams {
   const float* x;        // [tokens, ld_x] after the convolution and SiLU
   const float* dt_pre;   // [tokens, ld_dt] the step sizes before bias and softplus
@@ -157,8 +159,8 @@ struct ScanParams {
   const int* q_start;
   const int* state_slot;
   int ld_x, ld_dt, ld_bc, ld_z, b_at, c_at, channels, N, n_slots, write, ld_out;
-  int vec;               // rows of all inputs (small states: of dt_pre, x and z) may be copied 16 bytes at a time
-  int vec_bc, vec_out, vec_state;      // small states: B's and C's, the output's, the state's
+  int vec;               // rows of all inputs may be copied 16 bytes at a time; the walks of small states: VEC_ bits (more
+                         // fields change the other walk's registers: 2,048 tokens, 768 channels of 128 entries 367 us, not 333)
   int segments;          // a request's rows are cut into at most that many segments of whole chunks
   float* states;         // [requests, segments, channels, N]: 0, a copy of the request's state; i, the state at the end
                          // of segment i - 1 (from zeros, of segment 0 from the request's state)
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(32 * WARPS) selective_walk_kernel(T* __restric
     const int nt = min(WTS, n - t0);
     const size_t row0 = (size_t)(first + t0);
     float *b_x = buf + WTS * WC, *b_z = b_x + WTS * WC, *b_b = b_z + WTS * WC, *b_c = b_b + WTS * LN;
-    if (p.vec) {
+    if (p.vec & VEC_ROWS) {
       for (int i = tid; i < nt * (WC / 4); i += THREADS) {
         const int cc = c0 + 4 * (i % (WC / 4));
         if (cc >= p.channels) continue;
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(32 * WARPS) selective_walk_kernel(T* __restric
         cp_async_f32(b_z + i, p.z + row * p.ld_z + cc);
       }
     }
-    if (p.vec_bc) {
+    if (p.vec & VEC_BC) {
       for (int i = tid; i < nt * (N / 4); i += THREADS) {
         const int e = 4 * (i % (N / 4)), t = i / (N / 4);
         const float* row = p.bc + (row0 + t) * p.ld_bc + e;
@@ -491,7 +493,7 @@ __global__ void __launch_bounds__(32 * WARPS) selective_walk_kernel(T* __restric
     const int nt = min(WTS, n - t0);
     const T* from = s_out + which * WTS * WC;
     constexpr int UNIT = 16 / (int)sizeof(T), PER = WC / UNIT;
-    if (PER > 0 && p.vec_out) {
+    if (PER > 0 && (p.vec & VEC_OUT)) {
       for (int i = tid; i < nt * PER; i += THREADS) {
         const int cc = c0 + UNIT * (i % (PER > 0 ? PER : 1)), t = i / (PER > 0 ? PER : 1);
         if (cc < p.channels)
@@ -614,12 +616,12 @@ __global__ void __launch_bounds__(kThreads) selective_step_kernel(T* __restrict_
     if (4 * q + 2 < N) v.z = from[2];
     if (4 * q + 3 < N) v.w = from[3];
   };
-  if (live && p.vec_state) {
+  if (live && (p.vec & VEC_STATE)) {
     if (4 * q < N) S = load4(st);
   } else if (live) {
     four(S, st);
   }
-  if (p.vec_bc) {
+  if (p.vec & VEC_BC) {
     if (4 * q < N) b = load4(row_b), cc = load4(row_c);
   } else {
     four(b, row_b), four(cc, row_c);
@@ -645,7 +647,7 @@ __global__ void __launch_bounds__(kThreads) selective_step_kernel(T* __restrict_
   if (!live) return;
   if (q == 0) out[(size_t)t * p.ld_out + c] = from_f32<T>(fmaf(D, x, (sum.x + sum.z) + (sum.y + sum.w)) * silu_f(z));
   if (!p.write) return;
-  if (p.vec_state) {
+  if (p.vec & VEC_STATE) {
     if (4 * q < N) store4(st, S);
     return;
   }
@@ -787,12 +789,13 @@ LAB_EXPORT int lab_selective_scan(void* out, int ld_out, const float* x, int ld_
   p.ld_x = ld_x; p.ld_dt = ld_dt; p.ld_bc = ld_bc; p.ld_z = ld_z; p.b_at = b_at; p.c_at = c_at; p.channels = channels;
   p.N = N; p.n_slots = n_slots; p.write = write; p.ld_out = ld_out;
   p.segments = segments; p.states = states; p.sums = sums;
-  p.vec = ((ld_x | ld_dt | ld_z | channels) & 3) == 0 && ((((uintptr_t)x) | ((uintptr_t)dt_pre) | ((uintptr_t)z)) & 15) == 0;
-  p.vec_bc = ((ld_bc | b_at | c_at | N) & 3) == 0 && (((uintptr_t)bc) & 15) == 0;
-  p.vec_state = N % 4 == 0 && (((uintptr_t)state) & 15) == 0;
   const int unit = dtype == LAB_F32 ? 4 : 8;
-  p.vec_out = channels % unit == 0 && ld_out % unit == 0 && (((uintptr_t)out) & 15) == 0;
-  if (N > SMALL_STATE || segments > 1) p.vec = p.vec && p.vec_bc;
+  auto on_16 = [](const void* a) { return ((uintptr_t)a & 15) == 0; };
+  const bool rows = ((ld_x | ld_dt | ld_z | channels) & 3) == 0 && on_16(x) && on_16(dt_pre) && on_16(z);
+  const bool both = ((ld_bc | b_at | c_at | N) & 3) == 0 && on_16(bc);
+  p.vec = N > SMALL_STATE || segments > 1 ? rows && both
+                                          : rows * VEC_ROWS + both * VEC_BC + (N % 4 == 0 && on_16(state)) * VEC_STATE +
+                                                (channels % unit == 0 && ld_out % unit == 0 && on_16(out)) * VEC_OUT;
   if (requests > 65535) return (int)cudaErrorInvalidValue;
   if (dtype == LAB_F32) return pick_scan<float>(out, a_log, skip, dt_bias, p, requests, longest, stream);
   return pick_scan<__nv_bfloat16>(out, a_log, skip, dt_bias, p, requests, longest, stream);
