@@ -1,24 +1,32 @@
-// 32-bit matrix product on the tensor cores: every operand is split into two numbers of 11 bits of significand, whose
-// products the tensor cores form exactly.
+// 32-bit matrix product on the tensor cores: every operand is cut into three bfloat16 numbers, whose products the tensor cores
+// form exactly.
 //
 //   out[m, n] = sum_k x[m, k] * w[n, k]  (+ bias[n]; activation)      or gated, as in gemm_plain.cu; w is [out, in]
 //
-// x = x_hi + x_lo, x_hi the nearest number of 11 bits; of x_lo, 12 bits and a sign at most, the tensor cores read the first
-// 11 bits, so what is lost is below 2^-23 |x|.  A product is w_hi x_hi + (w_hi x_lo + w_lo x_hi); what is dropped, w_lo x_lo,
-// is at most 2^-24 of it.  The sum over k: the tensor cores add up chunks of 32 k's (four steps, at each of which a sum loses
-// what lies below its last bit), w_hi x_hi and the two small products apart; the chunks go one after the other into a sum kept
-// in registers, rounded to nearest.  K is cut into F32_PARTS parts of whole chunks, which are added pairwise, as a tree.  None
-// of this depends on the rows that come together or on the tile, so neither does any bit of the output.
+// A number's first 8 bits, the first 8 of what is left and the rest, 8 at most, make it up exactly: x = x1 + x2 + x3, |x2| <
+// 2^-7 |x|, |x3| < 2^-15 |x|.  A product is w1 x1 + (w1 x2 + w2 x1 + w2 x2 + w1 x3 + w3 x1 + w2 x3 + w3 x2); what is dropped,
+// w3 x3, is below 2^-30 of it.  Both operands enter times 2^24: the tensor cores take numbers below the smallest normal one for
+// zero, and so neither a part of an operand nor a product that counts is below it.  The sum over k: the tensor cores add up
+// chunks of 32 k's, w1 x1 and the small products apart, in steps of 16 k's at which a sum loses what lies below its last bit;
+// the chunks go one after the other into a sum kept in registers, rounded to nearest.  K is cut into F32_PARTS parts of whole
+// chunks, which are added pairwise, as a tree.  None of this depends on the rows that come together or on the tile, so neither
+// does any bit of the output.  A row of x whose one entry is a power of two gives w's column back, bit for bit.  2-norm of the
+// error (multiply-adds in brackets, in the order of gemm_plain.cu): normal operands, 896 k's 7.9e-8 (2.0e-7), 4,864 1.1e-7
+// (4.5e-7); operands from 0.5 to 1.5 3.7e-8 (6.0e-8) and 5.0e-8 (1.4e-7); over eight decades 9.6e-8 (1.4e-7) and 1.2e-7
+// (3.0e-7); operands of 1e-38, or 1e-40 by 1e18, likewise.
 //
-// What bounds it: the chain of hand-overs a chunk passes (brought, split, multiplied, summed), which takes 850 to 1,200 cycles
-// a chunk whatever the tile, though the tensor cores need 100 to 400 of them; deeper rings, more sums in tensor memory, two
-// chunks at a time and two CTAs a multiprocessor did not shorten it.  Measured on a B200, weights from memory, against tiles of
-// 64 x 64 by fused multiply-adds, which reach half of the units' rate (us): 517 x 4,864 x 896 gated 131 (266), 517 x 896 x
-// 4,864 47 (156), 517 x 1,152 x 896 29 (42), 517 x 896 x 896 16 (34), 100 x 896 x 4,864 16 (75), 8 x 896 x 4,864 12 (19), 8 x
-// 1,152 x 896 5.4 (4.4), 8 x 4,864 x 896 gated 17.5 (13.6).
+// What bounds it: the products' issue and the chain of hand-overs a chunk passes (brought, cut, multiplied, summed), 850 to
+// 1,300 cycles a chunk whatever the tile; 512 of them are products where a tile has 64 rows.  Three products instead of eight
+// would save 15 %, a third part that is neither formed nor stored 4 to 10 %; deeper rings, more sums in tensor memory, two
+// chunks at a time and two CTAs a multiprocessor did not shorten the chain.  Sums of parts that wait for their neighbour's lie
+// in local memory in the larger tiles, touched once a part.  Measured on a B200, weights from memory, against tiles of 64 x 64
+// by fused multiply-adds, which reach half of the units' rate (us): 517 x 4,864 x 896 gated 146 (266), 517 x 896 x 4,864 56
+// (157), 517 x 1,152 x 896 31 (43), 517 x 896 x 896 18 (34), 100 x 896 x 4,864 18 (75), 8 x 896 x 4,864 13 (17); few rows with
+// short K are slower, 8 x 1,152 x 896 6.1 (5.1), 8 x 4,864 x 896 gated 18.5 (13.2), 1 x 4,864 x 896 gated 18 (9.3), rows on no 16
+// bytes 1 x 4,864 x 898 gated 36 (31), but a row's bits may not depend on how many come with it.
 //
-// A result that is no finite number is formed again by fused multiply-adds one after the other: an infinite operand, or
-// one that the split rounds up to infinity, leaves differences of infinities behind.
+// A result that is no finite number, or beyond 2^79, is formed again by fused multiply-adds, in gemm_plain.cu's order: an
+// infinite operand, or a sum that outgrows 32 bits times 2^48, leaves differences of infinities behind.
 #pragma once
 #include "tcgen05.cuh"
 
@@ -29,32 +37,37 @@ constexpr int F32_FEATURES = 128;   // rows of w a tile holds (gated: 64 gate an
 constexpr int F32_GROUP = 128;      // threads of a group that splits operands
 constexpr int F32_THREADS = 128 + 2 * F32_GROUP + 64;      // sums; two such groups; issue; loads
 
-// D[tmem] (+)= A[tmem] * B[smem]^T, operands of 11 bits in 32-bit words, 32-bit accumulate; 8 k's.  A's lane is its row, a
-// column one k.
-__device__ __forceinline__ void umma_tf32_tmem_a(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
-                                                 uint32_t accumulate) {
+// Whether this lane issues (one of a converged warp).  Asked once for a run of products: an election in each took a third of
+// their issue.
+__device__ __forceinline__ uint32_t elected() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\tselp.u32 %0, 1, 0, e;\n\t}" : "=r"(e));
+  return e;
+}
+// D[tmem] (+)= A[tmem] * B[smem]^T by the lane that `issues`, as umma_bf16_tmem_a.
+template <bool ADD>
+__device__ __forceinline__ void f32_mma(uint32_t issues, uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc) {
   asm volatile(
       "{\n\t.reg .pred p, e;\n\t"
-      "elect.sync _|e, 0xffffffff;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "@e tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(tmem_d),
-      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u)
+      "setp.ne.b32 e, %4, 0;\n\t"
+      "setp.ne.b32 p, %5, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%6, %6, %6, %6}, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(issues), "n"(ADD ? 1 : 0), "r"(0u)
       : "memory");
-}
-// Instruction descriptor: 11-bit operands (both K-major) -> 32-bit, M = m, N = n.
-__host__ __device__ constexpr uint32_t tf32_instr_desc(int m, int n) {
-  return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
 }
 __device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
   return v;
 }
-// The nearest number of 11 bits, by Dekker's splitting (not for |v| > 2^115: no number then, see above).
-__device__ __forceinline__ float head_of(float v) {
-  const float c = __fmul_rn(v, 8193.f);
-  return __fsub_rn(c, __fsub_rn(c, v));
+// The first 8 bits of each of two numbers side by side; the two become what is left of them, exactly.
+__device__ __forceinline__ uint32_t heads_of(unsigned long long& pair) {
+  const uint32_t a = (uint32_t)pair, b = (uint32_t)(pair >> 32);
+  const unsigned long long heads = (unsigned long long)(b & 0xffff0000u) << 32 | (a & 0xffff0000u);
+  pair = fma2(heads, pair_of(-1.f, -1.f), pair);
+  return __byte_perm(a, b, 0x7632);
 }
+constexpr float F32_SCALE = 16777216.f;      // 2^24: what both operands enter the product times
 
 struct F32Params {
   float* out;
@@ -73,15 +86,15 @@ __device__ __forceinline__ void f32_copy4(uint32_t dst, const void* src, bool ha
 
 template <int NT> struct F32Tile {      // NT rows of x
   static constexpr int A_BYTES = F32_FEATURES * 128, B_BYTES = NT * 128;
-  static constexpr int STAGE = A_BYTES + 2 * B_BYTES;          // w's rows as they are, x's heads, x's tails
+  static constexpr int STAGE = A_BYTES + 2 * B_BYTES;          // w's rows as they are; x1 beside x2, x3 in half a row
   static constexpr int STAGES = 220 * 1024 / STAGE;            // 11, 9 or 6
   static constexpr int SMEM = STAGES * STAGE + 1024 + 512;
-  static constexpr int SUMS = 2 * NT;                          // columns of a chunk's sums: heads' products, small ones
-  // chunks in tensor memory: their sums, and behind those their w's heads and tails
+  static constexpr int SUMS = 2 * NT;                          // columns of a chunk's sums: w1 x1, the small products
+  // chunks in tensor memory: their sums, and behind those their w1, w2, w3 (two k's a column)
   static constexpr int SUM_BUFS = NT <= 32 ? 4 : 3, W_BUFS = NT <= 32 ? 4 : 2;
-  static constexpr int W_HI = SUM_BUFS * SUMS, W_COLUMNS = 2 * F32_CHUNK;
+  static constexpr int W_AT = SUM_BUFS * SUMS, W_COLUMNS = 3 * F32_CHUNK / 2;
   static constexpr int TMEM = 512;
-  static_assert(W_HI + W_BUFS * W_COLUMNS <= TMEM, "tensor memory");
+  static_assert(W_AT + W_BUFS * W_COLUMNS <= TMEM, "tensor memory");
   static_assert(NT * F32_FEATURES * 4 <= STAGES * STAGE, "the parts' sums lie in the stages");
   static_assert((3 * STAGES + 2 * SUM_BUFS) * 8 + 8 <= 512, "the barriers outgrow their 512 bytes");
 };
@@ -146,16 +159,24 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const __grid_c
     const float bias = !GATED && p.bias != nullptr && n < p.N ? p.bias[n] : 0.f;
     unsigned long long again = 0ull;
 #pragma unroll
-    for (int j = 0; j < COUNT; ++j)
+    for (int j = 0; j < COUNT; ++j) {
+      v[j] *= 1.f / (F32_SCALE * F32_SCALE);
       if (!(fabsf(v[j]) <= 3.402823466e38f) && m + j < p.M && n < p.N) again |= 1ull << j;
+    }
     while (again != 0ull) {
       const int j = __ffsll((long long)again) - 1;
       again &= again - 1;
       const float *a = p.w + (size_t)(GATED && (r & 16) ? p.N + n : n) * p.K, *b = p.x + (size_t)(m + j) * p.ldx;
-      float s = 0.f;
-      for (int k = 0; k < p.K; ++k) s = fmaf(__ldg(a + k), __ldg(b + k), s);
+      float s[8] = {};
+#pragma unroll 1
+      for (int k = 0; k < p.K; ++k) {
+        const int q = k / 16 % 4 * 2 + k % 2;
 #pragma unroll
-      for (int i = 0; i < COUNT; ++i) v[i] = i == j ? s : v[i];
+        for (int i = 0; i < 8; ++i) s[i] = i == q ? fmaf(__ldg(a + k), __ldg(b + k), s[i]) : s[i];
+      }
+      const float sum = (s[0] + s[1] + (s[2] + s[3])) + (s[4] + s[5] + (s[6] + s[7]));
+#pragma unroll
+      for (int i = 0; i < COUNT; ++i) v[i] = i == j ? sum : v[i];
     }
     __syncwarp();
 #pragma unroll
@@ -194,12 +215,12 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const __grid_c
           tc_fence_after();
 #pragma unroll
           for (int g = 0; g < NT; g += 16) {
-            uint32_t heads[16], small[16];
-            tmem_ld16_issue(mine + buf * Tile::SUMS + g, heads);
+            uint32_t large[16], small[16];
+            tmem_ld16_issue(mine + buf * Tile::SUMS + g, large);
             tmem_ld16_issue(mine + buf * Tile::SUMS + NT + g, small);
             tmem_wait();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) acc[g + j] += __uint_as_float(heads[j]) + __uint_as_float(small[j]);
+            for (int j = 0; j < 16; ++j) acc[g + j] += __uint_as_float(large[j]) + __uint_as_float(small[j]);
           }
           tc_fence_before();
           __syncwarp();
@@ -223,7 +244,10 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const __grid_c
     const int group = (warp - 4) / (F32_GROUP / 32), t = tid % F32_GROUP, unit = t & 7, row0 = t >> 3;
     const uint32_t at = row0 * 128 + ((unit ^ (row0 & 7)) << 4);      // (STEP rows on: the same place in the swizzle)
     constexpr int W_BUFS = Tile::W_BUFS;
-    const uint32_t w_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Tile::W_HI;
+    // where a unit's parts go: 8 bytes of x1, of x2 64 bytes on in the row, of x3 in the second array
+    const uint32_t at1 = row0 * 128 + (((unit >> 1) ^ (row0 & 7)) << 4) + (unit & 1) * 8;
+    const uint32_t at2 = row0 * 128 + (((4 + (unit >> 1)) ^ (row0 & 7)) << 4) + (unit & 1) * 8;
+    const uint32_t w_tmem = tmem + ((uint32_t)((warp & 3) * 32) << 16) + Tile::W_AT;
     // where row t of tensor memory lies in a stage (gated: all gate rows come first)
     const int w_row = GATED ? (t & 16) * 4 + (t >> 5) * 16 + (t & 15) : t;
     auto multiplied = [&](int c) {
@@ -258,33 +282,39 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const __grid_c
           if (group == 0) asm volatile("bar.sync 1, %0;" ::"n"(F32_GROUP) : "memory");      // the group's copies are here
           else asm volatile("bar.sync 2, %0;" ::"n"(F32_GROUP) : "memory");
         }
-        uint32_t hi[F32_CHUNK], lo[F32_CHUNK];      // of row t of w
+        unsigned long long v[F32_CHUNK / 2];      // row t of w
 #pragma unroll
         for (int u = 0; u < F32_CHUNK / 4; ++u) {
-          const uint4 v = *reinterpret_cast<const uint4*>(stage + w_row * 128 + ((u ^ (w_row & 7)) << 4));
-          lo[4 * u] = v.x, lo[4 * u + 1] = v.y, lo[4 * u + 2] = v.z, lo[4 * u + 3] = v.w;
+          const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(stage + w_row * 128 + ((u ^ (w_row & 7)) << 4));
+          v[2 * u] = q.x, v[2 * u + 1] = q.y;
         }
         float4 x[NB];
 #pragma unroll
         for (int i = 0; i < NB; ++i) x[i] = *reinterpret_cast<const float4*>(x_stage + i * STEP * 128 + at);
+        __syncwarp();      // a row's parts take the row's place; its eight units are this warp's
+        uint32_t w12[F32_CHUNK], w3[F32_CHUNK / 2];
 #pragma unroll
-        for (int e = 0; e < F32_CHUNK; ++e) {
-          const float v = __uint_as_float(lo[e]), h = head_of(v);
-          hi[e] = __float_as_uint(h), lo[e] = __float_as_uint(v - h);
+        for (int e = 0; e < F32_CHUNK / 2; ++e) {
+          v[e] = mul2(v[e], pair_of(F32_SCALE, F32_SCALE));
+          w12[e] = heads_of(v[e]), w12[F32_CHUNK / 2 + e] = heads_of(v[e]), w3[e] = heads_of(v[e]);
         }
-#pragma unroll
-        for (int i = 0; i < NB; ++i) {
-          const float4 h = make_float4(head_of(x[i].x), head_of(x[i].y), head_of(x[i].z), head_of(x[i].w));
-          float4* into = reinterpret_cast<float4*>(x_stage + i * STEP * 128 + at);
-          *into = h;
-          into[Tile::B_BYTES / 16] = make_float4(x[i].x - h.x, x[i].y - h.y, x[i].z - h.z, x[i].w - h.w);
-        }
-        proxy_fence();
         if (!multiplied(c - W_BUFS)) break;      // its place in tensor memory is free
         tc_fence_after();
         const uint32_t to = w_tmem + c % W_BUFS * Tile::W_COLUMNS;
-        tmem_st32(to, hi);
-        tmem_st32(to + F32_CHUNK, lo);
+        tmem_st32(to, w12);
+        tmem_st16(to + F32_CHUNK, w3);
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+          uint8_t* into = x_stage + i * STEP * 128;
+          unsigned long long lo = pair_of(x[i].x * F32_SCALE, x[i].y * F32_SCALE), hi = pair_of(x[i].z * F32_SCALE, x[i].w * F32_SCALE);
+          uint2 part[3];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) part[q].x = heads_of(lo), part[q].y = heads_of(hi);
+          *reinterpret_cast<uint2*>(into + at1) = part[0];
+          *reinterpret_cast<uint2*>(into + at2) = part[1];
+          *reinterpret_cast<uint2*>(into + Tile::B_BYTES + at1) = part[2];
+        }
+        proxy_fence();
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
@@ -296,22 +326,27 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const __grid_c
     auto wait_all = [&](uint64_t* bar, uint32_t parity) {
       return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
     };
-    constexpr uint32_t BOTH = tf32_instr_desc(F32_FEATURES, 2 * NT), ONE = tf32_instr_desc(F32_FEATURES, NT);
+    constexpr uint32_t idesc = umma_instr_desc(F32_FEATURES, NT);
     // (places and phases are counted on: divisions by the numbers of stages and buffers would be a third of the loop)
     int s = 0, buf = 0, w_buf = 0;
     uint32_t phase = 0, sum_phase = 1;
     const int all = own_tiles * n_chunks;
+    const uint32_t issues = elected();
     for (int c = 0; c < all; ++c) {
       if (!wait_all(&sum_empty[buf], sum_phase) || !wait_all(&full[s], phase)) break;
       tc_fence_after();
-      const uint32_t sums = tmem + buf * Tile::SUMS, w = tmem + Tile::W_HI + w_buf * Tile::W_COLUMNS;
-      // x's heads' rows, then the tails'
-      const uint64_t x = smem_desc_sw128(smem_u32(tiles + s * Tile::STAGE + Tile::A_BYTES));
+      const uint32_t large = tmem + buf * Tile::SUMS, small = large + NT, w = tmem + Tile::W_AT + w_buf * Tile::W_COLUMNS;
+      const uint64_t x1 = smem_desc_sw128(smem_u32(tiles + s * Tile::STAGE + Tile::A_BYTES));
+      const uint64_t x[3] = {x1, x1 + 4, x1 + Tile::B_BYTES / 16};      // (x2 lies 64 bytes on in x1's rows)
+      // w1 x1 of both halves of the chunk; the small ones
+      constexpr int HALF = F32_CHUNK / 2;
+      f32_mma<false>(issues, large, w, x[0], idesc);
+      f32_mma<true>(issues, large, w + 8, x[0] + 2, idesc);
+      f32_mma<false>(issues, small, w, x[1], idesc);
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {      // (8 k's are 32 bytes of a row)
-        umma_tf32_tmem_a(sums, w + 8 * k, x + 2 * k, BOTH, k > 0);
-        umma_tf32_tmem_a(sums + NT, w + F32_CHUNK + 8 * k, x + 2 * k, ONE, 1);
-      }
+      for (int q = 1; q < 8; ++q)      // w1 x2, w1 x3, w2 x1, w2 x2, w2 x3, w3 x1, w3 x2: 16 k's are 8 columns of w, 32 bytes of x
+#pragma unroll
+        for (int k = q == 1 ? 1 : 0; k < 2; ++k) f32_mma<true>(issues, small, w + HALF * (q / 3) + 8 * k, x[q % 3] + 2 * k, idesc);
       umma_commit(&empty[s]);
       umma_commit(&sum_full[buf]);
       if (++s == STAGES) s = 0, phase ^= 1;
@@ -438,14 +473,13 @@ int launch_f32_as(F32Params p, cudaStream_t stream) {
 }
 
 // Whether products with these sizes of w go through the tensor cores, by w alone, so that a row's bits depend on nothing that
-// comes beside it.  Below 768 k's a chain of multiply-adds is as close to 64-bit (2-norm of the error, random operands: 896
-// k's 1.45e-7 here and 1.96e-7 there, 4,864 1.6e-7 and 4.5e-7, 512 1.42e-7 and 1.52e-7; of a gated product 2.6e-7 and
-// 2.9e-7, 514 k's 2.6e-7 and 2.3e-7).  Very wide outputs (heads) are asked for few rows, which the weights' way from memory
-// bounds there: 1 x 151,936 x 896 116 us here, 82 there.
+// comes beside it.  Below 768 k's the fixed cost of a tile leaves little to gain.  Very wide outputs (heads) are asked for few
+// rows, which the weights' way from memory bounds there: 1 x 32,768 x 896 36 us here, 22 by multiply-adds, 1 x 151,936 x 896 82
+// by multiply-adds.
 inline bool f32_on_tensor_cores(int N, int K, bool gated) { return K >= 768 && (gated ? 2ll : 1ll) * N <= 32768; }
 
-// Rows of x a tile holds and CTAs that share the parts of K, by what a launch takes (us): a CTA of 16, 32 or 64 rows 0.45,
-// 0.49 or 0.62 a chunk and 3.5 a tile, in clusters 5 and a round more where not all find room at once.
+// Rows of x a tile holds and CTAs that share the parts of K, by what a launch takes (us): a CTA of 16, 32 or 64 rows 0.47,
+// 0.53 or 0.72 a chunk and 3.5 a tile, in clusters 5 and a round more where not all find room at once.
 inline void f32_plan(long long M, long long N, bool gated, int chunks, int part_chunks, int& nt, int& spread) {
   const long long sms = lab_sm_count(), blocks = (N + (gated ? 63 : 127)) / (gated ? 64 : 128);
   double best = 0;
@@ -454,21 +488,22 @@ inline void f32_plan(long long M, long long N, bool gated, int chunks, int part_
       const long long room = ctas == 8 ? sms * 7 / 8 : sms;
       const long long rounds = ((M + rows - 1) / rows * blocks * ctas + room - 1) / room;
       const int own = F32_PARTS / ctas * part_chunks < chunks ? F32_PARTS / ctas * part_chunks : chunks;
-      const double chunk = rows == 16 ? 0.45 : rows == 32 ? 0.49 : 0.62;
+      const double chunk = rows == 16 ? 0.47 : rows == 32 ? 0.53 : 0.72;
       const double us = ctas == 1 ? rounds * (own * chunk + 3.5) + 4 : rounds * (own * chunk + 5) + 2;
       if (best == 0 || us < best) best = us, nt = rows, spread = ctas;
     }
 }
 
 inline int launch_f32(void* out, const void* x, const void* w, const void* bias, int M, int N, int K, int ldx, int ldo,
-                      bool gated, int act, float gate_limit, int nt, int spread, cudaStream_t stream) {
+                      bool gated, int act, float gate_limit, cudaStream_t stream) {
   F32Params p;
   p.out = (float*)out; p.x = (const float*)x; p.w = (const float*)w; p.bias = (const float*)bias;
   p.M = M; p.N = N; p.K = K; p.ldx = ldx; p.ldo = ldo; p.act = act; p.gate_limit = gate_limit;
   p.chunks = (K + F32_CHUNK - 1) / F32_CHUNK;
   p.part_chunks = (p.chunks + F32_PARTS - 1) / F32_PARTS;
   const bool vec = K % 4 == 0 && ldx % 4 == 0 && ldx >= K && (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
-  if (nt == 0) f32_plan(M, N, gated, p.chunks, p.part_chunks, nt, spread);
+  int nt = 0, spread = 0;
+  f32_plan(M, N, gated, p.chunks, p.part_chunks, nt, spread);
 #define LAB_F32_AS(GATED_, NT_, VEC_)                                                       \
   return spread == 8   ? launch_f32_as<GATED_, NT_, VEC_, 8>(p, stream)                      \
          : spread == 4 ? launch_f32_as<GATED_, NT_, VEC_, 4>(p, stream)                      \

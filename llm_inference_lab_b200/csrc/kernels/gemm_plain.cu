@@ -1,7 +1,7 @@
 // Plain matrix product on the ordinary arithmetic units (no reduced precision): the
 // yardstick the bfloat16 tensor-core kernels are tested against, and the matrix product of
 // the 32-bit path where w's rows are short, its outputs very wide, or rows come in batches
-// and groups.  (Other 32-bit products run on the tensor cores in split operands, gemm_f32.cuh.)
+// and groups.  (Other 32-bit products run on the tensor cores, operands cut in three, gemm_f32.cuh.)
 //
 //   out[m, n] = OutT( sum_k x[m, k] * w[n, k]  (+ bias[n]) )          w is [out, in]
 //   gated:      out[m, n] = T( silu(g) * u ),  g = x . w[n], u = x . w[inter + n]   (32-bit, one rounding)
@@ -641,7 +641,7 @@ int launch(void* out, const void* x, const void* w, const void* bias, int M, int
                      (((uintptr_t)x | (uintptr_t)w) & 15) == 0;
   if constexpr (std::is_same_v<T, float>) {
     if (batch == 1 && row_src == nullptr && tile_group == nullptr && f32_on_tensor_cores(N, K, gate))
-      return launch_f32(out, x, w, bias, M, N, K, ldx, ldo, gate, act, gate_limit, 0, 0, stream);
+      return launch_f32(out, x, w, bias, M, N, K, ldx, ldo, gate, act, gate_limit, stream);
     if (M <= FR_ROWS && batch == 1 && row_src == nullptr && tile_group == nullptr && units)
       return launch_few_rows(out, x, w, bias, M, N, K, ldx, ldo, gate, act, gate_limit, stream);
   }

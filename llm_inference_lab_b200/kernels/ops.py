@@ -273,8 +273,8 @@ def rope_kv_write_table(qkv, table, rotary_dim, slots, cache_k, cache_v, n_q, n_
 def gemm_plain(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, gated: bool = False,
                out_f32: bool = False, out: torch.Tensor | None = None, gelu: bool = False,
                gate_limit: float = 0.0, gate_act: str = "silu") -> torch.Tensor:
-    """out = x @ w.T (+ bias) on the ordinary arithmetic units (32-bit operands with long rows: on the tensor cores, each split
-    in two, with no larger an error); `gated`: silu(x@wg.T) * (x@wu.T), w = [wg; wu]
+    """out = x @ w.T (+ bias) on the ordinary arithmetic units (32-bit operands with long rows: on the tensor cores, each cut
+    in three numbers of 16 bits, which make it up exactly); `gated`: silu(x@wg.T) * (x@wu.T), w = [wg; wu]
     (`gate_limit`, `gate_act`: see `linear_gated`); `gelu`: the tanh form of GELU after the bias, before
     the rounding."""
     assert not (gated and gelu)
