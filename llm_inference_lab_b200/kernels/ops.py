@@ -1069,11 +1069,20 @@ def delta_rule_supported(head_dim: int) -> bool:
 
 
 def delta_rule_blocks(longest: int) -> bool:
-    """Whether `delta_rule` walks a step's rows four at a time (16-bit storage, heads of 32, 64, 128 or 256): from 32 rows of
-    a request on.  Measured with the mixer around it (us, from a graph, blocks / row by row), 14 heads of 64: three requests
-    of 500 rows 184 / 204, one of 2,048 443 / 520, eight of 250 170 / 210, one of 100 55 / 66, two of 24 39 / 39; 12 heads
-    of 128: one of 700 rows 283 / 410, four of 500 410 / 642."""
+    """Whether `delta_rule` may walk a step's rows four at a time (16-bit storage, heads of 32, 64, 128 or 256; where
+    `delta_blocks_pay`): from 32 rows of a request on."""
     return longest >= 32
+
+
+def delta_blocks_pay(longest: int, tokens: int, requests: int, head_dim: int) -> bool:
+    """Whether blocks of four rows beat the walk row by row: a request costs a block's preparation however few rows it
+    brings, and a row of the longest one saves what the larger heads save more of.  Measured (us, from a graph, blocks / row by
+    row), 14 heads of 64: one request of 48 rows 18.2 / 17.1, 64 20.2 / 20.5, 500 rows three times 146 / 191, 250 eight times 134 /
+    167; beside 64 single rows 100 rows 43.1 / 42.5, 32 rows 33 / 24, 500 rows 124 / 175; 12 heads of 128: 48 rows 28.0 / 26.5, 64
+    30.8 / 32.0, 700 rows 216 / 354; beside 64 single rows 100 rows 124 / 100, 200 163 / 150, 500 259 / 312; four heads of 256 beside
+    64 single rows 100 rows 187 / 148; 28 heads of 32: 100 rows 22.0 / 20.4, 500 rows 74 / 82."""
+    base, each = {32: (150, 1.0), 64: (60, 2.0)}.get(head_dim, (56, 4.3))
+    return longest + (tokens - longest) / 6 >= base + each * (requests - 1)
 
 
 def tanh_cast(x: torch.Tensor, dtype: torch.dtype, head_dim: int = 64) -> torch.Tensor:
@@ -1110,7 +1119,8 @@ def delta_rule(proj: torch.Tensor, decay_pre: torch.Tensor, decay_bias: torch.Te
     L = lib("delta_rule", {"LAB_HEAD_DIM": head_dim})
     L.lab_delta_rule_scratch.restype = ctypes.c_longlong
     blocks = 0
-    if dt != torch.float32 and state.data_ptr() % 8 == 0 and delta_rule_blocks(ctx.max_q_len):
+    if (dt != torch.float32 and state.data_ptr() % 8 == 0 and delta_rule_blocks(ctx.max_q_len)
+            and delta_blocks_pay(ctx.max_q_len, tokens, ctx.n_requests, head_dim)):
         blocks = int(L.lab_delta_rule_blocks())
     raw = torch.empty((int(L.lab_delta_rule_scratch(tokens, heads, ctx.n_requests, blocks)),), dtype=torch.float32,
                       device=proj.device)

@@ -22,8 +22,9 @@ def plain(r, k, v, a, decay, S):
 
 @pytest.mark.parametrize("D,heads", [(32, 3), (64, 9), (128, 2), (256, 1)])
 @pytest.mark.parametrize("lens", [[32], [33, 1, 2, 67], [1, 130, 35, 4, 3], [34, 36]])
-def test_blocks_of_four_tokens(D, heads, lens):
+def test_blocks_of_four_tokens(D, heads, lens, monkeypatch):
     assert ops().delta_rule_blocks(max(lens))
+    monkeypatch.setattr(ops(), "delta_blocks_pay", lambda *a: True)
     g = torch.Generator(device=DEV).manual_seed(D + sum(lens))
     rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
     T, hd, rate = sum(lens), heads * D, 0.6
@@ -65,10 +66,11 @@ def test_blocks_of_four_tokens(D, heads, lens):
 @pytest.mark.parametrize("D,heads", [(32, 1), (64, 2)])
 @pytest.mark.parametrize("bad", [float("inf"), float("nan")])
 @pytest.mark.parametrize("row", [0, 1, 2, 3, 8, 17, 22, 31])
-def test_rows_before_a_non_finite_one_are_as_they_were(D, heads, bad, row):
+def test_rows_before_a_non_finite_one_are_as_they_were(D, heads, bad, row, monkeypatch):
     """Every place of a block, of a portion's first block and of later ones; one entry of r, k, v, the gate, the rate or the decay."""
     T, hd = 35, heads * D
     assert ops().delta_rule_blocks(T)
+    monkeypatch.setattr(ops(), "delta_blocks_pay", lambda *a: True)
     g = torch.Generator(device=DEV).manual_seed(row)
     rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
     proj, decay_pre, start = rand(T, 5 * hd), rand(T, hd), rand(1, heads, D, D)
@@ -91,3 +93,24 @@ def test_rows_before_a_non_finite_one_are_as_they_were(D, heads, bad, row):
     spoilt[row, 5] = bad
     assert torch.equal(run(proj, spoilt)[:row], clean[:row])
     ops().take_device_errors()
+
+
+@pytest.mark.parametrize("D,heads", [(32, 3), (64, 9), (128, 2), (256, 1)])
+def test_blocks_and_single_rows_agree(D, heads, monkeypatch):
+    """The two walks of the same step, single rows beside a portion: 32-bit roundings of the states, one of the outputs."""
+    lens = [1, 50, 1, 3, 33, 1]
+    g = torch.Generator(device=DEV).manual_seed(D)
+    T, hd = sum(lens), heads * D
+    proj, decay_pre = torch.randn(T, 5 * hd, device=DEV, generator=g), torch.randn(T, hd, device=DEV, generator=g)
+    bias, weight = (torch.randn(hd, device=DEV, generator=g).bfloat16() for _ in range(2))
+    start, got = torch.randn(6, heads, D, D, device=DEV, generator=g), {}
+    for blocks in (True, False):
+        monkeypatch.setattr(ops(), "delta_blocks_pay", lambda *a: blocks)
+        state = start.clone()
+        out = ops().delta_rule(proj, decay_pre, bias, bias, weight, state, context(lens, [4, 0, 5, 2, 1, 3]), heads, D, 1e-6, 0.6)
+        got[blocks] = out.float(), state
+    ops().take_device_errors()
+    (a, S), (b, R) = got[True], got[False]
+    assert not torch.equal(S, R) and float((S - R).abs().max()) <= 1e-5 * float(R.abs().max())
+    # (an entry near zero takes the error of the whole row's)
+    assert bool(((a - b).abs() <= 2.0 ** -7 * b.abs() + 1e-5 * b.abs().amax(1, keepdim=True)).all())

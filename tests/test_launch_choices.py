@@ -104,6 +104,17 @@ def test_small_states_are_walked_in_segments_where_that_was_faster():
                                      (5120, 16, 1, 2048), (512, 16, 4, 500), (3072, 8, 1, 2048), (5120, 4, 1, 2048), (1792, 16, 64, 400)))
 
 
+def test_rows_go_in_blocks_of_four_where_that_was_faster():
+    """(rows of the longest portion, single rows beside it, head size)"""
+    def pays(longest, singles, dim, portions=1):
+        return ops.delta_rule_blocks(longest) and ops.delta_blocks_pay(longest, longest * portions + singles, portions + singles, dim)
+
+    assert all(pays(*c) for c in ((64, 0, 64), (100, 8, 64), (500, 64, 64), (64, 0, 128), (400, 64, 128), (64, 0, 256), (500, 0, 32),
+                                  (48, 0, 64, 8), (250, 0, 128, 7), (250, 0, 32, 8)))
+    assert not any(pays(*c) for c in ((31, 0, 64), (48, 0, 64), (32, 64, 64), (100, 64, 64), (100, 64, 128), (200, 64, 128), (32, 0, 256),
+                                      (100, 64, 256), (100, 0, 32)))
+
+
 def test_gated_products_take_the_kind_of_tile_whose_rounds_take_less_time():
     """By the measured costs of a round (pairs of SMs 0.9 of the small tiles' where K is long, the same where it is short),
     for every number of tokens."""
