@@ -1626,14 +1626,33 @@ def decay_scan_supported(keys: int) -> bool:
     return 1 <= keys <= 256
 
 
-def decay_scan_chunks(ctas: int, keys: int, longest: int) -> bool:
+DECAY_SCAN_CHUNK_BYTES = 256 << 20      # what a step's chunks may keep of states
+
+
+def decay_scan_chunks(ctas: int, keys: int, longest: int, heads: int, vdim: int, tokens: int, requests: int) -> bool:
     """Whether `decay_scan` takes a step's rows in chunks of 64 side by side (three launches), `ctas` CTAs walking the step in
     one piece.  Measured with the matrix memory around it, 14 heads of 64 x 68 (us, kernel by kernel, chunks / walk, the walk
     of 450 rows on in segments): two requests of 1,000 rows 126 / 202, one of 2,048 137 / 241, eight of 250 118 / 135; 12 heads
     of 128 x 132: one of 1,500 187 / 376, four of 300 170 / 182.  Shorter portions save device time (from a graph one of 420
     rows 59 / 104, 200 56 / 66, 100 64 / 68, 64 55 / 45), but there the mixer launched kernel by kernel is bound by the
-    host, which two more launches and the scratch cost 12 us (420 rows 108 / 105, 200 108 / 96)."""
-    return keys <= 128 and (longest >= 450 or (longest >= 200 and ctas >= sm_count()))
+    host, which two more launches and the scratch cost 12 us (420 rows 108 / 105, 200 108 / 96).
+
+    Every request takes a chunk of its own, however few rows it brings, whose state per head is written and read: beside many
+    single rows the walk is the faster one, by what either takes (us; a chunk and head 0.013 and some by its state, a request
+    its state once more; a row of the walk's longest request, and all rows once they are too many to go side by side).
+    Measured alone (from a graph, chunks / walk): 500 rows beside 32 single rows, 14 heads of 64 x 68 66 / 78, 12 of 128 x 132
+    210 / 173; beside 64 112 / 81 and 378 / 182, 32 heads of 128 x 128 976 / 235; 2,048 rows beside 64 144 / 302; 20 requests of 20
+    beside one of 200 53 / 45; 24 requests of 500, 14 heads of 64 x 68 258 / 416, 32 of 128 x 128 2,198 / 1,865.  Beyond
+    DECAY_SCAN_CHUNK_BYTES of states, too, the walk is taken: it is the one that needs no room for them."""
+    if keys > 128 or not (longest >= 450 or (longest >= 200 and ctas >= sm_count())):
+        return False
+    places, state = tokens // 64 + requests, keys * vdim
+    if 4 * places * heads * state > DECAY_SCAN_CHUNK_BYTES:
+        return False
+    entry = 1.47e-5 if keys <= 64 else 1.75e-5
+    row, all_rows = (0.08, 3e-4) if keys <= 16 else (0.15, 1e-3) if keys <= 64 else (0.37, 1.8e-3)
+    chunks = 15 + heads * (places * (0.013 + entry * state) + 0.35 * entry * state * requests)
+    return chunks < max(5 + row * longest, all_rows * tokens * heads * -(-vdim // 32))
 
 
 def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) -> int:
@@ -1691,7 +1710,7 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
     vs = min(vs, max(8, 1 << (vdim - 1).bit_length()))
     segments, chunk_tokens, launches = 1, 0, 1
     states = decays = None
-    if not in_order and decay_scan_chunks(pairs * -(-vdim // vs), keys, ctx.max_q_len):
+    if not in_order and decay_scan_chunks(pairs * -(-vdim // vs), keys, ctx.max_q_len, heads, vdim, tokens, ctx.n_requests):
         places = lib("linear_state").lab_decay_scan_places(tokens, ctx.n_requests)
         scratch, (states, decays) = _segment_scratch(v.device, places * heads * keys * vdim, places * heads)
         chunk_tokens, launches = tokens, 3

@@ -115,6 +115,23 @@ def test_rows_go_in_blocks_of_four_where_that_was_faster():
                                       (100, 64, 256), (100, 0, 32)))
 
 
+def test_decayed_recurrences_go_in_chunks_where_that_was_faster():
+    """(heads, key channels, value columns, the requests' rows)"""
+    def chunks(heads, keys, vdim, rows):
+        return ops.decay_scan_chunks(len(rows) * heads * -(-vdim // 32), keys, max(rows), heads, vdim, sum(rows), len(rows))
+
+    one = [1]
+    assert all(chunks(*c) for c in ((14, 64, 68, [2048]), (14, 64, 68, [1000] * 2), (14, 64, 68, [250] * 8), (12, 128, 132, [1500]),
+                                    (12, 128, 132, [300] * 4), (14, 64, 68, [500] + one * 32), (14, 64, 68, [2048] + one * 64),
+                                    (14, 64, 68, [500] * 24), (4, 64, 64, [2048]), (32, 64, 64, [500] * 24)))
+    assert not any(chunks(*c) for c in ((14, 64, 68, [449]), (14, 64, 68, [199] * 8), (14, 200, 68, [2048]), (14, 64, 68, [500] + one * 64),
+                                        (12, 128, 132, [500] + one * 32), (32, 128, 128, [700] + one * 32), (64, 64, 64, [200] + [20] * 20)))
+    # 16,384 rows of 64 heads of 128 x 128 would keep 1.1 GB of states
+    assert not chunks(64, 128, 128, [16384]) and chunks(12, 128, 132, [16384])
+    for heads, keys, vdim, rows in itertools.product((1, 14, 64), (16, 64, 128), (16, 132, 256), ([500], [450] + one * 200, [9000] * 8)):
+        assert not chunks(heads, keys, vdim, rows) or 4 * (sum(rows) // 64 + len(rows)) * heads * keys * vdim <= ops.DECAY_SCAN_CHUNK_BYTES
+
+
 def test_gated_products_take_the_kind_of_tile_whose_rounds_take_less_time():
     """By the measured costs of a round (pairs of SMs 0.9 of the small tiles' where K is long, the same where it is short),
     for every number of tokens."""
