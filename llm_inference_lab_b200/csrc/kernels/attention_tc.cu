@@ -679,7 +679,7 @@ LAB_EXPORT int lab_attention_decode_rotated(void* out, int out_stride, const voi
                                             int page_size, int num_pages, int window, float scale, int splits,
                                             float* scratch, int cluster_merge, cudaStream_t stream) {
   if (rows == nullptr || positions == nullptr || inv_freq == nullptr || slots == nullptr || parts < 0 ||
-      width != (n_q + 2 * n_kv) * D)
+      width != (n_q + 2 * n_kv) * D || (((uintptr_t)rows | (uintptr_t)bias) & 15) != 0)      // (four columns a load)
     return (int)cudaErrorInvalidValue;
   Rotate rot;
   rot.rows = rows; rot.parts = parts; rot.width = width; rot.part_stride = (size_t)tokens * width;

@@ -59,3 +59,18 @@ def test_a_slot_beyond_the_pages_is_an_error():
     with pytest.raises(ops().KernelError):
         ops().take_device_errors()
     assert not ck.any()
+
+
+def test_rows_or_a_bias_off_16_bytes_are_refused():
+    ck = torch.zeros(4, 2, 16, 64, device=DEV, dtype=torch.bfloat16)
+    t = lambda a: torch.tensor(a, dtype=torch.int32, device=DEV)  # noqa: E731
+    ctx = SimpleNamespace(q_start=t([0, 1]), kv_len=t([5]), n_requests=1, q_lens=[1], max_q_len=1, max_kv_len=5)
+    width, bf = 18 * 64, torch.bfloat16
+    run = lambda rows, bias: ops().attention_rotated(rows, bias, t([4]), torch.ones(32, device=DEV), t([4]), ck, ck.clone(), ctx,  # noqa: E731
+                                                     SimpleNamespace(block_table=t([[0]])), 14, 2, 64, 0, 0.125)
+    run(torch.zeros(2, 1, width, device=DEV), torch.zeros(width, device=DEV, dtype=bf))
+    for rows, bias in ((torch.zeros(width + 1, device=DEV, dtype=bf)[1:].view(1, width), None),
+                       (torch.zeros(2, 1, width, device=DEV), torch.zeros(width + 1, device=DEV, dtype=bf)[1:])):
+        with pytest.raises(ops().KernelError):
+            run(rows, bias)
+    ops().take_device_errors()
