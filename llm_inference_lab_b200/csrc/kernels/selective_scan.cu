@@ -734,9 +734,6 @@ int pick_scan(void* out, const void* a_log, const void* skip, const void* dt_bia
 }
 }  // namespace
 
-// The largest state that is walked an entry a lane, in one piece.
-LAB_EXPORT int lab_selective_scan_small_state() { return SMALL_STATE; }
-
 // The largest state (entries per channel) the walk takes.
 LAB_EXPORT int lab_selective_scan_max_state() { return SCAN_MAX_STATE; }
 

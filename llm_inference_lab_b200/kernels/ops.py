@@ -1655,20 +1655,16 @@ def decay_scan_chunks(ctas: int, keys: int, longest: int, heads: int, vdim: int,
     return chunks < max(5 + row * longest, all_rows * tokens * heads * -(-vdim // 32))
 
 
-def decay_scan_segments(ctas: int, longest: int, requests: int, keys: int = 64) -> int:
+def decay_scan_segments(ctas: int, longest: int, requests: int) -> int:
     """Into how many segments `decay_scan` cuts a request's rows of more than 128 key channels (fewer go in chunks), `ctas`
-    CTAs walking the step in one piece; a multiprocessor holds three.  Segments cost most of the walk's work
-    once more, so they pay while multiprocessors are idle.  Measured with the matrix memory around it (us, from a graph,
-    states of 64 key channels, which went this way): 42
-    CTAs and 2,048 tokens 418 in one piece, 288 in 4, 236 in 8, 239 in 15; 460 tokens 113, 82 in 8; 84 CTAs and 1,000 tokens
-    236, 201 in 4, 198 in 8; 420 tokens 113, 105 in 4; 168 CTAs and 500 tokens 182, 186 in 2, 176 in 4; 336 and 250 tokens
-    137, 169 in 2.  Below 450 tokens they would still save the device time (42 CTAs and 300 tokens 84, 67 in 8), but there
-    the mixer launched kernel by kernel, as prompts of such models are, is bound by the host, which a second launch and its
-    scratch cost 8 us (94 us in one piece, 101 in segments)."""
-    if ctas >= sm_count() or longest < 450:
+    CTAs walking the step in one piece.  Segments cost most of the walk's work once more, so they pay while multiprocessors are
+    idle.  Measured (us, from a graph), 12 CTAs (3 heads of 256 x 128) and 2,048 tokens 763 in one piece, 319 in 4, 222 in 8, 210 in 12,
+    261 in 16; 8 CTAs (4 heads of 192 x 64) and 1,000 tokens 374, 175 in 4, 144 in 8, 160 in 12, 186 in 16; 460 tokens 177, 110 in 4,
+    112 in 8, 139 in 14; 64 CTAs (8 heads of 256 x 256) and 2,048 tokens 767, 565 in 2, 582 in 4, 632 in 6; (16 of 256 x 128) 1,000
+    tokens 379, 300 in 2, 309 in 4, 354 in 6; 80 CTAs (two requests, 8 heads of 160 x 160) and 700 tokens 265, 335 in 2, 301 in 4."""
+    if longest < 450:
         return 1
-    room = (9 * sm_count() // 2 if keys <= 64 else 3 * sm_count()) // max(1, ctas)
-    return max(1, min(longest // 32, room, 16, 65535 // max(1, requests)))
+    return max(1, min(longest // 96, sm_count() // max(1, ctas), 16, 65535 // max(1, requests)))
 
 
 def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, ctx, heads: int, groups: int,
@@ -1715,7 +1711,7 @@ def decay_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.T
         scratch, (states, decays) = _segment_scratch(v.device, places * heads * keys * vdim, places * heads)
         chunk_tokens, launches = tokens, 3
     elif not in_order and keys > 128:
-        segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests, keys)
+        segments = decay_scan_segments(pairs * -(-vdim // vs), ctx.max_q_len, ctx.n_requests)
         if segments > 1:
             scratch, (states, decays) = _segment_scratch(v.device, pairs * segments * keys * vdim, pairs * segments)
             launches = 2
@@ -1852,7 +1848,9 @@ def scan_segments(ctas: int, longest: int) -> int:
     4, 128 in 6; 224 CTAs and 500 tokens 246, 235 in 2, 209 in 6; 448 CTAs and 250 tokens 173, 196 in 2.  Below 320 tokens
     they would still save the device time (319 tokens 114, 91 in 8; 130 tokens 76, 71 in 8), but there the mixer launched
     kernel by kernel, as prompts of such models are, is bound by the host, which a second launch and its scratch cost 8 us
-    (130 tokens 99 us in one piece, 107 in segments)."""
+    (130 tokens 99 us in one piece, 107 in segments).  Larger states, alone: 56 CTAs of 32 entries and 2,048 tokens 496, 212 in 6,
+    218 in 11, 225 in 32; 48 of 64 entries 690, 324 in 6, 355 in 13, 433 in 32; 48 of 128 entries 737, 300 in 6, 334 in 13; 16 of
+    64 683, 134 in 16, 158 in 32; 192 of 64 and 500 tokens 217, 356 in 3 (not faster there)."""
     if longest < 320:
         return 1
     return max(1, min(longest // 32, 9 * sm_count() // (2 * max(1, ctas)), 32))

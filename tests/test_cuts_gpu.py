@@ -71,7 +71,7 @@ def test_32_bit_bits_depend_on_neither_cut_nor_batch(kind):
 
 def recurrence(name, T):
     """(a walk over rows a .. b of a prompt of T tokens from the states it is given, the states' shapes, the number of
-    segments the whole prompt is cut into)"""
+    segments or chunks the whole prompt is cut into)"""
     g = torch.Generator(device=DEV).manual_seed(9)
     rand = lambda *s: torch.randn(s, device=DEV, generator=g)  # noqa: E731
     if name == "selective_scan":
@@ -79,7 +79,8 @@ def recurrence(name, T):
         x, dt_pre, z, bc, a_log, skip, bias = rand(T, C), rand(T, C) - 4, rand(T, C), rand(T, 2 * N), rand(C, N), rand(C), rand(C)
         walk = lambda a, b, s: ops().selective_scan(x[a:b], dt_pre[a:b], bc[a:b], 0, N, z[a:b], a_log, skip, bias, s[0],  # noqa: E731
                                                     context([b - a], [0]))
-        return walk, [(1, C, N)], ops().scan_segments(3, T)
+        n = ops().scan_segments(3, T)
+        return walk, [(1, C, N)], n if ops().scan_segments_pay(n, C, N, 1, T) else 1
     H, D, V = 3, 64, 64
     if name == "gated_delta":
         taps, G = 4, 3
@@ -106,7 +107,8 @@ def recurrence(name, T):
         o = ops().decay_scan(qk[a:b, : H * D], qk[a:b, H * D:], v[a:b], s[0], ctx, H, H, D, V, **how)
         return o if name != "matrix_memory" else o.view(-1, H, V) * torch.exp(m.clamp(-20, 20))[:, :, None]
 
-    return walk, [(1, H, D, V), (1, H)], ops().decay_scan_segments(H * 2, T, 1, D)
+    # (chunks of 64 rows)
+    return walk, [(1, H, D, V), (1, H)], -(-T // 64) if ops().decay_scan_chunks(H * 2, D, T, H, V, T, 1) else 1
 
 
 @pytest.mark.parametrize("name", ["selective_scan", "linear_state", "matrix_memory", "gated_delta"])

@@ -88,8 +88,8 @@ def test_segments_of_recurrences_cover_the_cases_they_were_measured_on():
     assert walk(12, 128, 128, 2048) == 4 and walk(14, 64, 64, 300) == 1 and walk(14, 256, 64, 2048) == 1
     assert ops.scan_segments(56, 2048) == 11 and ops.scan_segments(112, 700) == 5 and ops.scan_segments(448, 250) == 1
     assert ops.scan_segments(56, 319) == 1 and ops.scan_segments(1, 5000) == 32
-    assert ops.decay_scan_segments(84, 1000, 2) == 7 and ops.decay_scan_segments(168, 500, 4) == 1
-    assert ops.decay_scan_segments(42, 449, 1) == 1 and ops.decay_scan_segments(60, 2048, 1, 128) == 7
+    assert [ops.decay_scan_segments(*c) for c in ((12, 2048, 1), (8, 1000, 1), (64, 2048, 1), (80, 700, 2), (8, 460, 1), (42, 449, 1))] \
+        == [12, 10, 2, 1, 4, 1]
 
 
 def test_small_states_are_walked_in_segments_where_that_was_faster():

@@ -65,7 +65,9 @@ def test_selective_scan_segments(channels, N, segments, monkeypatch):
 @pytest.mark.parametrize("segments", [1, 2, 3, 5, 9])
 @pytest.mark.parametrize("heads,groups,keys,vdim,per_token,silu", [(4, 2, 64, 68, True, False), (3, 3, 16, 20, False, True),
                                                                    (2, 1, 50, 33, True, False), (2, 2, 128, 128, True, False),
-                                                                   (1, 1, 200, 8, False, False)])
+                                                                   (1, 1, 200, 8, False, False), (2, 1, 130, 33, True, False),
+                                                                   (3, 3, 256, 96, True, True), (4, 2, 144, 68, True, False),
+                                                                   (1, 1, 129, 1, False, True)])
 def test_decay_scan_segments(heads, groups, keys, vdim, per_token, silu, segments, monkeypatch):
     monkeypatch.setattr(ops(), "decay_scan_segments", lambda *a: segments)
     g = torch.Generator(device=DEV).manual_seed(keys + vdim)
@@ -78,8 +80,11 @@ def test_decay_scan_segments(heads, groups, keys, vdim, per_token, silu, segment
     start, ctx = state.clone(), context(Q_LENS, SLOTS)
     how = dict(a_tok=gates[:, 0], s_tok=gates[:, 1]) if per_token else dict(a_head=fixed)
     for write in (False, True):
+        before = ops().COUNTER.launches
         out = ops().decay_scan(qk[:, : groups * keys], qk[:, groups * keys:], v, state, ctx, heads, groups, keys, vdim, silu=silu,
                                write=write, **how)
+        # (up to 128 key channels never go in segments)
+        assert ops().COUNTER.launches - before == (min(segments, 2) if keys > 128 else 1)
         assert write or torch.equal(state, start)
     ops().take_device_errors()
     n = lambda t: t.double().cpu().numpy()  # noqa: E731
