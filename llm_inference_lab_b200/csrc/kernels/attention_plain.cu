@@ -491,7 +491,8 @@ int launch_rows(RowsParams p, cudaStream_t stream) {
 // Sixteen rows a CTA halve what it reads, eight give twice the CTAs: sixteen once they fill every multiprocessor twice.  With
 // heads of 64 thirty-two, sixteen to a warp, once they fill every multiprocessor four times: fewer leave the long rows' CTAs
 // alone at the end.  Measured (us, 32 / 16 rows, 14 and 2 heads): one prompt of 1,200 143 / 162, 1,600 246 / 268, 800 85 / 84,
-// 517 59 / 43, two of 1,000 208 / 234, three of 400 85 / 81, eight of 250 120 / 127.
+// 517 59 / 43, two of 1,000 208 / 234, three of 400 85 / 81, eight of 250 120 / 127.  (Heads of 128 have no tile of thirty-two: a
+// lane's sums of four rows by sixteen entries and four keys' products would take all the registers that four CTAs leave.)
 template <typename T>
 int pick_rows(RowsParams p, bool single, cudaStream_t stream) {
   const int group = p.n_q / p.n_kv;

@@ -9,7 +9,7 @@
 //
 // Kernels: the causal convolution of x with the request's last inputs kept between steps (+ SiLU), and
 // the walk, of which there are three: states of up to 16 entries an entry a lane, in one piece; steps of single
-// tokens of such states; larger states a share of the entries a lane, in segments.  The walk is sequential in
+// tokens of such states; larger states, and such of few channels and many tokens, a share of the entries a lane, in segments.  The walk is sequential in
 // tokens; a CTA takes some channels of one request, WL lanes a channel,
 // each lane a share of the state's entries in registers.  A chunk of tokens waits in shared memory while the
 // next one arrives there (cp.async); step sizes are formed once per channel and token before the chunk is
@@ -17,7 +17,7 @@
 // over the state in shared memory, and the sums, the skip term and the gate are formed after the chunk, a
 // thread per channel and token.
 //
-// A long portion of larger states is cut into segments of tokens that are walked side by side, in two launches: the first walks every
+// A long portion is there cut into segments of tokens that are walked side by side, in two launches: the first walks every
 // segment but the last from zeros (the first one from the request's state) for its closing state and the sum of its
 // step sizes, the second takes every segment again from its opening state, which follows from the segments before it
 // (S <- exp(A sum dt) S + S_segment), and leaves the outputs.  Everything stays 32-bit; the errors against 64-bit are
@@ -394,8 +394,8 @@ __global__ void __launch_bounds__(WTHREADS) selective_scan_kernel(T* __restrict_
 // A lane an entry: LN lanes a channel, 32 / LN channels a warp.  A warp forms its channels' step sizes for a chunk of WTS
 // tokens, walks it, and forms its channels' outputs; only the chunk's inputs, brought by cp.async, are shared by the CTA's
 // warps, so they meet once a chunk.  Inputs lie so that a lane reads four tokens at a time; every lane leaves its
-// share of the sum over the state in shared memory.  A request's rows are walked in one piece, whatever their number: a
-// channel's numbers depend on neither the cut nor the batch.
+// share of the sum over the state in shared memory.  A request's rows are walked in one piece: its numbers depend on neither
+// the cut nor the batch.
 // What bounds it: the issue of instructions, most of them the exponential's, by the few warps that a request's channels make
 // (six a multiprocessor for 1,792 channels of 16; they issue in two cycles of five).  The mixer around it (us, from a graph)
 // against four entries a lane, in segments from 320 tokens on: 1,792 channels, one request of 2,048 tokens 212 (220), of 700
